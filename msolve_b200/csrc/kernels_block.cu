@@ -1544,61 +1544,75 @@ __global__ void __launch_bounds__(kMWarps * 32, 1)
   }
 }
 
-// ---------------------------------------------------------------- packed level operator (level 0)
+// ---------------------------------------------------------------- packed level operator
 // k_lvl_op with two realizations per lane in float2 registers: the element and
 // node arithmetic issues Blackwell's packed FP32 instructions (one issue slot
-// for both), halving the instructions per realization of an issue-bound
-// kernel. A 3 x 3 tile of node pencils with its 16 element warps for 64
-// realizations, at most 128 registers a thread (16 warps fill the register
-// file: 4 warps per SM sub-partition), and no separate producer warp: lane 0
-// of warp 0 issues the TMA loads two planes ahead (the 3-stage ring refills
-// the stage of the plane before the current one; its readers have arrived on
-// its "empty" barrier, a bounded wait). The exchange buffer holds corners 1..3
-// of each element (corner 0 stays in the registers of the warp that owns its
-// node pencil), which leaves room for the 5 x 5 node patches. Modes, barriers
-// and bounded waits as k_lvl_op otherwise.
-constexpr int kQJ = 3, kQK = 3;                     // node pencils per tile (y, z)
-constexpr int kQEJ = kQJ + 1, kQEK = kQK + 1;       // element pencils 4 x 4
-constexpr int kQWarps = kQEJ * kQEK;                // 16 element warps
+// for both). A work item is a 7 x 3 tile of node pencils for 16 realizations;
+// a warp holds 4 of its 8 x 4 element pencils (8 lanes each). At 128 registers
+// a thread two CTAs of 8 warps fill an SM's register file, so one CTA's plane
+// barrier is filled by the other's work. What bounds it is the latency of a
+// plane's chain (loads, modes, exchange, barrier, node sums) at 16 warps an SM:
+// issue slots and the FMA pipe are both at 45-47 %, DRAM at 60 % of its
+// measured rate. Against one CTA of 16 warps on a 3 x 3 tile of 64
+// realizations, which computed 16 element pencils for 9 nodes (1.78; here 32
+// for 21, 1.52) and had 3 times fewer, longer items: search-direction launch
+// 134 -> 103 us at 24^3 x 256 (2.2 rounds of items there took 3), 22.6 ->
+// 18.5 us at 8^3 x 64 (24 CTAs instead of 9), 776 -> 755 us at 32^3 x 1024.
+// Four items of one tile follow each other, so that CTAs next to each other
+// read whole 256-byte rows (a 16-realization row is 64 bytes; one group after
+// another re-read 35 % of the DRAM bytes). There is no producer warp: lane 0
+// of warp 0 issues the TMA loads two planes ahead. The exchange buffer holds
+// corners 1..3 of each element (corner 0 stays in the registers of the lanes
+// that own its node pencil). Modes and bounded waits as k_lvl_op otherwise.
+constexpr int kQJ = 7, kQK = 3;                     // node pencils per tile (y, z)
+constexpr int kQEJ = kQJ + 1, kQEK = kQK + 1;       // element pencils 8 x 4
+constexpr int kQR = 16;                             // realizations per work item
+constexpr int kQLanes = kQR / 2;                    // lanes of a pencil, two realizations each
+constexpr int kQPencils = 32 / kQLanes;             // pencils per warp, along y
+constexpr int kQWarps = kQEJ * kQEK / kQPencils;    // 8 warps
 constexpr int kQThreads = 32 * kQWarps;
-constexpr int kQPJ = kQJ + 2, kQPK = kQK + 2;       // node patch 5 x 5
-constexpr int kQR = 64;                             // realizations per work item
+constexpr int kQCtas = 2;                           // CTAs per SM
+constexpr int kQQuad = 64 / kQR;                    // items of one tile next to each other: 64 realizations, whole 256-byte rows
+constexpr int kQPJ = kQJ + 2, kQPK = kQK + 2;       // node patch 9 x 5
+static_assert(kQEJ % kQPencils == 0, "a warp's pencils lie in one row");
+constexpr int pad128(int floats) { return (floats + 31) / 32 * 32; }  // TMA destinations: 128-byte boundaries
 constexpr int kQPlane = kQR * 3 * kQPJ * kQPK;      // vector patch (floats)
 constexpr int kQNode = kQR * kQPJ * kQPK;           // dinv patch
 constexpr int kQE = kQR * kQEJ * kQEK;              // E patch
-constexpr int kQD = kQR * 3 * kQJ * kQK;            // d of the tile's own nodes
-// exchange buffer: corners 1..3 of every element warp (corner 0 belongs to the
-// node pencil of the warp itself and stays in its registers)
-constexpr int kQX = kQWarps * 3 * 3 * kQR;
+constexpr int kQD = kQR * 3 * kQJ * kQK;            // d (or b) of the tile's own nodes
+constexpr int kQO = kQR * kQJ * kQK;                // dinv of the tile's own nodes
+// exchange buffer: corners 1..3 of every element pencil (corner 0 belongs to the
+// node pencil of the same lanes and stays in their registers)
+constexpr int kQX = kQEJ * kQEK * 3 * 3 * kQR;
 template <int kMode> struct LvlStage2 {
   static constexpr bool kTwo = kMode == kLvlStart || kMode == kLvlPcgZ;
   // Smooth and Resid also stage b of the tile's own nodes (Smooth its dinv as
   // well), read by the node phase one plane later: their stages are released
-  // after that node phase, so the ring has 4 stages (loads still go two planes ahead)
+  // after that node phase, so the ring has 4 stages (loads go two planes ahead either way)
   static constexpr bool kOwn = kMode == kLvlSmooth || kMode == kLvlResid;
   static constexpr bool kOwnD = kMode == kLvlSmooth;
+  static constexpr bool kNodes = kMode == kLvlStart;   // dinv patch with halo
+  static constexpr bool kDir = kMode == kLvlPcgZ;      // d of the own nodes
   static constexpr int kStages = kOwn ? 4 : kMStages;
   static constexpr int kOffA = 0;
-  static constexpr int kOffB = kQPlane;
-  static constexpr int kOffN = (kTwo ? 2 : 1) * kQPlane;
-  static constexpr int kOffE = kOffN + (kMode == kLvlStart ? kQNode : 0);
-  static constexpr int kOffD = kOffE + kQE;  // d (direction) or own b (smooth, resid)
-  static constexpr int kOffO = kOffD + (kOwn ? kQD : 0);  // own dinv (smooth)
-  static constexpr int kFloats = kOffO + (kMode == kLvlPcgZ ? kQD : 0) + (kOwnD ? kQR * kQJ * kQK : 0);
-  static constexpr uint32_t kBytes = kFloats * 4;
+  static constexpr int kOffB = pad128(kQPlane);
+  static constexpr int kOffN = (kTwo ? 2 : 1) * pad128(kQPlane);
+  static constexpr int kOffE = kOffN + (kNodes ? pad128(kQNode) : 0);
+  static constexpr int kOffD = kOffE + pad128(kQE);  // d (direction) or own b (smooth, resid)
+  static constexpr int kOffO = kOffD + (kOwn ? pad128(kQD) : 0);  // own dinv (smooth)
+  static constexpr int kFloats = kOffO + (kDir ? pad128(kQD) : 0) + (kOwnD ? pad128(kQO) : 0);
+  static constexpr uint32_t kBytes = 4 * ((kTwo ? 2 : 1) * kQPlane + (kNodes ? kQNode : 0) + kQE +
+                                          (kDir || kOwn ? kQD : 0) + (kOwnD ? kQO : 0));  // loaded per stage
   static constexpr size_t kSmem = 128 + sizeof(float) * ((size_t)kStages * kFloats + 2 * (size_t)kQX) +
-                                  sizeof(double) * kQJ * kQK * kQR + sizeof(uint64_t) * (2 * kStages);
+                                  sizeof(double) * kQJ * kQK * kQR + sizeof(uint64_t) * kStages + sizeof(int) * 6;
 };
-static_assert(LvlStage2<kLvlStart>::kBytes % 128 == 0 && LvlStage2<kLvlSmooth>::kBytes % 128 == 0 &&
-                  LvlStage2<kLvlPcgZ>::kBytes % 128 == 0 && LvlStage2<kLvlResid>::kBytes % 128 == 0 &&
-                  LvlStage2<kLvlResid>::kSmem <= 227 * 1024,
-              "stage alignment");
-static_assert(LvlStage2<kLvlPcgZ>::kSmem <= 227 * 1024 && LvlStage2<kLvlStart>::kSmem <= 227 * 1024 &&
-                  LvlStage2<kLvlSmooth>::kSmem <= 227 * 1024 && (kQR * kQJ * kQK * 4) % 128 == 0,
+// two CTAs an SM: 227 KB together, 1 KB of system use each
+static_assert(LvlStage2<kLvlPcgZ>::kSmem <= 112 * 1024 && LvlStage2<kLvlStart>::kSmem <= 112 * 1024 &&
+                  LvlStage2<kLvlSmooth>::kSmem <= 112 * 1024 && LvlStage2<kLvlResid>::kSmem <= 112 * 1024,
               "smem");
 
 template <int kMode, bool kMass>
-__global__ void __maxnreg__(128)
+__global__ void __launch_bounds__(kQThreads, kQCtas)
     k_lvl_op2(Lattice L, const __grid_constant__ ModalCT<float2> C, const __grid_constant__ CUtensorMap tm_a,
               const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_n,
               const __grid_constant__ CUtensorMap tm_e, const __grid_constant__ CUtensorMap tm_d, int tiles_j,
@@ -1612,67 +1626,87 @@ __global__ void __maxnreg__(128)
   float* smem = smem_dyn + (((128u - (smem_u32(smem_dyn) & 127u)) & 127u) >> 2);
   constexpr int kSt = S::kStages;
   float* xbuf = smem + kSt * S::kFloats;
-  double* red = reinterpret_cast<double*>(xbuf + 2 * kQX);  // [node pencils][64]
+  double* red = reinterpret_cast<double*>(xbuf + 2 * kQX);  // [node pencils][kQR]
   uint64_t* full = reinterpret_cast<uint64_t*>(red + kQJ * kQK * kQR);
-  uint64_t* empty = full + kSt;
+  int* next = reinterpret_cast<int*>(full + kSt);  // the producer's next load: item, plane, J0, K0, realization
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int NX = L.NX, Rp = L.Rp, Rp2 = L.Rp >> 1;
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < kSt; ++st) {
-      mbar_init(&full[st], 1);
-      mbar_init(&empty[st], kQWarps);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  // producer role: global step q loads (item, plane) = (blockIdx.x + (q / NX) gridDim.x, q % NX + 1)
-  // into stage q % 3
+  const auto item_tile = [&](int item) { return (item / kQQuad) % n_tiles; };
+  const auto item_col = [&](int item) { return (item / (kQQuad * n_tiles) * kQQuad + item % kQQuad) * kQR; };
+  // The producer (lane 0 of warp 0, whose pencils own no nodes) loads the
+  // planes of the CTA's items in order, plane q into stage q % kSt: planes 0, 1
+  // and 2 at the start and plane c + 2 after the c-th plane barrier, when the
+  // readers of the stage it refills (plane c - 1, or c - 2 with kOwn's four
+  // stages) have all passed that barrier. The position is stepped, not divided
+  // out of q, and kept in shared memory: on the critical path of warp 0 the
+  // divisions took 1,100 of 3,500 cycles a plane.
   const bool producer = w == 0 && lane == 0;
-  auto produce = [&](uint32_t q) {
-    const int item = blockIdx.x + (int)(q / (uint32_t)NX) * gridDim.x;
+  uint32_t n_loads = 0;  // of the producer: planes loaded so far
+  const auto produce = [&]() {
+    const int item = next[0];
     if (item >= n_items) return;
-    const int P = (int)(q % (uint32_t)NX) + 1;
-    const int tile = item % n_tiles, g64 = (item / n_tiles) * kQR;
-    const int J0 = 1 + (tile % tiles_j) * kQJ, K0 = 1 + (tile / tiles_j) * kQK;
-    const int st = q % kSt;
-    const uint32_t use = q / kSt;
-    if (use > 0 && !mbar_wait(&empty[st], (use - 1) & 1)) {
-      atomicExch(err, 1);
-      return;
-    }
+    const int P = next[1], J0 = next[2], K0 = next[3], g16 = next[4];
+    const int st = n_loads % kSt;
+    ++n_loads;
     float* dst = smem + st * S::kFloats;
     mbar_expect_tx(&full[st], S::kBytes);
-    tma_load_5d(dst + S::kOffA, &tm_a, g64, 0, P, J0 - 1, K0 - 1, &full[st]);
-    if constexpr (S::kTwo) tma_load_5d(dst + S::kOffB, &tm_b, g64, 0, P, J0 - 1, K0 - 1, &full[st]);
-    if constexpr (kMode == kLvlStart) tma_load_4d(dst + S::kOffN, &tm_n, g64, P, J0 - 1, K0 - 1, &full[st]);
-    tma_load_4d(dst + S::kOffE, &tm_e, g64, P - 1, J0 - 1, K0 - 1, &full[st]);
-    if constexpr (kMode == kLvlPcgZ) tma_load_5d(dst + S::kOffD, &tm_d, g64, 0, P, J0, K0, &full[st]);
-    if constexpr (S::kOwn) tma_load_5d(dst + S::kOffD, &tm_b, g64, 0, P, J0, K0, &full[st]);
-    if constexpr (S::kOwnD) tma_load_4d(dst + S::kOffO, &tm_n, g64, P, J0, K0, &full[st]);
+    tma_load_5d(dst + S::kOffA, &tm_a, g16, 0, P, J0 - 1, K0 - 1, &full[st]);
+    if constexpr (S::kTwo) tma_load_5d(dst + S::kOffB, &tm_b, g16, 0, P, J0 - 1, K0 - 1, &full[st]);
+    if constexpr (kMode == kLvlStart) tma_load_4d(dst + S::kOffN, &tm_n, g16, P, J0 - 1, K0 - 1, &full[st]);
+    tma_load_4d(dst + S::kOffE, &tm_e, g16, P - 1, J0 - 1, K0 - 1, &full[st]);
+    if constexpr (kMode == kLvlPcgZ) tma_load_5d(dst + S::kOffD, &tm_d, g16, 0, P, J0, K0, &full[st]);
+    if constexpr (S::kOwn) tma_load_5d(dst + S::kOffD, &tm_b, g16, 0, P, J0, K0, &full[st]);
+    if constexpr (S::kOwnD) tma_load_4d(dst + S::kOffO, &tm_n, g16, P, J0, K0, &full[st]);
+    if (P < NX) {
+      next[1] = P + 1;
+      return;
+    }
+    const int it = item + gridDim.x, tile = item_tile(it);
+    next[0] = it;
+    next[1] = 1;
+    next[2] = 1 + (tile % tiles_j) * kQJ;
+    next[3] = 1 + (tile / tiles_j) * kQK;
+    next[4] = item_col(it);
   };
-  if (producer) {
-    produce(0);
-    produce(1);
+  if (threadIdx.x == 0) {
+    for (int st = 0; st < kSt; ++st) mbar_init(&full[st], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    const int it = blockIdx.x, tile = item_tile(it);
+    next[0] = it;
+    next[1] = 1;
+    next[2] = 1 + (tile % tiles_j) * kQJ;
+    next[3] = 1 + (tile / tiles_j) * kQK;
+    next[4] = item_col(it);
+    for (int q = 0; q < 3; ++q) produce();
   }
-  const int ej = w % kQEJ, ek = w / kQEJ;
-  const bool node_warp = ej >= 1 && ek >= 1;
+  __syncthreads();
+  // this lane's element pencil and realization pair
+  constexpr int kRow = kQEJ / kQPencils;  // warps per row of pencils
+  const int l2 = lane % kQLanes;
+  const int ej = (w % kRow) * kQPencils + lane / kQLanes, ek = w / kRow;
+  const int pid = ek * kQEJ + ej;
+  const bool node_warp = ek >= 1;                // warps with node pencils
+  const bool node_lane = node_warp && ej >= 1;
   uint32_t seq = 0;
   int xsel = 0;
   bool dead = false;
   auto csync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kQWarps * 32) : "memory"); };
+  // the barrier of a plane between the element and the node phase; the stage it frees is refilled
+  auto plane_sync = [&]() {
+    csync();
+    if (producer && !dead) produce();
+  };
   const float2 z2 = make_float2(0.f, 0.f);
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int tile = item % n_tiles, g64 = (item / n_tiles) * kQR;
+    const int tile = item_tile(item), g16 = item_col(item);
     const int J0 = 1 + (tile % tiles_j) * kQJ, K0 = 1 + (tile / tiles_j) * kQK;
     const int Je = J0 - 1 + ej, Ke = K0 - 1 + ek;
     auto realj = [&](int j) { return j >= 1 && j <= L.NY - 1; };
     auto realk = [&](int k) { return k >= 1 && k <= L.NZ - 1; };
     const bool real = realj(Je) && realk(Ke);
-    const bool node_ok = node_warp && Je <= L.NY && Ke <= L.NZ;
-    const bool r00 = real, r10 = realj(Je - 1) && realk(Ke);
-    const bool r01 = realj(Je) && realk(Ke - 1), r11 = realj(Je - 1) && realk(Ke - 1);
+    const bool node_ok = node_lane && Je <= L.NY && Ke <= L.NZ;
     const size_t nrow = ((size_t)Je + (size_t)L.NYp * Ke) * L.NXp;
-    const int rr2 = (g64 >> 1) + lane;  // float2 index of this lane's realization pair
+    const int rr2 = (g16 >> 1) + l2;  // float2 index of this lane's realization pair
     float2 al = z2, be = z2;
     if constexpr (kMode == kLvlStart || kMode == kLvlPcgZ) al = reinterpret_cast<const float2*>(alpha)[rr2];
     if constexpr (kMode == kLvlPcgZ) be = reinterpret_cast<const float2*>(beta)[rr2];
@@ -1688,27 +1722,32 @@ __global__ void __maxnreg__(128)
 #pragma unroll
       for (int qq = 0; qq < 4; ++qq) T0[c][qq] = z2;
     double acc0 = 0.0, acc1 = 0.0;
-    uint32_t mreg = 0;
+    uint32_t mreg = 0;  // constraint bits of 4 planes of the own pencil
     auto node_phase = [&](int X, uint32_t seq_x) {
       [[maybe_unused]] const float* px = smem + (seq_x % kSt) * S::kFloats;
       [[maybe_unused]] const int od = (ek - 1) * kQJ + (ej - 1);
-      if (((X - 1) & 31) == 0) {
-        const int pl = X + lane;
-        mreg = (pl <= NX) ? mask[nrow + pl] : 0u;
+      if (((X - 1) & (4 * kQLanes - 1)) == 0) {  // the next 32 planes, 4 a lane
+        mreg = 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int pl = X + 4 * l2 + i;
+          if (node_ok && pl <= NX) mreg |= (uint32_t)mask[nrow + pl] << (8 * i);
+        }
       }
-      const uint32_t mk = __shfl_sync(0xffffffffu, mreg, (X - 1) & 31);
+      const int mx = (X - 1) & (4 * kQLanes - 1);
+      const uint32_t mk = __shfl_sync(0xffffffffu, mreg, mx >> 2, kQLanes) >> (8 * (mx & 3));
+      if (!node_ok) return;
       const float2* xb = xb2 + xsel * (kQX / 2);
       const size_t node = nrow + X;
       float2 wdv = z2;
-      if constexpr (kMode == kLvlSmooth) wdv = om2 * reinterpret_cast<const float2*>(px + S::kOffO)[od * 32 + lane];
+      if constexpr (kMode == kLvlSmooth) wdv = om2 * reinterpret_cast<const float2*>(px + S::kOffO)[od * kQLanes + l2];
       double s0 = 0.0, s1 = 0.0;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        float2 y = z2;
-        if (r00) y = y + own[c];
-        if (r10) y = y + xb[(((w - 1) * 3 + 0) * 3 + c) * 32 + lane];
-        if (r01) y = y + xb[(((w - kQEJ) * 3 + 1) * 3 + c) * 32 + lane];
-        if (r11) y = y + xb[(((w - kQEJ - 1) * 3 + 2) * 3 + c) * 32 + lane];
+        float2 y = own[c];
+        y = y + xb[(((pid - 1) * 3 + 0) * 3 + c) * kQLanes + l2];
+        y = y + xb[(((pid - kQEJ) * 3 + 1) * 3 + c) * kQLanes + l2];
+        y = y + xb[(((pid - kQEJ - 1) * 3 + 2) * 3 + c) * kQLanes + l2];
         const size_t o = (node * 3 + c) * Rp2 + rr2;
         const bool fixed = (mk >> c) & 1;
         float2 v;
@@ -1717,9 +1756,9 @@ __global__ void __maxnreg__(128)
           s0 = fma((double)orc[c].x, (double)orc[c].x, s0);
           s1 = fma((double)orc[c].y, (double)orc[c].y, s1);
         } else if constexpr (kMode == kLvlResid) {
-          v = fixed ? z2 : reinterpret_cast<const float2*>(px + S::kOffD)[(od * 3 + c) * 32 + lane] - y;
+          v = fixed ? z2 : reinterpret_cast<const float2*>(px + S::kOffD)[(od * 3 + c) * kQLanes + l2] - y;
         } else if constexpr (kMode == kLvlSmooth) {
-          const float2 bv = reinterpret_cast<const float2*>(px + S::kOffD)[(od * 3 + c) * 32 + lane];
+          const float2 bv = reinterpret_cast<const float2*>(px + S::kOffD)[(od * 3 + c) * kQLanes + l2];
           v = fixed ? z2 : fmx(wdv, bv - y, ou[c]);
           s0 = fma((double)v.x, (double)bv.x, s0);
           s1 = fma((double)v.y, (double)bv.y, s1);
@@ -1740,14 +1779,13 @@ __global__ void __maxnreg__(128)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         own[c] = y[0][0][c];
-        xb[((w * 3 + 0) * 3 + c) * 32 + lane] = y[1][0][c];
-        xb[((w * 3 + 1) * 3 + c) * 32 + lane] = y[0][1][c];
-        xb[((w * 3 + 2) * 3 + c) * 32 + lane] = y[1][1][c];
+        xb[((pid * 3 + 0) * 3 + c) * kQLanes + l2] = y[1][0][c];
+        xb[((pid * 3 + 1) * 3 + c) * kQLanes + l2] = y[0][1][c];
+        xb[((pid * 3 + 2) * 3 + c) * kQLanes + l2] = y[1][1][c];
       }
     };
     for (int P = 1; P <= NX; ++P, ++seq) {
       const int st = seq % kSt;
-      if (producer && !dead) produce(seq + 2);
       if (!dead && !mbar_wait(&full[st], (seq / kSt) & 1)) {
         atomicExch(err, 1);
         dead = true;
@@ -1763,10 +1801,10 @@ __global__ void __maxnreg__(128)
           const int o = (ek + az) * kQPJ + (ej + ay);
           float2 wdv = z2;
           if constexpr (kMode == kLvlStart)
-            wdv = om2 * reinterpret_cast<const float2*>(pt + S::kOffN)[o * 32 + lane];
+            wdv = om2 * reinterpret_cast<const float2*>(pt + S::kOffN)[o * kQLanes + l2];
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            const int i = (o * 3 + c) * 32 + lane;
+            const int i = (o * 3 + c) * kQLanes + l2;
             if constexpr (kMode == kLvlStart) {
               const float2 rn = fmx(nal, pb[i], pa[i]);
               u[ay][az][c] = wdv * rn;
@@ -1778,7 +1816,7 @@ __global__ void __maxnreg__(128)
             }
           }
         }
-      const float2 E = reinterpret_cast<const float2*>(pt + S::kOffE)[w * 32 + lane];
+      const float2 E = reinterpret_cast<const float2*>(pt + S::kOffE)[pid * kQLanes + l2];
       if constexpr (kMode == kLvlStart || kMode == kLvlPcgZ) {
         if (node_ok) {
           const size_t node = nrow + P;
@@ -1790,35 +1828,37 @@ __global__ void __maxnreg__(128)
               if (out3 != nullptr) reinterpret_cast<float2*>(out3)[o] = u[0][0][c];
             } else {
               const int op = ek * kQPJ + ej, od = (ek - 1) * kQJ + (ej - 1);
-              const float2 pold = pb[(op * 3 + c) * 32 + lane];
-              const float2 dold = reinterpret_cast<const float2*>(pt + S::kOffD)[(od * 3 + c) * 32 + lane];
+              const float2 pold = pb[(op * 3 + c) * kQLanes + l2];
+              const float2 dold = reinterpret_cast<const float2*>(pt + S::kOffD)[(od * 3 + c) * kQLanes + l2];
               reinterpret_cast<float2*>(out2)[o] = u[0][0][c];
               reinterpret_cast<float2*>(d)[o] = fmx(al, pold, dold);
             }
           }
         }
       }
-      __syncwarp();
-      if (!S::kOwn && lane == 0) mbar_arrive(&empty[st]);
       float2 Bc[3][4];
       yz_forward(u, Bc);
       if (P >= 2) {
-        if (real) {
+        {
+          // ghost pencils have E = 0 and emit zeros (the mass term, which does not
+          // scale with E, is left out of them below)
           float2 C1[3][4];
           modal_apply<kMass>(C, E, Bp, Bc, T0, C1);
+          if (kMass && !real) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+              for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq] = z2;
+          }
           emit_corners(T0);
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
         }
-        csync();
-        if (node_ok) node_phase(P - 1, seq - 1);
+        plane_sync();
+        if (node_warp) node_phase(P - 1, seq - 1);
         xsel ^= 1;
-        if constexpr (S::kOwn) {  // the node phase of plane P - 1 is done with its stage
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&empty[(seq - 1) % kSt]);
-        }
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -1828,27 +1868,23 @@ __global__ void __maxnreg__(128)
         for (int qq = 0; qq < 4; ++qq) Bp[c][qq] = Bc[c][qq];
       }
     }
-    if (real) emit_corners(T0);
-    csync();
-    if (node_ok) node_phase(NX, seq - 1);
+    emit_corners(T0);
+    plane_sync();
+    if (node_warp) node_phase(NX, seq - 1);
     xsel ^= 1;
-    if constexpr (S::kOwn) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[(seq - 1) % kSt]);
-    }
     if (kMode != kLvlResid && partial != nullptr) {
-      if (node_warp) {
+      if (node_lane) {
         const int nw = (ek - 1) * kQJ + (ej - 1);
-        red[nw * kQR + 2 * lane] = acc0;
-        red[nw * kQR + 2 * lane + 1] = acc1;
+        red[nw * kQR + 2 * l2] = acc0;
+        red[nw * kQR + 2 * l2 + 1] = acc1;
       }
       csync();
-      if (w < 2) {
-        const int rl = w * 32 + lane;  // realization within the item
+      if (threadIdx.x < kQR) {
+        const int rl = threadIdx.x;  // realization within the item
         double sum = 0.0;
 #pragma unroll
         for (int i = 0; i < kQJ * kQK; ++i) sum += red[i * kQR + rl];
-        partial[((size_t)tile * Rp + g64 + rl) * pstride] = sum;
+        partial[((size_t)tile * Rp + g16 + rl) * pstride] = sum;
       }
     }
   }
@@ -2888,7 +2924,7 @@ struct BlockSys {
   GmgLevel lv[kGmgMaxLevels];
   WSlot xs, arena;
   CUtensorMap tm_xs;
-  // packed level-0 operator (k_lvl_op2: 64 realizations per item, 3 x 3 tiles)
+  // packed level-0 operator (k_lvl_op2: 16 realizations per item, 7 x 3 tiles)
   bool pack = false;
   ModalCT<float2> MC2;
   int tiles_j2 = 0, n_tiles2 = 0, n_items2 = 0, grid2 = 0;
@@ -3340,7 +3376,7 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
       B->tc = ctx->tensor_op != 0 && !B->mass;
       if (B->tc) MSG_TRY(tc_setup(ctx, B, K576));
       // packed level-0 operator: realizations in multiples of 64
-      B->pack = ctx->mg_packed && (Rp % kQR) == 0;
+      B->pack = ctx->mg_packed && (Rp % (kQQuad * kQR)) == 0;
       if (B->pack) {
         auto b2 = [](float v) { return make_float2(v, v); };
         auto pack_c = [&](const ModalC& f, ModalCT<float2>& g2) {
@@ -3352,10 +3388,11 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
         B->tiles_j2 = (L.NY + kQJ - 1) / kQJ;
         B->n_tiles2 = B->tiles_j2 * ((L.NZ + kQK - 1) / kQK);
         B->n_items2 = B->n_tiles2 * (Rp / kQR);
-        B->grid2 = B->X.persistent ? std::min(B->n_items2, ctx->sm_count) : B->n_items2;
-        // the loop's partials: [tile][Rp][2] and [tile][Rp] over the packed tiles
-        const size_t need = sizeof(double) * (size_t)std::max({B->n_tiles * 2, B->n_tiles_m * kMParts,
-                                                                B->n_tiles2 * 3}) * Rp;
+        B->grid2 = B->X.persistent ? std::min(B->n_items2, kQCtas * ctx->sm_count) : B->n_items2;
+        // the loop's partials: [tile][Rp][2] and [tile][Rp] over the packed tiles (the
+        // tensor-core direction launch writes its [tile][Rp] over its own tiles)
+        const size_t need = sizeof(double) * (size_t)std::max({B->n_tiles * 2, B->n_tiles_m * kMParts, B->n_tiles2 * 3,
+                                                                B->tc ? B->n_tiles2 * 2 + B->n_tiles_m : 0}) * Rp;
         MSG_TRY(B->slot_alloc(ctx, 9, need, &B->part_op.ptr));
         const cuuint32_t pb2[5] = {kQR, 3, 1, kQPJ, kQPK};
         const cuuint32_t nb2[4] = {kQR, 1, kQPJ, kQPK};
@@ -3380,7 +3417,7 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
           g.tiles_j2 = (Lc.NY + kQJ - 1) / kQJ;
           g.n_tiles2 = g.tiles_j2 * ((Lc.NZ + kQK - 1) / kQK);
           g.n_items2 = g.n_tiles2 * (Rp / kQR);
-          g.grid2 = B->X.persistent ? std::min(g.n_items2, ctx->sm_count) : g.n_items2;
+          g.grid2 = B->X.persistent ? std::min(g.n_items2, kQCtas * ctx->sm_count) : g.n_items2;
           const cuuint64_t cpd[5] = {(cuuint64_t)Rp, 3, (cuuint64_t)Lc.NXp, (cuuint64_t)Lc.NYp, (cuuint64_t)Lc.NZp};
           const cuuint64_t cps[4] = {Rp * fb, 3 * Rp * fb, 3 * Rp * fb * Lc.NXp, 3 * Rp * fb * Lc.NXp * Lc.NYp};
           const cuuint64_t ced[4] = {(cuuint64_t)Rp, (cuuint64_t)Lc.NXp, (cuuint64_t)Lc.NYp, (cuuint64_t)Lc.NZp};
@@ -3661,7 +3698,7 @@ void gmg_iteration(BlockSys* B, const LoopCfg& c, int it, cudaStream_t st) {
          B->d.as<float>(), part1, 1);
   }
   if (it == 0) cudaEventRecordWithFlags(ev[5], st, cudaEventRecordExternal);
-  k_gmg_alpha<<<c.sblocks, 1024, 0, st>>>(Rp, nt0, part1, s);
+  k_gmg_alpha<<<c.sblocks, 1024, 0, st>>>(Rp, B->tc ? B->n_tiles_m : nt0, part1, s);
   if (it == 0) cudaEventRecordWithFlags(ev[7], st, cudaEventRecordExternal);
 }
 
