@@ -359,9 +359,9 @@ typedef struct {
  * reference's SolverPCG with the diagonal preconditioner) with the iterate in
  * FP64 and FP64 true residuals, to ||b - K x||/||b|| < tol in FP64 for each
  * realization. With the multigrid option on (the default), a system whose mesh
- * has the numbering of an nx x ny x nz lattice with every side even and >= 4
- * (moved nodes allowed) is preconditioned instead by the V-cycle of its cube
- * lattice, and then the whole batch runs standard PCG (the operator, scalar
+ * has the numbering of an nx x ny x nz lattice that coarsens (every side at
+ * least 3; with an odd side, at least 216 elements; moved nodes allowed) is
+ * preconditioned instead by the V-cycle of its cube lattice, and then the whole batch runs standard PCG (the operator, scalar
  * and vector launches shared, one V-cycle per such system, the diagonal for
  * the others; two iterations to a graph launch). A system's results do not
  * depend on the other systems in the batch: the same bits alone and in any mix
@@ -461,9 +461,11 @@ int MSG_SERVE_STOP(MSG_CTX ctx);
  * batched lattice loop: 1, default, a geometric multigrid V-cycle for systems
  * without a mass term (static solves, serving), Jacobi for those with one
  * (Newmark); 2: the V-cycle for both; 0: Jacobi for both. The V-cycle needs a
- * lattice whose element counts are even at least once; otherwise Jacobi runs),
+ * lattice with every side at least 3 and, with an odd side, at least 216
+ * elements; otherwise Jacobi runs),
  * "multigrid_levels" (lattice levels at most, fine level included, 2..6,
- * default 6; a level halves every axis while each keeps at least 2 elements),
+ * default 6; a level halves every axis, rounding up, while the shortest has more
+ * than 2 elements),
  * "multigrid_sweeps" (damped Jacobi sweeps on the coarsest level, default 20),
  * "multigrid_omega" (Jacobi damping of every level, 0 = derived from the
  * element stiffness, default), "multigrid_delta" (reliable-update factor of the
@@ -471,7 +473,7 @@ int MSG_SERVE_STOP(MSG_CTX ctx);
  * (1, default: the three level-0 operator passes of an iteration work on two
  * realizations per thread with packed FP32 arithmetic; 0: one per thread),
  * "multigrid_fused_coarse" (1, default: every sweep of the coarsest level in
- * one launch when that level has at most 3 x 3 nodes across y and z; 0: one
+ * one launch when that level fits a CTA's shared memory; 0: one
  * launch per sweep; the results are identical), "serve_persistent" (serving
  * lanes created afterwards: 1, default, persistent grids of one CTA per SM;
  * 0: one CTA per work item of their level operators, so other lanes' launches

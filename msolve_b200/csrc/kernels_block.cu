@@ -1402,17 +1402,20 @@ __global__ void __launch_bounds__(kMThreads, 1)
 }
 
 // ---------------------------------------------------------------- coarsest-level sweeps
-// All damped Jacobi sweeps of the coarsest level in one launch. That level has
-// at most 3 x 3 node pencils in (y, z), one k_lvl_op tile, so a CTA holds the
-// whole level for its 32 realizations in shared memory (the iterate in two
-// buffers, b, omega dinv, E and the mask, real nodes only) and consecutive
-// sweeps are separated by CTA barriers instead of launches. Every sweep is the
-// arithmetic of k_lvl_op<kLvlSmooth> in the same order (element warps over the
-// x-planes, the same exchange and the same node sums), so the iterates are
-// identical to the launch-per-sweep loop.
+// All damped Jacobi sweeps of the coarsest level in one launch: a CTA holds the
+// whole level for its 32 realizations in shared memory (the iterate, b, omega
+// dinv, E and the mask, real nodes only). A sweep is two phases with a CTA
+// barrier after each: every (element pencil, x-plane) pair, one a warp, forms
+// the plane's corner contributions from the two elements next to it; then every
+// node sums the four pencils around it and steps the iterate in place. It is
+// bound by the latency of these two phases (0.6 us a sweep on 2 x 2 x 2
+// elements; 19 sweeps 41 -> 14 us against marching along x with a barrier a
+// plane). Every sweep is the arithmetic of k_lvl_op<kLvlSmooth> in the same
+// order, so the iterates are identical to the launch-per-sweep loop.
+constexpr int kCsX = 4 * 3 * 32;  // corner contributions of one (pencil, plane) pair
 inline size_t coarse_sweep_smem(const Lattice& L) {
-  const size_t nn = (size_t)L.NX * L.NY * L.NZ, ne = (size_t)(L.NX - 1) * (L.NY - 1) * (L.NZ - 1);
-  return sizeof(float) * (nn * 32 * 10 + ne * 32 + 2 * (size_t)kMXFloats) + nn;
+  const size_t nn = (size_t)L.NX * L.NY * L.NZ, np = (size_t)(L.NY - 1) * (L.NZ - 1), ne = np * (L.NX - 1);
+  return sizeof(float) * (nn * 32 * 7 + ne * 32 + np * L.NX * kCsX) + sizeof(int2) * (nn + np * L.NX);
 }
 template <bool kMass>
 __global__ void __launch_bounds__(kMWarps * 32, 1)
@@ -1421,126 +1424,117 @@ __global__ void __launch_bounds__(kMWarps * 32, 1)
                     float omega, int n_sweeps, const float* __restrict__ x, float* __restrict__ out) {
   extern __shared__ __align__(16) float smem_cs[];
   const int NX = L.NX, NY = L.NY, NZ = L.NZ, Rp = L.Rp;
-  const int nn = NX * NY * NZ, ne = (NX - 1) * (NY - 1) * (NZ - 1);
-  float* src = smem_cs;           // iterate [node][c][32]
-  float* dst = src + nn * 96;
-  float* bs = dst + nn * 96;      // b [node][c][32]
+  const int nn = NX * NY * NZ, np = (NY - 1) * (NZ - 1), ne = np * (NX - 1);
+  float* it = smem_cs;            // iterate [node][c][32]
+  float* bs = it + nn * 96;       // b [node][c][32]
   float* ws = bs + nn * 96;       // omega dinv [node][32]
   float* es = ws + nn * 32;       // E [element][32]
-  float* xbuf = es + ne * 32;     // two exchange buffers
-  uint8_t* mks = reinterpret_cast<uint8_t*>(xbuf + 2 * kMXFloats);
+  float* xbuf = es + ne * 32;     // [pencil][plane][corner][c][32]
+  // index tables, so that the sweeps divide nothing: (pencil, plane) pair u -> its
+  // node 0 and element (X - 1 below, X above; bit 30, 31: there is one); node i ->
+  // offset of the exchange of pencil (J - 1, K - 1), and its neighbours and mask
+  int2* utab = reinterpret_cast<int2*>(xbuf + np * NX * kCsX);
+  int2* ntab = utab + np * NX;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int rr = blockIdx.x * 32 + lane;
-  auto cn = [&](int X, int J, int K) { return (X - 1) + NX * ((J - 1) + NY * (K - 1)); };
-  auto ce = [&](int X, int J, int K) { return (X - 1) + (NX - 1) * ((J - 1) + (NY - 1) * (K - 1)); };
-  auto pn = [&](int X, int J, int K) { return (size_t)X + (size_t)L.NXp * ((size_t)J + (size_t)L.NYp * K); };
+  // 0-based node (X, J, K), element (X, j, k) and pencil (j, k)
+  auto cn = [&](int X, int J, int K) { return X + NX * (J + NY * K); };
+  auto pn = [&](int X, int J, int K) { return (size_t)(X + 1) + (size_t)L.NXp * ((size_t)(J + 1) + (size_t)L.NYp * (K + 1)); };
   for (int i = w; i < nn; i += kMWarps) {
-    const int X = i % NX + 1, J = (i / NX) % NY + 1, K = i / (NX * NY) + 1;
+    const int X = i % NX, J = (i / NX) % NY, K = i / (NX * NY);
     const size_t pi = pn(X, J, K);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      src[(i * 3 + c) * 32 + lane] = x[(pi * 3 + c) * Rp + rr];
+      it[(i * 3 + c) * 32 + lane] = x[(pi * 3 + c) * Rp + rr];
       bs[(i * 3 + c) * 32 + lane] = b[(pi * 3 + c) * Rp + rr];
     }
     ws[i * 32 + lane] = omega * dinv[pi * Rp + rr];
-    if (lane == 0) mks[i] = mask[pi];
+    if (lane == 0)
+      ntab[i] = make_int2(((J - 1 + (NY - 1) * (K - 1)) * NX + X) * kCsX,
+                          (J < NY - 1) | (J > 0) << 1 | (K < NZ - 1) << 2 | (K > 0) << 3 | mask[pi] << 4);
+  }
+  for (int u = threadIdx.x; u < np * NX; u += kMWarps * 32) {
+    const int X = u % NX, p = u / NX;
+    utab[u] = make_int2(cn(X, p % (NY - 1), p / (NY - 1)) | (X > 0) << 30, (p * (NX - 1) + X) | (X < NX - 1) << 30);
   }
   for (int i = w; i < ne; i += kMWarps) {
-    const int X = i % (NX - 1) + 1, J = (i / (NX - 1)) % (NY - 1) + 1, K = i / ((NX - 1) * (NY - 1)) + 1;
-    es[i * 32 + lane] = E[pn(X, J, K) * Rp + rr];
+    const int X = i % (NX - 1), p = i / (NX - 1);
+    es[i * 32 + lane] = E[pn(X, p % (NY - 1), p / (NY - 1)) * Rp + rr];
   }
   __syncthreads();
-  // the tile starts at node pencil (1, 1): element pencil (Je, Ke) = (ej, ek)
-  const int Je = w % kMEJ, Ke = w / kMEJ;
-  auto realj = [&](int j) { return j >= 1 && j <= NY - 1; };
-  auto realk = [&](int k) { return k >= 1 && k <= NZ - 1; };
-  const bool real = realj(Je) && realk(Ke);
-  const bool node_ok = Je >= 1 && Ke >= 1 && Je <= NY && Ke <= NZ;
-  const bool r00 = real, r10 = realj(Je - 1) && realk(Ke);
-  const bool r01 = realj(Je) && realk(Ke - 1), r11 = realj(Je - 1) && realk(Ke - 1);
-  int xsel = 0;
   for (int sw = 0; sw < n_sweeps; ++sw) {
-    float Bp[3][4], T0[3][4], ou[3] = {0.f, 0.f, 0.f};
+    // corner contributions of plane X of pencil p: the part of the element below
+    // it (upper face), then that of the element above it (lower face)
+    for (int u = w; u < np * NX; u += kMWarps) {
+      const int2 t = utab[u];
+      const bool below = t.x >> 30, above = t.y >> 30;
+      const float* i0 = it + (t.x & 0x3fffffff) * 96 + lane;
+      auto plane = [&](int d, float (&B)[3][4]) {
+        float v[2][2][3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+        for (int ay = 0; ay < 2; ++ay)
 #pragma unroll
-      for (int qq = 0; qq < 4; ++qq) T0[c][qq] = 0.f;
-    auto node_phase = [&](int X) {
-      const int i = cn(X, Je, Ke);
-      const uint32_t mk = mks[i];
-      const float* xb = xbuf + xsel * kMXFloats;
-      const float wdv = ws[i * 32 + lane];
+          for (int az = 0; az < 2; ++az)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        float y = 0.f;
-        if (r00) y += xb[((w * 4 + 0) * 3 + c) * 32 + lane];
-        if (r10) y += xb[(((w - 1) * 4 + 1) * 3 + c) * 32 + lane];
-        if (r01) y += xb[(((w - kMEJ) * 4 + 2) * 3 + c) * 32 + lane];
-        if (r11) y += xb[(((w - kMEJ - 1) * 4 + 3) * 3 + c) * 32 + lane];
-        const float bv = bs[(i * 3 + c) * 32 + lane];
-        dst[(i * 3 + c) * 32 + lane] = ((mk >> c) & 1) ? 0.f : fmaf(wdv, bv - y, ou[c]);
+            for (int c = 0; c < 3; ++c) v[ay][az][c] = i0[(d + ay * NX + az * NX * NY) * 96 + c * 32];
+        yz_forward(v, B);
+      };
+      const float* ep = es + (t.y & 0x3fffffff) * 32 + lane;
+      float T0[3][4], C1[3][4], Bo[3][4], Bc[3][4];
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq] = 0.f;
+      plane(0, Bc);
+      if (below) {
+        plane(-1, Bo);
+        modal_apply<kMass>(C, ep[-32], Bo, Bc, T0, C1);
       }
-    };
-    auto emit_corners = [&](const float (&B)[3][4]) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
+      if (above) {
+        plane(1, Bo);
+        modal_apply<kMass>(C, ep[0], Bc, Bo, T0, C1);
+      }
       float y[2][2][3];
-      yz_inverse(B, y);
-      float* xb = xbuf + xsel * kMXFloats;
+      yz_inverse(T0, y);
+      float* xb = xbuf + (size_t)u * kCsX + lane;
 #pragma unroll
       for (int ay = 0; ay < 2; ++ay)
 #pragma unroll
         for (int az = 0; az < 2; ++az)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) xb[((w * 4 + ay + 2 * az) * 3 + c) * 32 + lane] = y[ay][az][c];
-    };
-    for (int P = 1; P <= NX; ++P) {
-      float u[2][2][3];
-#pragma unroll
-      for (int ay = 0; ay < 2; ++ay)
-#pragma unroll
-        for (int az = 0; az < 2; ++az) {
-          const int J = Je + ay, K = Ke + az;
-          const bool in = J >= 1 && J <= NY && K >= 1 && K <= NZ;  // ghost nodes are zero
-          const int i = in ? cn(P, J, K) : 0;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) u[ay][az][c] = in ? src[(i * 3 + c) * 32 + lane] : 0.f;
-        }
-      float Bc[3][4];
-      yz_forward(u, Bc);
-      if (P >= 2) {
-        if (real) {
-          float C1[3][4];
-          modal_apply<kMass>(C, es[ce(P - 1, Je, Ke) * 32 + lane], Bp, Bc, T0, C1);
-          emit_corners(T0);
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
-        }
-        __syncthreads();
-        if (node_ok) node_phase(P - 1);
-        xsel ^= 1;
-      }
+          for (int c = 0; c < 3; ++c) xb[((ay + 2 * az) * 3 + c) * 32] = y[ay][az][c];
+    }
+    __syncthreads();
+    for (int i = w; i < nn; i += kMWarps) {
+      const int2 t = ntab[i];
+      const uint32_t mk = t.y >> 4;
+      const float wdv = ws[i * 32 + lane];
+      // pencils around the node: (J, K), (J - 1, K), (J, K - 1), (J - 1, K - 1)
+      const bool jh = t.y & 1, jl = t.y & 2, kh = t.y & 4, kl = t.y & 8;
+      const float* xb = xbuf + t.x + lane;
+      const int sj = NX * kCsX, sk = (NY - 1) * NX * kCsX;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        ou[c] = u[0][0][c];
-#pragma unroll
-        for (int qq = 0; qq < 4; ++qq) Bp[c][qq] = Bc[c][qq];
+        float y = 0.f;
+        if (jh && kh) y += xb[sj + sk + (0 * 3 + c) * 32];
+        if (jl && kh) y += xb[sk + (1 * 3 + c) * 32];
+        if (jh && kl) y += xb[sj + (2 * 3 + c) * 32];
+        if (jl && kl) y += xb[(3 * 3 + c) * 32];
+        const int o = (i * 3 + c) * 32 + lane;
+        it[o] = ((mk >> c) & 1) ? 0.f : fmaf(wdv, bs[o] - y, it[o]);
       }
     }
-    if (real) emit_corners(T0);
-    __syncthreads();
-    if (node_ok) node_phase(NX);
-    xsel ^= 1;
     __syncthreads();  // the sweep's iterate is complete before the next one reads it
-    float* tmp = src;
-    src = dst;
-    dst = tmp;
   }
   for (int i = w; i < nn; i += kMWarps) {
-    const int X = i % NX + 1, J = (i / NX) % NY + 1, K = i / (NX * NY) + 1;
+    const int X = i % NX, J = (i / NX) % NY, K = i / (NX * NY);
     const size_t pi = pn(X, J, K);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) out[(pi * 3 + c) * Rp + rr] = src[(i * 3 + c) * 32 + lane];
+    for (int c = 0; c < 3; ++c) out[(pi * 3 + c) * Rp + rr] = it[(i * 3 + c) * 32 + lane];
   }
 }
 
@@ -2122,140 +2116,133 @@ __global__ void __launch_bounds__(kRThreads, 1)
 
 // Full-weighting restriction b_c = P^T t_f (P: trilinear prolongation), masked
 // at the coarse level, and x_c = omega dinv_c b_c (the first Jacobi sweep from
-// zero). Coarse node (I, J, K) (padded) sits on fine node (2I-1, 2J-1, 2K-1);
-// the fine ghost layer is zero. Grid: x = coarse interior node, y = chunks of
-// 128 float4 realization groups; one thread per node and four realizations.
-// Offsets are 32-bit and relative to the centre node (the 27 loads of a
-// component share one base address).
-constexpr int kXferThreads = 128;
-constexpr int kProlongNodes = 2;  // fine nodes of one k_prolong_add CTA
-__global__ void __launch_bounds__(kXferThreads, 8) k_restrict(Lattice Lf, Lattice Lc, const int* __restrict__ interior_c,
-                                                              const uint8_t* __restrict__ mask_c,
-                                                              const float* __restrict__ tf,
-                                                              const float* __restrict__ dinv_c, float omega,
-                                                              float* __restrict__ bc, float* __restrict__ xc) {
+// zero). Coarse node (I, J, K) (padded) sits on fine node (2I-1, 2J-1, 2K-1),
+// on the ghost layer at the end of an axis with an odd number of elements; the
+// fine ghost layer is zero. Grid: x = coarse interior node, y = chunks of
+// 64 float4 realization groups; one thread per component and four realizations.
+// Offsets are 32-bit and relative to the centre node (the 27 loads share one
+// base address). Bound by the latency of the loads on small levels (components
+// one after another in a thread: 12 us at 5^3 nodes x 64), by HBM on the fine
+// one.
+constexpr int kXferThreads = 64;  // float4 realization groups of a CTA (x three components)
+__global__ void __launch_bounds__(3 * kXferThreads, 5) k_restrict(Lattice Lf, Lattice Lc, const int* __restrict__ interior_c,
+                                                                  const uint8_t* __restrict__ mask_c,
+                                                                  const float* __restrict__ tf,
+                                                                  const float* __restrict__ dinv_c, float omega,
+                                                                  float* __restrict__ bc, float* __restrict__ xc) {
   const int Q = Lf.Rp >> 2;
-  const int q = blockIdx.y * kXferThreads + threadIdx.x;
+  const int q = blockIdx.y * kXferThreads + threadIdx.x, c = threadIdx.y;
   if (q >= Q) return;
   const int nc = interior_c[blockIdx.x];
   const int I = nc % Lc.NXp, J = (nc / Lc.NXp) % Lc.NYp, K = nc / (Lc.NXp * Lc.NYp);
   const int fc = (2 * I - 1) + Lf.NXp * ((2 * J - 1) + Lf.NYp * (2 * K - 1));
   const int sx = 3 * Q, sy = Lf.NXp * sx, sz = Lf.NYp * sy;  // float4 strides between fine nodes
-  const float4* t4 = reinterpret_cast<const float4*>(tf) + (size_t)fc * sx + q;
-  const uint32_t mk = mask_c[nc];
-  const size_t oc = (size_t)nc * sx + q;
-  const float4* dv4 = reinterpret_cast<const float4*>(dinv_c) + (size_t)nc * Q + q;
-  float4* b4 = reinterpret_cast<float4*>(bc) + oc;
-  float4* x4 = reinterpret_cast<float4*>(xc) + oc;
-#pragma unroll 1
-  for (int c = 0; c < 3; ++c) {
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  // a last coarse node on the ghost layer has no fine node beyond: the layer's
+  // own zeros are read again there
+  const int px = 2 * I < Lf.NXp ? sx : 0, py = 2 * J < Lf.NYp ? sy : 0, pz = 2 * K < Lf.NZp ? sz : 0;
+  const float4* t4 = reinterpret_cast<const float4*>(tf) + (size_t)fc * sx + c * Q + q;
+  const size_t oc = (size_t)nc * sx + c * Q + q;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
+  for (int dz = -1; dz <= 1; ++dz)
 #pragma unroll
-      for (int dy = -1; dy <= 1; ++dy)
+    for (int dy = -1; dy <= 1; ++dy)
 #pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const float wgt = (dx ? 0.5f : 1.f) * (dy ? 0.5f : 1.f) * (dz ? 0.5f : 1.f);
-          const float4 v = t4[dx * sx + dy * sy + dz * sz + c * Q];
-          s.x = fmaf(wgt, v.x, s.x);
-          s.y = fmaf(wgt, v.y, s.y);
-          s.z = fmaf(wgt, v.z, s.z);
-          s.w = fmaf(wgt, v.w, s.w);
-        }
-    if ((mk >> c) & 1) s = make_float4(0.f, 0.f, 0.f, 0.f);
-    b4[c * Q] = s;
-    const float4 dv = *dv4;  // loaded after the sums: no register held across the 27 loads
-    x4[c * Q] = make_float4(omega * dv.x * s.x, omega * dv.y * s.y, omega * dv.z * s.z, omega * dv.w * s.w);
-  }
+      for (int dx = -1; dx <= 1; ++dx) {
+        const float wgt = (dx ? 0.5f : 1.f) * (dy ? 0.5f : 1.f) * (dz ? 0.5f : 1.f);
+        const float4 v = t4[(dx < 0 ? -sx : dx * px) + (dy < 0 ? -sy : dy * py) + (dz < 0 ? -sz : dz * pz)];
+        s.x = fmaf(wgt, v.x, s.x);
+        s.y = fmaf(wgt, v.y, s.y);
+        s.z = fmaf(wgt, v.z, s.z);
+        s.w = fmaf(wgt, v.w, s.w);
+      }
+  if ((mask_c[nc] >> c) & 1) s = make_float4(0.f, 0.f, 0.f, 0.f);
+  reinterpret_cast<float4*>(bc)[oc] = s;
+  const float4 dv = reinterpret_cast<const float4*>(dinv_c)[(size_t)nc * Q + q];
+  reinterpret_cast<float4*>(xc)[oc] = make_float4(omega * dv.x * s.x, omega * dv.y * s.y, omega * dv.z * s.z,
+                                                  omega * dv.w * s.w);
 }
 
 // x_f += P x_c: trilinear prolongation of the coarse correction (per axis, a
 // fine node with even coordinate takes the coincident coarse node, an odd one
-// the mean of its two neighbours), masked at the fine level. Grid as
-// k_restrict over the fine interior nodes; the 8 corner terms are summed in a
-// fixed order (the terms of an even axis's second neighbour, weight 0, are skipped).
-// With r0 given, the iterate before the correction is not read from x_f but
-// formed as the first Jacobi sweep from zero, x0 = (omega dinv0) r0, with the
-// arithmetic of the start pass (which then need not write it), and x_f is
-// written at every component (the constrained ones without the correction).
-__global__ void __launch_bounds__(kXferThreads, 8) k_prolong_add(Lattice Lf, Lattice Lc,
-                                                                 const int* __restrict__ interior_f, int n_int,
-                                                                 const uint8_t* __restrict__ mask_f,
-                                                                 const float* __restrict__ xc, float* __restrict__ xf,
-                                                                 const float* __restrict__ r0,
-                                                                 const float* __restrict__ dinv0, float omega) {
+// the mean of its two neighbours), masked at the fine level. The corner terms
+// are summed in a fixed order (z, y, x; the terms of an even axis's second
+// neighbour, weight 0, are skipped). With r0 given, the iterate before the
+// correction is not read from x_f but formed as the first Jacobi sweep from
+// zero, x0 = (omega dinv0) r0, with the arithmetic of the start pass (which
+// then need not write it), and x_f is written at every component (the
+// constrained ones without the correction). Grid: x = pairs of nodes along x
+// (2i, 2i + 1: they share the coarse nodes at i, and their loads are in flight
+// together), y = chunks of 64 float4 realization groups; a thread per component
+// and four realizations. Bound by HBM on the fine level (258 us at 32^3 x 1024
+// with three components and two nodes of any place a thread, 328 one node a CTA,
+// 223 now: 4.6 TB/s of its 1.03 GB), by load latency on the others (10 -> 5 us at
+// 8^3 x 64).
+__global__ void __launch_bounds__(3 * kXferThreads, 5)
+    k_prolong_add(Lattice Lf, Lattice Lc, const uint8_t* __restrict__ mask_f, const float* __restrict__ xc,
+                  float* __restrict__ xf, const float* __restrict__ r0, const float* __restrict__ dinv0, float omega) {
   const int Q = Lf.Rp >> 2;
-  const int q = blockIdx.y * kXferThreads + threadIdx.x;
+  const int q = blockIdx.y * kXferThreads + threadIdx.x, c = threadIdx.y;
   if (q >= Q) return;
   const int sx = 3 * Q, sy = Lc.NXp * sx, sz = Lc.NYp * sy;  // float4 strides between coarse nodes
-  // kProlongNodes fine nodes a CTA, their loads in flight together
-#pragma unroll
-  for (int u = 0; u < kProlongNodes; ++u) {
-    const int t = blockIdx.x * kProlongNodes + u;
-    if (t >= n_int) break;
-    const int nf = interior_f[t];
-    const uint32_t mk = mask_f[nf];
-    if (mk == 7u && r0 == nullptr) continue;
-    const int gi = nf % Lf.NXp - 1, gj = (nf / Lf.NXp) % Lf.NYp - 1, gk = nf / (Lf.NXp * Lf.NYp) - 1;
-    const int c0 = ((gi >> 1) + 1) + Lc.NXp * (((gj >> 1) + 1) + Lc.NYp * ((gk >> 1) + 1));
-    const int oi = (gi & 1) * sx, oj = (gj & 1) * sy, ok = (gk & 1) * sz;  // offset of the second neighbour (or 0)
-    const float wi[2] = {(gi & 1) ? 0.5f : 1.f, (gi & 1) ? 0.5f : 0.f};
-    const float wj[2] = {(gj & 1) ? 0.5f : 1.f, (gj & 1) ? 0.5f : 0.f};
-    const float wk[2] = {(gk & 1) ? 0.5f : 1.f, (gk & 1) ? 0.5f : 0.f};
-    const float4* c4 = reinterpret_cast<const float4*>(xc) + (size_t)c0 * sx + q;
-    float4* f4 = reinterpret_cast<float4*>(xf) + (size_t)nf * sx + q;
-    float4 wdv = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r0 != nullptr) {
-      const float4 dv = reinterpret_cast<const float4*>(dinv0)[(size_t)nf * Q + q];
-      wdv = make_float4(omega * dv.x, omega * dv.y, omega * dv.z, omega * dv.w);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      float4 s;
-      if (r0 != nullptr) {
-        const float4 rv = reinterpret_cast<const float4*>(r0)[((size_t)nf * 3 + c) * Q + q];
-        s = make_float4(wdv.x * rv.x, wdv.y * rv.y, wdv.z * rv.z, wdv.w * rv.w);
-        if ((mk >> c) & 1) {
-          f4[c * Q] = s;
-          continue;
-        }
-      } else {
-        if ((mk >> c) & 1) continue;
-        s = f4[c * Q];
-      }
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int bb = 0; bb < 2; ++bb)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            // an even coordinate has one coarse neighbour on that axis: skip the zero-weight loads
-            if ((e && !(gi & 1)) || (bb && !(gj & 1)) || (a && !(gk & 1))) continue;
-            const float wgt = wk[a] * wj[bb] * wi[e];
-            const float4 v = c4[(e ? oi : 0) + (bb ? oj : 0) + (a ? ok : 0) + c * Q];
-            s.x = fmaf(wgt, v.x, s.x);
-            s.y = fmaf(wgt, v.y, s.y);
-            s.z = fmaf(wgt, v.z, s.z);
-            s.w = fmaf(wgt, v.w, s.w);
-          }
-      f4[c * Q] = s;
-    }
+  const int npx = (Lf.NX + 1) >> 1;
+  const int ip = blockIdx.x % npx, gj = (blockIdx.x / npx) % Lf.NY, gk = blockIdx.x / (npx * Lf.NY);
+  const int nf = 2 * ip + 1 + Lf.NXp * (gj + 1 + Lf.NYp * (gk + 1));
+  const bool two = 2 * ip + 1 < Lf.NX;  // node 2i + 1 exists (and with it coarse node i + 1)
+  const int c0 = ip + 1 + Lc.NXp * ((gj >> 1) + 1 + Lc.NYp * ((gk >> 1) + 1));
+  const float4* c4 = reinterpret_cast<const float4*>(xc) + (size_t)c0 * sx + c * Q + q;
+  float4* f4 = reinterpret_cast<float4*>(xf) + (size_t)nf * sx + c * Q + q;
+  const bool oj = gj & 1, ok = gk & 1;
+  const bool fix0 = (mask_f[nf] >> c) & 1, fix1 = !two || ((mask_f[nf + 1] >> c) & 1);
+  float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+  if (r0 != nullptr) {
+    const float4* r4 = reinterpret_cast<const float4*>(r0) + (size_t)nf * sx + c * Q + q;
+    const float4* d4 = reinterpret_cast<const float4*>(dinv0) + (size_t)nf * Q + q;
+    auto first = [&](const float4& dv, const float4& rv) {
+      return make_float4(omega * dv.x * rv.x, omega * dv.y * rv.y, omega * dv.z * rv.z, omega * dv.w * rv.w);
+    };
+    s0 = first(d4[0], r4[0]);
+    if (two) s1 = first(d4[Q], r4[sx]);
+  } else {
+    if (fix0 && fix1) return;
+    s0 = f4[0];
+    if (two) s1 = f4[sx];
   }
+  const float wjk = (oj ? 0.5f : 1.f) * (ok ? 0.5f : 1.f);
+  auto add = [](float4& s, float w, const float4& v) {
+    s.x = fmaf(w, v.x, s.x);
+    s.y = fmaf(w, v.y, s.y);
+    s.z = fmaf(w, v.z, s.z);
+    s.w = fmaf(w, v.w, s.w);
+  };
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int bb = 0; bb < 2; ++bb) {
+      if ((bb && !oj) || (a && !ok)) continue;
+      const float4* p = c4 + (bb ? sy : 0) + (a ? sz : 0);
+      const float4 v0 = p[0];
+      if (!fix0) add(s0, wjk, v0);
+      if (!fix1) {
+        add(s1, 0.5f * wjk, v0);
+        add(s1, 0.5f * wjk, p[sx]);
+      }
+    }
+  f4[0] = s0;
+  if (two) f4[sx] = s1;
 }
 
-// grid of the transfer kernels: x = interior node, y = chunks of kXferThreads float4 groups
+// launch shape of the transfer kernels: x = interior node, y = chunks of kXferThreads
+// float4 groups; a thread per float4 group and component
 inline dim3 xfer_grid(int n_int, int Rp) {
   return dim3((unsigned)n_int, (unsigned)((Rp / 4 + kXferThreads - 1) / kXferThreads));
 }
-inline int xfer_block(int Rp) { return std::min(kXferThreads, (Rp / 4 + 31) / 32 * 32); }
-inline dim3 prolong_grid(int n_int, int Rp) {
-  return dim3((unsigned)((n_int + kProlongNodes - 1) / kProlongNodes),
-              (unsigned)((Rp / 4 + kXferThreads - 1) / kXferThreads));
-}
+inline int prolong_pairs(const Lattice& L) { return (L.NX + 1) / 2 * L.NY * L.NZ; }
+inline dim3 xfer_block(int Rp) { return dim3((unsigned)std::min(kXferThreads, Rp / 4), 3); }
 
 // Coarse element field: the mean of the 8 fine elements it covers (elements
-// are stored at their lower-corner padded node). One CTA per coarse element.
+// are stored at their lower-corner padded node; those beyond the end of an odd
+// axis are ghosts with E = 0). One CTA per coarse element.
 __global__ void __launch_bounds__(128) k_coarsen_E(Lattice Lf, Lattice Lc, int nxc, int nyc,
                                                    const float* __restrict__ Ef, float* __restrict__ Ec) {
   const int e = blockIdx.x;
@@ -2870,6 +2857,7 @@ struct GmgLevel {
   int nx = 0, ny = 0, nz = 0;  // elements per axis
   ModalC MC;
   double kdiag = 0.0, mdiag = 0.0;
+  float omega = 0.f;  // Jacobi damping of the level
   const int* interior = nullptr;
   const uint8_t* mask = nullptr;
   float *b = nullptr, *x = nullptr, *t = nullptr, *E32 = nullptr, *dinv = nullptr;
@@ -3011,13 +2999,13 @@ double element_jacobi_lambda(const double* K576) {
 
 // Coarse-level maps of a structured mesh for levels 1..n_lvl-1 (built once per
 // mesh, under its lock): a coarse node is constrained in component c when the
-// fine node it sits on is.
+// fine node it sits on (the last one of its axis, when it lies beyond) is.
 int gmg_maps(Context* ctx, Mesh* m, int n_lvl) {
   std::lock_guard<std::mutex> lock(m->gmg_mu);
   if (m->gmg_levels >= n_lvl) return MSG_OK;
   const int NXf = m->nx + 1, NYf = m->ny + 1;
   for (int l = m->gmg_levels; l < n_lvl; ++l) {
-    const int nx = m->nx >> l, ny = m->ny >> l, nz = m->nz >> l;
+    const int nx = gmg_side(m->nx, l), ny = gmg_side(m->ny, l), nz = gmg_side(m->nz, l);
     const int NX = nx + 1, NY = ny + 1, NZ = nz + 1, NXp = NX + 2, NYp = NY + 2, NZp = NZ + 2;
     std::vector<uint8_t> mask((size_t)NXp * NYp * NZp, 7);
     std::vector<int> interior((size_t)NX * NY * NZ);
@@ -3026,7 +3014,8 @@ int gmg_maps(Context* ctx, Mesh* m, int n_lvl) {
       for (int j = 0; j < NY; ++j)
         for (int i = 0; i < NX; ++i, ++t) {
           const int p = (i + 1) + NXp * ((j + 1) + NYp * (k + 1));
-          const size_t f = ((size_t)i << l) + (size_t)NXf * (((size_t)j << l) + (size_t)NYf * ((size_t)k << l));
+          const size_t fi = std::min(i << l, m->nx), fj = std::min(j << l, m->ny), fk = std::min(k << l, m->nz);
+          const size_t f = fi + (size_t)NXf * (fj + (size_t)NYf * fk);
           uint8_t mk = 0;
           for (int c = 0; c < 3; ++c)
             if (m->dof[3 * f + c] < 0) mk |= (uint8_t)(1 << c);
@@ -3266,26 +3255,30 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
   }
   if (e != CUDA_SUCCESS) return set_error(ctx, MSG_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)e);
 
-  // multigrid levels: halve the lattice while every axis is even and keeps at
-  // least 2 elements
   B->gmg = false;
   B->n_lvl = 1;
   // (by default only without a mass term: a mass-dominated system, as in implicit
   // dynamics, is close to diagonal and the Jacobi loop needs few cheaper iterations)
   if (B->modal && (ctx->multigrid == 2 || (ctx->multigrid == 1 && !B->mass))) {
-    int n_lvl = 1;
-    while (n_lvl < ctx->mg_levels) {
-      const int nx = m->nx >> (n_lvl - 1), ny = m->ny >> (n_lvl - 1), nz = m->nz >> (n_lvl - 1);
-      if ((nx & 1) || (ny & 1) || (nz & 1) || nx < 4 || ny < 4 || nz < 4) break;
-      ++n_lvl;
-    }
+    const int n_lvl = gmg_level_count(m->nx, m->ny, m->nz, ctx->mg_levels);
     if (n_lvl >= 2) {
       MSG_TRY(gmg_maps(ctx, m, n_lvl));
       B->gmg = true;
       B->n_lvl = n_lvl;
       B->sweeps = ctx->mg_sweeps;
       const double lam = element_jacobi_lambda(K576);
-      B->omega = (float)(ctx->mg_omega > 0.0 ? ctx->mg_omega : std::min(0.6, 3.19 / lam));
+      // Damping. An axis that halves evenly keeps the Jacobi-scaled spectrum of the
+      // fine lattice (below 3.2 of the element bound lam = 5.3 at nu = 0.3), and 0.6
+      // holds there. A level with a half-empty last element does not (3.5 for 2 x 2 x
+      // n elements; the V-cycle lost definiteness at 0.6 on 5 x 5 x 20), and neither
+      // need any level of a lattice that starts with an odd axis be trusted further
+      // than the Jacobi loop it would otherwise take: there 1.99 / lam, positive
+      // definite for every positive element field.
+      const double om_even = std::min(0.6, 3.19 / lam), om_odd = std::min(0.6, 1.99 / lam);
+      const bool odd0 = (m->nx | m->ny | m->nz) & 1;
+      auto level_omega = [&](bool odd) { return (float)(ctx->mg_omega > 0.0 ? ctx->mg_omega : odd ? om_odd : om_even); };
+      B->omega = level_omega(odd0);
+      bool odd = odd0;
       MSG_TRY(B->slot_alloc(ctx, 30, sizeof(float) * nvec, &B->xs.ptr));
       MSG_CUDA(ctx, cudaMemsetAsync(B->xs.ptr, 0, sizeof(float) * nvec, st));
       const cuuint32_t pbm[5] = {32, 3, 1, kMPJ, kMPK};
@@ -3300,9 +3293,11 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
       size_t off[kGmgMaxLevels][5];
       for (int l = 1; l < n_lvl; ++l) {
         GmgLevel& g = B->lv[l];
-        g.nx = m->nx >> l;
-        g.ny = m->ny >> l;
-        g.nz = m->nz >> l;
+        g.nx = gmg_side(m->nx, l);
+        g.ny = gmg_side(m->ny, l);
+        g.nz = gmg_side(m->nz, l);
+        odd = odd || ((gmg_side(m->nx, l - 1) | gmg_side(m->ny, l - 1) | gmg_side(m->nz, l - 1)) & 1);
+        g.omega = level_omega(odd);
         Lattice& Lc = g.L;
         Lc.NX = g.nx + 1; Lc.NY = g.ny + 1; Lc.NZ = g.nz + 1;
         Lc.NXp = Lc.NX + 2; Lc.NYp = Lc.NY + 2; Lc.NZp = Lc.NZ + 2;
@@ -3358,7 +3353,7 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
       {  // coarsest level: one launch for all its sweeps when it fits a CTA
         GmgLevel& g = B->lv[n_lvl - 1];
         const size_t sm = coarse_sweep_smem(g.L);
-        g.sweep_smem = (ctx->mg_fused_coarse && g.L.NY <= kMJ && g.L.NZ <= kMK && sm <= 200 * 1024) ? sm : 0;
+        g.sweep_smem = (ctx->mg_fused_coarse && sm <= 200 * 1024) ? sm : 0;
         if (g.sweep_smem) {
           static std::once_flag cs_once;
           static cudaError_t cs_err = cudaSuccess;
@@ -3561,12 +3556,12 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
   const bool mass = B->mass;
   auto lvl = [&](auto mode, const Lattice& L, const ModalC& C, const CUtensorMap& ta, const CUtensorMap& tb,
                  const CUtensorMap& tn, const CUtensorMap& te, const CUtensorMap& td, int tiles_j, int n_tiles,
-                 int n_items, int grid, const uint8_t* mask, const float* b, const float* dinv, float* out,
+                 int n_items, int grid, const uint8_t* mask, const float* b, const float* dinv, float omega, float* out,
                  float* out2, float* out3, float* d, double* partial, int pstride) {
     constexpr int kMode = decltype(mode)::value;
     auto k = mass ? k_lvl_op<kMode, true> : k_lvl_op<kMode, false>;
     k<<<grid, kMThreads, LvlStage<kMode>::kSmem, st>>>(L, C, ta, tb, tn, te, td, tiles_j, n_tiles, n_items, mask, b,
-                                                       dinv, om, s.alpha, s.beta, out, out2, out3, d, partial,
+                                                       dinv, omega, s.alpha, s.beta, out, out2, out3, d, partial,
                                                        pstride, s.err);
   };
   // level 0 with two realizations per lane (k_lvl_op2) where the batch allows it
@@ -3584,7 +3579,7 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
           om, s.alpha, s.beta, out, out2, out3, d, partial, pstride, s.err);
     } else {
       lvl(mode, B->L, B->MC, ta, tb, B->tm_dinvm, B->tm_em, B->tm_dm, B->tiles_jm, B->n_tiles_m, B->n_items_m,
-          B->grid_m, B->mask, b, dinv, out, out2, out3, d, partial, pstride);
+          B->grid_m, B->mask, b, dinv, om, out, out2, out3, d, partial, pstride);
     }
   };
   // coarse level l: residual (out = b - A x) or post-sweep (out = x + omega dinv (b - A x)) of x into t
@@ -3594,10 +3589,10 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
       auto k = mass ? k_lvl_op2<kMode, true> : k_lvl_op2<kMode, false>;
       k<<<g.grid2, kQThreads, LvlStage2<kMode>::kSmem, st>>>(
           g.L, g.MC2, g.tm2_x, g.tm2_bo, g.tm2_dinvo, g.tm2_e, g.tm2_x, g.tiles_j2, g.n_tiles2, g.n_items2, g.mask, g.b,
-          g.dinv, om, s.alpha, s.beta, g.t, nullptr, nullptr, nullptr, nullptr, 1, s.err);
+          g.dinv, g.omega, s.alpha, s.beta, g.t, nullptr, nullptr, nullptr, nullptr, 1, s.err);
     } else {
       lvl(mode, g.L, g.MC, g.tm_x, g.tm_x, g.tm_x, g.tm_e, g.tm_x, g.tiles_j, g.n_tiles, g.n_items, g.grid, g.mask,
-          g.b, kMode == kLvlSmooth ? g.dinv : nullptr, g.t, nullptr, nullptr, nullptr, nullptr, 1);
+          g.b, kMode == kLvlSmooth ? g.dinv : nullptr, g.omega, g.t, nullptr, nullptr, nullptr, nullptr, 1);
     }
   };
   using Start = std::integral_constant<int, kLvlStart>;
@@ -3612,8 +3607,8 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
     GmgLevel& g = B->lv[l];
     const Lattice& Lf = l == 1 ? B->L : B->lv[l - 1].L;
     const float* tf = l == 1 ? qB : B->lv[l - 1].t;
-    k_restrict<<<xfer_grid(g.L.n_int, Rp), xfer_block(Rp), 0, st>>>(Lf, g.L, g.interior, g.mask, tf, g.dinv, om, g.b,
-                                                                     g.x);
+    k_restrict<<<xfer_grid(g.L.n_int, Rp), xfer_block(Rp), 0, st>>>(Lf, g.L, g.interior, g.mask, tf, g.dinv, g.omega,
+                                                                     g.b, g.x);
     if (l < nl - 1) lvlc(Resid{}, g);
   }
   // coarsest level: the restriction made the first sweep; sweeps - 1 more, x and t alternating
@@ -3623,7 +3618,7 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
     res_c = g.x;
     if (B->sweeps > 1) {
       auto k = mass ? k_coarse_sweeps<true> : k_coarse_sweeps<false>;
-      k<<<Rp / 32, kMWarps * 32, g.sweep_smem, st>>>(g.L, g.MC, g.mask, g.b, g.dinv, g.E32, om, B->sweeps - 1, g.x,
+      k<<<Rp / 32, kMWarps * 32, g.sweep_smem, st>>>(g.L, g.MC, g.mask, g.b, g.dinv, g.E32, g.omega, B->sweeps - 1, g.x,
                                                       g.t);
       res_c = g.t;
     }
@@ -3632,7 +3627,7 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
     bool in_x = true;
     for (int k = 1; k < B->sweeps; ++k) {
       lvl(Smooth{}, g.L, g.MC, in_x ? g.tm_x : g.tm_t, g.tm_x, g.tm_x, g.tm_e, g.tm_x, g.tiles_j, g.n_tiles,
-          g.n_items, g.grid, g.mask, g.b, g.dinv, in_x ? g.t : g.x, nullptr, nullptr, nullptr, nullptr, 1);
+          g.n_items, g.grid, g.mask, g.b, g.dinv, g.omega, in_x ? g.t : g.x, nullptr, nullptr, nullptr, nullptr, 1);
       in_x = !in_x;
     }
     res_c = in_x ? g.x : g.t;
@@ -3640,17 +3635,14 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
   // up: prolongate into the level's iterate, one sweep (result in t)
   for (int l = nl - 2; l >= 1; --l) {
     GmgLevel& g = B->lv[l];
-    k_prolong_add<<<prolong_grid(g.L.n_int, Rp), xfer_block(Rp), 0, st>>>(g.L, B->lv[l + 1].L, g.interior,
-                                                                          g.L.n_int, g.mask, res_c, g.x, nullptr,
-                                                                          nullptr, 0.f);
+    k_prolong_add<<<xfer_grid(prolong_pairs(g.L), Rp), xfer_block(Rp), 0, st>>>(g.L, B->lv[l + 1].L, g.mask, res_c,
+                                                                                g.x, nullptr, nullptr, 0.f);
     lvlc(Smooth{}, g);
     res_c = g.t;
   }
   // level 0: x0 = omega dinv r' formed here (the start pass does not write it)
-  k_prolong_add<<<prolong_grid(B->L.n_int, Rp), xfer_block(Rp), 0, st>>>(B->L, B->lv[1].L, B->interior,
-                                                                          B->L.n_int, B->mask, res_c,
-                                                                          B->xs.as<float>(), r_out,
-                                                                          B->dinv.as<float>(), om);
+  k_prolong_add<<<xfer_grid(prolong_pairs(B->L), Rp), xfer_block(Rp), 0, st>>>(
+      B->L, B->lv[1].L, B->mask, res_c, B->xs.as<float>(), r_out, B->dinv.as<float>(), om);
   // level 0 post-sweep: z (into qB) and the partial z.r'
   lvl0(Smooth{}, B->tm_xs, B->tm_xs, B->tm2_xs, B->tm2_xs, r_out, B->dinv.as<float>(), qB, nullptr, nullptr, nullptr,
        part2 + 1, 2);

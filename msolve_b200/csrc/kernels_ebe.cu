@@ -1426,7 +1426,7 @@ int ebe_solve(Context* ctx, const std::vector<RgInput>& in, int max_it, double t
     const int nx = m->structured ? m->nx : m->tnx, ny = m->structured ? m->ny : m->tny,
               nz = m->structured ? m->nz : m->tnz;
     const bool lattice = m->structured || m->topo_lattice;
-    vc[i] = lattice && nx % 2 == 0 && ny % 2 == 0 && nz % 2 == 0 && nx >= 4 && ny >= 4 && nz >= 4;
+    vc[i] = lattice && gmg_level_count(nx, ny, nz, ctx->mg_levels) >= 2;
     any = any || vc[i];
   }
   // the loop publishes one request word a system into the mapped flag page

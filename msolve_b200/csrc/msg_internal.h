@@ -33,6 +33,26 @@ __host__ __device__ constexpr int corner_id(int ax, int ay, int az) {
 constexpr int kGmgMaxLevels = 6;  // multigrid lattice levels at most (fine level included)
 constexpr int kWorkSlots = 40;    // context workspace slots (see workspace())
 
+// Elements of an axis of n on multigrid level l: halved, rounded up, per level (on
+// an odd axis the last coarse element reaches one fine element beyond the lattice).
+inline int gmg_side(int n, int l) {
+  for (; l > 0; --l) n = (n + 1) / 2;
+  return n;
+}
+// Lattice levels of an nx x ny x nz lattice, the fine one included (1: it does not
+// coarsen), at most max_levels: every axis halves while the shortest has more than
+// two elements. Below that the 20 coarsest-level sweeps (one launch) are cheaper
+// than a level: 2 x 2 x 2 elements from a cube of any side. Lattices with an odd
+// axis (and more of the Jacobi loop's cheaper iterations than V-cycles: 140 to 600
+// against 25 to 30) coarsen from 216 elements on: 5^3 x 64 took 3.3 ms by Jacobi and
+// 3.7 by V-cycles, 7^3 4.6 and 3.8, 15^3 13.6 and 5.6, 33^3 72 and 13.3.
+inline int gmg_level_count(int nx, int ny, int nz, int max_levels) {
+  if (((nx | ny | nz) & 1) && (int64_t)nx * ny * nz < 216) return 1;
+  int n = 1;
+  for (int m = nx < ny ? (nx < nz ? nx : nz) : (ny < nz ? ny : nz); n < max_levels && m > 2; m = (m + 1) / 2) ++n;
+  return n;
+}
+
 struct Context;
 
 // Device allocation charged against the context's memory budget.
@@ -243,7 +263,8 @@ struct Mesh {
   DevMem d_pad_mask;       // [padded nodes] constrained bits, ghosts = 7
   DevMem d_pad_interior;   // [interior nodes] padded index of interior node t (generator order)
   // coarse lattices of the multigrid preconditioner, level l = 1..gmg_levels-1
-  // (node (i, j, k) of level l sits on fine node 2^l (i, j, k)): constrained
+  // (node (i, j, k) of level l sits on fine node 2^l (i, j, k), at the end of an
+  // odd axis beyond the last one): constrained
   // bits of the padded nodes (ghosts 7) and the interior list; built on first use
   std::mutex gmg_mu;
   int gmg_levels = 1;
