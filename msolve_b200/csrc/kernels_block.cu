@@ -221,76 +221,6 @@ __device__ __forceinline__ void pencil_of(const Lattice& L, int& J, int& Kz, boo
   Kz = k + 1;
 }
 
-// ---------------------------------------------------------------- polynomial-chaos Galerkin product
-// y_j = sum over the terms t of block j of c_t K(E_pos_t) u_k_t, FP64: the
-// stochastic Galerkin matrix-vector product of PolynomialChaosSolverPCGMatrixCalculator.
-// MultiplyWithMatrix (ISAAR.MSolve.Analyzers/PolynomialChaosSolverPCGMatrixCalculator.cs:1062-1089)
-// on a structured lattice, each K_pos applied element by element from its
-// field E_pos (value-class stencil, the pencil sweep of the FP64 residual).
-// One thread per node pencil and output block (lane = block j); terms are
-// accumulated in the reference's order (matrix, then input block) into the
-// thread's own outputs.
-__global__ void __launch_bounds__(128)
-    k_pc_matvec(Lattice L, const __grid_constant__ KhatD K, const double* __restrict__ u,
-                const double* __restrict__ Epc, int Mp, const uint8_t* __restrict__ mask,
-                const int* __restrict__ term_ptr, const int* __restrict__ term_pos, const int* __restrict__ term_k,
-                const double* __restrict__ term_c, int P, double* __restrict__ y) {
-  int J, Kz;
-  bool valid;
-  pencil_of(L, J, Kz, valid);
-  const int Pp = L.Rp;
-  const int j = blockIdx.y * 32 + threadIdx.x;
-  if (!valid || j >= P) return;
-  Lattice LE = L;
-  LE.Rp = Mp;  // the pencil sweep strides the element field by Rp
-  for (int t = term_ptr[j]; t < term_ptr[j + 1]; ++t) {
-    const int pos = term_pos[t], k = term_k[t];
-    const double c = term_c[t];
-    const bool first = t == term_ptr[j];
-    auto load = [&](size_t node, double* o) {
-#pragma unroll
-      for (int cc = 0; cc < 3; ++cc) o[cc] = u[(node * 3 + cc) * Pp + k];
-    };
-    auto own = [](size_t, const double*) {};
-    auto emit = [&](size_t node, const double*, const double* yy) {
-      const uint32_t mk = mask[node];
-#pragma unroll
-      for (int cc = 0; cc < 3; ++cc) {
-        const size_t o = (node * 3 + cc) * Pp + j;
-        const double v = ((mk >> cc) & 1) ? 0.0 : c * yy[cc];
-        y[o] = first ? v : y[o] + v;
-      }
-    };
-    pencil_sweep<double>(LE, K, J, Kz, Epc + pos, load, own, emit);
-  }
-}
-
-// E_pc[row(e)][0] = mean, E_pc[row(e)][1 + i] = mean * psi[i][e] (the field of
-// the i-th expansion term, GaussianFileStochasticCoefficientsProvider
-// GetCoefficientInternal scaled by the mean modulus)
-__global__ void k_pc_fields(int ne, int m, int Mp, double mean, const double* __restrict__ psi,
-                            const int* __restrict__ elem_row, double* __restrict__ Epc) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  const size_t row = (size_t)elem_row[e];
-  Epc[row * Mp] = mean;
-  for (int i = 0; i < m; ++i) Epc[row * Mp + 1 + i] = mean * psi[(size_t)i * ne + e];
-}
-
-// block-major DOF vectors [P][n_dofs] <-> lattice layout [padded node][3][Pp]
-__global__ void k_pc_scatter(int n_dofs, int P, int Pp, const int* __restrict__ rows, const double* __restrict__ in,
-                             double* __restrict__ out) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y;
-  if (d < n_dofs && j < P) out[(size_t)rows[d] * Pp + j] = in[(size_t)j * n_dofs + d];
-}
-__global__ void k_pc_gather(int n_dofs, int P, int Pp, const int* __restrict__ rows, const double* __restrict__ in,
-                            double* __restrict__ out) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y;
-  if (d < n_dofs && j < P) out[(size_t)j * n_dofs + d] = in[(size_t)rows[d] * Pp + j];
-}
-
 // ---------------------------------------------------------------- mbarrier and TMA helpers
 // Every wait on an mbarrier is bounded: on expiry the kernel raises *err and
 // stops streaming (the host reads the flag and returns MSG_ERR_TIMEOUT).
@@ -528,6 +458,129 @@ __device__ __forceinline__ void modal_apply(const ModalCT<T>& C, T E, const T (&
       T0[c][q] = (T0[c][q] + y0[c][q]) - y1[c][q];
       C1[c][q] = y0[c][q] + y1[c][q];
     }
+}
+
+// ---------------------------------------------------------------- polynomial-chaos Galerkin product
+// y_j = sum over the terms t of block j of c_t K(E_pos_t) u_k_t, FP64: the
+// stochastic Galerkin matrix-vector product of PolynomialChaosSolverPCGMatrixCalculator.
+// MultiplyWithMatrix (ISAAR.MSolve.Analyzers/PolynomialChaosSolverPCGMatrixCalculator.cs:1062-1089)
+// on a structured lattice. K(E) is linear in E and in u, so an element's terms
+// are summed before its stiffness is applied once, in the Walsh modes:
+//   y_e = Khat sum_pos E_pos(e) (sum over the terms of pos of c_t u_k_t).
+// A CTA takes one output block and a tile of 8 x 4 x 4 nodes with the 9 x 5 x 5
+// elements around them, one a thread. Per matrix it stages the term sum at the
+// tile's nodes (read and written in the caller's DOF numbering, no lattice copy)
+// and adds it, times the element's modulus, to the thread's 24 values; the
+// elements' corner forces meet in the same shared memory and every node sums
+// its eight in fixed order. Bound by latency (a few staged rounds a CTA):
+// 12^3 elements, 35 blocks: 143 us with a dense stencil per term and a thread a
+// block, 32 us now (the call 3.1 -> 0.66 ms: nine allocations went too).
+constexpr int kPcX = 8, kPcY = 4, kPcZ = 4;
+constexpr int kPcEX = kPcX + 1, kPcEY = kPcY + 1, kPcEZ = kPcZ + 1, kPcE = kPcEX * kPcEY * kPcEZ;  // 225 elements
+constexpr int kPcNX = kPcX + 2, kPcNY = kPcY + 2, kPcNZ = kPcZ + 2, kPcN = kPcNX * kPcNY * kPcNZ;  // 360 nodes
+constexpr int kPcThreads = 256;
+constexpr int kPcPer = (3 * kPcN + kPcThreads - 1) / kPcThreads;  // staged values a thread
+static_assert(kPcE <= kPcThreads, "one element a thread");
+struct PcArgs {
+  int nx, ny, nz, n_dofs, P, tiles_x, tiles_y;
+  double mean;
+  const double* psi;    // [m][n_elems]
+  const int* dof;       // [n_nodes][3], -1 constrained
+  const int* term_ptr;  // [P + 1]
+  const int* term_pos;  // matrix of a term, ascending within a block: 0 the mean, i + 1 the i-th expansion term
+  const int* term_k;
+  const double* term_c;
+  const double* u;      // [P][n_dofs]
+  double* y;            // [P][n_dofs]
+};
+__global__ void __launch_bounds__(kPcThreads, 2) k_pc_matvec(PcArgs A, const __grid_constant__ ModalCD C) {
+  __shared__ double sh[24 * kPcE];  // 3 x 360 staged values, then the corner forces [corner][c][element]
+  const int tid = threadIdx.x;
+  const int j = blockIdx.x % A.P, tile = blockIdx.x / A.P;
+  const int x0 = tile % A.tiles_x * kPcX, y0 = tile / A.tiles_x % A.tiles_y * kPcY;
+  const int z0 = tile / (A.tiles_x * A.tiles_y) * kPcZ;
+  const int NX = A.nx + 1, NY = A.ny + 1, NZ = A.nz + 1;
+  // this thread's staged values: DOFs of the patch from node (x0 - 1, y0 - 1, z0 - 1)
+  int dof[kPcPer];
+#pragma unroll
+  for (int q = 0; q < kPcPer; ++q) {
+    const int i = tid + q * kPcThreads, n = i / 3;
+    const int X = x0 - 1 + n % kPcNX, Y = y0 - 1 + n / kPcNX % kPcNY, Z = z0 - 1 + n / (kPcNX * kPcNY);
+    const bool in = i < 3 * kPcN && X >= 0 && X < NX && Y >= 0 && Y < NY && Z >= 0 && Z < NZ;
+    dof[q] = in ? A.dof[3 * ((size_t)X + (size_t)NX * (Y + (size_t)NY * Z)) + i % 3] : -1;
+  }
+  // its element (lower corner at patch node (ex, ey, ez))
+  const int ex = tid % kPcEX, ey = tid / kPcEX % kPcEY, ez = tid / (kPcEX * kPcEY);
+  const int EX = x0 - 1 + ex, EY = y0 - 1 + ey, EZ = z0 - 1 + ez;
+  const bool real = tid < kPcE && EX >= 0 && EX < A.nx && EY >= 0 && EY < A.ny && EZ >= 0 && EZ < A.nz;
+  const size_t ne = (size_t)A.nx * A.ny * A.nz;
+  const size_t e = real ? (size_t)EX + (size_t)A.nx * (EY + (size_t)A.ny * EZ) : 0;
+  double v[2][2][2][3];  // [ax][ay][az][c]
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[a >> 2][a >> 1 & 1][a & 1][c] = 0.0;
+  const int t1 = A.term_ptr[j + 1];
+  for (int t = A.term_ptr[j]; t < t1;) {
+    const int pos = A.term_pos[t];
+    double w[kPcPer];
+#pragma unroll
+    for (int q = 0; q < kPcPer; ++q) w[q] = 0.0;
+    for (; t < t1 && A.term_pos[t] == pos; ++t) {  // the terms of one matrix
+      const double c = A.term_c[t];
+      const double* uk = A.u + (size_t)A.term_k[t] * A.n_dofs;
+#pragma unroll
+      for (int q = 0; q < kPcPer; ++q)
+        if (dof[q] >= 0) w[q] = fma(c, uk[dof[q]], w[q]);
+    }
+    __syncthreads();  // the last matrix's values have been read
+#pragma unroll
+    for (int q = 0; q < kPcPer; ++q)
+      if (tid + q * kPcThreads < 3 * kPcN) sh[tid + q * kPcThreads] = w[q];
+    const double E = !real ? 0.0 : pos == 0 ? A.mean : A.mean * A.psi[(size_t)(pos - 1) * ne + e];
+    __syncthreads();
+    if (real) {
+      const double* p = sh + 3 * (ex + kPcNX * (ey + kPcNY * ez));
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int ax = a >> 2, ay = a >> 1 & 1, az = a & 1;
+          v[ax][ay][az][c] = fma(E, p[3 * (ax + kPcNX * (ay + kPcNY * az)) + c], v[ax][ay][az][c]);
+        }
+    }
+  }
+  double B0[3][4], B1[3][4], T0[3][4], C1[3][4];
+  yz_forward(v[0], B0);
+  yz_forward(v[1], B1);
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) T0[c][q] = 0.0;
+  modal_apply<false>(C, 1.0, B0, B1, T0, C1);
+  yz_inverse(T0, v[0]);
+  yz_inverse(C1, v[1]);
+  __syncthreads();
+  if (tid < kPcE) {
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) sh[(a * 3 + c) * kPcE + tid] = v[a >> 2][a >> 1 & 1][a & 1][c];
+  }
+  __syncthreads();
+  for (int i = tid; i < 3 * kPcX * kPcY * kPcZ; i += kPcThreads) {
+    const int c = i % 3, n = i / 3, nx = n % kPcX, ny = n / kPcX % kPcY, nz = n / (kPcX * kPcY);
+    if (x0 + nx >= NX || y0 + ny >= NY || z0 + nz >= NZ) continue;
+    const int d = A.dof[3 * ((size_t)(x0 + nx) + (size_t)NX * (y0 + ny + (size_t)NY * (z0 + nz))) + c];
+    if (d < 0) continue;
+    double s = 0.0;  // the node is corner (ax, ay, az) of element (nx + 1 - ax, ...) of the tile; ghosts hold zeros
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const int ax = a >> 2, ay = a >> 1 & 1, az = a & 1;
+      s += sh[(a * 3 + c) * kPcE + (nx + 1 - ax) + kPcEX * ((ny + 1 - ay) + kPcEY * (nz + 1 - az))];
+    }
+    A.y[(size_t)j * A.n_dofs + d] = s;
+  }
 }
 
 // One whole inner PCG iteration per launch (single-reduction form). Launch k+1
@@ -3988,56 +4041,49 @@ int pc_matvec(Context* ctx, Mesh* m, double nu, const MSG_KL* kl, int mo, int po
   std::vector<double> tc;
   MSG_TRY(pc_gaussian_terms(mo, po, tptr, tpos, tk, tc));
   const int P = (int)tptr.size() - 1;
-  const int Pp = (P + 31) / 32 * 32, Mp = mo + 1;
   cudaStream_t st = ctx->stream;
   double K576[576];
   MSG_TRY(unit_cube_khat(ctx, m->h, nu, K576));
-  KhatD KD;
-  for (int c = 0; c < kKhatClasses; ++c) KD.v[c] = K576[kKhatRep[c]];
+  ModalC MC;
+  ModalCD MCD;
+  MSG_TRY(modal_coefficients(ctx, K576, nullptr, 1.0, 0.0, &MC, &MCD));
   KLDevice kd;
   MSG_TRY(kl_prepare(ctx, m, kl, &kd));
-  const size_t npad = (size_t)m->NXp * m->NYp * m->NZp;
-  DevMem dE, du, dy, dlat_u, dlat_y, dptr, dpos, dk, dc;
-  MSG_TRY(dE.alloc(ctx, sizeof(double) * npad * Mp));
-  MSG_TRY(du.alloc(ctx, sizeof(double) * (size_t)P * std::max(1, m->n_dofs)));
-  MSG_TRY(dy.alloc(ctx, sizeof(double) * (size_t)P * std::max(1, m->n_dofs)));
-  MSG_TRY(dlat_u.alloc(ctx, sizeof(double) * npad * 3 * Pp));
-  MSG_TRY(dlat_y.alloc(ctx, sizeof(double) * npad * 3 * Pp));
-  MSG_TRY(dptr.alloc(ctx, sizeof(int) * tptr.size()));
-  MSG_TRY(dpos.alloc(ctx, sizeof(int) * std::max<size_t>(1, tpos.size())));
-  MSG_TRY(dk.alloc(ctx, sizeof(int) * std::max<size_t>(1, tk.size())));
-  MSG_TRY(dc.alloc(ctx, sizeof(double) * std::max<size_t>(1, tc.size())));
-  MSG_CUDA(ctx, cudaMemcpyAsync(dptr.ptr, tptr.data(), sizeof(int) * tptr.size(), cudaMemcpyHostToDevice, st));
-  MSG_CUDA(ctx, cudaMemcpyAsync(dpos.ptr, tpos.data(), sizeof(int) * tpos.size(), cudaMemcpyHostToDevice, st));
-  MSG_CUDA(ctx, cudaMemcpyAsync(dk.ptr, tk.data(), sizeof(int) * tk.size(), cudaMemcpyHostToDevice, st));
-  MSG_CUDA(ctx, cudaMemcpyAsync(dc.ptr, tc.data(), sizeof(double) * tc.size(), cudaMemcpyHostToDevice, st));
-  MSG_CUDA(ctx, cudaMemcpyAsync(du.ptr, u_host, sizeof(double) * (size_t)P * m->n_dofs, cudaMemcpyHostToDevice, st));
-  MSG_CUDA(ctx, cudaMemsetAsync(dE.ptr, 0, sizeof(double) * npad * Mp, st));
-  MSG_CUDA(ctx, cudaMemsetAsync(dlat_u.ptr, 0, sizeof(double) * npad * 3 * Pp, st));
-  MSG_CUDA(ctx, cudaMemsetAsync(dlat_y.ptr, 0, sizeof(double) * npad * 3 * Pp, st));
-  k_pc_fields<<<(m->n_elems + 127) / 128, 128, 0, st>>>(m->n_elems, mo, Mp, kl->mean, kd.psi,
-                                                        m->d_pad_elem_row.as<int>(), dE.as<double>());
-  const dim3 gd((m->n_dofs + 255) / 256, P);
-  if (m->n_dofs > 0)
-    k_pc_scatter<<<gd, 256, 0, st>>>(m->n_dofs, P, Pp, m->d_pad_free_rows.as<int>(), du.as<double>(),
-                                     dlat_u.as<double>());
-  Lattice L;
-  L.NX = m->nx + 1; L.NY = m->ny + 1; L.NZ = m->nz + 1;
-  L.NXp = m->NXp; L.NYp = m->NYp; L.NZp = m->NZp;
-  L.Rp = Pp;
-  L.tiles_j = (L.NY + kTJ - 1) / kTJ;
-  L.n_pad = (int)npad;
-  L.n_int = L.NX * L.NY * L.NZ;
-  const int n_tiles = L.tiles_j * ((L.NZ + kTK - 1) / kTK);
-  k_pc_matvec<<<dim3(n_tiles, Pp / 32), dim3(32, kWarps), 0, st>>>(
-      L, KD, dlat_u.as<double>(), dE.as<double>(), Mp, m->d_pad_mask.as<uint8_t>(), dptr.as<int>(), dpos.as<int>(),
-      dk.as<int>(), dc.as<double>(), P, dlat_y.as<double>());
-  if (m->n_dofs > 0)
-    k_pc_gather<<<gd, 256, 0, st>>>(m->n_dofs, P, Pp, m->d_pad_free_rows.as<int>(), dlat_y.as<double>(),
-                                    dy.as<double>());
-  count_launch(ctx, 4);
+  const size_t nv = (size_t)P * m->n_dofs, nt = tpos.size();
+  const int tx = (m->nx + kPcX) / kPcX, ty = (m->ny + kPcY) / kPcY, tz = (m->nz + kPcZ) / kPcZ;
+  if ((int64_t)tx * ty * tz * P > INT32_MAX)
+    return set_error(ctx, MSG_ERR_INVALID_ARGUMENT, "polynomial chaos: lattice and basis too large");
+  // u, y, the terms' weights, then their index lists: one context buffer, kept between calls
+  const size_t bytes = sizeof(double) * (2 * nv + nt) + sizeof(int) * (2 * nt + P + 1);
+  void* buf = nullptr;
+  MSG_TRY(workspace(ctx, 38, bytes, &buf));
+  double* du = static_cast<double*>(buf);
+  double* dy = du + nv;
+  double* dc = dy + nv;
+  int* dpos = reinterpret_cast<int*>(dc + nt);
+  std::vector<int> lists(tpos);
+  lists.insert(lists.end(), tk.begin(), tk.end());
+  lists.insert(lists.end(), tptr.begin(), tptr.end());
+  MSG_CUDA(ctx, cudaMemcpyAsync(dc, tc.data(), sizeof(double) * nt, cudaMemcpyHostToDevice, st));
+  MSG_CUDA(ctx, cudaMemcpyAsync(dpos, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice, st));
+  MSG_CUDA(ctx, cudaMemcpyAsync(du, u_host, sizeof(double) * nv, cudaMemcpyHostToDevice, st));
+  PcArgs A;
+  A.nx = m->nx; A.ny = m->ny; A.nz = m->nz;
+  A.n_dofs = m->n_dofs; A.P = P;
+  A.tiles_x = tx; A.tiles_y = ty;
+  A.mean = kl->mean;
+  A.psi = kd.psi;
+  A.dof = m->d_dof.as<int>();
+  A.term_pos = dpos;
+  A.term_k = dpos + nt;
+  A.term_ptr = dpos + 2 * nt;
+  A.term_c = dc;
+  A.u = du;
+  A.y = dy;
+  k_pc_matvec<<<tx * ty * tz * P, kPcThreads, 0, st>>>(A, MCD);
+  count_launch(ctx, 1);
   MSG_CUDA(ctx, cudaGetLastError());
-  MSG_CUDA(ctx, cudaMemcpyAsync(y_host, dy.ptr, sizeof(double) * (size_t)P * m->n_dofs, cudaMemcpyDeviceToHost, st));
+  MSG_CUDA(ctx, cudaMemcpyAsync(y_host, dy, sizeof(double) * nv, cudaMemcpyDeviceToHost, st));
   MSG_CUDA(ctx, cudaStreamSynchronize(st));
   return MSG_OK;
 }
