@@ -143,9 +143,9 @@ int MSG_MAT_DESTROY(MSG_MAT mat);
  * (ISAAR.MSolve.Solvers/PCG/SolverPCG.cs:105-149, simple search vector
  * SolverPCGSimpleSearchVectorCalculator.cs:18-41): x0 = 0, r0 = b, stop when
  * ||r_k|| / ||b|| < tol on the recursively updated r, skip if ||b|| <= 1e-25.
- * The whole loop runs on the device: one CUDA graph launch a solve, whose
- * conditional WHILE node repeats 8-iteration rounds until the solve ends (no
- * host round trip between iterations or rounds).
+ * The whole loop runs on the device: one cooperative launch a solve (no host
+ * round trip between iterations); MSG_ERR_TIMEOUT if its CTAs' bounded waits for
+ * each other expire.
  * iterations = the reference's count (loop index at the break); rel_res = last
  * ||r||/||b||. Returns MSG_ERR_NOT_CONVERGED if max_it was reached. */
 int MSG_PCG_SOLVE(MSG_MAT mat, const double* b, double* x, int max_it, double tol, int* iterations,
@@ -161,8 +161,8 @@ int MSG_PCG_SOLVE(MSG_MAT mat, const double* b, double* x, int max_it, double to
  * the search direction is kept, and the solve stops only when
  * ||b - K x|| / ||b|| < tol in FP64 (rel_res). iterations counts as
  * MSG_PCG_SOLVE. The FP32 copy of the values is built on first use. Like
- * MSG_PCG_SOLVE, one CUDA graph launch a solve; the true-residual step is a
- * conditional node of that graph. No counterpart in the reference. */
+ * MSG_PCG_SOLVE, one cooperative launch a solve, true-residual steps included.
+ * No counterpart in the reference. */
 int MSG_PCG_SOLVE_MIXED(MSG_MAT mat, const double* b, double* x, int max_it, double tol, int* iterations,
                         double* rel_res);
 
@@ -197,7 +197,7 @@ int MSG_PCG_SOLVE_REORTH(MSG_MAT mat, MSG_SVS store, const double* b, double* x,
  * work would stall), and a host that hands the library a fixed share of device
  * memory may forbid allocations outside it. b_dev and x_dev are the caller's
  * device buffers (n_dofs doubles, DOF numbering); the solve's working vectors
- * live in one fixed device array of the library (about 9.5 MB, held on every
+ * live in one fixed device array of the library (about 11 MB, held on every
  * GPU that loads the library until the process exits), which limits the mesh
  * to 65536 nodes (larger meshes: MSG_ERR_INVALID_ARGUMENT). MSG_CREATE looks up
  * that array's device address, so the solve itself does no set-up. Stream
@@ -481,9 +481,8 @@ int MSG_SERVE_STOP(MSG_CTX ctx);
  * afterwards: 0, default, equal stream priorities; 1: priority grows as the
  * model shrinks, shortest solves first: with serve_persistent = 0 small
  * models' latency under load halves while the largest models wait longer),
- * "spmv32_shape" (launch shape of the FP32 SpMV of MSG_PCG_SOLVE_MIXED on
- * large matrices: 0, default, 4 slots per load group and 8 slices per CTA;
- * 1: 8 and 8; 2: 4 and 4; 3: 8 and 4; results are identical),
+ * "spmv32_shape" (0 to 3; accepted and read back, no longer of effect: the
+ * mixed solve's launch shape follows from the matrix),
  * "tensor_operator" (0, default: every element product in the element's Walsh
  * modes on the FP32 cores; 1: the multigrid loop's level-0 search-direction
  * launch forms E_e Khat u_e on the tensor cores, tcgen05.mma in TF32 with a

@@ -120,410 +120,466 @@ __global__ void k_node_to_dof(int n_dofs, const int* __restrict__ free_rows, con
 }
 
 // ------------------------------------------------------------------ PCG
-// Device-resident Jacobi-PCG. Two kernels per iteration, each ending with a
-// last-block-done reduction that updates the scalar state in fixed block order
-// (deterministic results):
-//   k_pcg_dir_spmv: p_new = dinv.r + beta p_old (recomputed for gathered
-//     columns, written for own rows), q = K p_new, partial p.q
-//     -> last block: alpha = z.r / p.q (breakdown check)
-//   k_pcg_update:   r -= alpha q, x += alpha p_new, partials r.r and (dinv r).r
-//     -> last block: err = ||r||/||b||, convergence / iteration bookkeeping, beta
+// Device-resident Jacobi-PCG: the whole solve is one cooperative launch. A CTA
+// owns a fixed set of 32-row slices; the phases of an iteration are separated by
+// grid-wide sums, in which every CTA adds all CTAs' partials itself in the same
+// fixed order, so that each holds the same scalars and takes the same branches
+// (deterministic results). FP64 loop, two sums an iteration:
+//   1: p_new = z + beta p_old (formed at the gathered columns, written for own
+//      rows), q = K p_new, sum p.q -> alpha = z.r / p.q (breakdown check)
+//   2: r -= alpha q, x += alpha p_new, z = D^-1 r, sums r.r and z.r -> err =
+//      ||r||/||b||, convergence, beta
 // p is double-buffered by iteration parity so gathered columns are never read
 // while being overwritten.
+//
+// k_pcg_resident: while a matrix' values fit the SMs' shared memory (3 slices an
+// SM in FP64, 6 in FP32: 14,000 and 28,000 lattice nodes) they are copied there
+// once and an iteration reads only vectors from L2; it is bound by the two sums
+// (2.5 us each). k_pcg streams them: bound by HBM, or by L2 for matrices that
+// stay there. Two kernels an iteration in a graph spent the launch latency of
+// each and the last block's serial sum. Per iteration, then -> now: 10 x 4 x 4
+// 14.7 -> 6.7 us, 20^3 17.2 -> 7.4, 37 x 22 x 29 19.6 -> 14.4 (mixed 22.4 ->
+// 11.0), 32^3 20.7 -> 18.2, 48^3 55.7 -> 47.6, 64^3 111.7 -> 102.8 (5.7 TB/s;
+// mixed 63.5 -> 60.4). Reading blocks below the diagonal from their mirror images
+// (half the HBM bytes) was slower at 48^3 (57-60 us): L2 delivers no faster here.
 
-constexpr int kPcgThreads = 256;
+constexpr int kPcgThreads = 256, kPcgWarps = kPcgThreads / 32;  // of the streaming kernels
+constexpr int kPcgMaxCtas = 4;     // CTAs an SM at most (sizes the partial sums)
+constexpr int kPcgSums = 3;        // values of a grid-wide sum at most
+constexpr int kPcgSpin = 1 << 22;  // polls of a grid-wide sum before it gives up
 
-__device__ __forceinline__ double block_sum(double v, double* sh) {
+// Grid-wide sums of one solve: the CTAs' partial sums (two buffers, used in turn: a
+// CTA can be at most one sum ahead of another) and the arrival counter, cleared
+// before the launch.
+struct PcgGrid {
+  double* part;       // [2][kPcgSums][grid]
+  unsigned* arrived;
+  unsigned target;    // arrivals that complete the next sum
+  int buf;
+};
+
+// out[k] = sum over the grid of v[k], every thread of every CTA; what the CTAs
+// wrote before is visible after. False when the bounded wait expired (the kernel
+// then returns). About 2.5 us over 26 to 592 CTAs; polling every CTA's partial sum
+// itself, without a counter, was faster below 30 CTAs only.
+template <int NW, int K>  // warps of the CTA, values
+__device__ __forceinline__ bool grid_sum(PcgGrid& g, const double (&v)[K], double (&out)[K]) {
+  __shared__ double sh[2][NW][K];
+  __shared__ int ok;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, G = gridDim.x;
+  double* part = g.part + (size_t)g.buf * kPcgSums * G;
+  g.buf ^= 1;
+  g.target += G;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  for (int k = 0; k < K; ++k) {
+    double t = v[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (l == 0) sh[0][w][k] = t;
+  }
+  __syncthreads();  // (and every thread's stores of this phase are ordered before the release)
+  if (w == 0) {
+    if (l < K) {
+      double t = 0;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) t += sh[0][i][l];
+      part[(size_t)l * G + blockIdx.x] = t;
+    }
+    __syncwarp();
+    if (l == 0) {
+      __threadfence();
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.arrived) : "memory");
+      int good = 0;
+      for (int i = 0; i < kPcgSpin && !good; ++i) {
+        unsigned n;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(g.arrived) : "memory");
+        good = (int)(n - g.target) >= 0;
+      }
+      __threadfence();
+      ok = good;
+    }
+  }
   __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double s = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += sh[i];
-  return s;  // valid in thread 0
-}
-
-// Whole-block sums of the K interleaved partials partial[i*K + k], i < n, in a
-// fixed order (thread t adds i = t, t + blockDim, ... in turn; then the block
-// tree): called by every thread of the last block, results valid in thread 0.
-// The loads of four rounds are issued before their adds (the order of the adds
-// is unchanged), so the last block waits for one L2 round trip, not n / blockDim.
-template <int K>
-__device__ __forceinline__ void sum_partials(const double* partial, int n, double (&out)[K], double* sh) {
-  double s[K];
+  if (!ok) return false;
+  // thread t adds the CTAs t, t + 32 NW, ... in order, then the block's fixed tree
+  double t[K];
 #pragma unroll
-  for (int k = 0; k < K; ++k) s[k] = 0;
-  const int B = blockDim.x;
-  int i = threadIdx.x;
-  for (; i + 3 * B < n; i += 4 * B) {
-    double v[4][K];
+  for (int k = 0; k < K; ++k) t[k] = threadIdx.x < G ? __ldcg(part + (size_t)k * G + threadIdx.x) : 0.0;
+  for (int i = threadIdx.x + (32 * NW); i < G; i += (32 * NW))
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int k = 0; k < K; ++k) t[k] += __ldcg(part + (size_t)k * G + i);
 #pragma unroll
-      for (int k = 0; k < K; ++k) v[u][k] = __ldcg(partial + (size_t)(i + u * B) * K + k);
+  for (int k = 0; k < K; ++k) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int k = 0; k < K; ++k) s[k] += v[u][k];
-  }
-  for (; i < n; i += B)
-#pragma unroll
-    for (int k = 0; k < K; ++k) s[k] += __ldcg(partial + (size_t)i * K + k);
-#pragma unroll
-  for (int k = 0; k < K; ++k) out[k] = block_sum(s[k], sh);
-}
-
-// Returns true in every thread of the last block to finish.
-__device__ __forceinline__ bool last_block(unsigned int* counter) {
-  __shared__ bool is_last;
-  __threadfence();
-  if (threadIdx.x == 0) {
-    const unsigned int ticket = atomicAdd(counter, 1u);
-    is_last = (ticket == gridDim.x - 1);
+    for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
+    if (l == 0) sh[1][w][k] = t[k];
   }
   __syncthreads();
-  return is_last;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double x = 0;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) x += sh[1][i][k];
+    out[k] = x;
+  }
+  return true;
 }
 
-__global__ void __launch_bounds__(kPcgThreads) k_pcg_init(int n_rows, const double* __restrict__ b,
-                                                          const double* __restrict__ dinv, double* __restrict__ r,
-                                                          double* __restrict__ x, double* __restrict__ p0,
-                                                          double* __restrict__ p1, double* __restrict__ partial,
-                                                          PcgState* st) {
-  __shared__ double sh[32];
-  double bb = 0, zr = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * n_rows; i += gridDim.x * blockDim.x) {
-    const double bi = b[i];
-    r[i] = bi; x[i] = 0; p0[i] = 0; p1[i] = 0;
-    bb += bi * bi;
-    zr += bi * dinv[i] * bi;
-  }
-  double s1 = block_sum(bb, sh);
-  double s2 = block_sum(zr, sh);
-  if (threadIdx.x == 0) { partial[2 * blockIdx.x] = s1; partial[2 * blockIdx.x + 1] = s2; }
-  if (!last_block(&st->counter)) return;
-  double tt[2];
-  sum_partials<2>(partial, gridDim.x, tt, sh);
-  const double tb = tt[0], tz = tt[1];
-  if (threadIdx.x == 0) {
-    st->bnorm = sqrt(tb);
-    st->zr = tz;
-    st->beta = 0; st->alpha = 0; st->err = 0;
-    st->it = 0; st->iterations = 0; st->matvecs = 0; st->status = 0;
-    st->done = (st->bnorm > 1e-25) ? 0 : 1;  // SolverPCG.cs:112
-    st->need = 0; st->err_ref = 1.0;
-    st->counter = 0;
+// y += the 3x3 block a times u. FP32 values multiply in FP32 and add in FP64.
+template <class V>
+__device__ __forceinline__ void block_row(const V (&a)[9], const V (&u)[3], double (&y)[3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    if constexpr (sizeof(V) == 8)
+      y[r] += a[3 * r] * u[0] + a[3 * r + 1] * u[1] + a[3 * r + 2] * u[2];
+    else
+      y[r] += (double)fmaf(a[3 * r + 2], u[2], fmaf(a[3 * r + 1], u[1], a[3 * r] * u[0]));
   }
 }
 
-// The loop's direction + SpMV kernel: p_new = dinv.r + beta p_old (formed for
-// gathered columns, written for own rows), q = K p_new, partial p.q -> last
-// block: alpha = z.r / p.q (breakdown check). A CTA is one 32-row slice, a
-// thread owns the 3 components of its row, so every slot streams 9 coalesced
-// 256-byte value lines per warp and the gathered p is formed once per column
-// (not once per output component). A CTA takes kS slices; a slice's slots are
-// dealt round-robin to kW warps (kW = 4 for small matrices, to keep enough
-// warps in flight; 1 for large ones) and the warp sums meet in shared memory
-// in fixed order. Slots are taken in groups
-// whose value loads are all issued before use (144 bytes in flight per
-// thread); values of matrices too large for L2 stream with evict-first loads
-// so the vectors stay in L2 (smaller ones stay in L2 across iterations);
-// padded positions (column -1) hold zero values and skip the gather.
-template <class V, int kS, int kSpmvWarps, bool kStream>
-__global__ void __launch_bounds__(32 * kS * kSpmvWarps) k_pcg_dir_spmv_rows(int n_rows, int n_slices,
-                                                                      const int64_t* __restrict__ slice_ptr,
-                                                                      const int* __restrict__ col,
-                                                                      const V* __restrict__ val,
-                                                                      const double* __restrict__ dinv,
-                                                                      const double* __restrict__ r, double* p0,
-                                                                      double* p1, double* __restrict__ q,
-                                                                      double* __restrict__ partial, PcgState* st) {
-  __shared__ double sh[32];
-  __shared__ double ys[kS][kSpmvWarps][3][32];
-  if (st->done) return;
-  const int it = st->it;
-  const double beta = st->beta;
-  const double* __restrict__ pold = (it & 1) ? p1 : p0;
-  double* __restrict__ pnew = (it & 1) ? p0 : p1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sl = warp / kSpmvWarps, w = warp % kSpmvWarps;
-  const int slice = blockIdx.x * kS + sl;
-  const int row = slice * 32 + lane;
-  const bool live = slice < n_slices && row < n_rows;
-  double y0 = 0, y1 = 0, y2 = 0;
-  auto fma9 = [&](const double (&a)[9], int cc) {
-    if (cc < 0) return;  // padding (its values are zero)
-    const double x0 = dinv[3 * cc] * r[3 * cc] + beta * pold[3 * cc];
-    const double x1 = dinv[3 * cc + 1] * r[3 * cc + 1] + beta * pold[3 * cc + 1];
-    const double x2 = dinv[3 * cc + 2] * r[3 * cc + 2] + beta * pold[3 * cc + 2];
-    y0 += a[0] * x0 + a[1] * x1 + a[2] * x2;
-    y1 += a[3] * x0 + a[4] * x1 + a[5] * x2;
-    y2 += a[6] * x0 + a[7] * x1 + a[8] * x2;
+// Part of a slice's row sums y = K u formed by warp w of the W that share the
+// slice (slots w, w + W, ...): U slots at a time, all their values requested
+// before use (kStream: evict-first, for matrices that do not stay in L2).
+// gather(c, u3) gives u at node c.
+template <int W, int U, bool kStream, class V, class Gather>
+__device__ __forceinline__ void slice_rows(int64_t s0, int64_t s1, int w, int lane, const int* __restrict__ col,
+                                           const V* __restrict__ val, Gather gather, double (&y)[3]) {
+  y[0] = y[1] = y[2] = 0.0;
+  for (int64_t s = s0 + w; s < s1; s += U * W) {
+    V a[U][9];
+    int c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      c[u] = -1;
+      if (s + u * W >= s1) continue;
+      c[u] = __ldg(col + (s + u * W) * 32 + lane);
+      const V* v = val + (s + u * W) * 288 + lane;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) a[u][k] = kStream ? __ldcs(v + k * 32) : __ldg(v + k * 32);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c[u] >= 0) {  // (padding: -1)
+        V x[3];
+        gather(c[u], x);
+        block_row(a[u], x, y);
+      }
+  }
+}
+
+struct PcgMat {
+  int n_rows, n_slices;
+  const int64_t* slice_ptr;
+  const int* col;
+};
+
+// Visits the CTA's slices: f(slice, live) by all warps together, W warps a slice
+// (kPcgWarps / W slices at a time). The set is the same in every phase.
+template <int W, class F>
+__device__ __forceinline__ void for_slices(int n_slices, F f) {
+  constexpr int S = kPcgWarps / W;
+  for (int base = blockIdx.x * S; base < n_slices; base += gridDim.x * S) f(base + (int)(threadIdx.x >> 5) / W);
+}
+
+// y of the W warps of each slice summed in warp order; valid in warp 0 of the slice.
+// (ys: [warps of the CTA][3][32] of shared memory.)
+template <int W>
+__device__ __forceinline__ void join_warps(double (&y)[3], double (*ys)[3][32]) {
+  if constexpr (W > 1) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 3; ++c) ys[warp][c][lane] = y[c];
+    __syncthreads();
+    if (warp % W == 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        for (int i = 1; i < W; ++i) y[c] += ys[warp + i][c][lane];
+    }
+  }
+}
+
+struct PcgEnd {  // how a solve ended (CTA 0 writes it)
+  __device__ static void write(PcgState* st, double err, int status, int iterations, int matvecs) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      st->err = err;
+      st->status = status;
+      st->iterations = iterations;
+      st->matvecs = matvecs;
+      st->done = 1;
+    }
+  }
+};
+
+template <int W, bool kStream>
+__global__ void __launch_bounds__(kPcgThreads, 3)
+    k_pcg(PcgMat M, const double* __restrict__ val, const double* __restrict__ b, const double* __restrict__ dinv,
+          double* x, double* r, double* z, double* p0, double* p1, double* q, PcgGrid grid, PcgState* st, double tol,
+          int max_it) {
+  __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = warp % W;
+  const int n3 = 3 * M.n_rows;
+  // elementwise phases: the 96 components of a slice, dealt to its W warps
+  auto own = [&](auto f) {
+    for_slices<W>(M.n_slices, [&](int slice) {
+      if (slice >= M.n_slices) return;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int i = slice * 96 + k * 32 + lane;
+        if (k % W == w && i < n3) f(i);
+      }
+    });
   };
-  if (live) {
-    const int64_t s0 = slice_ptr[slice], s1 = slice_ptr[slice + 1];
-    constexpr int U = 16 / (int)sizeof(V);  // 2 FP64 / 4 FP32 slots per group
-    int64_t s = s0 + w;
-    for (; s + (U - 1) * kSpmvWarps < s1; s += U * kSpmvWarps) {
-      int cu[U];
-      double a[U][9];
+  double s2[2] = {0.0, 0.0}, t2[2], t1[1];
+  own([&](int i) {
+    const double bi = b[i], zi = dinv[i] * bi;
+    r[i] = bi; x[i] = 0; z[i] = zi; p0[i] = 0;
+    s2[0] += bi * bi;
+    s2[1] += zi * bi;
+  });
+  if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
+  const double bnorm = sqrt(t2[0]);
+  double zr = t2[1], beta = 0.0, err = 0.0;
+  if (!(bnorm > 1e-25)) {  // SolverPCG.cs:112
+    PcgEnd::write(st, 0.0, MSG_OK, 0, 0);
+    return;
+  }
+  for (int it = 0;; ++it) {
+    double* pold = (it & 1) ? p1 : p0;
+    double* pnew = (it & 1) ? p0 : p1;
+    double pq = 0.0;
+    for_slices<W>(M.n_slices, [&](int slice) {
+      const int row = slice * 32 + lane;
+      const bool live = slice < M.n_slices && row < M.n_rows;
+      double y[3] = {0.0, 0.0, 0.0};
+      auto dir = [&](int c, double (&u)[3]) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t su = s + u * kSpmvWarps;
-        cu[u] = __ldg(col + su * 32 + lane);
-        const V* vu = val + su * 9 * 32 + lane;
+        for (int k = 0; k < 3; ++k) u[k] = z[3 * c + k] + beta * pold[3 * c + k];
+      };
+      if (live) slice_rows<W, 2, kStream>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val, dir, y);
+      join_warps<W>(y, ys);
+      if (w == 0 && live) {
+        double pn[3];
+        dir(row, pn);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) a[u][k] = (double)(kStream ? __ldcs(vu + k * 32) : __ldg(vu + k * 32));
+        for (int k = 0; k < 3; ++k) {
+          pnew[3 * row + k] = pn[k];
+          q[3 * row + k] = y[k];
+        }
+        pq += pn[0] * y[0] + pn[1] * y[1] + pn[2] * y[2];
+      }
+    });
+    const double v1[1] = {pq};
+    if (!grid_sum<kPcgWarps, 1>(grid, v1, t1)) return;
+    if (!(t1[0] > 0) || isnan(t1[0])) {  // breakdown: p.q <= 0 or NaN
+      PcgEnd::write(st, err, MSG_ERR_BREAKDOWN, it, it + 1);
+      return;
+    }
+    const double alpha = zr / t1[0];
+    s2[0] = s2[1] = 0.0;
+    own([&](int i) {
+      const double ri = r[i] - alpha * q[i], zi = dinv[i] * ri;
+      r[i] = ri;
+      x[i] += alpha * pnew[i];
+      z[i] = zi;
+      s2[0] += ri * ri;
+      s2[1] += zi * ri;
+    });
+    if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
+    err = sqrt(t2[0]) / bnorm;
+    if (err < tol) {
+      PcgEnd::write(st, err, MSG_OK, it, it + 1);
+      return;
+    }
+    if (it + 1 >= max_it) {
+      PcgEnd::write(st, err, MSG_ERR_NOT_CONVERGED, max_it, it + 1);
+      return;
+    }
+    beta = t2[1] / zr;
+    zr = t2[1];
+  }
+}
+
+// The same loop for matrices whose values fit the SMs' shared memory: a CTA, alone
+// on its SM, copies the values and columns of its S slices there once (W warps a
+// slice), and each thread keeps the r, x, D^-1 of its own component in registers,
+// so that an iteration reads only z and p_old at the gathered columns from L2.
+constexpr int kPcgResidentSmem = 204 * 1024;
+template <class V>
+inline size_t pcg_resident_smem(int64_t slots) {  // of a CTA with that many slots
+  return (size_t)slots * 32 * (9 * sizeof(V) + sizeof(int));
+}
+
+// What the two resident kernels share: the copy of a CTA's slices, and a row's sum
+// from it.
+template <int S, int W, class V>
+struct Resident {
+  V* vals;
+  int* cols;
+  int sl, w, lane, slice, row, t0, t1, n_slots;
+  bool have, live;
+  __device__ Resident(const PcgMat& M, const V* __restrict__ val, void* smem) {
+    const int warp = threadIdx.x >> 5, first = blockIdx.x * S;
+    lane = threadIdx.x & 31;
+    w = warp % W;
+    sl = warp / W;
+    slice = first + sl;
+    row = slice * 32 + lane;
+    have = slice < M.n_slices;
+    live = have && row < M.n_rows;
+    const int64_t a0 = M.slice_ptr[first], a1 = M.slice_ptr[min(first + S, M.n_slices)];
+    n_slots = (int)(a1 - a0);
+    t0 = have ? (int)(M.slice_ptr[slice] - a0) : 0;
+    t1 = have ? (int)(M.slice_ptr[slice + 1] - a0) : 0;
+    vals = static_cast<V*>(smem);
+    cols = reinterpret_cast<int*>(vals + (size_t)n_slots * 288);
+    for (int i = threadIdx.x; i < n_slots * 32; i += 32 * S * W) cols[i] = M.col[a0 * 32 + i];
+    for (int i = threadIdx.x; i < n_slots * 288; i += 32 * S * W) vals[i] = val[a0 * 288 + i];
+    __syncthreads();
+  }
+  // y = the part of the row's sum in the slots of this warp, four slots' gathers at a time
+  template <class Gather>
+  __device__ __forceinline__ void sum(Gather gather, double (&y)[3]) const {
+    constexpr int U = 4;
+    y[0] = y[1] = y[2] = 0.0;
+    if (!live) return;
+    for (int s = t0 + w; s < t1; s += U * W) {
+      V u[U][3];
+      int c[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        c[q] = s + q * W < t1 ? cols[(s + q * W) * 32 + lane] : -1;
+        if (c[q] >= 0) gather(c[q], u[q]);
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) fma9(a[u], cu[u]);
-    }
-    for (; s < s1; s += kSpmvWarps) {
-      const int c0 = __ldg(col + s * 32 + lane);
-      const V* v0 = val + s * 9 * 32 + lane;
-      double a0[9];
+      for (int q = 0; q < U; ++q)
+        if (c[q] >= 0) {
+          V a[9];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) a0[k] = (double)(kStream ? __ldcs(v0 + k * 32) : __ldg(v0 + k * 32));
-      fma9(a0, c0);
+          for (int k = 0; k < 9; ++k) a[k] = vals[(s + q * W) * 288 + k * 32 + lane];
+          block_row(a, u[q], y);
+        }
     }
   }
-  ys[sl][w][0][lane] = y0;
-  ys[sl][w][1][lane] = y1;
-  ys[sl][w][2][lane] = y2;
-  __syncthreads();
-  double pq = 0;
-  if (w == 0 && live) {
-    double yc[3], pn[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      double t = ys[sl][0][c][lane];
-#pragma unroll
-      for (int ww = 1; ww < kSpmvWarps; ++ww) t += ys[sl][ww][c][lane];
-      yc[c] = t;
-      pn[c] = dinv[3 * row + c] * r[3 * row + c] + beta * pold[3 * row + c];
-      pnew[3 * row + c] = pn[c];
-      q[3 * row + c] = t;
-    }
-    pq = pn[0] * yc[0] + pn[1] * yc[1] + pn[2] * yc[2];
+};
+
+template <int S, int W>
+__global__ void __launch_bounds__(32 * S * W, 1)
+    k_pcg_resident(PcgMat M, const double* __restrict__ val, const double* __restrict__ b,
+                   const double* __restrict__ dinv, double* x, double* z, double* p0, double* p1, PcgGrid grid,
+                   PcgState* st, double tol, int max_it) {
+  constexpr int NW = S * W;
+  extern __shared__ __align__(16) unsigned char pcg_smem[];
+  __shared__ double ys[NW][3][32];
+  __shared__ double qs[S][96], ps[S][96];
+  const Resident<S, W, double> A(M, val, pcg_smem);
+  const int lane = A.lane, sl = A.sl, row = A.row;
+  // the thread's own component of its slice (warps 0, 1, 2 of it)
+  const int e = A.w * 32 + lane, i = A.slice * 96 + e;
+  const bool own = A.have && A.w < 3 && i < 3 * M.n_rows;
+  double r = 0.0, xi = 0.0, dv = 0.0;
+  double s2[2] = {0.0, 0.0}, t2[2], u1[1];
+  if (own) {
+    r = b[i];
+    dv = dinv[i];
+    const double zi = dv * r;
+    z[i] = zi;
+    p0[i] = 0;
+    s2[0] = r * r;
+    s2[1] = zi * r;
   }
-  const double bs = block_sum(pq, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = bs;
-  if (!last_block(&st->counter)) return;
-  double tt[1];
-  sum_partials<1>(partial, gridDim.x, tt, sh);
-  const double t = tt[0];
-  if (threadIdx.x == 0) {
-    st->pq = t;
-    st->matvecs += 1;
-    if (!(t > 0) || isnan(t)) {  // breakdown: p.q <= 0 or NaN
-      st->status = MSG_ERR_BREAKDOWN; st->done = 1; st->iterations = it;
-    } else {
-      st->alpha = st->zr / t;
+  if (!grid_sum<NW, 2>(grid, s2, t2)) return;
+  const double bnorm = sqrt(t2[0]);
+  double zr = t2[1], beta = 0.0, err = 0.0;
+  int status = MSG_OK, iterations = 0, it = 0;
+  const bool solve = bnorm > 1e-25;  // SolverPCG.cs:112
+  while (solve) {
+    double* pold = (it & 1) ? p1 : p0;
+    double* pnew = (it & 1) ? p0 : p1;
+    auto dir = [&](int c, double (&u)[3]) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) u[k] = z[3 * c + k] + beta * pold[3 * c + k];
+    };
+    double y[3], pn[3] = {0.0, 0.0, 0.0};
+    const bool first = A.w == 0 && A.live;
+    if (first) dir(row, pn);
+    A.sum(dir, y);
+    join_warps<W>(y, ys);
+    const double v1[1] = {first ? pn[0] * y[0] + pn[1] * y[1] + pn[2] * y[2] : 0.0};
+    if (first) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        pnew[3 * row + k] = pn[k];
+        ps[sl][3 * lane + k] = pn[k];
+        qs[sl][3 * lane + k] = y[k];
+      }
     }
-    st->counter = 0;
+    if (!grid_sum<NW, 1>(grid, v1, u1)) return;
+    if (!(u1[0] > 0) || isnan(u1[0])) {  // breakdown: p.q <= 0 or NaN
+      status = MSG_ERR_BREAKDOWN;
+      iterations = it;
+      break;
+    }
+    const double alpha = zr / u1[0];
+    s2[0] = s2[1] = 0.0;
+    if (own) {
+      r -= alpha * qs[sl][e];
+      xi += alpha * ps[sl][e];
+      const double zi = dv * r;
+      z[i] = zi;
+      s2[0] = r * r;
+      s2[1] = zi * r;
+    }
+    if (!grid_sum<NW, 2>(grid, s2, t2)) return;
+    err = sqrt(t2[0]) / bnorm;
+    if (err < tol) {
+      iterations = it;
+      break;
+    }
+    if (++it >= max_it) {
+      iterations = max_it;
+      status = MSG_ERR_NOT_CONVERGED;
+      break;
+    }
+    beta = t2[1] / zr;
+    zr = t2[1];
   }
+  if (own) x[i] = xi;
+  PcgEnd::write(st, err, status, iterations, it);
 }
 
 // ------------------------------------------------------------------ mixed-precision PCG
 // MSG_PCG_SOLVE_MIXED's loop: FP32 matrix values and FP32 vectors (r, p, q, the
 // correction d and D^-1) inside the loop, the iterate x in FP64 (x += d at each
-// FP64 true residual) and FP64 sums for every dot product. Two kernels an
-// iteration:
-//   k_pcgm_spmv:   q = K32 p (p gathered in FP32), partials p.q, (D r).q and
-//     q.D q -> last block: alpha = gamma / p.q (breakdown check) and, since
-//     r' = r - alpha q, gamma' = (D r').r' = gamma - 2 alpha (D r).q +
-//     alpha^2 q.D q, hence beta = gamma' / gamma before the update;
-//   k_pcgm_update: r -= alpha q, d += alpha p, z = D r, p = z + beta p (the
-//     next direction, formed in the same pass) and the exact z.r, r.r ->
-//     last block: gamma = z.r, ||r||/||b||, pause for an FP64 true residual
-//     when it has dropped by delta since the last one or below tol.
-// On a pause the host runs k_pcgm_fold (x += d, d = 0), y = K64 x with the FP64
-// values and k_pcgm_true (r = b - y into the FP32 r, gamma = (D r).r; stop
-// when ||r||/||b|| < tol in FP64). The direction is kept across the
-// replacement. Per iteration the vectors cost 48 bytes a DOF besides the
-// matrix (16 in the SpMV pass, 32 in the update; with FP64 vectors and a
-// separate direction pass they would cost 108).
-// A warp owns one slice at a time; with kSpmvWarps = 1 the CTAs are persistent
-// (the grid fills the SMs once) and a warp strides over the slices, summing its
-// partials across them; with kSpmvWarps > 1 (small matrices) a CTA takes one
-// slice whose slots are dealt to its warps, whose sums meet in shared memory.
-template <int kS, int kSpmvWarps, bool kStream, int U = 4>
-__global__ void __launch_bounds__(32 * kS * kSpmvWarps, kSpmvWarps > 1 ? 1 : (U > 4 ? 3 : 4)) k_pcgm_spmv(int n_rows, int n_slices,
-                                                              const int64_t* __restrict__ slice_ptr,
-                                                              const int* __restrict__ col,
-                                                              const float* __restrict__ val,
-                                                              const float* __restrict__ p32,
-                                                              const float* __restrict__ r32,
-                                                              const float* __restrict__ dinv32,
-                                                              float* __restrict__ q32, double* __restrict__ partial,
-                                                              PcgState* st) {
-  __shared__ double sh[32];
-  __shared__ double ys[kSpmvWarps > 1 ? kS : 1][kSpmvWarps][3][32];
-  if (st->done) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sl = warp / kSpmvWarps, w = warp % kSpmvWarps;
-  double pq = 0, dq = 0, qdq = 0;
-  const int stride = kSpmvWarps > 1 ? n_slices : gridDim.x * kS;
-  for (int slice = blockIdx.x * kS + sl; slice < n_slices || (kSpmvWarps > 1 && slice == blockIdx.x * kS + sl);
-       slice += stride) {
-    const int row = slice * 32 + lane;
-    const bool live = slice < n_slices && row < n_rows;
-    double y0 = 0, y1 = 0, y2 = 0;
-    auto fma9 = [&](const float (&a)[9], int cc) {
-      if (cc < 0) return;  // padding (its values are zero)
-      const float x0 = __ldg(p32 + 3 * cc), x1 = __ldg(p32 + 3 * cc + 1), x2 = __ldg(p32 + 3 * cc + 2);
-      y0 += (double)fmaf(a[2], x2, fmaf(a[1], x1, a[0] * x0));
-      y1 += (double)fmaf(a[5], x2, fmaf(a[4], x1, a[3] * x0));
-      y2 += (double)fmaf(a[8], x2, fmaf(a[7], x1, a[6] * x0));
-    };
-    if (live) {
-      const int64_t s0 = slice_ptr[slice], s1 = slice_ptr[slice + 1];
-      // U slots per group: 36 U bytes of values in flight per thread
-      int64_t s = s0 + w;
-      for (; s + (U - 1) * kSpmvWarps < s1; s += U * kSpmvWarps) {
-        int cu[U];
-        float a[U][9];
+// FP64 true residual) and FP64 sums for every dot product. Two sums an iteration:
+//   1: q = K32 p, sums p.q, (D r).q and q.D q -> alpha = gamma / p.q (breakdown
+//      check) and, since r' = r - alpha q, gamma' = (D r').r' = gamma - 2 alpha
+//      (D r).q + alpha^2 q.D q, hence beta = gamma' / gamma before the update;
+//   2: r -= alpha q, d += alpha p, z = D r, p = z + beta p (the next direction,
+//      formed in the same pass), exact sums z.r and r.r -> gamma = z.r, and a
+//      true residual when ||r||/||b|| has dropped by delta since the last one or
+//      below tol: x += d, r = b - K64 x with the FP64 values (stop when
+//      ||r||/||b|| < tol in FP64), the direction kept.
+template <int W, bool kStream>
+__global__ void __launch_bounds__(kPcgThreads, 4)
+    k_pcg_mixed(PcgMat M, const double* __restrict__ val, const float* __restrict__ val32, const double* __restrict__ b,
+                const double* __restrict__ dinv, double* x, float* r32, float* p32, float* q32, float* d32,
+                float* dinv32, PcgGrid grid, PcgState* st, double tol, double delta, int max_it) {
+  __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = warp % W;
+  const int n3 = 3 * M.n_rows;
+  auto own = [&](auto f) {
+    for_slices<W>(M.n_slices, [&](int slice) {
+      if (slice >= M.n_slices) return;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int64_t su = s + u * kSpmvWarps;
-          cu[u] = __ldg(col + su * 32 + lane);
-          const float* vu = val + su * 9 * 32 + lane;
-#pragma unroll
-          for (int k = 0; k < 9; ++k) a[u][k] = kStream ? __ldcs(vu + k * 32) : __ldg(vu + k * 32);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) fma9(a[u], cu[u]);
+      for (int k = 0; k < 3; ++k) {
+        const int i = slice * 96 + k * 32 + lane;
+        if (k % W == w && i < n3) f(i);
       }
-      for (; s < s1; s += kSpmvWarps) {
-        const int c0 = __ldg(col + s * 32 + lane);
-        const float* v0 = val + s * 9 * 32 + lane;
-        float a0[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) a0[k] = kStream ? __ldcs(v0 + k * 32) : __ldg(v0 + k * 32);
-        fma9(a0, c0);
-      }
-    }
-    double yc[3] = {y0, y1, y2};
-    if constexpr (kSpmvWarps > 1) {
-      ys[sl][w][0][lane] = y0;
-      ys[sl][w][1][lane] = y1;
-      ys[sl][w][2][lane] = y2;
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        double t = ys[sl][0][c][lane];
-#pragma unroll
-        for (int ww = 1; ww < kSpmvWarps; ++ww) t += ys[sl][ww][c][lane];
-        yc[c] = t;
-      }
-    }
-    if (w == 0 && live) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int i = 3 * row + c;
-        const float qf = (float)yc[c], dv = dinv32[i];
-        q32[i] = qf;
-        pq += (double)p32[i] * (double)qf;
-        dq += (double)(dv * r32[i]) * (double)qf;
-        qdq += (double)(dv * qf) * (double)qf;
-      }
-    }
-    if constexpr (kSpmvWarps > 1) break;
-  }
-  const double b0 = block_sum(pq, sh), b1 = block_sum(dq, sh), b2 = block_sum(qdq, sh);
-  if (threadIdx.x == 0) {
-    partial[3 * blockIdx.x] = b0;
-    partial[3 * blockIdx.x + 1] = b1;
-    partial[3 * blockIdx.x + 2] = b2;
-  }
-  if (!last_block(&st->counter)) return;
-  double tt[3];
-  sum_partials<3>(partial, gridDim.x, tt, sh);
-  const double t = tt[0], tdq = tt[1], tqdq = tt[2];
-  if (threadIdx.x == 0) {
-    st->pq = t;
-    st->matvecs += 1;
-    if (!(t > 0) || isnan(t)) {  // breakdown: p.q <= 0 or NaN
-      st->status = MSG_ERR_BREAKDOWN; st->done = 1; st->iterations = st->it;
-    } else {
-      const double al = st->zr / t;
-      const double g1 = st->zr - 2.0 * al * tdq + al * al * tqdq;
-      st->alpha = al;
-      st->beta = g1 > 0.0 ? g1 / st->zr : 0.0;  // a non-positive estimate restarts from z
-    }
-    st->counter = 0;
-  }
-}
-
-// The vectors start at 16-byte boundaries: four components a thread at a
-// time (float4), the n3 % 4 tail one at a time.
-__global__ void __launch_bounds__(kPcgThreads) k_pcgm_update(int n3, const float* __restrict__ dinv32,
-                                                             float* __restrict__ r32, float* __restrict__ p32,
-                                                             const float* __restrict__ q32, float* __restrict__ d32,
-                                                             double* __restrict__ partial, PcgState* st) {
-  __shared__ double sh[32];
-  if (st->done) return;
-  const float al = (float)st->alpha, be = (float)st->beta;
-  double zr = 0, rr = 0;
-  auto step = [&](float pv, float qv, float rv, float dv, float dd, float& pn, float& rn, float& dn) {
-    rn = fmaf(-al, qv, rv);
-    const float zv = dv * rn;
-    dn = fmaf(al, pv, dd);
-    pn = fmaf(be, pv, zv);
-    zr += (double)zv * (double)rn;
-    rr += (double)rn * (double)rn;
+    });
   };
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-  const int n4 = n3 >> 2;
-  for (int i = tid; i < n4; i += nt) {
-    const float4 p = reinterpret_cast<const float4*>(p32)[i], q = reinterpret_cast<const float4*>(q32)[i];
-    const float4 r = reinterpret_cast<const float4*>(r32)[i], dv = reinterpret_cast<const float4*>(dinv32)[i];
-    const float4 d = reinterpret_cast<const float4*>(d32)[i];
-    float4 pn, rn, dn;
-    step(p.x, q.x, r.x, dv.x, d.x, pn.x, rn.x, dn.x);
-    step(p.y, q.y, r.y, dv.y, d.y, pn.y, rn.y, dn.y);
-    step(p.z, q.z, r.z, dv.z, d.z, pn.z, rn.z, dn.z);
-    step(p.w, q.w, r.w, dv.w, d.w, pn.w, rn.w, dn.w);
-    reinterpret_cast<float4*>(p32)[i] = pn;
-    reinterpret_cast<float4*>(r32)[i] = rn;
-    reinterpret_cast<float4*>(d32)[i] = dn;
-  }
-  for (int i = 4 * n4 + tid; i < n3; i += nt) step(p32[i], q32[i], r32[i], dinv32[i], d32[i], p32[i], r32[i], d32[i]);
-  const double s1 = block_sum(rr, sh), s2 = block_sum(zr, sh);
-  if (threadIdx.x == 0) { partial[2 * blockIdx.x] = s1; partial[2 * blockIdx.x + 1] = s2; }
-  if (!last_block(&st->counter)) return;
-  double tt[2];
-  sum_partials<2>(partial, gridDim.x, tt, sh);
-  const double tr = tt[0], tz = tt[1];
-  if (threadIdx.x == 0) {
-    const int it = st->it;
-    st->err = sqrt(tr) / st->bnorm;
-    st->rr = tr;
-    st->zr = tz;
-    if (st->err < st->tol || st->err < st->delta * st->err_ref) {
-      st->need = 1; st->done = 1;  // pause for an FP64 true residual
-    } else if (it + 1 >= st->max_it) {
-      st->done = 1; st->iterations = st->max_it; st->status = MSG_ERR_NOT_CONVERGED;
-    } else {
-      st->it = it + 1;
-    }
-    st->counter = 0;
-  }
-}
-
-// Start of the mixed loop: x = 0, d = 0, r = (float) b, D^-1 in FP32, p = z =
-// D^-1 r, gamma = z.r, ||b|| in FP64.
-__global__ void __launch_bounds__(kPcgThreads) k_pcgm_init(int n3, const double* __restrict__ b,
-                                                           const double* __restrict__ dinv, double* __restrict__ x,
-                                                           float* __restrict__ r32, float* __restrict__ p32,
-                                                           float* __restrict__ d32, float* __restrict__ dinv32,
-                                                           double* __restrict__ partial, PcgState* st) {
-  __shared__ double sh[32];
-  double bb = 0, zr = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
+  double s2[2] = {0.0, 0.0}, t2[2], t3[3];
+  own([&](int i) {
     const double bi = b[i];
     const float rv = (float)bi, dv = (float)dinv[i], zv = dv * rv;
     x[i] = 0;
@@ -531,128 +587,229 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcgm_init(int n3, const double*
     dinv32[i] = dv;
     p32[i] = zv;
     d32[i] = 0.f;
-    bb += bi * bi;
-    zr += (double)zv * (double)rv;
-  }
-  const double s1 = block_sum(bb, sh), s2 = block_sum(zr, sh);
-  if (threadIdx.x == 0) { partial[2 * blockIdx.x] = s1; partial[2 * blockIdx.x + 1] = s2; }
-  if (!last_block(&st->counter)) return;
-  double tt[2];
-  sum_partials<2>(partial, gridDim.x, tt, sh);
-  const double tb = tt[0], tz = tt[1];
-  if (threadIdx.x == 0) {
-    st->bnorm = sqrt(tb);
-    st->zr = tz;
-    st->beta = 0; st->alpha = 0; st->err = 0;
-    st->it = 0; st->iterations = 0; st->matvecs = 0; st->status = 0;
-    st->done = (st->bnorm > 1e-25) ? 0 : 1;  // SolverPCG.cs:112
-    st->need = 0; st->err_ref = 1.0;
-    st->counter = 0;
-  }
-}
-
-// x += d, d = 0 (the FP32 correction into the FP64 iterate)
-__global__ void k_pcgm_fold(int n3, double* __restrict__ x, float* __restrict__ d32) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-    x[i] += (double)d32[i];
-    d32[i] = 0.f;
-  }
-}
-
-// FP64 true residual r = b - y (y = K x with the FP64 values) into the FP32 r:
-// stop when ||r||/||b|| < tol, else gamma = (D r).r and the loop resumes with
-// its direction.
-__global__ void __launch_bounds__(kPcgThreads) k_pcgm_true(int n3, const double* __restrict__ b,
-                                                           const double* __restrict__ y,
-                                                           const float* __restrict__ dinv32, float* __restrict__ r32,
-                                                           double* __restrict__ partial, PcgState* st) {
-  __shared__ double sh[32];
-  double rr = 0, zr = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x) {
-    const double ri = b[i] - y[i];
-    const float rv = (float)ri;
-    r32[i] = rv;
-    rr += ri * ri;
-    zr += (double)(dinv32[i] * rv) * (double)rv;
-  }
-  const double s1 = block_sum(rr, sh), s2 = block_sum(zr, sh);
-  if (threadIdx.x == 0) { partial[2 * blockIdx.x] = s1; partial[2 * blockIdx.x + 1] = s2; }
-  if (!last_block(&st->counter)) return;
-  double tt[2];
-  sum_partials<2>(partial, gridDim.x, tt, sh);
-  const double tr = tt[0], tz = tt[1];
-  if (threadIdx.x == 0) {
-    const int it = st->it;
-    st->err = sqrt(tr) / st->bnorm;
-    st->need = 0;
-    if (st->err < st->tol) {
-      st->done = 1; st->iterations = it;
-    } else if (it + 1 >= st->max_it) {
-      st->done = 1; st->iterations = st->max_it; st->status = MSG_ERR_NOT_CONVERGED;
-    } else {
-      st->zr = tz;
-      st->it = it + 1;
-      st->err_ref = st->err;
-      st->done = 0;
+    s2[0] += bi * bi;
+    s2[1] += (double)zv * (double)rv;
+  });
+  if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
+  const double bnorm = sqrt(t2[0]);
+  double zr = t2[1], err = 0.0, err_ref = 1.0;
+  int status = MSG_OK, iterations = 0, it = 0, products = 0;
+  bool done = !(bnorm > 1e-25);  // SolverPCG.cs:112
+  while (!done) {
+    double s3[3] = {0.0, 0.0, 0.0};
+    for_slices<W>(M.n_slices, [&](int slice) {
+      const int row = slice * 32 + lane;
+      const bool live = slice < M.n_slices && row < M.n_rows;
+      double y[3] = {0.0, 0.0, 0.0};
+      auto dir = [&](int c, float (&u)[3]) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[k] = p32[3 * c + k];
+      };
+      if (live) slice_rows<W, 2, kStream>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val32, dir, y);
+      join_warps<W>(y, ys);
+      if (w == 0 && live) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const int i = 3 * row + k;
+          const float qf = (float)y[k], dv = dinv32[i];
+          q32[i] = qf;
+          s3[0] += (double)p32[i] * (double)qf;
+          s3[1] += (double)(dv * r32[i]) * (double)qf;
+          s3[2] += (double)(dv * qf) * (double)qf;
+        }
+      }
+    });
+    if (!grid_sum<kPcgWarps, 3>(grid, s3, t3)) return;
+    ++products;
+    if (!(t3[0] > 0) || isnan(t3[0])) {  // breakdown: p.q <= 0 or NaN
+      status = MSG_ERR_BREAKDOWN;
+      iterations = it;
+      break;
     }
-    st->counter = 0;
+    const double alpha = zr / t3[0];
+    const double g1 = zr - 2.0 * alpha * t3[1] + alpha * alpha * t3[2];
+    const float al = (float)alpha, be = (float)(g1 > 0.0 ? g1 / zr : 0.0);  // a non-positive estimate restarts from z
+    s2[0] = s2[1] = 0.0;
+    own([&](int i) {
+      const float pv = p32[i], rn = fmaf(-al, q32[i], r32[i]), zv = dinv32[i] * rn;
+      d32[i] = fmaf(al, pv, d32[i]);
+      p32[i] = fmaf(be, pv, zv);
+      r32[i] = rn;
+      s2[0] += (double)rn * (double)rn;
+      s2[1] += (double)zv * (double)rn;
+    });
+    if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
+    err = sqrt(t2[0]) / bnorm;
+    zr = t2[1];
+    if (err < tol || err < delta * err_ref) {
+      own([&](int i) {
+        x[i] += (double)d32[i];
+        d32[i] = 0.f;
+      });
+      s2[0] = s2[1] = 0.0;
+      if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;  // x is complete
+      for_slices<W>(M.n_slices, [&](int slice) {
+        const int row = slice * 32 + lane;
+        const bool live = slice < M.n_slices && row < M.n_rows;
+        double y[3] = {0.0, 0.0, 0.0};
+        auto at = [&](int c, double (&u)[3]) {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) u[k] = x[3 * c + k];
+        };
+        if (live) slice_rows<W, 1, true>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val, at, y);
+        join_warps<W>(y, ys);
+        if (w == 0 && live) {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int i = 3 * row + k;
+            const double ri = b[i] - y[k];
+            const float rv = (float)ri;
+            r32[i] = rv;
+            s2[0] += ri * ri;
+            s2[1] += (double)(dinv32[i] * rv) * (double)rv;
+          }
+        }
+      });
+      if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
+      err = sqrt(t2[0]) / bnorm;
+      if (err < tol) {
+        iterations = it;
+        done = true;
+      } else {
+        zr = t2[1];
+        err_ref = err;
+      }
+    }
+    if (!done && it + 1 >= max_it) {
+      iterations = max_it;
+      status = MSG_ERR_NOT_CONVERGED;
+      done = true;
+    }
+    ++it;
   }
+  own([&](int i) { x[i] += (double)d32[i]; });  // a correction left by a solve that ended without a true residual
+  PcgEnd::write(st, err, status, iterations, products);
 }
 
-__global__ void __launch_bounds__(kPcgThreads) k_pcg_update(int n_rows, const double* __restrict__ dinv,
-                                                            double* __restrict__ r, double* __restrict__ x,
-                                                            const double* __restrict__ p0,
-                                                            const double* __restrict__ p1,
-                                                            const double* __restrict__ q, double* __restrict__ partial,
-                                                            PcgState* st) {
-  __shared__ double sh[32];
-  if (st->done) return;
-  const int it = st->it;
-  const double alpha = st->alpha;
-  const double* __restrict__ pnew = (it & 1) ? p0 : p1;
-  double rr = 0, zr = 0;
-  // two components a thread at a time (double2; the vectors start at 16-byte boundaries)
-  const int n3 = 3 * n_rows, n2 = n3 >> 1;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-  for (int i = tid; i < n2; i += nt) {
-    const double2 rv = reinterpret_cast<const double2*>(r)[i], qv = reinterpret_cast<const double2*>(q)[i];
-    const double2 xv = reinterpret_cast<const double2*>(x)[i], pv = reinterpret_cast<const double2*>(pnew)[i];
-    const double2 dv = reinterpret_cast<const double2*>(dinv)[i];
-    const double r0 = rv.x - alpha * qv.x, r1 = rv.y - alpha * qv.y;
-    reinterpret_cast<double2*>(r)[i] = make_double2(r0, r1);
-    reinterpret_cast<double2*>(x)[i] = make_double2(xv.x + alpha * pv.x, xv.y + alpha * pv.y);
-    rr += r0 * r0;
-    zr += dv.x * r0 * r0;
-    rr += r1 * r1;
-    zr += dv.y * r1 * r1;
+// The mixed loop on resident FP32 values (Resident): the thread keeps r, p, d, D^-1,
+// b and x of its component in registers; the FP64 values of the true residuals
+// stream from memory.
+template <int S, int W>
+__global__ void __launch_bounds__(32 * S * W, 1)
+    k_pcg_mixed_resident(PcgMat M, const double* __restrict__ val, const float* __restrict__ val32,
+                         const double* __restrict__ b, const double* __restrict__ dinv, double* x, float* p32,
+                         PcgGrid grid, PcgState* st, double tol, double delta, int max_it) {
+  constexpr int NW = S * W;
+  extern __shared__ __align__(16) unsigned char pcg_smem[];
+  __shared__ double ys[NW][3][32];
+  __shared__ double qs[S][96];
+  const Resident<S, W, float> A(M, val32, pcg_smem);
+  const int lane = A.lane, sl = A.sl;
+  const int e = A.w * 32 + lane, i = A.slice * 96 + e;
+  const bool own = A.have && A.w < 3 && i < 3 * M.n_rows, first = A.w == 0 && A.live;
+  double bi = 0.0, xi = 0.0;
+  float r = 0.f, p = 0.f, d = 0.f, dv = 0.f;
+  double s2[2] = {0.0, 0.0}, t2[2], t3[3];
+  if (own) {
+    bi = b[i];
+    r = (float)bi;
+    dv = (float)dinv[i];
+    p = dv * r;
+    p32[i] = p;
+    s2[0] = bi * bi;
+    s2[1] = (double)p * (double)r;
   }
-  for (int i = 2 * n2 + tid; i < n3; i += nt) {
-    const double ri = r[i] - alpha * q[i];
-    r[i] = ri;
-    x[i] = x[i] + alpha * pnew[i];
-    rr += ri * ri;
-    zr += dinv[i] * ri * ri;
-  }
-  double s1 = block_sum(rr, sh);
-  double s2 = block_sum(zr, sh);
-  if (threadIdx.x == 0) { partial[2 * blockIdx.x] = s1; partial[2 * blockIdx.x + 1] = s2; }
-  if (!last_block(&st->counter)) return;
-  double tt[2];
-  sum_partials<2>(partial, gridDim.x, tt, sh);
-  const double tr = tt[0], tz = tt[1];
-  if (threadIdx.x == 0) {
-    st->err = sqrt(tr) / st->bnorm;
-    if (st->err < st->tol) {
-      st->done = 1; st->iterations = it;
-    } else if (it + 1 >= st->max_it) {
-      st->done = 1; st->iterations = st->max_it; st->status = MSG_ERR_NOT_CONVERGED;
-    } else {
-      st->beta = tz / st->zr;
-      st->zr = tz;
-      st->it = it + 1;
+  if (!grid_sum<NW, 2>(grid, s2, t2)) return;
+  const double bnorm = sqrt(t2[0]);
+  double zr = t2[1], err = 0.0, err_ref = 1.0;
+  int status = MSG_OK, iterations = 0, it = 0, products = 0;
+  bool done = !(bnorm > 1e-25);  // SolverPCG.cs:112
+  // the row sums of the slices' first warps, as the components of the own threads
+  auto spread = [&](double (&y)[3]) {
+    join_warps<W>(y, ys);
+    if (first)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) qs[sl][3 * lane + k] = y[k];
+    __syncthreads();
+  };
+  while (!done) {
+    double y[3], s3[3] = {0.0, 0.0, 0.0};
+    A.sum([&](int c, float (&u)[3]) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) u[k] = p32[3 * c + k];
+    }, y);
+    spread(y);
+    float q = 0.f;
+    if (own) {
+      q = (float)qs[sl][e];
+      s3[0] = (double)p * (double)q;
+      s3[1] = (double)(dv * r) * (double)q;
+      s3[2] = (double)(dv * q) * (double)q;
     }
-    st->counter = 0;
+    if (!grid_sum<NW, 3>(grid, s3, t3)) return;
+    ++products;
+    if (!(t3[0] > 0) || isnan(t3[0])) {  // breakdown: p.q <= 0 or NaN
+      status = MSG_ERR_BREAKDOWN;
+      iterations = it;
+      break;
+    }
+    const double alpha = zr / t3[0];
+    const double g1 = zr - 2.0 * alpha * t3[1] + alpha * alpha * t3[2];
+    const float al = (float)alpha, be = (float)(g1 > 0.0 ? g1 / zr : 0.0);  // a non-positive estimate restarts from z
+    s2[0] = s2[1] = 0.0;
+    if (own) {
+      r = fmaf(-al, q, r);
+      const float zv = dv * r;
+      d = fmaf(al, p, d);
+      p = fmaf(be, p, zv);
+      p32[i] = p;
+      s2[0] = (double)r * (double)r;
+      s2[1] = (double)zv * (double)r;
+    }
+    if (!grid_sum<NW, 2>(grid, s2, t2)) return;
+    err = sqrt(t2[0]) / bnorm;
+    zr = t2[1];
+    if (err < tol || err < delta * err_ref) {
+      if (own) {
+        xi += (double)d;
+        d = 0.f;
+        x[i] = xi;
+      }
+      s2[0] = s2[1] = 0.0;
+      if (!grid_sum<NW, 2>(grid, s2, t2)) return;  // x is complete
+      y[0] = y[1] = y[2] = 0.0;
+      if (A.live)
+        slice_rows<W, 1, true>(M.slice_ptr[A.slice], M.slice_ptr[A.slice + 1], A.w, lane, M.col, val,
+                               [&](int c, double (&u)[3]) {
+#pragma unroll
+                                 for (int k = 0; k < 3; ++k) u[k] = x[3 * c + k];
+                               }, y);
+      spread(y);
+      if (own) {
+        const double ri = bi - qs[sl][e];
+        r = (float)ri;
+        s2[0] = ri * ri;
+        s2[1] = (double)(dv * r) * (double)r;
+      }
+      if (!grid_sum<NW, 2>(grid, s2, t2)) return;
+      err = sqrt(t2[0]) / bnorm;
+      if (err < tol) {
+        iterations = it;
+        done = true;
+      } else {
+        zr = t2[1];
+        err_ref = err;
+      }
+    }
+    if (!done && it + 1 >= max_it) {
+      iterations = max_it;
+      status = MSG_ERR_NOT_CONVERGED;
+      done = true;
+    }
+    ++it;
   }
+  if (own) x[i] = xi + (double)d;  // (a correction left by a solve that ended without a true residual)
+  PcgEnd::write(st, err, status, iterations, products);
 }
 
 __global__ void k_to_f32(size_t n, const double* __restrict__ a, float* __restrict__ b) {
@@ -720,260 +877,169 @@ int launch_node_to_dof(Context* ctx, const Mesh* m, const double* d_in, double* 
   return MSG_OK;
 }
 
-// The FP64 loop's direction + SpMV launch (shape chosen by size).
-static void launch_pcg_dir_spmv(Context* ctx, const Mesh* m, double* v64, double* dv, double* rv, double* p0,
-                                double* p1, double* qv, double* pa, PcgState* st, cudaStream_t stream) {
-  const int nr = m->n_nodes;
-  const int ns = m->pat.n_slices;
-  const bool small = ns < ctx->sm_count * 32;  // fewer slices than 32 warps per SM: 4 warps per slice
-  const int64_t* sp = m->d_slice_ptr.as<int64_t>();
-  const int* cl = m->d_col.as<int>();
-  // FP64 values stream through with evict-first loads (measured faster at every size)
-  if (small)
-    k_pcg_dir_spmv_rows<double, 1, 4, true><<<ns, 128, 0, stream>>>(nr, ns, sp, cl, v64, dv, rv, p0, p1, qv, pa, st);
-  else
-    k_pcg_dir_spmv_rows<double, 8, 1, true><<<(ns + 7) / 8, 256, 0, stream>>>(nr, ns, sp, cl, v64, dv, rv, p0, p1, qv,
-                                                                              pa, st);
+namespace {
+
+// Warps that share a slice: 4 where the slices are fewer than 32 warps an SM
+// (a warp alone takes 27 slots one after another), 2 above (a CTA's share of the
+// slices is then even to a few percent: 64^3 is 9.7 rounds of 4 slices a CTA).
+bool pcg_small(const Context* ctx, const Mesh* m) { return m->pat.n_slices < ctx->sm_count * 32; }
+
+PcgMat pcg_mat(const Mesh* m) {
+  return {m->n_nodes, m->pat.n_slices, m->d_slice_ptr.as<int64_t>(), m->d_col.as<int>()};
 }
 
-// The mixed loop's FP32 SpMV launch: small matrices one slice per CTA with 4
-// warps; large ones by the "spmv32_shape" option (slots per group / slices per
-// CTA: 0: 4 / 8, 1: 8 / 8, 2: 4 / 4, 3: 8 / 4). FP32 values of matrices up to
-// ~60 % of L2 stay there across iterations, larger ones stream (evict-first).
-static void launch_pcgm_spmv(Context* ctx, const Mesh* m, const float* v32, const float* p32, const float* r32,
-                             const float* dinv32, float* q32, double* pa, PcgState* st, cudaStream_t stream) {
-  const int nr = m->n_nodes;
-  const int ns = m->pat.n_slices;
-  const bool small = ns < ctx->sm_count * 32;
-  const int64_t* sp = m->d_slice_ptr.as<int64_t>();
-  const int* cl = m->d_col.as<int>();
-  const bool strm = (size_t)m->pat.n_slots * 32 * 9 * 4 > (size_t)76 << 20;
-  const int shape = ctx->spmv32_shape;
-  // persistent grid (W = 1): the resident CTAs of every SM once
-  auto fill = [&](const void* k, int threads, int n_ctas) {
-    int occ = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, threads, 0) != cudaSuccess || occ < 1) occ = 1;
-    return std::max(1, std::min(n_ctas, ctx->sm_count * occ));
-  };
-#define MSG_SPMV32(S, W, U)                                                                                       \
-  do {                                                                                                           \
-    const int grid = W > 1 ? (ns + S - 1) / S                                                                    \
-                           : fill((const void*)k_pcgm_spmv<S, W, true, U>, 32 * S * W, (ns + S - 1) / S);        \
-    if (strm)                                                                                                    \
-      k_pcgm_spmv<S, W, true, U><<<grid, 32 * S * W, 0, stream>>>(nr, ns, sp, cl, v32, p32, r32, dinv32, q32, pa, \
-                                                                  st);                                           \
-    else                                                                                                         \
-      k_pcgm_spmv<S, W, false, U><<<grid, 32 * S * W, 0, stream>>>(nr, ns, sp, cl, v32, p32, r32, dinv32, q32,    \
-                                                                   pa, st);                                      \
-  } while (0)
-  if (small) MSG_SPMV32(1, 4, 4);
-  else if (shape == 1) MSG_SPMV32(8, 1, 8);
-  else if (shape == 2) MSG_SPMV32(4, 1, 4);
-  else if (shape == 3) MSG_SPMV32(4, 1, 8);
-  else MSG_SPMV32(8, 1, 4);
-#undef MSG_SPMV32
+// CTAs of a solve: one per group of slices, at most those resident at once
+// (the kernels' CTAs wait for each other).
+int pcg_grid(Context* ctx, const Mesh* m, const void* kernel, bool small) {
+  const int per = small ? kPcgWarps / 4 : kPcgWarps / 2;
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kPcgThreads, 0) != cudaSuccess || occ < 1) occ = 1;
+  return std::max(1, std::min((m->pat.n_slices + per - 1) / per, ctx->sm_count * std::min(occ, kPcgMaxCtas)));
 }
 
-// The device loop's control (one thread each, inside the solve's graph):
-// another round of iterations while the solve runs, at most
-// max_it / chunk + 2 max_it + 4 rounds (every round but a paused one advances
-// the iteration count, every pause ends or advances it, so the bound is never
-// the reason to stop); and, in the mixed loop, the FP64 true-residual step
-// when the round paused for one.
-__global__ void k_pcg_loop_while(PcgState* st, cudaGraphConditionalHandle h, int chunk) {
-  const long long r = ++st->rounds;
-  const long long cap = (long long)st->max_it / chunk + 2LL * st->max_it + 4;
-  cudaGraphSetConditional(h, (!st->done && r < cap) ? 1u : 0u);
+// bytes of the partial sums, then the state
+size_t pcg_head_bytes(const Context* ctx) { return sizeof(double) * 2 * kPcgSums * kPcgMaxCtas * ctx->sm_count + 256; }
+PcgState* pcg_state(const Context* ctx, void* head) {
+  return reinterpret_cast<PcgState*>(static_cast<char*>(head) + pcg_head_bytes(ctx) - 256);
 }
 
-__global__ void k_pcg_loop_if(PcgState* st, cudaGraphConditionalHandle h) {
-  const int need = st->need;
-  if (need) st->pauses += 1;
-  cudaGraphSetConditional(h, need ? 1u : 0u);
+// Values that do not stay in L2 between iterations stream through it evict-first
+// (a 71 MB matrix: 18.2 us an iteration without, 18.7 with; 240 MB: 56 and 48).
+bool pcg_stream(const Mesh* m, size_t value_bytes) { return (size_t)m->pat.n_slots * 288 * value_bytes > (size_t)100 << 20; }
+
+// Slices an SM (at most `most`, the kernels' widest CTA) if the CTAs of a resident
+// solve fit, one an SM, with their slots in shared memory; 0 otherwise.
+template <class V>
+int pcg_resident(const Context* ctx, const Mesh* m, int most, size_t* smem) {
+  const std::vector<int64_t>& sp = m->pat.slice_ptr;
+  const int ns = m->pat.n_slices, S = (ns + ctx->sm_count - 1) / ctx->sm_count;
+  if (S > most) return 0;
+  int64_t slots = 0;
+  for (int i = 0; i < ns; i += S) slots = std::max(slots, sp[std::min(i + S, ns)] - sp[i]);
+  *smem = pcg_resident_smem<V>(slots);
+  return *smem <= (size_t)kPcgResidentSmem ? S : 0;
 }
 
-// Runs the device PCG on node-layout vectors, the whole solve one graph
-// launch: a WHILE node repeats a round of `chunk` iterations (2 kernels each,
-// captured once per matrix) until the state says done, with no host round
-// trip between rounds. Kernels after convergence return immediately, so the
-// recorded iteration count is exact. Mixed precision: the FP32 loop
-// (k_pcgm_*); when it pauses (need), an IF node runs x += d, y = K x with the
-// FP64 values and k_pcgm_true, which replace the recursive residual (or end
-// the solve on the true residual).
+struct PcgLaunch {
+  const void* kernel = nullptr;
+  int grid = 0, threads = kPcgThreads;
+  size_t smem = 0;
+};
+
+int pcg_cooperative(Context* ctx, const PcgLaunch& l, void** args, cudaStream_t s) {
+  MSG_CUDA(ctx, cudaFuncSetAttribute(l.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
+  MSG_CUDA(ctx, cudaLaunchCooperativeKernel(l.kernel, dim3(l.grid), dim3(l.threads), args, l.smem, s));
+  count_launch(ctx);
+  return MSG_OK;
+}
+
+// One FP64 solve on stream s: partial sums and state cleared, one cooperative launch.
+int pcg_launch(Context* ctx, const Mesh* m, const double* val, const double* b, const double* dinv, double* x,
+               double* r, double* z, double* p0, double* p1, double* q, void* head, double tol, int max_it,
+               cudaStream_t s) {
+  PcgMat M = pcg_mat(m);
+  PcgState* st = pcg_state(ctx, head);
+  PcgGrid g{static_cast<double*>(head), &st->counter, 0u, 0};
+  MSG_CUDA(ctx, cudaMemsetAsync(head, 0, pcg_head_bytes(ctx), s));
+  PcgLaunch l;
+  if (const int S = pcg_resident<double>(ctx, m, 3, &l.smem)) {
+    l.kernel = S == 1 ? (const void*)k_pcg_resident<1, 8> : S == 2 ? (const void*)k_pcg_resident<2, 4>
+                                                                   : (const void*)k_pcg_resident<3, 4>;
+    l.threads = S == 1 ? 256 : 128 * S;
+    l.grid = (m->pat.n_slices + S - 1) / S;
+    void* args[] = {&M, &val, &b, &dinv, &x, &z, &p0, &p1, &g, &st, &tol, &max_it};
+    return pcg_cooperative(ctx, l, args, s);
+  }
+  l.smem = 0;
+  const bool small = pcg_small(ctx, m), stream = pcg_stream(m, sizeof(double));
+  l.kernel = small ? (stream ? (const void*)k_pcg<4, true> : (const void*)k_pcg<4, false>)
+                   : (stream ? (const void*)k_pcg<2, true> : (const void*)k_pcg<2, false>);
+  l.grid = pcg_grid(ctx, m, l.kernel, small);
+  void* args[] = {&M, &val, &b, &dinv, &x, &r, &z, &p0, &p1, &q, &g, &st, &tol, &max_it};
+  return pcg_cooperative(ctx, l, args, s);
+}
+
+// The state after a solve (its copy on the host); a solve whose grid barrier
+// expired leaves it not done.
+int pcg_finish(Context* ctx, PcgState* st, PcgState* host, cudaStream_t s) {
+  MSG_CUDA(ctx, cudaMemcpyAsync(host, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
+  MSG_CUDA(ctx, cudaStreamSynchronize(s));
+  if (!host->done) return set_error(ctx, MSG_ERR_TIMEOUT, "PCG: a bounded grid barrier expired");
+  return MSG_OK;
+}
+
+}  // namespace
+
+// Runs the device PCG on node-layout vectors (k_pcg, or k_pcg_mixed), one launch a solve.
 int pcg_solve_device(Context* ctx, Matrix* A, const double* d_b, double* d_x, int max_it, double tol, int* iterations,
                      double* rel_res, int* status, bool mixed) {
   Mesh* m = A->mesh;
-  const int nr = m->n_nodes;
-  const int n = 3 * nr;
+  const size_t n = 3 * (size_t)m->n_nodes;
   cudaStream_t s = ctx->stream;
   MSG_TRY(context_resources(ctx));
-  if (!A->d_r.ptr) {
-    MSG_TRY(A->d_r.alloc(ctx, sizeof(double) * n));
-    MSG_TRY(A->d_p0.alloc(ctx, sizeof(double) * n));
-    MSG_TRY(A->d_p1.alloc(ctx, sizeof(double) * n));
-    MSG_TRY(A->d_q.alloc(ctx, sizeof(double) * n));
-    // partials: one per FP64 SpMV CTA (slice), three per FP32 SpMV CTA or two per update CTA
-    MSG_TRY(A->d_partial.alloc(ctx, sizeof(double) * std::max<size_t>(2 * 4096, 3 * (size_t)m->pat.n_slices)));
-    MSG_TRY(A->d_state.alloc(ctx, sizeof(PcgState)));
-    MSG_CUDA(ctx, cudaMemsetAsync(A->d_state.ptr, 0, sizeof(PcgState), s));
-  }
-  if (mixed && !A->d_val32.ptr) {
-    const size_t nv = (size_t)m->pat.n_slots * 32 * 9;
-    MSG_TRY(A->d_val32.alloc(ctx, sizeof(float) * std::max<size_t>(1, nv)));
-    MSG_TRY(A->d_tmp.alloc(ctx, sizeof(double) * n));   // y = K x of the true residual
-    MSG_TRY(A->d_tmp2.alloc(ctx, sizeof(float) * n));   // p (FP32)
-    MSG_TRY(A->d_m32.alloc(ctx, sizeof(float) * 4 * (((size_t)n + 31) / 32 * 32)));
-    k_to_f32<<<ctx->sm_count * 8, 256, 0, s>>>(nv, A->d_val.as<double>(), A->d_val32.as<float>());
-    count_launch(ctx);
-  }
-  PcgState* st = A->d_state.as<PcgState>();
-  const int grid_v = std::min(4096, std::max(1, std::min((n + kPcgThreads - 1) / kPcgThreads, ctx->sm_count * 8)));
-  // the update passes: float4 (mixed) or double2 (FP64) a thread, at most 4 CTAs an SM
-  const int grid_u = std::max(1, std::min((n / (mixed ? 4 : 2) + kPcgThreads - 1) / kPcgThreads, ctx->sm_count * 4));
-  double* pa = A->d_partial.as<double>();
-  float *p32 = nullptr, *r32 = nullptr, *q32 = nullptr, *d32 = nullptr, *dinv32 = nullptr;
+  // one allocation for the partial sums, the state and the solve's vectors: r, z, p
+  // (two), q in FP64, or in the mixed loop r, p, q, d and D^-1 in FP32
+  const size_t nv = (n + 31) / 32 * 32, head = pcg_head_bytes(ctx);
+  if (!A->d_work.ptr) MSG_TRY(A->d_work.alloc(ctx, head + sizeof(double) * 5 * nv));
+  PcgState* st = pcg_state(ctx, A->d_work.ptr);
+  double* v = reinterpret_cast<double*>(A->d_work.as<char>() + head);
   if (mixed) {
-    const size_t n32 = ((size_t)n + 31) / 32 * 32;  // 128-byte aligned vectors
-    p32 = A->d_tmp2.as<float>();
-    r32 = A->d_m32.as<float>();
-    q32 = r32 + n32;
-    d32 = q32 + n32;
-    dinv32 = d32 + n32;
-    k_pcgm_init<<<grid_v, kPcgThreads, 0, s>>>(n, d_b, A->d_dinv.as<double>(), d_x, r32, p32, d32, dinv32, pa, st);
+    const size_t nval = (size_t)m->pat.n_slots * 32 * 9;
+    if (!A->d_val32.ptr) {
+      MSG_TRY(A->d_val32.alloc(ctx, sizeof(float) * std::max<size_t>(1, nval)));
+      k_to_f32<<<ctx->sm_count * 8, 256, 0, s>>>(nval, A->d_val.as<double>(), A->d_val32.as<float>());
+      count_launch(ctx);
+    }
+    float* f = reinterpret_cast<float*>(v);
+    PcgMat M = pcg_mat(m);
+    PcgGrid g{A->d_work.as<double>(), &st->counter, 0u, 0};
+    const double *val = A->d_val.as<double>(), *dinv = A->d_dinv.as<double>();
+    const float* val32 = A->d_val32.as<float>();
+    float *r32 = f, *p32 = f + nv, *q32 = f + 2 * nv, *d32 = f + 3 * nv, *dinv32 = f + 4 * nv;
+    double delta = ctx->reliable_delta;
+    MSG_CUDA(ctx, cudaMemsetAsync(A->d_work.ptr, 0, head, s));
+    PcgLaunch l;
+    if (const int S = pcg_resident<float>(ctx, m, 6, &l.smem)) {
+      const void* ks[] = {(const void*)k_pcg_mixed_resident<1, 8>, (const void*)k_pcg_mixed_resident<2, 4>,
+                          (const void*)k_pcg_mixed_resident<3, 4>, (const void*)k_pcg_mixed_resident<4, 3>,
+                          (const void*)k_pcg_mixed_resident<5, 3>, (const void*)k_pcg_mixed_resident<6, 3>};
+      l.kernel = ks[S - 1];
+      l.threads = S == 1 ? 256 : S < 4 ? 128 * S : 96 * S;
+      l.grid = (m->pat.n_slices + S - 1) / S;
+      void* args[] = {&M, &val, &val32, &d_b, &dinv, &d_x, &p32, &g, &st, &tol, &delta, &max_it};
+      MSG_TRY(pcg_cooperative(ctx, l, args, s));
+    } else {
+      l.smem = 0;
+      const bool small = pcg_small(ctx, m), stream = pcg_stream(m, sizeof(float));
+      l.kernel = small ? (stream ? (const void*)k_pcg_mixed<4, true> : (const void*)k_pcg_mixed<4, false>)
+                       : (stream ? (const void*)k_pcg_mixed<2, true> : (const void*)k_pcg_mixed<2, false>);
+      l.grid = pcg_grid(ctx, m, l.kernel, small);
+      void* args[] = {&M,   &val, &val32,  &d_b, &dinv, &d_x, &r32,   &p32,
+                      &q32, &d32, &dinv32, &g,   &st,   &tol, &delta, &max_it};
+      MSG_TRY(pcg_cooperative(ctx, l, args, s));
+    }
   } else {
-    k_pcg_init<<<grid_v, kPcgThreads, 0, s>>>(nr, d_b, A->d_dinv.as<double>(), A->d_r.as<double>(), d_x,
-                                              A->d_p0.as<double>(), A->d_p1.as<double>(), pa, st);
+    MSG_TRY(pcg_launch(ctx, m, A->d_val.as<double>(), d_b, A->d_dinv.as<double>(), d_x, v, v + nv, v + 2 * nv,
+                       v + 3 * nv, v + 4 * nv, A->d_work.ptr, tol, max_it, s));
   }
-  count_launch(ctx);
-  // tol, max_it and the mixed-precision settings into the state (after init so the counter reset does not race)
-  {
-    const int mx = mixed ? 1 : 0;
-    const double delta = ctx->reliable_delta;
-    MSG_CUDA(ctx, cudaMemcpyAsync(&st->tol, &tol, sizeof(double), cudaMemcpyHostToDevice, s));
-    MSG_CUDA(ctx, cudaMemcpyAsync(&st->max_it, &max_it, sizeof(int), cudaMemcpyHostToDevice, s));
-    MSG_CUDA(ctx, cudaMemcpyAsync(&st->mixed, &mx, sizeof(int), cudaMemcpyHostToDevice, s));
-    MSG_CUDA(ctx, cudaMemcpyAsync(&st->delta, &delta, sizeof(double), cudaMemcpyHostToDevice, s));
-    // the pageable copies above are staged before they return
-  }
-  const int chunk = 8;
-  const int graph_kind = mixed ? 1 + ctx->spmv32_shape : 0;  // the captured loop's kernels and shapes
-  if (!A->graph || A->graph_chunk != chunk || A->graph_x != (const void*)d_x || A->graph_mixed != graph_kind ||
-      (mixed && A->graph_b != (const void*)d_b)) {
-    if (A->graph) { cudaGraphExecDestroy(A->graph); A->graph = nullptr; }
-    struct Graphs {
-      cudaGraph_t round = nullptr, pause = nullptr, loop = nullptr;
-      ~Graphs() {
-        if (round) cudaGraphDestroy(round);
-        if (pause) cudaGraphDestroy(pause);
-        if (loop) cudaGraphDestroy(loop);
-      }
-    } G;
-    // one round: `chunk` iterations
-    MSG_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < chunk; ++k) {
-      if (mixed) {
-        launch_pcgm_spmv(ctx, m, A->d_val32.as<float>(), p32, r32, dinv32, q32, pa, st, s);
-        k_pcgm_update<<<grid_u, kPcgThreads, 0, s>>>(n, dinv32, r32, p32, q32, d32, pa, st);
-      } else {
-        launch_pcg_dir_spmv(ctx, m, A->d_val.as<double>(), A->d_dinv.as<double>(), A->d_r.as<double>(),
-                            A->d_p0.as<double>(), A->d_p1.as<double>(), A->d_q.as<double>(), pa, st, s);
-        k_pcg_update<<<grid_u, kPcgThreads, 0, s>>>(nr, A->d_dinv.as<double>(), A->d_r.as<double>(), d_x,
-                                                    A->d_p0.as<double>(), A->d_p1.as<double>(), A->d_q.as<double>(),
-                                                    pa, st);
-      }
-    }
-    MSG_CUDA(ctx, cudaStreamEndCapture(s, &G.round));
-    if (mixed) {
-      // the pause: x += d in FP64, y = K x, the true residual (resume or stop)
-      MSG_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      k_pcgm_fold<<<grid_v, kPcgThreads, 0, s>>>(n, d_x, d32);
-      k_bsr_spmv3<<<m->pat.n_slices, 96, 0, s>>>(nr, m->d_slice_ptr.as<int64_t>(), m->d_col.as<int>(),
-                                                  A->d_val.as<double>(), d_x, A->d_tmp.as<double>());
-      k_pcgm_true<<<grid_v, kPcgThreads, 0, s>>>(n, d_b, A->d_tmp.as<double>(), dinv32, r32, pa, st);
-      MSG_CUDA(ctx, cudaStreamEndCapture(s, &G.pause));
-    }
-    MSG_CUDA(ctx, cudaGraphCreate(&G.loop, 0));
-    cudaGraphConditionalHandle h_while = 0, h_if = 0;
-    MSG_CUDA(ctx, cudaGraphConditionalHandleCreate(&h_while, G.loop, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams wp = {};
-    wp.type = cudaGraphNodeTypeConditional;
-    wp.conditional.handle = h_while;
-    wp.conditional.type = cudaGraphCondTypeWhile;
-    wp.conditional.size = 1;
-    cudaGraphNode_t wn = nullptr, last = nullptr;
-    MSG_CUDA(ctx, cudaGraphAddNode(&wn, G.loop, nullptr, 0, &wp));
-    cudaGraph_t body = wp.conditional.phGraph_out[0];
-    MSG_CUDA(ctx, cudaGraphAddChildGraphNode(&last, body, nullptr, 0, G.round));
-    auto add_kernel = [&](void* fn, void** args) -> int {
-      cudaKernelNodeParams kp = {};
-      kp.func = fn;
-      kp.gridDim = dim3(1);
-      kp.blockDim = dim3(1);
-      kp.kernelParams = args;
-      cudaGraphNode_t kn = nullptr;
-      MSG_CUDA(ctx, cudaGraphAddKernelNode(&kn, body, &last, 1, &kp));
-      last = kn;
-      return MSG_OK;
-    };
-    if (mixed) {
-      MSG_CUDA(ctx, cudaGraphConditionalHandleCreate(&h_if, body, 0, 0));
-      void* a_if[] = {&st, &h_if};
-      MSG_TRY(add_kernel((void*)k_pcg_loop_if, a_if));
-      cudaGraphNodeParams ip = {};
-      ip.type = cudaGraphNodeTypeConditional;
-      ip.conditional.handle = h_if;
-      ip.conditional.type = cudaGraphCondTypeIf;
-      ip.conditional.size = 1;
-      cudaGraphNode_t in = nullptr, pn = nullptr;
-      MSG_CUDA(ctx, cudaGraphAddNode(&in, body, &last, 1, &ip));
-      MSG_CUDA(ctx, cudaGraphAddChildGraphNode(&pn, ip.conditional.phGraph_out[0], nullptr, 0, G.pause));
-      last = in;
-    }
-    int chunk_arg = chunk;
-    void* a_while[] = {&st, &h_while, &chunk_arg};
-    MSG_TRY(add_kernel((void*)k_pcg_loop_while, a_while));
-    cudaError_t e = cudaGraphInstantiate(&A->graph, G.loop, 0);
-    if (e != cudaSuccess) {
-      A->graph = nullptr;
-      return cuda_error(ctx, e, "cudaGraphInstantiate");
-    }
-    A->graph_chunk = chunk;
-    A->graph_x = d_x;
-    A->graph_b = d_b;
-    A->graph_mixed = graph_kind;
-  }
-  MSG_CUDA(ctx, cudaMemsetAsync(&st->rounds, 0, 2 * sizeof(int), s));  // rounds, pauses
-  {
-    cudaError_t e = cudaGraphLaunch(A->graph, s);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "cudaGraphLaunch");
-  }
-  if (mixed) {  // a correction left by a solve that ended without a true residual
-    k_pcgm_fold<<<grid_v, kPcgThreads, 0, s>>>(n, d_x, d32);
-    count_launch(ctx);
-  }
-  MSG_CUDA(ctx, cudaGetLastError());
   PcgState hs;
-  MSG_CUDA(ctx, cudaMemcpyAsync(&hs, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
-  MSG_CUDA(ctx, cudaStreamSynchronize(s));
-  count_launch(ctx, hs.rounds * (2 * chunk + (mixed ? 2 : 1)) + 3 * hs.pauses);
+  MSG_TRY(pcg_finish(ctx, st, &hs, s));
   if (iterations) *iterations = hs.iterations;
   if (rel_res) *rel_res = hs.err;
-  if (status) *status = hs.done ? hs.status : MSG_ERR_NOT_CONVERGED;
+  if (status) *status = hs.status;
   return MSG_OK;
 }
 
 // ------------------------------------------------------------------ PCG without allocation
 // Scratch of MSG_PCG_SOLVE_NOALLOC: a fixed array in device memory, so the call
-// needs no cudaMalloc. Sized for meshes of up to kNoAllocMaxNodes nodes: six
-// node-layout FP64 vectors (b, x, r, two search directions, K p), the per-CTA
-// partial sums and the scalar state, about 9.5 MB. Every GPU that loads the
+// needs no cudaMalloc. Sized for meshes of up to kNoAllocMaxNodes nodes: seven
+// node-layout FP64 vectors (b, x, r, z, two search directions, K p), the CTAs'
+// partial sums and the scalar state, about 11 MB. Every GPU that loads the
 // library holds this array until the process exits.
 constexpr int kNoAllocMaxNodes = 65536;
 constexpr size_t kNoAllocVecBytes = sizeof(double) * 3 * (size_t)kNoAllocMaxNodes;
-constexpr size_t kNoAllocPartials = 2 * 4096;  // >= max(2 * update CTAs, slices of 65536 nodes)
-constexpr size_t kNoAllocStateOff = 6 * kNoAllocVecBytes + sizeof(double) * kNoAllocPartials;
-constexpr size_t kNoAllocBytes = kNoAllocStateOff + 256;
-static_assert(sizeof(PcgState) <= 256, "the scalar state fits its slot of the scratch");
+constexpr size_t kNoAllocBytes = 7 * kNoAllocVecBytes + sizeof(double) * 2 * kPcgSums * kPcgMaxCtas * 256 + 256;  // up to 256 SMs
+static_assert(sizeof(PcgState) <= 256, "the scalar state fits its slot");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -995,8 +1061,8 @@ using namespace msg;
 // The device Jacobi-PCG of MSG_PCG_SOLVE, for callers that must not allocate
 // device memory during the solve: the solve's working vectors live in the
 // fixed scratch array above instead of buffers from cudaMalloc, and the
-// right-hand side and solution are the caller's device buffers. Kernels and
-// their order are those of MSG_PCG_SOLVE, launched one by one.
+// right-hand side and solution are the caller's device buffers. The kernel and
+// its launch shape are MSG_PCG_SOLVE's.
 extern "C" int MSG_PCG_SOLVE_NOALLOC(MSG_MAT A, const double* b_dev, double* x_dev, int max_it, double tol,
                                      int* iterations, double* rel_res) {
   if (!A || !b_dev || !x_dev || max_it <= 0 || !(tol > 0)) return MSG_ERR_INVALID_ARGUMENT;
@@ -1014,37 +1080,20 @@ extern "C" int MSG_PCG_SOLVE_NOALLOC(MSG_MAT A, const double* b_dev, double* x_d
   const size_t n = 3 * (size_t)nr;
   double* bn = reinterpret_cast<double*>(base);
   double* xn = reinterpret_cast<double*>(base + kNoAllocVecBytes);
-  double* r = reinterpret_cast<double*>(base + 2 * kNoAllocVecBytes);
-  double* p0 = reinterpret_cast<double*>(base + 3 * kNoAllocVecBytes);
-  double* p1 = reinterpret_cast<double*>(base + 4 * kNoAllocVecBytes);
-  double* q = reinterpret_cast<double*>(base + 5 * kNoAllocVecBytes);
-  double* partial = reinterpret_cast<double*>(base + 6 * kNoAllocVecBytes);
-  PcgState* st = reinterpret_cast<PcgState*>(base + kNoAllocStateOff);
+  double* v[5];  // r, z, p (two), q
+  for (int i = 0; i < 5; ++i) v[i] = reinterpret_cast<double*>(base + (2 + i) * kNoAllocVecBytes);
+  void* head = base + 7 * kNoAllocVecBytes;
+  if (ctx->sm_count > 256) return set_error(ctx, MSG_ERR_INVALID_ARGUMENT, "MSG_PCG_SOLVE_NOALLOC: device too large");
+  PcgState* st = pcg_state(ctx, head);
   cudaStream_t s = ctx->stream;
   // the array keeps the previous call's contents: clear what must start at zero
   MSG_CUDA(ctx, cudaMemsetAsync(bn, 0, sizeof(double) * n, s));
-  MSG_CUDA(ctx, cudaMemsetAsync(st, 0, sizeof(PcgState), s));
   MSG_TRY(launch_dof_to_node(ctx, m, b_dev, bn, 1, 0, 0));
-  const int grid_v = std::min(4096, std::max(1, std::min((int)((n + kPcgThreads - 1) / kPcgThreads), ctx->sm_count * 8)));
-  k_pcg_init<<<grid_v, kPcgThreads, 0, s>>>(nr, bn, A->d_dinv.as<double>(), r, xn, p0, p1, partial, st);
-  count_launch(ctx);
-  MSG_CUDA(ctx, cudaMemcpyAsync(&st->tol, &tol, sizeof(double), cudaMemcpyHostToDevice, s));
-  MSG_CUDA(ctx, cudaMemcpyAsync(&st->max_it, &max_it, sizeof(int), cudaMemcpyHostToDevice, s));
-  int done = 0;
-  for (int it = 0; it < max_it + 8 && !done; it += 8) {
-    for (int k = 0; k < 8; ++k) {
-      launch_pcg_dir_spmv(ctx, m, A->d_val.as<double>(), A->d_dinv.as<double>(), r, p0, p1, q, partial, st, s);
-      k_pcg_update<<<grid_v, kPcgThreads, 0, s>>>(nr, A->d_dinv.as<double>(), r, xn, p0, p1, q, partial, st);
-    }
-    count_launch(ctx, 16);
-    MSG_CUDA(ctx, cudaMemcpyAsync(&done, &st->done, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MSG_CUDA(ctx, cudaStreamSynchronize(s));
-  }
-  MSG_CUDA(ctx, cudaGetLastError());
+  MSG_TRY(pcg_launch(ctx, m, A->d_val.as<double>(), bn, A->d_dinv.as<double>(), xn, v[0], v[1], v[2], v[3], v[4],
+                     head, tol, max_it, s));
   MSG_TRY(launch_node_to_dof(ctx, m, xn, x_dev, 1, 0, 0));
   PcgState hs;
-  MSG_CUDA(ctx, cudaMemcpyAsync(&hs, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
-  MSG_CUDA(ctx, cudaStreamSynchronize(s));
+  MSG_TRY(pcg_finish(ctx, st, &hs, s));
   if (iterations) *iterations = hs.iterations;
   if (rel_res) *rel_res = hs.err;
   if (hs.status != MSG_OK)

@@ -62,10 +62,6 @@ int DevMem::alloc(Context* c, size_t n) {
   return MSG_OK;
 }
 
-Matrix::~Matrix() {
-  if (graph) cudaGraphExecDestroy(graph);
-}
-
 Context::~Context() {
   delete static_cast<msg_matrix*>(mc_matrix);
   delete mc_ke;

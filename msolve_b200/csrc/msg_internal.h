@@ -106,7 +106,7 @@ struct Context {
   int mg_packed = 1;            // 1: level-0 operator with two realizations per lane (packed FP32)
   int mg_fused_coarse = 1;      // 1: all coarsest-level sweeps in one launch (when the level fits a CTA)
   int tensor_op = 0;            // 1: the multigrid loop's level-0 search-direction launch on the tensor cores
-  int spmv32_shape = 0;         // launch shape of the mixed assembled loop's FP32 SpMV (slots per group, slices per CTA)
+  int spmv32_shape = 0;         // accepted, of no effect (the mixed solve's launch shape follows from the matrix)
   int element_batch = 1;        // mixed mode on non-lattice meshes: 1 batched element-by-element loop, 0 per realization
   int element_groups = 0;       // realization groups of 32 per CTA of the element-by-element FP32 operator (0 auto)
   int ragged_lattice_loop = 1;  // ragged batches: cube lattices through the lattice loop (1) or the shared loop (0)
@@ -279,20 +279,12 @@ struct Mesh {
   std::mutex shadow_mu;
 };
 
+// How a device PCG solve ended, and the arrival counter of its grid-wide sums
+// (cleared before the launch; done stays 0 when their bounded wait expired).
 struct PcgState {
-  double zr, pq, rr, bnorm, alpha, beta, err;
-  // need (mixed precision) follows done: the host reads both as one pair
-  int it, done, need, status, iterations, matvecs, max_it;
-  double tol;
+  double err;
+  int status, iterations, matvecs, done;
   unsigned int counter;
-  // mixed precision (FP32 matrix values and vectors, FP64 iterate): the loop
-  // pauses (need = 1) when the recursive residual has dropped by delta since
-  // err_ref or below tol, and the host replaces it with the FP64 true residual
-  double delta, err_ref;
-  int mixed;
-  // rounds of the graph's device loop (chunks of iterations) and the FP64
-  // true-residual pauses among them
-  int rounds, pauses, pad;
 };
 
 struct Matrix {
@@ -301,15 +293,8 @@ struct Matrix {
   DevMem d_val32; // SELL values FP32 (mixed-precision solves; built on first use)
   DevMem d_bn, d_xn, d_bd;  // node-layout b and x, DOF-layout staging of the host entry points
   DevMem d_dinv;  // [n_nodes*3]
-  // PCG workspace (node layout, 3 per node)
-  DevMem d_r, d_p0, d_p1, d_q, d_partial, d_state, d_tmp, d_tmp2;
-  DevMem d_m32;  // mixed loop: FP32 r, q, d and D^-1 ([4][n_nodes*3]; p32 in d_tmp2)
-  cudaGraphExec_t graph = nullptr;
-  int graph_chunk = 0;
-  int graph_mixed = 0;
-  const void* graph_x = nullptr;  // output vector the captured graph writes (not owned)
-  const void* graph_b = nullptr;  // right-hand side its true-residual steps read (not owned)
-  ~Matrix();
+  DevMem d_work;  // PCG workspace: partial sums, state, vectors (node layout)
+
 };
 
 // Search vectors (p, K p) kept across solves for the re-orthogonalised PCG
