@@ -4091,7 +4091,7 @@ int pc_matvec(Context* ctx, Mesh* m, double nu, const MSG_KL* kl, int mo, int po
   k_pc_matvec<<<tx * ty * tz * P, kPcThreads, 0, st>>>(A, MCD);
   count_launch(ctx, 1);
   MSG_CUDA(ctx, cudaGetLastError());
-  MSG_CUDA(ctx, cudaMemcpyAsync(y_host, dy, sizeof(double) * nv, cudaMemcpyDeviceToHost, st));
+  MSG_TRY(copy_out(ctx, y_host, dy, sizeof(double) * nv, st));
   MSG_CUDA(ctx, cudaStreamSynchronize(st));
   return MSG_OK;
 }

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstring>
 #include <numeric>
+#include <thread>
 
 #include "msg_internal.h"
 
@@ -87,6 +88,9 @@ Context::~Context() {
   if (pipe_ready) cudaEventDestroy(pipe_ready);
   if (h_flags) cudaFreeHost(h_flags);
   if (h_stage) cudaFreeHost(h_stage);
+  if (h_copy) cudaFreeHost(h_copy);
+  for (auto& e : copy_ev)
+    if (e) cudaEventDestroy(e);
 }
 
 int context_resources(Context* ctx) {
@@ -116,6 +120,86 @@ int workspace(Context* ctx, int slot, size_t bytes, void** out) {
   if (w->bytes < bytes) MSG_TRY(w->alloc(ctx, bytes));
   *out = w->ptr;
   return MSG_OK;
+}
+
+// Device-to-host copies of outputs on stream st. Pageable memory is filled by a few
+// host threads, each through its own pair of pinned pieces: a plain copy is staged
+// by the driver on one thread, which also takes the page faults of an output that
+// was just allocated (3.8 GB/s; 92 MB of displacements in 20 ms, 6 ms here).
+// Complete on return then, otherwise (pinned or short outputs) enqueued on st.
+int copy_out(Context* ctx, const std::vector<HostCopy>& outs, cudaStream_t st) {
+  struct Piece {
+    char* dst;
+    const char* src;
+    size_t bytes;
+  };
+  std::vector<Piece> pieces;
+  size_t total = 0;
+  std::vector<int> staged(outs.size(), 0);
+  for (size_t i = 0; i < outs.size(); ++i) {
+    cudaPointerAttributes at{};
+    const bool known = cudaPointerGetAttributes(&at, outs[i].dst) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    staged[i] = !known || at.type == cudaMemoryTypeUnregistered;
+    if (staged[i]) total += outs[i].bytes;
+  }
+  const int threads = std::min<int>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency() / 2));
+  const bool pool_copy = total >= kCopyMin && threads > 1;
+  for (size_t i = 0; i < outs.size(); ++i) {
+    const HostCopy& o = outs[i];
+    if (!pool_copy || !staged[i]) {
+      if (o.bytes) MSG_CUDA(ctx, cudaMemcpyAsync(o.dst, o.src, o.bytes, cudaMemcpyDeviceToHost, st));
+      continue;
+    }
+    for (size_t at = 0; at < o.bytes; at += kCopyPiece)
+      pieces.push_back({static_cast<char*>(o.dst) + at, static_cast<const char*>(o.src) + at,
+                        std::min(kCopyPiece, o.bytes - at)});
+  }
+  if (pieces.empty()) return MSG_OK;
+  // pinned pieces and their events, kept in the context
+  if (!ctx->h_copy) MSG_CUDA(ctx, cudaMallocHost(&ctx->h_copy, 2 * kCopyThreads * kCopyPiece));
+  for (auto& e : ctx->copy_ev)
+    if (!e) MSG_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  std::atomic<int> failed{cudaSuccess};
+  auto work = [&](int t) {
+    cudaError_t e = cudaSetDevice(ctx->device);
+    const Piece* held[2] = {nullptr, nullptr};  // piece in each of this thread's buffers
+    auto buffer = [&](int k) { return ctx->h_copy + (size_t)(2 * t + k) * kCopyPiece; };
+    auto take = [&](int k) {  // the buffer's piece goes to its place
+      if (!held[k] || e != cudaSuccess) return;
+      e = cudaEventSynchronize(ctx->copy_ev[2 * t + k]);
+      if (e == cudaSuccess) std::memcpy(held[k]->dst, buffer(k), held[k]->bytes);
+      held[k] = nullptr;
+    };
+    int k = 0;
+    for (size_t p = t; p < pieces.size() && e == cudaSuccess; p += threads, k ^= 1) {
+      take(k);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(buffer(k), pieces[p].src, pieces[p].bytes, cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaEventRecord(ctx->copy_ev[2 * t + k], st);
+      held[k] = &pieces[p];
+    }
+    take(k);
+    take(k ^ 1);
+    if (e != cudaSuccess) failed = e;
+  };
+  std::vector<std::thread> pool;
+  int started = 1;
+  try {
+    for (; started < threads; ++started) pool.emplace_back(work, started);
+  } catch (...) {  // threads that cannot start: their share is done here
+  }
+  work(0);
+  for (int t = started; t < threads; ++t) work(t);
+  for (std::thread& t : pool) t.join();
+  if (failed != cudaSuccess) {
+    cudaStreamSynchronize(st);  // no copy into the pieces is left in flight
+    return cuda_error(ctx, static_cast<cudaError_t>(failed.load()), "copy of the outputs");
+  }
+  return MSG_OK;
+}
+
+int copy_out(Context* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  return copy_out(ctx, {{dst, src, bytes}}, st);
 }
 
 void retain(Context* ctx) { ctx->refs++; }
@@ -847,7 +931,7 @@ int MSG_H8_KE_BATCH(MSG_CTX ctx, int n, const double* xyz, const double* E, doub
   MSG_CUDA(ctx, cudaMemsetAsync(ds.ptr, 0, sizeof(int), ctx->stream));
   MSG_TRY(launch_h8_ke(ctx, n, dx.as<double>(), dE.as<double>(), 0.0, nu, dK.as<double>(), ds.as<int>()));
   int st = 0;
-  MSG_CUDA(ctx, cudaMemcpyAsync(Ke, dK.ptr, sizeof(double) * 300 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+  MSG_TRY(copy_out(ctx, Ke, dK.ptr, sizeof(double) * 300 * (size_t)n, ctx->stream));
   MSG_CUDA(ctx, cudaMemcpyAsync(&st, ds.ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   MSG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st != 0) return set_error(ctx, st, "negative or tiny Jacobian determinant (H8)");
@@ -865,7 +949,7 @@ int MSG_H8_ME_BATCH(MSG_CTX ctx, int n, const double* xyz, double rho, double* M
   MSG_CUDA(ctx, cudaMemsetAsync(ds.ptr, 0, sizeof(int), ctx->stream));
   MSG_TRY(launch_h8_me(ctx, n, dx.as<double>(), rho, dM.as<double>(), ds.as<int>()));
   int st = 0;
-  MSG_CUDA(ctx, cudaMemcpyAsync(Me, dM.ptr, sizeof(double) * 300 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+  MSG_TRY(copy_out(ctx, Me, dM.ptr, sizeof(double) * 300 * (size_t)n, ctx->stream));
   MSG_CUDA(ctx, cudaMemcpyAsync(&st, ds.ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   MSG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st != 0) return set_error(ctx, st, "negative or tiny Jacobian determinant (H8)");
@@ -893,12 +977,11 @@ int MSG_H8_STRESS_BATCH(MSG_CTX ctx, int n, const double* xyz, const double* E, 
                            dT.as<double>(), dF.as<double>(), ds.as<int>()));
   int st = 0;
   if (strains)
-    MSG_CUDA(ctx, cudaMemcpyAsync(strains, dS.ptr, sizeof(double) * 48 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+    MSG_TRY(copy_out(ctx, strains, dS.ptr, sizeof(double) * 48 * (size_t)n, ctx->stream));
   if (stresses)
-    MSG_CUDA(ctx, cudaMemcpyAsync(stresses, dT.ptr, sizeof(double) * 48 * (size_t)n, cudaMemcpyDeviceToHost,
-                                  ctx->stream));
+    MSG_TRY(copy_out(ctx, stresses, dT.ptr, sizeof(double) * 48 * (size_t)n, ctx->stream));
   if (forces)
-    MSG_CUDA(ctx, cudaMemcpyAsync(forces, dF.ptr, sizeof(double) * 24 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+    MSG_TRY(copy_out(ctx, forces, dF.ptr, sizeof(double) * 24 * (size_t)n, ctx->stream));
   MSG_CUDA(ctx, cudaMemcpyAsync(&st, ds.ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   MSG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (st != 0) return set_error(ctx, st, "negative or tiny Jacobian determinant (H8)");
@@ -1218,7 +1301,7 @@ int MSG_KL_FIELD(MSG_MESH m, const MSG_KL* kl, int R, const double* xi, double* 
   MSG_TRY(upload(ctx, dxi, xi, (size_t)R * kl->n_terms));
   MSG_TRY(dE.alloc(ctx, sizeof(double) * (size_t)R * m->n_elems));
   MSG_TRY(launch_kl_field(ctx, m, &kd, R, Rp, dxi.as<double>(), nullptr, nullptr, dE.as<double>()));
-  MSG_CUDA(ctx, cudaMemcpyAsync(E, dE.ptr, sizeof(double) * (size_t)R * m->n_elems, cudaMemcpyDeviceToHost, ctx->stream));
+  MSG_TRY(copy_out(ctx, E, dE.ptr, sizeof(double) * (size_t)R * m->n_elems, ctx->stream));
   MSG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return MSG_OK;
 }
@@ -1249,7 +1332,7 @@ int MSG_MC_SOLVE_BATCH(MSG_MESH m, double nu, const MSG_KL* kl, int R, const dou
                     X ? static_cast<double*>(dX) : nullptr, tip, iterations, rel_res);
   // per-realization outcomes (not converged, breakdown): the other realizations' results are valid
   if (X && (st == MSG_OK || st == MSG_ERR_NOT_CONVERGED || st == MSG_ERR_BREAKDOWN)) {
-    MSG_CUDA(ctx, cudaMemcpyAsync(X, dX, sizeof(double) * (size_t)R * m->n_dofs, cudaMemcpyDeviceToHost, ctx->stream));
+    MSG_TRY(copy_out(ctx, X, dX, sizeof(double) * (size_t)R * m->n_dofs, ctx->stream));
     MSG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
   return st;
@@ -1415,11 +1498,11 @@ int MSG_MC_SOLVE_RAGGED(MSG_CTX ctx, int n_systems, const MSG_RAGGED_SYSTEM* sys
     const int st = ebe_solve(ctx, in, max_it, tol);
     if (!outcome(st)) return st;
   }
+  std::vector<HostCopy> outs;
   for (int i = 0; i < n_systems; ++i)
     if (systems[i].X)
-      MSG_CUDA(ctx, cudaMemcpyAsync(systems[i].X, base + off[3 * i + 2],
-                                    sizeof(double) * (size_t)systems[i].R * systems[i].mesh->n_dofs,
-                                    cudaMemcpyDeviceToHost, ctx->stream));
+      outs.push_back({systems[i].X, base + off[3 * i + 2], sizeof(double) * (size_t)systems[i].R * systems[i].mesh->n_dofs});
+  MSG_TRY(copy_out(ctx, outs, ctx->stream));
   cudaEventRecord(e1, ctx->stream);
   cudaEventSynchronize(e1);
   float ms = 0;
@@ -1466,7 +1549,7 @@ int MSG_NEWMARK_BATCH(MSG_MESH m, double nu, const MSG_KL* kl, int R, const doub
   int st = block_newmark(ctx, m, nu, &kd, static_cast<double*>(dxi), R, Rp, p, static_cast<double*>(df), max_it, tol,
                          tip_dof, tip_hist, static_cast<double*>(dU), iterations);
   if (U && st == MSG_OK) {
-    MSG_CUDA(ctx, cudaMemcpyAsync(U, dU, sizeof(double) * (size_t)R * m->n_dofs, cudaMemcpyDeviceToHost, ctx->stream));
+    MSG_TRY(copy_out(ctx, U, dU, sizeof(double) * (size_t)R * m->n_dofs, ctx->stream));
     MSG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
   cudaEventRecord(e1, ctx->stream);

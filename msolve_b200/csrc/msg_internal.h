@@ -53,6 +53,12 @@ inline int gmg_level_count(int nx, int ny, int nz, int max_levels) {
   return n;
 }
 
+// Outputs copied to pageable host memory (copy_out): host threads, bytes of a
+// pinned piece (two a thread), and the shortest outputs they are worth it for
+// (1.7 MB: 0.14 ms more than a plain copy, the threads' start).
+constexpr int kCopyThreads = 8;
+constexpr size_t kCopyPiece = (size_t)512 << 10, kCopyMin = (size_t)8 << 20;
+
 struct Context;
 
 // Device allocation charged against the context's memory budget.
@@ -130,6 +136,8 @@ struct Context {
   int* h_flags = nullptr;           // 4 KB of pinned host memory, mapped into the device
   int* d_hflags = nullptr;          // the device's address of h_flags
   double* h_stage = nullptr;        // 8 KB of pinned host memory: small uploads issued as true async copies
+  char* h_copy = nullptr;           // pinned pieces of copy_out (8 MB, on the first large output)
+  cudaEvent_t copy_ev[2 * kCopyThreads] = {nullptr};
   // unit-cube element matrices already computed (kind 0: stiffness at E = 1
   // for (h, nu); 1: consistent mass for (h, rho)): later batches read no
   // device data and free no device memory while setting up
@@ -176,6 +184,14 @@ int context_resources(Context* ctx);
 
 // Workspace slot `slot` of at least `bytes` bytes (grown, never shrunk).
 int workspace(Context* ctx, int slot, size_t bytes, void** out);
+// Device-to-host copies of outputs on stream st (synchronise st after it).
+struct HostCopy {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+int copy_out(Context* ctx, const std::vector<HostCopy>& outs, cudaStream_t st);
+int copy_out(Context* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);
 // Waits for every displacement copy of the pipelined batches still in flight.
 int pipe_flush(Context* ctx);
 // h_host[0 .. n) = d_src[0 .. n) on stream st, written by a one-block kernel
