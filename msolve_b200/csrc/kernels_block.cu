@@ -15,7 +15,7 @@
 // checks. A warp is 32 realizations of one node: every access is one coalesced
 // 128-byte line and per-realization dot products need no cross-lane reduction.
 //
-// Operator kernels (k_op_modal, k_lvl_op, k_lvl_op2, k_resid_modal): a CTA owns
+// Operator kernels (k_jacobi_op, k_lvl_op, k_lvl_op2, k_resid_modal): a CTA owns
 // a tile of node pencils along x and walks the x-planes, staging each plane's
 // patch with TMA; the element product is applied in the element's Walsh modes
 // (below), and the four elements around a node meet in a shared-memory
@@ -23,7 +23,7 @@
 // results are deterministic and independent of the batch mix. k_lvl_tc applies
 // the same product on the tensor cores (option "tensor_operator").
 //
-// Solvers: the single-reduction FP32 Jacobi-PCG loop (k_op_modal +
+// Solvers: the single-reduction FP32 Jacobi-PCG loop (k_jacobi_op +
 // k_alpha_gamma per iteration) and the multigrid-preconditioned loop
 // (gmg_iteration), each captured as one CUDA graph of `chunk` iterations, with
 // reliable updates in FP64: x += d + alpha p (the pending term), d = 0,
@@ -299,26 +299,18 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* tm, in
 // per axis (sum and difference of two values), and the yz part of a plane
 // is shared by the elements on both sides of it along x.
 //
-// A CTA owns a 3 x 3 tile of node pencils for 32 realizations and runs one
-// warp per element pencil of the 4 x 4 that touch it (the tile's own
-// elements plus one halo row and column below; the 7 halo pencils are also
-// computed by the neighbouring CTA). Per x-plane P every element warp turns
-// its 4 plane nodes into 4 yz-modes per component, combines them with the
-// previous plane's modes into the element's 24 modes, applies the blocks,
-// and folds the result back onto the yz-modes of planes P-1 and P; the P-1
-// part completes that plane and goes back to its 4 corner nodes. The corner
-// contributions meet in a shared-memory exchange buffer, where the warp that
-// owns node pencil (J, K) sums the four elements around it in fixed order,
-// so results stay deterministic. About 150 FP32 operations per element and
-// plane instead of the 576 FMAs of a dense Khat row block per node. The
-// output is not masked here: constrained components of p are zero, so p.q
-// is unaffected, and k_update leaves the constrained components of r at zero.
-//
-// The kernel is persistent (one CTA per SM walks work items, a tile and a
-// realization group each), with a dedicated TMA producer warp filling the
-// same 4-stage mbarrier ring as the dense operator, and an mbarrier (bounded
-// waits, like every other wait here) in place of a CTA barrier between the
-// element and node phases of a plane.
+// A CTA owns a tile of node pencils for a group of realizations (7 x 3 for 16:
+// k_lvl_op2, k_jacobi_op) and computes every element pencil that touches it (the
+// tile's own elements plus one halo row and column below, which the neighbouring
+// CTA computes too). Per x-plane P an element pencil's lanes turn its 4 plane
+// nodes into 4 yz-modes per component, combine them with the previous plane's
+// modes into the element's 24 modes, apply the blocks, and fold the result back
+// onto the yz-modes of planes P-1 and P; the P-1 part completes that plane and
+// goes back to its 4 corner nodes. The corner contributions meet in a
+// shared-memory exchange buffer, where the lanes that own node pencil (J, K) sum
+// the four elements around it in fixed order, so results stay deterministic.
+// About 150 FP32 operations per element and plane instead of the 576 FMAs of a
+// dense Khat row block per node.
 template <class T> struct ModalCT {
   T vd, vb;  // V: a - b, b
   T sa, sb;  // S: a, b
@@ -350,17 +342,9 @@ constexpr int kMPlaneFloats = 32 * 3 * kMPJ * kMPK;   // r, q or p patch of a pl
 constexpr int kMNodeFloats = 32 * kMPJ * kMPK;        // dinv patch: 800
 constexpr int kMEFloats = 32 * kMEJ * kMEK;           // E patch: 512
 constexpr int kMDFloats = 32 * 3 * kMJ * kMK;         // d of the tile's own nodes: 864
-// stage: r | q | p | dinv | E | d (each patch a multiple of 128 bytes)
-constexpr int kMOffR = 0, kMOffQ = kMPlaneFloats, kMOffP = 2 * kMPlaneFloats, kMOffDinv = 3 * kMPlaneFloats;
-constexpr int kMOffE = kMOffDinv + kMNodeFloats, kMOffD = kMOffE + kMEFloats;
-constexpr int kMStageFloats = kMOffD + kMDFloats;     // 9,376 floats, 37,504 bytes
-constexpr uint32_t kMStageBytes = kMStageFloats * 4;
 constexpr int kMStages = 3;
 constexpr int kMXFloats = kMWarps * 4 * 3 * 32;       // exchange buffer: element x corner x component x lane
 constexpr int kMThreads = 32 * (kMWarps + 1);         // + 1 TMA producer warp
-constexpr size_t kMSmem = 128 + sizeof(float) * ((size_t)kMStages * kMStageFloats + 2 * (size_t)kMXFloats) +
-                          sizeof(double) * 4 * kMJ * kMK * 32 + sizeof(uint64_t) * (2 * kMStages);
-static_assert(kMSmem <= 227 * 1024, "modal operator shared memory");
 
 // yz transform of one plane's 4 nodes u[ay][az] into the modes B[my + 2 mz]
 template <class T>
@@ -583,237 +567,11 @@ __global__ void __launch_bounds__(kPcThreads, 2) k_pc_matvec(PcArgs A, const __g
   }
 }
 
-// One whole inner PCG iteration per launch (single-reduction form). Launch k+1
-// receives r_k, q_k = K p_k, p_k, alpha_k and beta_{k+1} and, at every node,
-//   r_{k+1} = r_k - alpha_k q_k,  p_{k+1} = dinv r_{k+1} + beta_{k+1} p_k,
-//   d += alpha_k p_k (the FP32 solution correction),
-// then q_{k+1} = K p_{k+1} (masked) with the partials p.q, (dinv r).q,
-// q.dinv.q and (dinv r).r of p_{k+1}, r_{k+1}, q_{k+1}. The scalar kernel that
-// follows forms alpha_{k+1} = gamma_{k+1} / p.q from the gamma of r_{k+1}
-// itself and the next gamma by the expansion of (dinv r_{k+2}).r_{k+2},
-//   gamma_{k+2} = gamma_{k+1} - 2 alpha (dinv r).q + alpha^2 q.dinv.q,
-// so r never needs a pass of its own (and the expansion never runs for more
-// than one step, which keeps the FP32 iteration count of the two-pass loop). Each stage carries the plane's r, q, p and dinv patches with halo (and
-// the tile's d); the element warps form p_{k+1} at their corners on the fly,
-// and the owner of a node pencil writes r, p and d back. r, q and p each have
-// a second buffer: neighbouring CTAs still read the old values in their halos.
-constexpr int kMParts = 4;  // partials per realization and tile: p.q, (dinv r).q, q.dinv.q, (dinv r).r
-template <bool kMass>
-__global__ void __launch_bounds__(kMThreads, 1)
-    k_op_modal(Lattice L, const __grid_constant__ ModalC C, const __grid_constant__ CUtensorMap tm_r,
-               const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_p,
-               const __grid_constant__ CUtensorMap tm_dinv, const __grid_constant__ CUtensorMap tm_e,
-               const __grid_constant__ CUtensorMap tm_d, int tiles_j, int n_tiles, int n_items,
-               const uint8_t* __restrict__ mask, const float* __restrict__ alpha, const float* __restrict__ beta,
-               float* __restrict__ r_out, float* __restrict__ p_out, float* __restrict__ q_out, float* __restrict__ d,
-               double* __restrict__ partial, int* __restrict__ err) {
-  extern __shared__ __align__(128) float smem_dyn[];
-  float* smem = smem_dyn + (((128u - (smem_u32(smem_dyn) & 127u)) & 127u) >> 2);
-  float* xbuf = smem + kMStages * kMStageFloats;                            // 2 exchange buffers
-  double* red = reinterpret_cast<double*>(xbuf + 2 * kMXFloats);            // [parts][node pencils][32]
-  uint64_t* full = reinterpret_cast<uint64_t*>(red + kMParts * kMJ * kMK * 32);
-  uint64_t* empty = full + kMStages;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int NX = L.NX, Rp = L.Rp;
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < kMStages; ++st) {
-      mbar_init(&full[st], 1);
-      mbar_init(&empty[st], kMWarps);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (w == kMWarps) {
-    // producer: plane P of every work item, in the consumers' order
-    if (lane == 0) {
-      uint32_t seq = 0;
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-        const int tile = item % n_tiles, g32 = (item / n_tiles) * 32;
-        const int J0 = 1 + (tile % tiles_j) * kMJ, K0 = 1 + (tile / tiles_j) * kMK;
-        for (int P = 1; P <= NX; ++P, ++seq) {
-          const int st = seq % kMStages;
-          const uint32_t use = seq / kMStages;
-          if (use > 0 && !mbar_wait(&empty[st], (use - 1) & 1)) {
-            atomicExch(err, 1);
-            return;
-          }
-          float* dst = smem + st * kMStageFloats;
-          mbar_expect_tx(&full[st], kMStageBytes);
-          tma_load_5d(dst + kMOffR, &tm_r, g32, 0, P, J0 - 1, K0 - 1, &full[st]);
-          tma_load_5d(dst + kMOffQ, &tm_q, g32, 0, P, J0 - 1, K0 - 1, &full[st]);
-          tma_load_5d(dst + kMOffP, &tm_p, g32, 0, P, J0 - 1, K0 - 1, &full[st]);
-          tma_load_4d(dst + kMOffDinv, &tm_dinv, g32, P, J0 - 1, K0 - 1, &full[st]);
-          tma_load_4d(dst + kMOffE, &tm_e, g32, P - 1, J0 - 1, K0 - 1, &full[st]);
-          tma_load_5d(dst + kMOffD, &tm_d, g32, 0, P, J0, K0, &full[st]);
-        }
-      }
-    }
-    return;
-  }
-  const int ej = w % kMEJ, ek = w / kMEJ;
-  const bool node_warp = ej >= 1 && ek >= 1;
-  uint32_t seq = 0;
-  int xsel = 0;
-  bool dead = false;  // a stage never arrived: finish the walk without data (err is set)
-  // barrier of the consumer warps between the element and the node phase of a
-  // plane; every consumer warp passes the same sequence of them, error or not
-  auto csync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kMWarps * 32) : "memory"); };
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int tile = item % n_tiles, g32 = (item / n_tiles) * 32;
-    const int J0 = 1 + (tile % tiles_j) * kMJ, K0 = 1 + (tile / tiles_j) * kMK;
-    const int Je = J0 - 1 + ej, Ke = K0 - 1 + ek;  // element pencil (lower corner), padded
-    // real elements have lower corners 1..NY-1 (1..NZ-1); others are ghosts
-    auto realj = [&](int j) { return j >= 1 && j <= L.NY - 1; };
-    auto realk = [&](int k) { return k >= 1 && k <= L.NZ - 1; };
-    const bool real = realj(Je) && realk(Ke);
-    const bool node_ok = node_warp && Je <= L.NY && Ke <= L.NZ;
-    const bool r00 = real, r10 = realj(Je - 1) && realk(Ke);
-    const bool r01 = realj(Je) && realk(Ke - 1), r11 = realj(Je - 1) && realk(Ke - 1);
-    const size_t nrow = ((size_t)Je + (size_t)L.NYp * Ke) * L.NXp;  // padded node (0, Je, Ke)
-    const int rr = g32 + lane;
-    const float al = alpha[rr], be = beta[rr];
-    float Bp[3][4], T0[3][4];
-    float op[3] = {0.f, 0.f, 0.f}, orr[3] = {0.f, 0.f, 0.f}, odv = 0.f;  // p, r, dinv at the own node
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int qq = 0; qq < 4; ++qq) T0[c][qq] = 0.f;
-    double acc_pq = 0.0, acc_zq = 0.0, acc_qq = 0.0, acc_zr = 0.0;
-    uint32_t mreg = 0;  // constraint bits of plane base + lane of the own pencil
-    // node phase of plane X: sum the corner contributions of the 4 elements
-    auto node_phase = [&](int X) {
-      if (((X - 1) & 31) == 0) {
-        const int pl = X + lane;
-        mreg = (pl <= NX) ? mask[nrow + pl] : 0u;
-      }
-      const uint32_t mk = __shfl_sync(0xffffffffu, mreg, (X - 1) & 31);
-      const float* xb = xbuf + xsel * kMXFloats;
-      const size_t node = nrow + X;
-      // products in FP64: a fast-converging realization drives r and q towards the
-      // bottom of the FP32 range, where FP32 squares would underflow
-      double spq = 0.0, szq = 0.0, sqq = 0.0, szr = 0.0;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        float y = 0.f;
-        if (r00) y += xb[((w * 4 + 0) * 3 + c) * 32 + lane];
-        if (r10) y += xb[(((w - 1) * 4 + 1) * 3 + c) * 32 + lane];
-        if (r01) y += xb[(((w - kMEJ) * 4 + 2) * 3 + c) * 32 + lane];
-        if (r11) y += xb[(((w - kMEJ - 1) * 4 + 3) * 3 + c) * 32 + lane];
-        y = ((mk >> c) & 1) ? 0.f : y;
-        q_out[(node * 3 + c) * Rp + rr] = y;
-        const double yd = (double)y, rd = (double)orr[c];
-        spq = fma((double)op[c], yd, spq);
-        szq = fma(rd, yd, szq);
-        sqq = fma(yd, yd, sqq);
-        szr = fma(rd, rd, szr);
-      }
-      const double dvd = (double)odv;
-      acc_pq += spq;
-      acc_zq += dvd * szq;
-      acc_qq += dvd * sqq;
-      acc_zr += dvd * szr;
-    };
-    auto emit_corners = [&](const float (&B)[3][4]) {
-      float y[2][2][3];
-      yz_inverse(B, y);
-      float* xb = xbuf + xsel * kMXFloats;
-#pragma unroll
-      for (int ay = 0; ay < 2; ++ay)
-#pragma unroll
-        for (int az = 0; az < 2; ++az)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) xb[((w * 4 + ay + 2 * az) * 3 + c) * 32 + lane] = y[ay][az][c];
-    };
-    for (int P = 1; P <= NX; ++P, ++seq) {
-      const int st = seq % kMStages;
-      if (!dead && !mbar_wait(&full[st], (seq / kMStages) & 1)) {
-        atomicExch(err, 1);
-        dead = true;
-      }
-      const float* pt = smem + st * kMStageFloats;
-      // p_{k+1} at the element's 4 plane corners: dinv (r - alpha q) + beta p_k
-      float u[2][2][3], rc[3], dvc = 0.f;
-#pragma unroll
-      for (int ay = 0; ay < 2; ++ay)
-#pragma unroll
-        for (int az = 0; az < 2; ++az) {
-          const int o = (ek + az) * kMPJ + (ej + ay);
-          const float dv = pt[kMOffDinv + o * 32 + lane];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const int i = (o * 3 + c) * 32 + lane;
-            const float rn = fmaf(-al, pt[kMOffQ + i], pt[kMOffR + i]);
-            u[ay][az][c] = fmaf(dv, rn, be * pt[kMOffP + i]);
-            if (ay == 0 && az == 0) rc[c] = rn;
-          }
-          if (ay == 0 && az == 0) dvc = dv;
-        }
-      const float E = pt[kMOffE + w * 32 + lane];  // element (P-1, Je, Ke)
-      if (node_ok) {
-        // the owner writes r_{k+1}, p_{k+1} and d += alpha_k p_k of node (P, Je, Ke)
-        const int o = ek * kMPJ + ej, od = (ek - 1) * kMJ + (ej - 1);
-        const size_t node = nrow + P;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const float pold = pt[kMOffP + (o * 3 + c) * 32 + lane];
-          const float dn = fmaf(al, pold, pt[kMOffD + (od * 3 + c) * 32 + lane]);
-          r_out[(node * 3 + c) * Rp + rr] = rc[c];
-          p_out[(node * 3 + c) * Rp + rr] = u[0][0][c];
-          d[(node * 3 + c) * Rp + rr] = dn;
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[st]);
-      float Bc[3][4];
-      yz_forward(u, Bc);
-      if (P >= 2) {
-        if (real) {
-          float C1[3][4];
-          modal_apply<kMass>(C, E, Bp, Bc, T0, C1);
-          emit_corners(T0);
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
-        }
-        csync();
-        if (node_ok) node_phase(P - 1);
-        xsel ^= 1;
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        op[c] = u[0][0][c];
-        orr[c] = rc[c];
-        odv = dvc;
-#pragma unroll
-        for (int qq = 0; qq < 4; ++qq) Bp[c][qq] = Bc[c][qq];
-      }
-    }
-    // plane NX: the slab above it is a ghost, so the pending part is complete
-    if (real) emit_corners(T0);
-    csync();
-    if (node_ok) node_phase(NX);
-    xsel ^= 1;
-    if (node_warp) {
-      const int nw = (ek - 1) * kMJ + (ej - 1);
-      red[(0 * kMJ * kMK + nw) * 32 + lane] = acc_pq;
-      red[(1 * kMJ * kMK + nw) * 32 + lane] = acc_zq;
-      red[(2 * kMJ * kMK + nw) * 32 + lane] = acc_qq;
-      red[(3 * kMJ * kMK + nw) * 32 + lane] = acc_zr;
-    }
-    csync();
-    if (w < kMParts) {
-      double sum = 0.0;
-#pragma unroll
-      for (int i = 0; i < kMJ * kMK; ++i) sum += red[(w * kMJ * kMK + i) * 32 + lane];
-      partial[((size_t)tile * Rp + rr) * kMParts + w] = sum;
-    }
-  }
-}
+constexpr int kMParts = 4;  // partials of the single-reduction loop: p.q, (dinv r).q, q.dinv.q, (dinv r).r
 
 // ---------------------------------------------------------------- multigrid level operator
 // The Walsh-mode operator of one lattice level (same tiling, TMA ring,
-// exchange buffer and bounded waits as k_op_modal), with the node phase of one
+// exchange buffer and bounded waits as described above), with the node phase of one
 // step of the multigrid-preconditioned loop:
 //   kLvlStart : level 0, first step of an iteration. Corner input
 //               x0 = omega dinv (r - alpha q) (the first Jacobi sweep from zero
@@ -1619,9 +1377,77 @@ constexpr int kQPencils = 32 / kQLanes;             // pencils per warp, along y
 constexpr int kQWarps = kQEJ * kQEK / kQPencils;    // 8 warps
 constexpr int kQThreads = 32 * kQWarps;
 constexpr int kQCtas = 2;                           // CTAs per SM
-constexpr int kQQuad = 64 / kQR;                    // items of one tile next to each other: 64 realizations, whole 256-byte rows
+constexpr int kQQuad = 64 / kQR;                    // items of one tile next to each other at most: 64 realizations, whole 256-byte rows
 constexpr int kQPJ = kQJ + 2, kQPK = kQK + 2;       // node patch 9 x 5
 static_assert(kQEJ % kQPencils == 0, "a warp's pencils lie in one row");
+// Work items of an operator launch: the planes of a tile of node pencils for a group
+// of realizations, whole (nseg = 1) or in segments of seg_len planes, which are
+// whole chunks. A segment walks one more plane on either side for the elements it
+// shares with its neighbours. Groups beyond the batch's last realization have no
+// items. Partial sums are per tile and chunk, and the chunks follow from the lattice
+// alone, so that a realization's sums do not depend on the batch it is in.
+// A plane costs about 1.3 us of latency however few CTAs there are, which is what
+// small batches pay for: 8^3 x 64 18.4 us a launch in whole walks, 12.3 in segments,
+// 16^3 x 20 28.7 and 14.4; 32^3 x 1024 is walked whole. Shorter chunks for long axes
+// gain nothing there (six at most: 16^3 x 20 16.1 us), and sums within the walk cost
+// 8 % of it, so that they are left in shared memory until its end.
+constexpr int kChunk = 2;       // planes of a chunk at least
+constexpr int kMaxChunks = 4;   // chunks of a lattice at most
+struct Walk {
+  int tiles_j, n_tiles, nseg, seg_len;
+  int chunk, n_chunk;  // planes of a chunk, chunks
+  uint32_t chunk_mul;  // ceil(2^32 / chunk): chunk_of without a division
+  __device__ __forceinline__ int chunk_of(int X) const { return (int)__umulhi((uint32_t)(X - 1), chunk_mul); }
+  int kq;       // realization groups whose items of one tile follow each other
+  int n_items;
+};
+struct WalkItem {
+  int tile, col, J0, K0;  // first realization, first node pencil
+  int a, b, p0, p1;       // node planes of the item, planes walked (1-based)
+};
+template <bool kSeg, int kTileJ, int kTileK, int kCols>
+__device__ __forceinline__ WalkItem walk_item(const Walk& W, int item, int NX) {
+  WalkItem I;
+  const int t = item / W.kq, u = kSeg ? t / W.nseg : t, quad = u / W.n_tiles;
+  I.tile = u - quad * W.n_tiles;
+  I.col = (quad * W.kq + (item - t * W.kq)) * kCols;
+  const int tk = I.tile / W.tiles_j;
+  I.J0 = 1 + (I.tile - tk * W.tiles_j) * kTileJ;
+  I.K0 = 1 + tk * kTileK;
+  I.a = I.p0 = 1;
+  I.b = I.p1 = NX;
+  if (kSeg) {
+    I.a = 1 + (t - u * W.nseg) * W.seg_len;
+    I.b = min(NX, I.a + W.seg_len - 1);
+    I.p0 = max(1, I.a - 1);
+    I.p1 = min(NX, I.b + 1);
+  }
+  return I;
+}
+// The segments that take the fewest rounds x planes on `slots` resident CTAs (two
+// planes more a segment, about 1.5 planes' time an item).
+inline Walk make_walk(int NX, int tiles_j, int n_tiles, int groups, int kq, int slots) {
+  Walk W;
+  W.tiles_j = tiles_j;
+  W.n_tiles = n_tiles;
+  W.kq = kq;
+  W.chunk = std::max(kChunk, (NX + kMaxChunks - 1) / kMaxChunks);
+  W.n_chunk = (NX + W.chunk - 1) / W.chunk;
+  W.chunk_mul = (uint32_t)(((1ull << 32) + W.chunk - 1) / W.chunk);
+  double best = 0.0;
+  for (int c = W.n_chunk; c >= 1; --c) {
+    const int len = c * W.chunk, nseg = (NX + len - 1) / len;
+    const int64_t items = (int64_t)n_tiles * groups * nseg;
+    const double cost = (double)((items + slots - 1) / slots) * (std::min(len, NX) + (nseg > 1 ? 2 : 0) + 1.5);
+    if (c == W.n_chunk || cost < 0.97 * best) {
+      best = cost;
+      W.nseg = nseg;
+      W.seg_len = len;
+      W.n_items = (int)items;
+    }
+  }
+  return W;
+}
 constexpr int pad128(int floats) { return (floats + 31) / 32 * 32; }  // TMA destinations: 128-byte boundaries
 constexpr int kQPlane = kQR * 3 * kQPJ * kQPK;      // vector patch (floats)
 constexpr int kQNode = kQR * kQPJ * kQPK;           // dinv patch
@@ -1631,6 +1457,7 @@ constexpr int kQO = kQR * kQJ * kQK;                // dinv of the tile's own no
 // exchange buffer: corners 1..3 of every element pencil (corner 0 belongs to the
 // node pencil of the same lanes and stays in their registers)
 constexpr int kQX = kQEJ * kQEK * 3 * 3 * kQR;
+constexpr int kQRed = kMaxChunks * (kQWarps - kQEJ / kQPencils) * kQR;  // partial sums of an item
 template <int kMode> struct LvlStage2 {
   static constexpr bool kTwo = kMode == kLvlStart || kMode == kLvlPcgZ;
   // Smooth and Resid also stage b of the tile's own nodes (Smooth its dinv as
@@ -1651,7 +1478,7 @@ template <int kMode> struct LvlStage2 {
   static constexpr uint32_t kBytes = 4 * ((kTwo ? 2 : 1) * kQPlane + (kNodes ? kQNode : 0) + kQE +
                                           (kDir || kOwn ? kQD : 0) + (kOwnD ? kQO : 0));  // loaded per stage
   static constexpr size_t kSmem = 128 + sizeof(float) * ((size_t)kStages * kFloats + 2 * (size_t)kQX) +
-                                  sizeof(double) * kQJ * kQK * kQR + sizeof(uint64_t) * kStages + sizeof(int) * 6;
+                                  sizeof(double) * kQRed + sizeof(uint64_t) * kStages + sizeof(int) * 8;
 };
 // two CTAs an SM: 227 KB together, 1 KB of system use each
 static_assert(LvlStage2<kLvlPcgZ>::kSmem <= 112 * 1024 && LvlStage2<kLvlStart>::kSmem <= 112 * 1024 &&
@@ -1662,8 +1489,8 @@ template <int kMode, bool kMass>
 __global__ void __launch_bounds__(kQThreads, kQCtas)
     k_lvl_op2(Lattice L, const __grid_constant__ ModalCT<float2> C, const __grid_constant__ CUtensorMap tm_a,
               const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_n,
-              const __grid_constant__ CUtensorMap tm_e, const __grid_constant__ CUtensorMap tm_d, int tiles_j,
-              int n_tiles, int n_items, const uint8_t* __restrict__ mask, const float* __restrict__ b,
+              const __grid_constant__ CUtensorMap tm_e, const __grid_constant__ CUtensorMap tm_d, Walk W,
+              const uint8_t* __restrict__ mask, const float* __restrict__ b,
               const float* __restrict__ dinv, float omega, const float* __restrict__ alpha,
               const float* __restrict__ beta, float* __restrict__ out, float* __restrict__ out2,
               float* __restrict__ out3, float* __restrict__ d, double* __restrict__ partial, int pstride,
@@ -1673,28 +1500,33 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
   float* smem = smem_dyn + (((128u - (smem_u32(smem_dyn) & 127u)) & 127u) >> 2);
   constexpr int kSt = S::kStages;
   float* xbuf = smem + kSt * S::kFloats;
-  double* red = reinterpret_cast<double*>(xbuf + 2 * kQX);  // [node pencils][kQR]
-  uint64_t* full = reinterpret_cast<uint64_t*>(red + kQJ * kQK * kQR);
-  int* next = reinterpret_cast<int*>(full + kSt);  // the producer's next load: item, plane, J0, K0, realization
+  double* red = reinterpret_cast<double*>(xbuf + 2 * kQX);  // [chunks][warps with nodes][kQR]
+  uint64_t* full = reinterpret_cast<uint64_t*>(red + kQRed);
+  int* next = reinterpret_cast<int*>(full + kSt);  // the producer's next load: item, plane, last plane, J0, K0, realization, stage
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int NX = L.NX, Rp = L.Rp, Rp2 = L.Rp >> 1;
-  const auto item_tile = [&](int item) { return (item / kQQuad) % n_tiles; };
-  const auto item_col = [&](int item) { return (item / (kQQuad * n_tiles) * kQQuad + item % kQQuad) * kQR; };
   // The producer (lane 0 of warp 0, whose pencils own no nodes) loads the
-  // planes of the CTA's items in order, plane q into stage q % kSt: planes 0, 1
-  // and 2 at the start and plane c + 2 after the c-th plane barrier, when the
-  // readers of the stage it refills (plane c - 1, or c - 2 with kOwn's four
-  // stages) have all passed that barrier. The position is stepped, not divided
-  // out of q, and kept in shared memory: on the critical path of warp 0 the
-  // divisions took 1,100 of 3,500 cycles a plane.
+  // planes of the CTA's items in order, plane q of the walk into stage q % kSt, as
+  // soon as a plane barrier shows that every reader of the stage's last plane has
+  // passed (with kOwn's four stages also the node phase after it). The position is
+  // stepped, not divided out of q, and kept in shared memory: on the critical path
+  // of warp 0 the divisions took 1,100 of 3,500 cycles a plane.
   const bool producer = w == 0 && lane == 0;
-  uint32_t n_loads = 0;  // of the producer: planes loaded so far
+  const auto place = [&](int item) {
+    const WalkItem I = walk_item<true, kQJ, kQK, kQR>(W, item, NX);
+    next[0] = item;
+    next[1] = I.p0;
+    next[2] = I.p1;
+    next[3] = I.J0;
+    next[4] = I.K0;
+    next[5] = I.col;
+  };
   const auto produce = [&]() {
     const int item = next[0];
-    if (item >= n_items) return;
-    const int P = next[1], J0 = next[2], K0 = next[3], g16 = next[4];
-    const int st = n_loads % kSt;
-    ++n_loads;
+    if (item >= W.n_items) return;
+    const int P = next[1], J0 = next[3], K0 = next[4], g16 = next[5];
+    const int st = next[6];
+    next[6] = st + 1 < kSt ? st + 1 : 0;
     float* dst = smem + st * S::kFloats;
     mbar_expect_tx(&full[st], S::kBytes);
     tma_load_5d(dst + S::kOffA, &tm_a, g16, 0, P, J0 - 1, K0 - 1, &full[st]);
@@ -1704,27 +1536,17 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
     if constexpr (kMode == kLvlPcgZ) tma_load_5d(dst + S::kOffD, &tm_d, g16, 0, P, J0, K0, &full[st]);
     if constexpr (S::kOwn) tma_load_5d(dst + S::kOffD, &tm_b, g16, 0, P, J0, K0, &full[st]);
     if constexpr (S::kOwnD) tma_load_4d(dst + S::kOffO, &tm_n, g16, P, J0, K0, &full[st]);
-    if (P < NX) {
+    if (P < next[2])
       next[1] = P + 1;
-      return;
-    }
-    const int it = item + gridDim.x, tile = item_tile(it);
-    next[0] = it;
-    next[1] = 1;
-    next[2] = 1 + (tile % tiles_j) * kQJ;
-    next[3] = 1 + (tile / tiles_j) * kQK;
-    next[4] = item_col(it);
+    else
+      place(item + gridDim.x);
   };
   if (threadIdx.x == 0) {
     for (int st = 0; st < kSt; ++st) mbar_init(&full[st], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    const int it = blockIdx.x, tile = item_tile(it);
-    next[0] = it;
-    next[1] = 1;
-    next[2] = 1 + (tile % tiles_j) * kQJ;
-    next[3] = 1 + (tile / tiles_j) * kQK;
-    next[4] = item_col(it);
-    for (int q = 0; q < 3; ++q) produce();
+    place(blockIdx.x);
+    next[6] = 0;
+    for (int st = 0; st < kSt - (S::kOwn ? 1 : 0); ++st) produce();
   }
   __syncthreads();
   // this lane's element pencil and realization pair
@@ -1735,24 +1557,37 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
   const bool node_warp = ek >= 1;                // warps with node pencils
   const bool node_lane = node_warp && ej >= 1;
   uint32_t seq = 0;
-  int xsel = 0;
   bool dead = false;
   auto csync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kQWarps * 32) : "memory"); };
-  // the barrier of a plane between the element and the node phase; the stage it frees is refilled
+  // the barrier of a plane (the walk's plane q has been read) between the element and
+  // the node phase; the stages it frees are refilled
   auto plane_sync = [&]() {
     csync();
     if (producer && !dead) produce();
   };
+  // partial sums: left by the node lanes in red at the end of a chunk, added by the
+  // first lanes at the end of the item (a flush within the walk cost 8 % of it)
+  constexpr int kPart = (kQWarps - kRow) * kQR;  // sums of a chunk: a row of every warp with nodes
+  auto flush = [&](const WalkItem& I) {
+    const int chunk = W.chunk_of(I.a) + threadIdx.x / kQR, rl = threadIdx.x % kQR;
+    if (kMode == kLvlResid || partial == nullptr || chunk > W.chunk_of(I.b)) return;
+    const double* rd = red + chunk * kPart + rl;
+    double sum = 0.0;
+#pragma unroll
+    for (int i = 0; i < kPart / kQR; ++i) sum += rd[i * kQR];
+    partial[(((int64_t)I.tile * W.n_chunk + chunk) * Rp + I.col + rl) * pstride] = sum;
+  };
   const float2 z2 = make_float2(0.f, 0.f);
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int tile = item_tile(item), g16 = item_col(item);
-    const int J0 = 1 + (tile % tiles_j) * kQJ, K0 = 1 + (tile / tiles_j) * kQK;
-    const int Je = J0 - 1 + ej, Ke = K0 - 1 + ek;
+  for (int item = blockIdx.x; item < W.n_items; item += gridDim.x) {
+    const WalkItem I = walk_item<true, kQJ, kQK, kQR>(W, item, NX);
+    const int g16 = I.col;
+    const int Je = I.J0 - 1 + ej, Ke = I.K0 - 1 + ek;
     auto realj = [&](int j) { return j >= 1 && j <= L.NY - 1; };
     auto realk = [&](int k) { return k >= 1 && k <= L.NZ - 1; };
     const bool real = realj(Je) && realk(Ke);
     const bool node_ok = node_lane && Je <= L.NY && Ke <= L.NZ;
-    const size_t nrow = ((size_t)Je + (size_t)L.NYp * Ke) * L.NXp;
+    // (32-bit offsets in pairs of realizations: a vector is far below 32 GB)
+    const uint32_t nrow = ((uint32_t)Je + (uint32_t)L.NYp * Ke) * L.NXp;
     const int rr2 = (g16 >> 1) + l2;  // float2 index of this lane's realization pair
     float2 al = z2, be = z2;
     if constexpr (kMode == kLvlStart || kMode == kLvlPcgZ) al = reinterpret_cast<const float2*>(alpha)[rr2];
@@ -1773,7 +1608,8 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
     auto node_phase = [&](int X, uint32_t seq_x) {
       [[maybe_unused]] const float* px = smem + (seq_x % kSt) * S::kFloats;
       [[maybe_unused]] const int od = (ek - 1) * kQJ + (ej - 1);
-      if (((X - 1) & (4 * kQLanes - 1)) == 0) {  // the next 32 planes, 4 a lane
+      const int mx = (X - I.a) & (4 * kQLanes - 1);
+      if (mx == 0) {  // the next 32 planes, 4 a lane
         mreg = 0u;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -1781,11 +1617,10 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
           if (node_ok && pl <= NX) mreg |= (uint32_t)mask[nrow + pl] << (8 * i);
         }
       }
-      const int mx = (X - 1) & (4 * kQLanes - 1);
       const uint32_t mk = __shfl_sync(0xffffffffu, mreg, mx >> 2, kQLanes) >> (8 * (mx & 3));
       if (!node_ok) return;
-      const float2* xb = xb2 + xsel * (kQX / 2);
-      const size_t node = nrow + X;
+      const float2* xb = xb2 + (X & 1) * (kQX / 2);
+      const uint32_t node = nrow + X;
       float2 wdv = z2;
       if constexpr (kMode == kLvlSmooth) wdv = om2 * reinterpret_cast<const float2*>(px + S::kOffO)[od * kQLanes + l2];
       double s0 = 0.0, s1 = 0.0;
@@ -1795,7 +1630,7 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
         y = y + xb[(((pid - 1) * 3 + 0) * 3 + c) * kQLanes + l2];
         y = y + xb[(((pid - kQEJ) * 3 + 1) * 3 + c) * kQLanes + l2];
         y = y + xb[(((pid - kQEJ - 1) * 3 + 2) * 3 + c) * kQLanes + l2];
-        const size_t o = (node * 3 + c) * Rp2 + rr2;
+        const uint32_t o = (node * 3 + c) * Rp2 + rr2;
         const bool fixed = (mk >> c) & 1;
         float2 v;
         if constexpr (kMode == kLvlStart) {
@@ -1819,10 +1654,24 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
       acc0 += s0;
       acc1 += s1;
     };
-    auto emit_corners = [&](const float2 (&B)[3][4]) {
+    auto leave = [&](int chunk) {  // partial sums of a chunk
+      if (kMode == kLvlResid || !node_warp) return;
+      double* rd = red + chunk * kPart + (w - kRow) * kQR + 2 * l2;
+#pragma unroll
+      for (int o = kQLanes; o < 32; o *= 2) {  // of the warp's four pencils (a ghost's are zero)
+        acc0 += __shfl_xor_sync(0xffffffffu, acc0, o);
+        acc1 += __shfl_xor_sync(0xffffffffu, acc1, o);
+      }
+      if (lane < kQLanes) {
+        rd[0] = acc0;
+        rd[1] = acc1;
+      }
+      acc0 = acc1 = 0.0;
+    };
+    auto emit_corners = [&](const float2 (&B)[3][4], int X) {  // of plane X
       float2 y[2][2][3];
       yz_inverse(B, y);
-      float2* xb = reinterpret_cast<float2*>(xbuf) + xsel * (kQX / 2);
+      float2* xb = reinterpret_cast<float2*>(xbuf) + (X & 1) * (kQX / 2);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         own[c] = y[0][0][c];
@@ -1831,7 +1680,9 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
         xb[((pid * 3 + 2) * 3 + c) * kQLanes + l2] = y[1][1][c];
       }
     };
-    for (int P = 1; P <= NX; ++P, ++seq) {
+    float2 u[2][2][3], rc[3] = {z2, z2, z2}, Bc[3][4], E = z2;
+    // plane P of the walk: the corner values and their yz modes; the owner writes
+    auto plane = [&](int P) {
       const int st = seq % kSt;
       if (!dead && !mbar_wait(&full[st], (seq / kSt) & 1)) {
         atomicExch(err, 1);
@@ -1840,7 +1691,6 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
       const float* pt = smem + st * S::kFloats;
       const float2* pa = reinterpret_cast<const float2*>(pt + S::kOffA);
       const float2* pb = reinterpret_cast<const float2*>(pt + S::kOffB);
-      float2 u[2][2][3], rc[3] = {z2, z2, z2};
 #pragma unroll
       for (int ay = 0; ay < 2; ++ay)
 #pragma unroll
@@ -1863,13 +1713,13 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
             }
           }
         }
-      const float2 E = reinterpret_cast<const float2*>(pt + S::kOffE)[pid * kQLanes + l2];
+      E = reinterpret_cast<const float2*>(pt + S::kOffE)[pid * kQLanes + l2];
       if constexpr (kMode == kLvlStart || kMode == kLvlPcgZ) {
-        if (node_ok) {
-          const size_t node = nrow + P;
+        if (node_ok && P >= I.a && P <= I.b) {
+          const uint32_t node = nrow + P;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            const size_t o = (node * 3 + c) * Rp2 + rr2;
+            const uint32_t o = (node * 3 + c) * Rp2 + rr2;
             if constexpr (kMode == kLvlStart) {
               reinterpret_cast<float2*>(out2)[o] = rc[c];
               if (out3 != nullptr) reinterpret_cast<float2*>(out3)[o] = u[0][0][c];
@@ -1883,30 +1733,9 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
           }
         }
       }
-      float2 Bc[3][4];
       yz_forward(u, Bc);
-      if (P >= 2) {
-        {
-          // ghost pencils have E = 0 and emit zeros (the mass term, which does not
-          // scale with E, is left out of them below)
-          float2 C1[3][4];
-          modal_apply<kMass>(C, E, Bp, Bc, T0, C1);
-          if (kMass && !real) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-              for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq] = z2;
-          }
-          emit_corners(T0);
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
-        }
-        plane_sync();
-        if (node_warp) node_phase(P - 1, seq - 1);
-        xsel ^= 1;
-      }
+    };
+    auto keep = [&]() {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         ou[c] = u[0][0][c];
@@ -1914,26 +1743,326 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
 #pragma unroll
         for (int qq = 0; qq < 4; ++qq) Bp[c][qq] = Bc[c][qq];
       }
-    }
-    emit_corners(T0);
-    plane_sync();
-    if (node_warp) node_phase(NX, seq - 1);
-    xsel ^= 1;
-    if (kMode != kLvlResid && partial != nullptr) {
-      if (node_lane) {
-        const int nw = (ek - 1) * kQJ + (ej - 1);
-        red[nw * kQR + 2 * l2] = acc0;
-        red[nw * kQR + 2 * l2 + 1] = acc1;
-      }
-      csync();
-      if (threadIdx.x < kQR) {
-        const int rl = threadIdx.x;  // realization within the item
-        double sum = 0.0;
+      ++seq;
+    };
+    plane(I.p0);
+    keep();
+    int P = I.p0 + 1, chunk = W.chunk_of(I.a);
+    for (;; ++chunk) {
+      const int ce = (chunk + 1) * W.chunk;  // the chunk's last plane
+      for (const int last = min(ce + 1, I.p1); P <= last; ++P) {
+        plane(P);
+        // ghost pencils have E = 0 and emit zeros (the mass term, which does not
+        // scale with E, is left out of them below)
+        float2 C1[3][4];
+        modal_apply<kMass>(C, E, Bp, Bc, T0, C1);
+        if (kMass && !real) {
 #pragma unroll
-        for (int i = 0; i < kQJ * kQK; ++i) sum += red[i * kQR + rl];
-        partial[((size_t)tile * Rp + g16 + rl) * pstride] = sum;
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq] = z2;
+        }
+        emit_corners(T0, P - 1);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
+        plane_sync();
+        if (node_warp && P > I.a) node_phase(P - 1, seq - 1);  // (plane a - 1 is the neighbour's)
+        keep();
+      }
+      if (ce >= I.b) break;
+      leave(chunk);
+    }
+    if (I.b == NX) {  // plane NX: the slab above it is a ghost
+      emit_corners(T0, NX);
+      csync();
+      if (node_warp) node_phase(NX, seq - 1);
+    }
+    leave(chunk);
+    plane_sync();
+    flush(I);
+  }
+}
+
+// ---------------------------------------------------------------- single-reduction Jacobi iteration
+// One whole inner PCG iteration per launch (single-reduction form). Launch k+1
+// receives r_k, q_k = K p_k, p_k, alpha_k and beta_{k+1} and, at every node,
+//   r_{k+1} = r_k - alpha_k q_k,  p_{k+1} = dinv r_{k+1} + beta_{k+1} p_k,
+//   d += alpha_k p_k (the FP32 solution correction),
+// then q_{k+1} = K p_{k+1} (masked) with the partials p.q, (dinv r).q,
+// q.dinv.q and (dinv r).r of p_{k+1}, r_{k+1}, q_{k+1}. The scalar kernel that
+// follows forms alpha_{k+1} = gamma_{k+1} / p.q from the gamma of r_{k+1}
+// itself and the next gamma by the expansion of (dinv r_{k+2}).r_{k+2},
+//   gamma_{k+2} = gamma_{k+1} - 2 alpha (dinv r).q + alpha^2 q.dinv.q,
+// so r never needs a pass of its own (and the expansion never runs for more
+// than one step, which keeps the FP32 iteration count of the two-pass loop).
+// Each stage carries the plane's r, q, p and dinv patches with halo (and the
+// tile's d); the element warps form p_{k+1} at their corners on the fly, and the
+// owner of a node pencil writes r, p and d back. r, q and p each have a second
+// buffer: neighbouring CTAs still read the old values in their halos.
+//
+// Tiles of 7 x 3 node pencils for 16 realizations as k_lvl_op2, one realization a
+// lane and two element pencils a warp: one CTA of 16 warps and a loading warp an
+// SM. It is bound by the latency of a plane's chain, like k_lvl_op2; two
+// realizations a lane spill here (r, p, D^-1 and eight partial sums live across
+// planes; 193 us). 24^3 x 256 with a mass term: 174 us on 3 x 3 tiles of 32
+// realizations (16 element pencils for 9 nodes, and 4.4 rounds of items that took
+// 5), 148 us now; 11^3 x 100: 24 us in whole walks, 18 in segments.
+constexpr int kJLanes = kQR;                      // lanes of a pencil
+constexpr int kJPencils = 32 / kJLanes;           // pencils per warp, along y
+constexpr int kJWarps = kQEJ * kQEK / kJPencils;  // 16 element warps
+constexpr int kJThreads = 32 * (kJWarps + 1);
+constexpr int kJPen = 4 * 3 * kQR + 16;           // exchange floats of a pencil (16 more: no bank conflicts)
+constexpr int kJX = kQEJ * kQEK * kJPen;
+struct JacStage {
+  static constexpr int kStages = 4;
+  static constexpr int kOffR = 0, kOffQ = pad128(kQPlane), kOffP = 2 * pad128(kQPlane), kOffN = 3 * pad128(kQPlane);
+  static constexpr int kOffE = kOffN + pad128(kQNode), kOffD = kOffE + pad128(kQE), kFloats = kOffD + pad128(kQD);
+  static constexpr uint32_t kBytes = 4 * (3 * kQPlane + kQNode + kQE + kQD);
+  static constexpr int kRed = kMaxChunks * kMParts * (kJWarps - kQEJ / kJPencils) * kQR;  // partial sums
+  static constexpr size_t kSmem = 128 + sizeof(float) * ((size_t)kStages * kFloats + 2 * (size_t)kJX) +
+                                  sizeof(double) * kRed + sizeof(uint64_t) * 2 * kStages;
+  static_assert(kSmem <= 227 * 1024, "shared memory");
+};
+template <bool kMass, bool kSeg>
+__global__ void __launch_bounds__(kJThreads, 1)
+    k_jacobi_op(Lattice L, const __grid_constant__ ModalC C, const __grid_constant__ CUtensorMap tm_r,
+                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_p,
+                const __grid_constant__ CUtensorMap tm_n, const __grid_constant__ CUtensorMap tm_e,
+                const __grid_constant__ CUtensorMap tm_d, Walk W, const uint8_t* __restrict__ mask,
+                const float* __restrict__ alpha, const float* __restrict__ beta,
+                float* __restrict__ r_out, float* __restrict__ p_out, float* __restrict__ q_out, float* __restrict__ d,
+                double* __restrict__ partial, int* __restrict__ err) {
+  using S = JacStage;
+  constexpr int kSt = S::kStages;
+  extern __shared__ __align__(128) float smem_dyn[];
+  float* smem = smem_dyn + (((128u - (smem_u32(smem_dyn) & 127u)) & 127u) >> 2);
+  float* xbuf = smem + kSt * S::kFloats;
+  double* red = reinterpret_cast<double*>(xbuf + 2 * kJX);  // [chunks][parts][warps with nodes][kQR]
+  uint64_t* full = reinterpret_cast<uint64_t*>(red + S::kRed);
+  uint64_t* empty = full + kSt;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int NX = L.NX, Rp = L.Rp;
+  if (threadIdx.x == 0) {
+    for (int st = 0; st < kSt; ++st) {
+      mbar_init(&full[st], 1);
+      mbar_init(&empty[st], kJWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (w == kJWarps) {
+    // loading warp: plane P of every work item, in the consumers' order
+    if (lane == 0) {
+      uint32_t seq = 0;
+      for (int item = blockIdx.x; item < W.n_items; item += gridDim.x) {
+        const WalkItem I = walk_item<kSeg, kQJ, kQK, kQR>(W, item, NX);
+        const int g16 = I.col, J0 = I.J0, K0 = I.K0;
+        for (int P = I.p0; P <= I.p1; ++P, ++seq) {
+          const int st = seq % kSt;
+          const uint32_t use = seq / kSt;
+          if (use > 0 && !mbar_wait(&empty[st], (use - 1) & 1)) {
+            atomicExch(err, 1);
+            return;
+          }
+          float* dst = smem + st * S::kFloats;
+          mbar_expect_tx(&full[st], S::kBytes);
+          tma_load_5d(dst + S::kOffR, &tm_r, g16, 0, P, J0 - 1, K0 - 1, &full[st]);
+          tma_load_5d(dst + S::kOffQ, &tm_q, g16, 0, P, J0 - 1, K0 - 1, &full[st]);
+          tma_load_5d(dst + S::kOffP, &tm_p, g16, 0, P, J0 - 1, K0 - 1, &full[st]);
+          tma_load_4d(dst + S::kOffN, &tm_n, g16, P, J0 - 1, K0 - 1, &full[st]);
+          tma_load_4d(dst + S::kOffE, &tm_e, g16, P - 1, J0 - 1, K0 - 1, &full[st]);
+          tma_load_5d(dst + S::kOffD, &tm_d, g16, 0, P, J0, K0, &full[st]);
+        }
       }
     }
+    return;
+  }
+  constexpr int kRow = kQEJ / kJPencils;  // warps per row of pencils
+  const int l = lane % kJLanes;
+  const int ej = (w % kRow) * kJPencils + lane / kJLanes, ek = w / kRow;
+  const int pid = ek * kQEJ + ej;
+  const bool node_warp = ek >= 1, node_lane = node_warp && ej >= 1;
+  uint32_t seq = 0;
+  bool dead = false;  // a stage never arrived: finish the walk without data (err is set)
+  // barrier of the element warps between the element and the node phase of a
+  // plane; every one passes the same sequence of them, error or not
+  auto csync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kJWarps * 32) : "memory"); };
+  constexpr int kPart = (kJWarps - kRow) * kQR;  // sums of a chunk: a row of every warp with nodes
+  auto flush = [&](const WalkItem& I) {  // partial sums of the item's chunks (as k_lvl_op2)
+    const int chunk = W.chunk_of(I.a) + threadIdx.x / (kMParts * kQR);
+    const int i = threadIdx.x / kQR % kMParts, rl = threadIdx.x % kQR;
+    if (chunk > W.chunk_of(I.b)) return;
+    const double* rd = red + (chunk * kMParts + i) * kPart + rl;
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < kPart / kQR; ++k) sum += rd[k * kQR];
+    partial[(((int64_t)I.tile * W.n_chunk + chunk) * Rp + I.col + rl) * kMParts + i] = sum;
+  };
+  for (int item = blockIdx.x; item < W.n_items; item += gridDim.x) {
+    const WalkItem I = walk_item<kSeg, kQJ, kQK, kQR>(W, item, NX);
+    const int g16 = I.col;
+    const int Je = I.J0 - 1 + ej, Ke = I.K0 - 1 + ek;  // element pencil (lower corner), padded
+    const bool real = Je >= 1 && Je <= L.NY - 1 && Ke >= 1 && Ke <= L.NZ - 1;
+    const bool node_ok = node_lane && Je <= L.NY && Ke <= L.NZ;
+    const uint32_t nrow = ((uint32_t)Je + (uint32_t)L.NYp * Ke) * L.NXp;  // padded node (0, Je, Ke)
+    const int rr = g16 + l;
+    const float al = alpha[rr], be = beta[rr];
+    float Bp[3][4], T0[3][4];
+    float op[3] = {0.f, 0.f, 0.f}, orr[3] = {0.f, 0.f, 0.f}, odv = 0.f;  // p, r, dinv at the own node
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int qq = 0; qq < 4; ++qq) T0[c][qq] = 0.f;
+    double acc_pq = 0.0, acc_zq = 0.0, acc_qq = 0.0, acc_zr = 0.0;
+    uint32_t mreg = 0;  // constraint bits of two planes of the own pencil
+    // node phase of plane X: sum the corner contributions of the 4 elements (ghosts emit zeros)
+    auto node_phase = [&](int X) {
+      const int mx = (X - I.a) & (2 * kJLanes - 1);
+      if (mx == 0) {  // the next 32 planes
+        mreg = 0u;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (node_ok && X + 2 * l + i <= NX) mreg |= (uint32_t)mask[nrow + X + 2 * l + i] << (8 * i);
+      }
+      const uint32_t mk = __shfl_sync(0xffffffffu, mreg, mx >> 1, kJLanes) >> (8 * (mx & 1));
+      if (!node_ok) return;
+      const float* xb = xbuf + (X & 1) * kJX + l;
+      const uint32_t node = nrow + X;
+      // products in FP64: a fast-converging realization drives r and q towards the
+      // bottom of the FP32 range, where FP32 squares would underflow
+      double spq = 0.0, szq = 0.0, sqq = 0.0, szr = 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        float y = xb[pid * kJPen + (0 * 3 + c) * kJLanes];
+        y += xb[(pid - 1) * kJPen + (1 * 3 + c) * kJLanes];
+        y += xb[(pid - kQEJ) * kJPen + (2 * 3 + c) * kJLanes];
+        y += xb[(pid - kQEJ - 1) * kJPen + (3 * 3 + c) * kJLanes];
+        y = ((mk >> c) & 1) ? 0.f : y;
+        q_out[(node * 3 + c) * Rp + rr] = y;
+        const double yd = (double)y, rd = (double)orr[c];
+        spq = fma((double)op[c], yd, spq);
+        szq = fma(rd, yd, szq);
+        sqq = fma(yd, yd, sqq);
+        szr = fma(rd, rd, szr);
+      }
+      const double dvd = (double)odv;
+      acc_pq += spq;
+      acc_zq += dvd * szq;
+      acc_qq += dvd * sqq;
+      acc_zr += dvd * szr;
+    };
+    auto leave = [&](int chunk) {  // partial sums of a chunk
+      if (!node_warp) return;
+      double* rd = red + chunk * kMParts * kPart + (w - kRow) * kQR + l;
+      const double v[kMParts] = {acc_pq, acc_zq, acc_qq, acc_zr};
+#pragma unroll
+      for (int i = 0; i < kMParts; ++i) {  // of the warp's two pencils (a ghost's are zero)
+        const double o = __shfl_xor_sync(0xffffffffu, v[i], kJLanes);
+        if (lane < kJLanes) rd[i * kPart] = v[i] + o;
+      }
+      acc_pq = acc_zq = acc_qq = acc_zr = 0.0;
+    };
+    auto emit_corners = [&](const float (&B)[3][4], int X) {  // of plane X
+      float y[2][2][3];
+      yz_inverse(B, y);
+      float* xb = xbuf + (X & 1) * kJX + pid * kJPen + l;
+#pragma unroll
+      for (int ay = 0; ay < 2; ++ay)
+#pragma unroll
+        for (int az = 0; az < 2; ++az)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) xb[((ay + 2 * az) * 3 + c) * kJLanes] = y[ay][az][c];
+    };
+    float u[2][2][3], rc[3], Bc[3][4], dvc = 0.f, E = 0.f;
+    // plane P of the walk: the corner values and their yz modes; the owner writes
+    auto plane = [&](int P) {
+      const int st = seq % kSt;
+      if (!dead && !mbar_wait(&full[st], (seq / kSt) & 1)) {
+        atomicExch(err, 1);
+        dead = true;
+      }
+      const float* pt = smem + st * S::kFloats + l;
+      // p_{k+1} at the element's 4 plane corners: dinv (r - alpha q) + beta p_k
+#pragma unroll
+      for (int ay = 0; ay < 2; ++ay)
+#pragma unroll
+        for (int az = 0; az < 2; ++az) {
+          const int o = (ek + az) * kQPJ + (ej + ay);
+          const float dv = pt[S::kOffN + o * kJLanes];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const int i = (o * 3 + c) * kJLanes;
+            const float rn = fmaf(-al, pt[S::kOffQ + i], pt[S::kOffR + i]);
+            u[ay][az][c] = fmaf(dv, rn, be * pt[S::kOffP + i]);
+            if (ay == 0 && az == 0) rc[c] = rn;
+          }
+          if (ay == 0 && az == 0) dvc = dv;
+        }
+      E = pt[S::kOffE + pid * kJLanes];
+      if (node_ok && (!kSeg || (P >= I.a && P <= I.b))) {
+        // the owner writes r_{k+1}, p_{k+1} and d += alpha_k p_k of node (P, Je, Ke)
+        const int o = ek * kQPJ + ej, od = (ek - 1) * kQJ + (ej - 1);
+        const uint32_t node = nrow + P;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float dn = fmaf(al, pt[S::kOffP + (o * 3 + c) * kJLanes], pt[S::kOffD + (od * 3 + c) * kJLanes]);
+          r_out[(node * 3 + c) * Rp + rr] = rc[c];
+          p_out[(node * 3 + c) * Rp + rr] = u[0][0][c];
+          d[(node * 3 + c) * Rp + rr] = dn;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
+      yz_forward(u, Bc);
+    };
+    auto keep = [&]() {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        op[c] = u[0][0][c];
+        orr[c] = rc[c];
+        odv = dvc;
+#pragma unroll
+        for (int qq = 0; qq < 4; ++qq) Bp[c][qq] = Bc[c][qq];
+      }
+      ++seq;
+    };
+    plane(I.p0);
+    keep();
+    int P = I.p0 + 1, chunk = W.chunk_of(I.a);
+    for (;; ++chunk) {
+      const int ce = (chunk + 1) * W.chunk;  // the chunk's last plane
+      for (const int last = min(ce + 1, I.p1); P <= last; ++P) {
+        plane(P);
+        float C1[3][4];
+        modal_apply<kMass>(C, E, Bp, Bc, T0, C1);
+        if (kMass && !real) {  // the mass term does not scale with a ghost's E = 0
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq] = 0.f;
+        }
+        emit_corners(T0, P - 1);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
+        csync();
+        if (node_warp && (!kSeg || P > I.a)) node_phase(P - 1);  // (plane a - 1 is the neighbour's)
+        keep();
+      }
+      if (ce >= I.b) break;
+      leave(chunk);
+    }
+    if (!kSeg || I.b == NX) {  // plane NX: the slab above it is a ghost, so the pending part is complete
+      emit_corners(T0, NX);
+      csync();
+      if (node_warp) node_phase(NX);
+    }
+    leave(chunk);
+    csync();
+    flush(I);
   }
 }
 
@@ -1948,7 +2077,7 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
 // needs about twice the registers of the FP32 operator: 3 warps per SM
 // sub-partition) and no separate producer warp: lane 0 of warp 0 issues the
 // TMA loads three planes ahead into the 4-stage ring; exchange and bounded
-// waits as k_op_modal. 24^3 x 256: 206 -> 196 us without divisions on the loading lane.
+// waits as k_jacobi_op. 24^3 x 256: 206 -> 196 us without divisions on the loading lane.
 constexpr int kRJ = 3, kRK = 2;
 constexpr int kREJ = kRJ + 1, kREK = kRK + 1, kRWarps = kREJ * kREK;
 constexpr int kRPJ = kRJ + 2, kRPK = kRK + 2;
@@ -1960,46 +2089,44 @@ constexpr uint32_t kRStageBytes = kROffE + 8 * kREPatch;  // 33,792 bytes
 constexpr int kRStages = 4;
 constexpr int kRXDoubles = kRWarps * 4 * 3 * 32;        // exchange buffer (doubles)
 constexpr size_t kRSmem = 128 + (size_t)kRStages * kRStageBytes + 2 * sizeof(double) * kRXDoubles +
-                          sizeof(double) * 2 * kRJ * kRK * 32 + sizeof(uint64_t) * kRStages + sizeof(int) * 6;
+                          sizeof(double) * kMaxChunks * 2 * kRJ * kRK * 32 + sizeof(uint64_t) * kRStages + sizeof(int) * 6;
 static_assert(kRStageBytes % 128 == 0 && kROffD % 128 == 0 && kROffP % 128 == 0 && kROffE % 128 == 0, "align");
 static_assert(kRSmem <= 227 * 1024, "FP64 residual shared memory");
 
-template <bool kMass, bool kBPerR, bool kUpdate>
+template <bool kMass, bool kBPerR, bool kUpdate, bool kSeg>
 __global__ void __launch_bounds__(kRThreads, 1)
     k_resid_modal(Lattice L, const __grid_constant__ ModalCD C, const __grid_constant__ CUtensorMap tm_x,
                   const __grid_constant__ CUtensorMap tm_d, const __grid_constant__ CUtensorMap tm_p,
-                  const __grid_constant__ CUtensorMap tm_e, int tiles_j, int n_tiles, int n_items,
-                  const uint8_t* __restrict__ mask, const double* __restrict__ b, const float* __restrict__ dinv,
+                  const __grid_constant__ CUtensorMap tm_e, Walk W, const uint8_t* __restrict__ mask,
+                  const double* __restrict__ b, const float* __restrict__ dinv,
                   const float* __restrict__ alpha, double* __restrict__ x_out, float* __restrict__ r32,
                   double* __restrict__ partial, int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   double* xbuf = reinterpret_cast<double*>(smem + (size_t)kRStages * kRStageBytes);
-  double* red = xbuf + 2 * kRXDoubles;  // [2][node pencils][32]
-  uint64_t* full = reinterpret_cast<uint64_t*>(red + 2 * kRJ * kRK * 32);
-  int* next = reinterpret_cast<int*>(full + kRStages);  // the producer's next load: item, plane, J0, K0, realization
+  double* red = xbuf + 2 * kRXDoubles;  // [chunks][2 sums][node pencils][32]
+  uint64_t* full = reinterpret_cast<uint64_t*>(red + kMaxChunks * 2 * kRJ * kRK * 32);
+  int* next = reinterpret_cast<int*>(full + kRStages);  // the producer's next load: item, plane, last plane, J0, K0, realization
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int NX = L.NX, Rp = L.Rp;
   constexpr uint32_t kBytes = kUpdate ? kRStageBytes : (8 * kRPatch + 8 * kREPatch);
-  // producer: lane 0 of warp 0 (no nodes of its own) loads the planes of the
-  // CTA's items in order, the first four at the start and plane c + 3 after the
-  // c-th plane barrier, which every reader of the stage it refills (plane c - 1)
-  // has passed; its position is stepped, not divided out of a counter (1,100
-  // cycles a plane on the critical path)
+  // producer: lane 0 of warp 0 (no nodes of its own) loads the planes of the CTA's
+  // items in order, as k_lvl_op2's
   const bool producer = w == 0 && lane == 0;
   uint32_t n_loads = 0;
   const auto place = [&](int item) {
-    const int tile = item % n_tiles;
+    const WalkItem I = walk_item<kSeg, kRJ, kRK, 32>(W, item, NX);
     next[0] = item;
-    next[1] = 1;
-    next[2] = 1 + (tile % tiles_j) * kRJ;
-    next[3] = 1 + (tile / tiles_j) * kRK;
-    next[4] = (item / n_tiles) * 32;
+    next[1] = I.p0;
+    next[2] = I.p1;
+    next[3] = I.J0;
+    next[4] = I.K0;
+    next[5] = I.col;
   };
   const auto produce = [&]() {
     const int item = next[0];
-    if (item >= n_items) return;
-    const int P = next[1], J0 = next[2], K0 = next[3], g32 = next[4];
+    if (item >= W.n_items) return;
+    const int P = next[1], J0 = next[3], K0 = next[4], g32 = next[5];
     const int st = n_loads % kRStages;
     ++n_loads;
     unsigned char* dst = smem + (size_t)st * kRStageBytes;
@@ -2010,7 +2137,7 @@ __global__ void __launch_bounds__(kRThreads, 1)
       tma_load_5d(dst + kROffP, &tm_p, g32, 0, P, J0 - 1, K0 - 1, &full[st]);
     }
     tma_load_4d(dst + (kUpdate ? kROffE : 8 * kRPatch), &tm_e, g32, P - 1, J0 - 1, K0 - 1, &full[st]);
-    if (P < NX)
+    if (P < next[2])
       next[1] = P + 1;
     else
       place(item + gridDim.x);
@@ -2019,30 +2146,39 @@ __global__ void __launch_bounds__(kRThreads, 1)
     for (int st = 0; st < kRStages; ++st) mbar_init(&full[st], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     place(blockIdx.x);
-    for (int q = 0; q < kRStages; ++q) produce();
+    for (int st = 0; st < kRStages; ++st) produce();
   }
   __syncthreads();
   const int ej = w % kREJ, ek = w / kREJ;
   const bool node_warp = ej >= 1 && ek >= 1;
   uint32_t seq = 0;
-  int xsel = 0;
   bool dead = false;
   auto csync = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kRWarps * 32) : "memory"); };
+  constexpr int kPart = kRJ * kRK * 32;
+  auto flush = [&](const WalkItem& I) {  // partial sums of the item's chunks (as k_lvl_op2)
+    const int chunk = W.chunk_of(I.a) + w / 2, i = w % 2;
+    if (chunk > W.chunk_of(I.b)) return;
+    const double* rd = red + (chunk * 2 + i) * kPart + lane;
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < kRJ * kRK; ++k) sum += rd[k * 32];
+    partial[(((int64_t)I.tile * W.n_chunk + chunk) * Rp + I.col + lane) * 2 + i] = sum;
+  };
   auto plane_sync = [&]() {
     csync();
     if (producer && !dead) produce();
   };
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int tile = item % n_tiles, g32 = (item / n_tiles) * 32;
-    const int J0 = 1 + (tile % tiles_j) * kRJ, K0 = 1 + (tile / tiles_j) * kRK;
-    const int Je = J0 - 1 + ej, Ke = K0 - 1 + ek;
+  for (int item = blockIdx.x; item < W.n_items; item += gridDim.x) {
+    const WalkItem I = walk_item<kSeg, kRJ, kRK, 32>(W, item, NX);
+    const int g32 = I.col;
+    const int Je = I.J0 - 1 + ej, Ke = I.K0 - 1 + ek;
     auto realj = [&](int j) { return j >= 1 && j <= L.NY - 1; };
     auto realk = [&](int k) { return k >= 1 && k <= L.NZ - 1; };
     const bool real = realj(Je) && realk(Ke);
     const bool node_ok = node_warp && Je <= L.NY && Ke <= L.NZ;
     const bool r00 = real, r10 = realj(Je - 1) && realk(Ke);
     const bool r01 = realj(Je) && realk(Ke - 1), r11 = realj(Je - 1) && realk(Ke - 1);
-    const size_t nrow = ((size_t)Je + (size_t)L.NYp * Ke) * L.NXp;
+    const uint32_t nrow = ((uint32_t)Je + (uint32_t)L.NYp * Ke) * L.NXp;
     const int rr = g32 + lane;
     double al = 0.0;
     if constexpr (kUpdate) al = (double)alpha[rr];
@@ -2059,19 +2195,19 @@ __global__ void __launch_bounds__(kRThreads, 1)
     float ndv = 0.f;
     auto prefetch = [&](int X) {
       if (!node_ok) return;
-      const size_t node = nrow + X;
+      const uint32_t node = nrow + X;
       ndv = dinv[node * Rp + rr];
 #pragma unroll
       for (int c = 0; c < 3; ++c) nb[c] = kBPerR ? b[(node * 3 + c) * Rp + rr] : b[node * 3 + c];
     };
     auto node_phase = [&](int X) {
-      if (((X - 1) & 31) == 0) {
+      if (((X - I.a) & 31) == 0) {
         const int pl = X + lane;
         mreg = (pl <= NX) ? mask[nrow + pl] : 0u;
       }
-      const uint32_t mk = __shfl_sync(0xffffffffu, mreg, (X - 1) & 31);
-      const double* xb = xbuf + xsel * kRXDoubles;
-      const size_t node = nrow + X;
+      const uint32_t mk = __shfl_sync(0xffffffffu, mreg, (X - I.a) & 31);
+      const double* xb = xbuf + (X & 1) * kRXDoubles;
+      const uint32_t node = nrow + X;
       const double dv = (double)ndv;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -2080,7 +2216,7 @@ __global__ void __launch_bounds__(kRThreads, 1)
         if (r10) y += xb[(((w - 1) * 4 + 1) * 3 + c) * 32 + lane];
         if (r01) y += xb[(((w - kREJ) * 4 + 2) * 3 + c) * 32 + lane];
         if (r11) y += xb[(((w - kREJ - 1) * 4 + 3) * 3 + c) * 32 + lane];
-        const size_t o = (node * 3 + c) * Rp + rr;
+        const uint32_t o = (node * 3 + c) * Rp + rr;
         const double bv = nb[c];
         const double rc = ((mk >> c) & 1) ? 0.0 : bv - y;
         const float rf = (float)rc;
@@ -2089,10 +2225,17 @@ __global__ void __launch_bounds__(kRThreads, 1)
         acc_dz = fma(dv * (double)rf, (double)rf, acc_dz);
       }
     };
-    auto emit_corners = [&](const double (&B)[3][4]) {
+    auto leave = [&](int chunk) {  // partial sums of a chunk
+      if (!node_warp) return;
+      double* rd = red + (chunk * 2 * kRK * kRJ + (ek - 1) * kRJ + (ej - 1)) * 32 + lane;
+      rd[0] = acc_rr;
+      rd[kPart] = acc_dz;
+      acc_rr = acc_dz = 0.0;
+    };
+    auto emit_corners = [&](const double (&B)[3][4], int X) {  // of plane X
       double y[2][2][3];
       yz_inverse(B, y);
-      double* xb = xbuf + xsel * kRXDoubles;
+      double* xb = xbuf + (X & 1) * kRXDoubles;
 #pragma unroll
       for (int ay = 0; ay < 2; ++ay)
 #pragma unroll
@@ -2100,19 +2243,20 @@ __global__ void __launch_bounds__(kRThreads, 1)
 #pragma unroll
           for (int c = 0; c < 3; ++c) xb[((w * 4 + ay + 2 * az) * 3 + c) * 32 + lane] = y[ay][az][c];
     };
-    for (int P = 1; P <= NX; ++P, ++seq) {
+    double u[2][2][3], Bc[3][4], E = 0.0;
+    // plane P of the walk: the corner values and their yz modes; the owner writes
+    auto plane = [&](int P) {
       const int st = seq % kRStages;
       if (!dead && !mbar_wait(&full[st], (seq / kRStages) & 1)) {
         atomicExch(err, 1);
         dead = true;
       }
-      if (P >= 2) prefetch(P - 1);
+      if (kSeg ? P > I.a : P > 1) prefetch(P - 1);
       const unsigned char* pt = smem + (size_t)st * kRStageBytes;
       const double* px = reinterpret_cast<const double*>(pt + kROffX);
       const float* pd = reinterpret_cast<const float*>(pt + kROffD);
       const float* pp = reinterpret_cast<const float*>(pt + kROffP);
       const double* pe = reinterpret_cast<const double*>(pt + (kUpdate ? kROffE : 8 * kRPatch));
-      double u[2][2][3];
 #pragma unroll
       for (int ay = 0; ay < 2; ++ay)
 #pragma unroll
@@ -2126,52 +2270,55 @@ __global__ void __launch_bounds__(kRThreads, 1)
             u[ay][az][c] = v;
           }
         }
-      const double E = pe[w * 32 + lane];
+      E = pe[w * 32 + lane];
       if constexpr (kUpdate) {
-        if (node_ok) {
-          const size_t node = nrow + P;
+        if (node_ok && (!kSeg || (P >= I.a && P <= I.b))) {
+          const uint32_t node = nrow + P;
 #pragma unroll
           for (int c = 0; c < 3; ++c) x_out[(node * 3 + c) * Rp + rr] = u[0][0][c];
         }
       }
-      double Bc[3][4];
       yz_forward(u, Bc);
-      if (P >= 2) {
+    };
+    auto keep = [&]() {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int qq = 0; qq < 4; ++qq) Bp[c][qq] = Bc[c][qq];
+      ++seq;
+    };
+    plane(I.p0);
+    keep();
+    int P = I.p0 + 1, chunk = W.chunk_of(I.a);
+    for (;; ++chunk) {
+      const int ce = (chunk + 1) * W.chunk;  // the chunk's last plane
+      for (const int last = min(ce + 1, I.p1); P <= last; ++P) {
+        plane(P);
         if (real) {
           double C1[3][4];
           modal_apply<kMass>(C, E, Bp, Bc, T0, C1);
-          emit_corners(T0);
+          emit_corners(T0, P - 1);
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int qq = 0; qq < 4; ++qq) T0[c][qq] = C1[c][qq];
         }
         plane_sync();
-        if (node_ok) node_phase(P - 1);
-        xsel ^= 1;
+        if (node_ok && (!kSeg || P > I.a)) node_phase(P - 1);  // (plane a - 1 is the neighbour's)
+        keep();
       }
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int qq = 0; qq < 4; ++qq) Bp[c][qq] = Bc[c][qq];
+      if (ce >= I.b) break;
+      leave(chunk);
     }
-    prefetch(NX);
-    if (real) emit_corners(T0);
+    if (!kSeg || I.b == NX) {  // plane NX: the slab above it is a ghost
+      prefetch(NX);
+      if (real) emit_corners(T0, NX);
+      csync();
+      if (node_ok) node_phase(NX);
+    }
+    leave(chunk);
     plane_sync();
-    if (node_ok) node_phase(NX);
-    xsel ^= 1;
-    if (node_warp) {
-      const int nw = (ek - 1) * kRJ + (ej - 1);
-      red[(0 * kRJ * kRK + nw) * 32 + lane] = acc_rr;
-      red[(1 * kRJ * kRK + nw) * 32 + lane] = acc_dz;
-    }
-    csync();
-    if (w < 2) {
-      double sum = 0.0;
-#pragma unroll
-      for (int i = 0; i < kRJ * kRK; ++i) sum += red[(w * kRJ * kRK + i) * 32 + lane];
-      partial[((size_t)tile * Rp + rr) * 2 + w] = sum;
-    }
+    flush(I);
   }
 }
 
@@ -2392,6 +2539,7 @@ struct Scal {
 // Per-realization sum of NV interleaved partials over n rows, 32 realizations x
 // 32 row-groups per CTA; fixed summation order (row-group sequential, then the
 // 32 groups in order), so results are reproducible and independent of the batch.
+// The result is warp 0's (the last sum by every warp took 4 us of shared loads).
 template <int NV>
 __device__ __forceinline__ void reduce_rows(const double* __restrict__ partial, int n, int Rp, double (&out)[NV]) {
   __shared__ double sh[32][NV][33];
@@ -2400,19 +2548,31 @@ __device__ __forceinline__ void reduce_rows(const double* __restrict__ partial, 
   double acc[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) acc[q] = 0.0;
-  for (int t = g; t < n; t += 32)
+  int t = g;
+  for (; t + 96 < n; t += 128) {  // four rows' loads in flight, added in order
+    double v[4][NV];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int q = 0; q < NV; ++q) v[u][q] = partial[((size_t)(t + 32 * u) * Rp + r) * NV + q];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int q = 0; q < NV; ++q) acc[q] += v[u][q];
+  }
+  for (; t < n; t += 32)
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q] += partial[((size_t)t * Rp + r) * NV + q];
 #pragma unroll
   for (int q = 0; q < NV; ++q) sh[g][q][lane] = acc[q];
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    double s = 0.0;
-#pragma unroll 4
-    for (int gg = 0; gg < 32; ++gg) s += sh[gg][q][lane];
-    out[q] = s;
-  }
+  for (int q = 0; q < NV; ++q) out[q] = 0.0;
+  if (g > 0) return;
+#pragma unroll 8
+  for (int gg = 0; gg < 32; ++gg)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) out[q] += sh[gg][q][lane];
 }
 
 // After a true-residual replacement: convergence test, new reference norm and
@@ -2453,7 +2613,7 @@ __global__ void __launch_bounds__(1024) k_resid_scalars(int Rp, int n_tiles, con
   if (threadIdx.x == 0 && active) atomicAdd(s.n_active, active);
 }
 
-// Scalars of the single-reduction loop after k_op_modal: with gamma = (dinv r).r
+// Scalars of the single-reduction loop after k_jacobi_op: with gamma = (dinv r).r
 // of the launch's r, alpha = gamma / p.q, gamma' = gamma - 2 alpha (dinv r).q +
 // alpha^2 q.dinv.q (the gamma of the next r), beta = gamma' / gamma;
 // a reliable update is requested once gamma has dropped by delta^2 since the
@@ -2927,7 +3087,8 @@ struct GmgLevel {
   size_t sweep_smem = 0;  // coarsest level: all sweeps in one k_coarse_sweeps launch (0: launch per sweep)
   // packed operator (k_lvl_op2) on this level: x patches, element patches, own b and dinv
   ModalCT<float2> MC2;
-  int tiles_j2 = 0, n_tiles2 = 0, n_items2 = 0, grid2 = 0;
+  Walk W2;
+  int grid2 = 0;
   CUtensorMap tm2_x, tm2_e, tm2_bo, tm2_dinvo;
 };
 
@@ -2949,6 +3110,15 @@ struct BlockSys {
   WSlot x, r32, p, q, d, dinv, blat, E64, E32, part_op, part_up, scal, pB, rB, qB;
   size_t scal_bytes = 0;
   Scal s;
+  int groups = 0, kq = 1;  // 16-wide realization groups with items, and how many follow each other
+  // items of an operator launch on lattice Lw (tiles of tj x tk node pencils, ctas an
+  // SM) and its grid
+  Walk walk(Context* ctx, const Lattice& Lw, int tj, int tk, int n_groups, int q, int ctas, int* grid) const {
+    const int tiles_j = (Lw.NY + tj - 1) / tj, n_tiles = tiles_j * ((Lw.NZ + tk - 1) / tk);
+    const Walk W = make_walk(Lw.NX, tiles_j, n_tiles, n_groups, q, ctas * ctx->sm_count);
+    *grid = X.persistent ? std::min(W.n_items, ctas * ctx->sm_count) : W.n_items;
+    return W;
+  }
   int slot_alloc(Context* ctx, int slot, size_t bytes, void** out) {
     if (!own) return workspace(ctx, slot, bytes, out);
     if (own[slot].bytes < bytes) {
@@ -2963,7 +3133,7 @@ struct BlockSys {
   // between x and xB (the step writes x + d + alpha p into the other buffer)
   WSlot xB;
   ModalCD MCD;
-  int tiles_jr = 0, n_tiles_r = 0, n_items_r = 0, grid_r = 0;
+  int grid_r = 0;
   CUtensorMap tm_xr, tm_xBr, tm_dr, tm_pr, tm_er;
   // multigrid preconditioner: levels 1..n_lvl-1 (level 0 is this lattice), the
   // level-0 pre-smoothed iterate xs, the damping and the coarsest-level sweeps
@@ -2976,7 +3146,8 @@ struct BlockSys {
   // packed level-0 operator (k_lvl_op2: 16 realizations per item, 7 x 3 tiles)
   bool pack = false;
   ModalCT<float2> MC2;
-  int tiles_j2 = 0, n_tiles2 = 0, n_items2 = 0, grid2 = 0;
+  Walk W2, WJ, WR;  // level operator, Jacobi operator, true residual
+  int grid2 = 0, grid_j = 0;
   CUtensorMap tm2_rA, tm2_rB, tm2_qA, tm2_qB, tm2_pA, tm2_pB, tm2_xs, tm2_dinv, tm2_e, tm2_d;
   CUtensorMap tm2_rAo, tm2_rBo, tm2_dinvo;  // own-tile boxes of r (both buffers) and dinv (post-sweep)
   // level-0 search-direction launch on the tensor cores (k_lvl_tc): the B operand
@@ -3185,8 +3356,25 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
   MSG_TRY(B->slot_alloc(ctx, 6, sizeof(double) * npad * Rp, &B->E64.ptr));
   MSG_TRY(B->slot_alloc(ctx, 7, sizeof(float) * npad * Rp, &B->E32.ptr));
   MSG_TRY(B->slot_alloc(ctx, 8, sizeof(double) * npad * 3, &B->blat.ptr));
-  MSG_TRY(B->slot_alloc(ctx, 9, sizeof(double) * (size_t)std::max(B->n_tiles * 2, B->n_tiles_m * kMParts) * Rp,
-                    &B->part_op.ptr));
+  // packed operators: 7 x 3 tiles of 16 realizations. Partials: [tile, chunk][Rp][parts]
+  // of the Jacobi loop, [tile, chunk][Rp][2] and [tile, chunk][Rp] of the multigrid
+  // loop (the tensor-core direction launch writes the latter over its own tiles),
+  // [tile, chunk][Rp][2] of the true residual over its smaller tiles
+  if (Rp % (kQQuad * kQR) != 0)
+    return set_error(ctx, MSG_ERR_INVALID_ARGUMENT, "batch of %d realizations is not padded to %d", Rp, kQQuad * kQR);
+  // realization groups with a realization of the batch (a multiple of four or two of
+  // them, or all when fewer, so that items of neighbouring groups share rows)
+  B->groups = (R + kQR - 1) / kQR;
+  if (B->groups > kQQuad) B->groups = (B->groups + 1) / 2 * 2;
+  B->kq = B->groups <= kQQuad ? B->groups : B->groups % 4 == 0 ? 4 : 2;
+  B->W2 = B->walk(ctx, L, kQJ, kQK, B->groups, B->kq, kQCtas, &B->grid2);
+  B->WJ = B->walk(ctx, L, kQJ, kQK, B->groups, B->kq, 1, &B->grid_j);
+  B->WR = B->walk(ctx, L, kRJ, kRK, (R + 31) / 32, 1, 1, &B->grid_r);
+  const size_t n_part = std::max({(size_t)B->n_tiles * 2, (size_t)B->n_tiles_m * 3,
+                                  (size_t)B->W2.n_tiles * B->W2.n_chunk * kMParts,
+                                  (size_t)B->W2.n_tiles * B->W2.n_chunk * 2 + B->n_tiles_m,
+                                  (size_t)B->WR.n_tiles * B->WR.n_chunk * 2});
+  MSG_TRY(B->slot_alloc(ctx, 9, sizeof(double) * n_part * Rp, &B->part_op.ptr));
   MSG_TRY(B->slot_alloc(ctx, 10, sizeof(double) * (size_t)std::max(B->n_upd, B->n_bsq) * Rp * 2, &B->part_up.ptr));
   B->scal_bytes = (sizeof(float) * 2 + sizeof(double) * 6 + sizeof(int) * 5) * (size_t)Rp + 64;
   MSG_TRY(B->slot_alloc(ctx, 11, B->scal_bytes, &B->scal.ptr));
@@ -3253,6 +3441,18 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
     return encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, ed, es, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
+  // boxes of the packed operators: patches with halo, elements, own nodes
+  const cuuint32_t pb2[5] = {kQR, 3, 1, kQPJ, kQPK};
+  const cuuint32_t nb2[4] = {kQR, 1, kQPJ, kQPK};
+  const cuuint32_t eb2[4] = {kQR, 1, kQEJ, kQEK};
+  const cuuint32_t db2[5] = {kQR, 3, 1, kQJ, kQK};
+  const cuuint32_t ob2[4] = {kQR, 1, kQJ, kQK};
+  auto pack_c = [](const ModalC& f, ModalCT<float2>& g2) {
+    auto b2 = [](float v) { return make_float2(v, v); };
+    g2.vd = b2(f.vd); g2.vb = b2(f.vb); g2.sa = b2(f.sa); g2.sb = b2(f.sb); g2.pa = b2(f.pa); g2.pb = b2(f.pb);
+    g2.td = b2(f.td); g2.tb = b2(f.tb); g2.da = b2(f.da);
+    for (int i = 0; i < 8; ++i) g2.m[i] = b2(f.m[i]);
+  };
   CUresult e = CUDA_SUCCESS;
   if (B->modal) {
     // modal loop: r, q, p (both buffers) and dinv patches with halo, the element patch, the tile's d
@@ -3260,6 +3460,14 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
     const cuuint32_t nbm[4] = {32, 1, kMPJ, kMPK};
     const cuuint32_t ebm[4] = {32, 1, kMEJ, kMEK};
     const cuuint32_t dbm[5] = {32, 3, 1, kMJ, kMK};
+    pack_c(B->MC, B->MC2);
+    const CUresult r2[9] = {enc5(&B->tm2_rA, B->r32.ptr, pb2), enc5(&B->tm2_rB, B->rB.ptr, pb2),
+                            enc5(&B->tm2_qA, B->q.ptr, pb2),   enc5(&B->tm2_qB, B->qB.ptr, pb2),
+                            enc5(&B->tm2_pA, B->p.ptr, pb2),   enc5(&B->tm2_pB, B->pB.ptr, pb2),
+                            enc4(&B->tm2_dinv, B->dinv.ptr, nb2), enc4(&B->tm2_e, B->E32.ptr, eb2),
+                            enc5(&B->tm2_d, B->d.ptr, db2)};
+    for (CUresult r : r2)
+      if (r != CUDA_SUCCESS) e = r;
     const CUresult rs[9] = {enc5(&B->tm_rAm, B->r32.ptr, pbm), enc5(&B->tm_rBm, B->rB.ptr, pbm),
                             enc5(&B->tm_qAm, B->q.ptr, pbm),   enc5(&B->tm_qBm, B->qB.ptr, pbm),
                             enc5(&B->tm_pAm, B->p.ptr, pbm),   enc5(&B->tm_pBm, B->pB.ptr, pbm),
@@ -3288,18 +3496,18 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)};
       for (CUresult r : r64)
         if (r != CUDA_SUCCESS) e = r;
-      B->tiles_jr = (L.NY + kRJ - 1) / kRJ;
-      B->n_tiles_r = B->tiles_jr * ((L.NZ + kRK - 1) / kRK);
-      B->n_items_r = B->n_tiles_r * (Rp / 32);
-      B->grid_r = B->X.persistent ? std::min(B->n_items_r, ctx->sm_count) : B->n_items_r;
     }
     static std::once_flag resid_once;
     static cudaError_t resid_err = cudaSuccess;
     std::call_once(resid_once, [] {
-      const void* fs[] = {(const void*)k_resid_modal<false, false, false>, (const void*)k_resid_modal<false, false, true>,
-                          (const void*)k_resid_modal<false, true, false>,  (const void*)k_resid_modal<false, true, true>,
-                          (const void*)k_resid_modal<true, false, false>,  (const void*)k_resid_modal<true, false, true>,
-                          (const void*)k_resid_modal<true, true, false>,   (const void*)k_resid_modal<true, true, true>};
+      const void* fs[] = {(const void*)k_resid_modal<false, false, false, false>, (const void*)k_resid_modal<false, false, true, false>,
+                          (const void*)k_resid_modal<false, false, false, true>, (const void*)k_resid_modal<false, false, true, true>,
+                          (const void*)k_resid_modal<false, true, false, false>, (const void*)k_resid_modal<false, true, true, false>,
+                          (const void*)k_resid_modal<false, true, false, true>, (const void*)k_resid_modal<false, true, true, true>,
+                          (const void*)k_resid_modal<true, false, false, false>, (const void*)k_resid_modal<true, false, true, false>,
+                          (const void*)k_resid_modal<true, false, false, true>, (const void*)k_resid_modal<true, false, true, true>,
+                          (const void*)k_resid_modal<true, true, false, false>, (const void*)k_resid_modal<true, true, true, false>,
+                          (const void*)k_resid_modal<true, true, false, true>, (const void*)k_resid_modal<true, true, true, true>};
       for (const void* f : fs)
         if (resid_err == cudaSuccess)
           resid_err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRSmem);
@@ -3308,9 +3516,11 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
     static std::once_flag attr_once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(attr_once, [] {
-      attr_err = cudaFuncSetAttribute(k_op_modal<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMSmem);
-      if (attr_err == cudaSuccess)
-        attr_err = cudaFuncSetAttribute(k_op_modal<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMSmem);
+      const void* fs[] = {(const void*)k_jacobi_op<false, false>, (const void*)k_jacobi_op<false, true>,
+                          (const void*)k_jacobi_op<true, false>, (const void*)k_jacobi_op<true, true>};
+      for (const void* f : fs)
+        if (attr_err == cudaSuccess)
+          attr_err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)JacStage::kSmem);
     });
     MSG_CUDA(ctx, attr_err);
   }
@@ -3434,46 +3644,15 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
       // packed level-0 operator: realizations in multiples of 64
       B->pack = ctx->mg_packed && (Rp % (kQQuad * kQR)) == 0;
       if (B->pack) {
-        auto b2 = [](float v) { return make_float2(v, v); };
-        auto pack_c = [&](const ModalC& f, ModalCT<float2>& g2) {
-          g2.vd = b2(f.vd); g2.vb = b2(f.vb); g2.sa = b2(f.sa); g2.sb = b2(f.sb); g2.pa = b2(f.pa); g2.pb = b2(f.pb);
-          g2.td = b2(f.td); g2.tb = b2(f.tb); g2.da = b2(f.da);
-          for (int i = 0; i < 8; ++i) g2.m[i] = b2(f.m[i]);
-        };
-        pack_c(B->MC, B->MC2);
-        B->tiles_j2 = (L.NY + kQJ - 1) / kQJ;
-        B->n_tiles2 = B->tiles_j2 * ((L.NZ + kQK - 1) / kQK);
-        B->n_items2 = B->n_tiles2 * (Rp / kQR);
-        B->grid2 = B->X.persistent ? std::min(B->n_items2, kQCtas * ctx->sm_count) : B->n_items2;
-        // the loop's partials: [tile][Rp][2] and [tile][Rp] over the packed tiles (the
-        // tensor-core direction launch writes its [tile][Rp] over its own tiles)
-        const size_t need = sizeof(double) * (size_t)std::max({B->n_tiles * 2, B->n_tiles_m * kMParts, B->n_tiles2 * 3,
-                                                                B->tc ? B->n_tiles2 * 2 + B->n_tiles_m : 0}) * Rp;
-        MSG_TRY(B->slot_alloc(ctx, 9, need, &B->part_op.ptr));
-        const cuuint32_t pb2[5] = {kQR, 3, 1, kQPJ, kQPK};
-        const cuuint32_t nb2[4] = {kQR, 1, kQPJ, kQPK};
-        const cuuint32_t eb2[4] = {kQR, 1, kQEJ, kQEK};
-        const cuuint32_t db2[5] = {kQR, 3, 1, kQJ, kQK};
-        const cuuint32_t ob2[4] = {kQR, 1, kQJ, kQK};
         if (enc5(&B->tm2_rAo, B->r32.ptr, db2) != CUDA_SUCCESS || enc5(&B->tm2_rBo, B->rB.ptr, db2) != CUDA_SUCCESS ||
-            enc4(&B->tm2_dinvo, B->dinv.ptr, ob2) != CUDA_SUCCESS)
+            enc4(&B->tm2_dinvo, B->dinv.ptr, ob2) != CUDA_SUCCESS || enc5(&B->tm2_xs, B->xs.ptr, pb2) != CUDA_SUCCESS)
           return set_error(ctx, MSG_ERR_CUDA, "cuTensorMapEncodeTiled failed (packed)");
-        const CUresult r2[10] = {enc5(&B->tm2_rA, B->r32.ptr, pb2), enc5(&B->tm2_rB, B->rB.ptr, pb2),
-                                 enc5(&B->tm2_qA, B->q.ptr, pb2),   enc5(&B->tm2_qB, B->qB.ptr, pb2),
-                                 enc5(&B->tm2_pA, B->p.ptr, pb2),   enc5(&B->tm2_pB, B->pB.ptr, pb2),
-                                 enc5(&B->tm2_xs, B->xs.ptr, pb2),  enc4(&B->tm2_dinv, B->dinv.ptr, nb2),
-                                 enc4(&B->tm2_e, B->E32.ptr, eb2),  enc5(&B->tm2_d, B->d.ptr, db2)};
-        for (CUresult r : r2)
-          if (r != CUDA_SUCCESS) return set_error(ctx, MSG_ERR_CUDA, "cuTensorMapEncodeTiled failed (packed)");
         // the coarse levels' residual and post-sweeps on the packed operator too
         for (int l = 1; l < n_lvl; ++l) {
           GmgLevel& g = B->lv[l];
           const Lattice& Lc = g.L;
           pack_c(g.MC, g.MC2);
-          g.tiles_j2 = (Lc.NY + kQJ - 1) / kQJ;
-          g.n_tiles2 = g.tiles_j2 * ((Lc.NZ + kQK - 1) / kQK);
-          g.n_items2 = g.n_tiles2 * (Rp / kQR);
-          g.grid2 = B->X.persistent ? std::min(g.n_items2, kQCtas * ctx->sm_count) : g.n_items2;
+          g.W2 = B->walk(ctx, Lc, kQJ, kQK, B->groups, B->kq, kQCtas, &g.grid2);
           const cuuint64_t cpd[5] = {(cuuint64_t)Rp, 3, (cuuint64_t)Lc.NXp, (cuuint64_t)Lc.NYp, (cuuint64_t)Lc.NZp};
           const cuuint64_t cps[4] = {Rp * fb, 3 * Rp * fb, 3 * Rp * fb * Lc.NXp, 3 * Rp * fb * Lc.NXp * Lc.NYp};
           const cuuint64_t ced[4] = {(cuuint64_t)Rp, (cuuint64_t)Lc.NXp, (cuuint64_t)Lc.NYp, (cuuint64_t)Lc.NZp};
@@ -3636,7 +3815,7 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
       const CUtensorMap& tn2 = kMode == kLvlSmooth ? B->tm2_dinvo : B->tm2_dinv;
       const CUtensorMap& tbb = kMode == kLvlSmooth ? (even ? B->tm2_rBo : B->tm2_rAo) : tb2;
       k<<<B->grid2, kQThreads, LvlStage2<kMode>::kSmem, st>>>(
-          B->L, B->MC2, ta2, tbb, tn2, B->tm2_e, B->tm2_d, B->tiles_j2, B->n_tiles2, B->n_items2, B->mask, b, dinv,
+          B->L, B->MC2, ta2, tbb, tn2, B->tm2_e, B->tm2_d, B->W2, B->mask, b, dinv,
           om, s.alpha, s.beta, out, out2, out3, d, partial, pstride, s.err);
     } else {
       lvl(mode, B->L, B->MC, ta, tb, B->tm_dinvm, B->tm_em, B->tm_dm, B->tiles_jm, B->n_tiles_m, B->n_items_m,
@@ -3649,7 +3828,7 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
     if (B->pack) {
       auto k = mass ? k_lvl_op2<kMode, true> : k_lvl_op2<kMode, false>;
       k<<<g.grid2, kQThreads, LvlStage2<kMode>::kSmem, st>>>(
-          g.L, g.MC2, g.tm2_x, g.tm2_bo, g.tm2_dinvo, g.tm2_e, g.tm2_x, g.tiles_j2, g.n_tiles2, g.n_items2, g.mask, g.b,
+          g.L, g.MC2, g.tm2_x, g.tm2_bo, g.tm2_dinvo, g.tm2_e, g.tm2_x, g.W2, g.mask, g.b,
           g.dinv, g.omega, s.alpha, s.beta, g.t, nullptr, nullptr, nullptr, nullptr, 1, s.err);
     } else {
       lvl(mode, g.L, g.MC, g.tm_x, g.tm_x, g.tm_x, g.tm_e, g.tm_x, g.tiles_j, g.n_tiles, g.n_items, g.grid, g.mask,
@@ -3714,7 +3893,7 @@ void gmg_iteration(BlockSys* B, const LoopCfg& c, int it, cudaStream_t st) {
   Scal& s = B->s;
   cudaEvent_t* ev = B->X.ev;
   const bool even = (it & 1) == 0;
-  const int nt0 = B->pack ? B->n_tiles2 : B->n_tiles_m;
+  const int nt0 = B->pack ? B->W2.n_tiles * B->W2.n_chunk : B->n_tiles_m;
   double* part2 = B->part_op.as<double>();
   double* part1 = part2 + (size_t)2 * nt0 * Rp;
   float* p_out = even ? B->pB.as<float>() : B->p.as<float>();
@@ -3729,7 +3908,7 @@ void gmg_iteration(BlockSys* B, const LoopCfg& c, int it, cudaStream_t st) {
     if (B->pack) {
       auto k = mass ? k_lvl_op2<kMode, true> : k_lvl_op2<kMode, false>;
       k<<<B->grid2, kQThreads, LvlStage2<kMode>::kSmem, st>>>(
-          B->L, B->MC2, ta2, tb2, B->tm2_dinv, B->tm2_e, B->tm2_d, B->tiles_j2, B->n_tiles2, B->n_items2, B->mask,
+          B->L, B->MC2, ta2, tb2, B->tm2_dinv, B->tm2_e, B->tm2_d, B->W2, B->mask,
           nullptr, nullptr, B->omega, s.alpha, s.beta, out, out2, nullptr, d, partial, pstride, s.err);
     } else {
       auto k = mass ? k_lvl_op<kMode, true> : k_lvl_op<kMode, false>;
@@ -3795,17 +3974,24 @@ int block_graph(Context* ctx, BlockSys* B, const LoopCfg& c, cudaGraphExec_t* ou
     mix(mm, sizeof(mm));
     const int gg[5] = {B->gmg ? 1 : 0, B->n_lvl, B->sweeps, B->pack ? 1 : 0, B->tc ? 1 : 0};
     mix(gg, sizeof(gg));
+    {
+      const CUtensorMap* t2[9] = {&B->tm2_rA, &B->tm2_rB, &B->tm2_qA, &B->tm2_qB, &B->tm2_pA,
+                                  &B->tm2_pB, &B->tm2_dinv, &B->tm2_e, &B->tm2_d};
+      for (const CUtensorMap* t : t2) mix(t, sizeof(CUtensorMap));
+      mix(&B->MC2, sizeof(B->MC2));
+      mix(&B->W2, sizeof(Walk));
+      mix(&B->WJ, sizeof(Walk));
+      const int m2[2] = {B->grid2, B->grid_j};
+      mix(m2, sizeof(m2));
+    }
     if (B->gmg) {
       mix(&B->omega, sizeof(B->omega));
       mix(&B->xs.ptr, sizeof(void*));
       mix(&B->tm_xs, sizeof(CUtensorMap));
       for (int l = 1; l < B->n_lvl; ++l) mix(&B->lv[l], sizeof(GmgLevel));
       if (B->pack) {
-        const CUtensorMap* t2[13] = {&B->tm2_rA, &B->tm2_rB, &B->tm2_qA, &B->tm2_qB, &B->tm2_pA,
-                                     &B->tm2_pB, &B->tm2_xs, &B->tm2_dinv, &B->tm2_e, &B->tm2_d,
-                                     &B->tm2_rAo, &B->tm2_rBo, &B->tm2_dinvo};
+        const CUtensorMap* t2[4] = {&B->tm2_xs, &B->tm2_rAo, &B->tm2_rBo, &B->tm2_dinvo};
         for (const CUtensorMap* t : t2) mix(t, sizeof(CUtensorMap));
-        mix(&B->MC2, sizeof(B->MC2));
       }
     }
     const double dd[2] = {c.delta2, c.tol2};
@@ -3831,16 +4017,18 @@ int block_graph(Context* ctx, BlockSys* B, const LoopCfg& c, cudaGraphExec_t* ou
         // alternate between their two buffers
         const bool even = (it & 1) == 0;
         if (it == 0) cudaEventRecordWithFlags(ev[4], st, cudaEventRecordExternal);
-        auto op = B->mass ? k_op_modal<true> : k_op_modal<false>;
-        op<<<B->grid_m, kMThreads, kMSmem, st>>>(
-            L, B->MC, even ? B->tm_rAm : B->tm_rBm, even ? B->tm_qAm : B->tm_qBm, even ? B->tm_pAm : B->tm_pBm,
-            B->tm_dinvm, B->tm_em, B->tm_dm, B->tiles_jm, B->n_tiles_m, B->n_items_m, mask, s.alpha, s.beta,
+        // whole walks without segment bounds in registers: 148 us against 152 at 24^3 x 256
+        auto op = B->WJ.nseg > 1 ? (B->mass ? k_jacobi_op<true, true> : k_jacobi_op<false, true>)
+                                 : (B->mass ? k_jacobi_op<true, false> : k_jacobi_op<false, false>);
+        op<<<B->grid_j, kJThreads, JacStage::kSmem, st>>>(
+            L, B->MC, even ? B->tm2_rA : B->tm2_rB, even ? B->tm2_qA : B->tm2_qB, even ? B->tm2_pA : B->tm2_pB,
+            B->tm2_dinv, B->tm2_e, B->tm2_d, B->WJ, mask, s.alpha, s.beta,
             even ? rB.as<float>() : r32.as<float>(), even ? pB.as<float>() : p.as<float>(),
             even ? qB.as<float>() : q.as<float>(), d.as<float>(), part_op.as<double>(), s.err);
         if (it == 0) cudaEventRecordWithFlags(ev[5], st, cudaEventRecordExternal);
         cudaMemsetAsync(s.n_active, 0, 32, st);  // n_active and n_update
         if (it == 0) cudaEventRecordWithFlags(ev[6], st, cudaEventRecordExternal);
-        k_alpha_gamma<<<c.sblocks, 1024, 0, st>>>(Rp, B->n_tiles_m, part_op.as<double>(), s, c.delta2, c.tol2);
+        k_alpha_gamma<<<c.sblocks, 1024, 0, st>>>(Rp, B->WJ.n_tiles * B->WJ.n_chunk, part_op.as<double>(), s, c.delta2, c.tol2);
         if (it == 0) cudaEventRecordWithFlags(ev[7], st, cudaEventRecordExternal);
       }
     }
@@ -3882,19 +4070,20 @@ int block_update(Context* ctx, BlockSys* B, const LoopCfg& c, const double* b, b
   }
   {
     // x += d + alpha p (into the other x buffer) and the FP64 residual in one pass
-    auto pick = [&](auto M, auto P, auto U) {
-      return k_resid_modal<decltype(M)::value, decltype(P)::value, decltype(U)::value>;
-    };
     using T1 = std::true_type;
     using F0 = std::false_type;
+    auto pick = [&](auto M, auto P, auto U) {
+      constexpr bool kM = decltype(M)::value, kP = decltype(P)::value, kU = decltype(U)::value;
+      // whole walks without segment bounds in registers: 1.32 ms against 1.39 at 32^3 x 1024
+      return B->WR.nseg > 1 ? k_resid_modal<kM, kP, kU, true> : k_resid_modal<kM, kP, kU, false>;
+    };
     const bool upd = !first;
     auto k = B->mass ? (b_per_r ? (upd ? pick(T1{}, T1{}, T1{}) : pick(T1{}, T1{}, F0{}))
                                 : (upd ? pick(T1{}, F0{}, T1{}) : pick(T1{}, F0{}, F0{})))
                      : (b_per_r ? (upd ? pick(F0{}, T1{}, T1{}) : pick(F0{}, T1{}, F0{}))
                                 : (upd ? pick(F0{}, F0{}, T1{}) : pick(F0{}, F0{}, F0{})));
-    k<<<B->grid_r, kRThreads, kRSmem, st>>>(L, B->MCD, B->tm_xr, B->tm_dr, B->tm_pr, B->tm_er, B->tiles_jr,
-                                             B->n_tiles_r, B->n_items_r, mask, b, dinv, s.alpha, B->xB.as<double>(),
-                                             r32, part, s.err);
+    k<<<B->grid_r, kRThreads, kRSmem, st>>>(L, B->MCD, B->tm_xr, B->tm_dr, B->tm_pr, B->tm_er, B->WR, mask, b,
+                                             dinv, s.alpha, B->xB.as<double>(), r32, part, s.err);
     if (upd) {
       MSG_CUDA(ctx, cudaMemsetAsync(B->d.ptr, 0, sizeof(float) * B->nvec, st));
       std::swap(B->x.ptr, B->xB.ptr);
@@ -3902,7 +4091,7 @@ int block_update(Context* ctx, BlockSys* B, const LoopCfg& c, const double* b, b
     }
   }
   MSG_CUDA(ctx, cudaMemsetAsync(s.n_active, 0, 32, st));
-  k_resid_scalars<<<c.sblocks, 1024, 0, st>>>(Rp, B->n_tiles_r, part, s, tol, first ? 1 : 0, B->gmg ? 2 : 1,
+  k_resid_scalars<<<c.sblocks, 1024, 0, st>>>(Rp, B->WR.n_tiles * B->WR.n_chunk, part, s, tol, first ? 1 : 0, B->gmg ? 2 : 1,
                                                max_it);
   count_launch(ctx, 2);
   MSG_CUDA(ctx, cudaGetLastError());
@@ -4722,7 +4911,7 @@ void gmg_precond_buffers(void* handle, float** r_lat, float** z_lat, const int**
   *Rp = P->B.Rp;
   // the level-0 post-sweep's partials z.r' ([tile][Rp][2], component 1)
   *zr_part = P->B.part_op.as<double>() + 1;
-  *zr_blocks = P->B.pack ? P->B.n_tiles2 : P->B.n_tiles_m;
+  *zr_blocks = P->B.pack ? P->B.W2.n_tiles * P->B.W2.n_chunk : P->B.n_tiles_m;
 }
 
 void gmg_precond_destroy(void* handle) { delete static_cast<GmgPrecondImpl*>(handle); }

@@ -75,3 +75,62 @@ def test_odd_moved_nodes(ctx):
         C.assemble(O.h8_stiffness_batch(model.element_xyz(), E[r], model.poisson)[0])
         xo, _ = C.pcg_jacobi(model.subdomains[0].RHS, tol=1e-13)
         assert np.abs(mc.Solutions[r] - xo).max() <= 1e-8 * np.abs(xo).max()
+
+
+def few_and_many(ctx, solve, few, many):
+    """Results of the first `few` realizations alone and within `many`."""
+    ctx.set_option("fixed_updates", 1)  # a realization's updates do not depend on the others
+    try:
+        return solve(few), solve(many)
+    finally:
+        ctx.set_option("fixed_updates", 0)
+
+
+# long axes are walked in segments by small batches, whole by large ones: partial
+# sums per chunk of planes, so that the same numbers come out to the last bit. Axes
+# of 6 to 40 elements: chunks of 3 to 10 planes, the last one short or of one plane
+@pytest.mark.parametrize("nx,ny,nz,many", [(6, 6, 6, 300), (12, 12, 12, 1000), (13, 10, 7, 900), (25, 4, 4, 1100),
+                                           (40, 5, 5, 700)])
+def test_segments_give_the_same_numbers(ctx, nx, ny, nz, many):
+    few, K = 2, 12
+    xi = np.random.default_rng(nx).standard_normal((many, K))
+    model = M.clamped_block_model(nx, ny=ny, nz=nz)
+    kl = M.LognormalStochasticCoefficientsProvider([nx, ny, nz], 0.3 * nx, K, 8)
+
+    def solve(R):
+        mc = M.MonteCarloAnalyzerWithStochasticMaterial(ctx, model, kl, expansion_order=K, simulations=R, seed=1,
+                                                        mode="mixed", tolerance=1e-10)
+        mc.Initialize()
+        mc.RandomNumbers = xi[:R]
+        mc.Solve()
+        return mc.Solutions[:few].copy(), mc.Iterations[:few].copy()
+
+    (xf, itf), (xm, itm) = few_and_many(ctx, solve, few, many)
+    assert np.array_equal(itf, itm)
+    assert np.array_equal(xf, xm)
+
+
+@pytest.mark.parametrize("n,R", [(5, 2), (9, 3), (10, 17)])
+def test_newmark_segments(ctx, n, R):
+    """The Jacobi loop in segments against the oracle's direct solves, with the
+    bounds of the batched Newmark parity test (tip 1e-8, final field 1e-7: each
+    step is solved to 1e-11)."""
+    steps, dt = 6, 0.01
+    model = M.clamped_block_model(n)
+    kl = M.LognormalStochasticCoefficientsProvider([n, n, n], 0.2 * n, 12, 6)
+    load = M.MassAccelerationSinusoidalLoad(1.0, dt, dt * steps, 0.1, dof=0)
+    corner = int(np.argmax(model.xyz.sum(1)))
+    nm = M.NewmarkDynamicAnalyzer(ctx, model, kl, 0.25, 0.5, dt, dt * steps, load, expansion_order=12,
+                                  simulations=R, density=1.0, rayleigh_alpha=0.01, rayleigh_beta=0.001,
+                                  tolerance=1e-11, tip_dof=int(model.dof[corner, 0]))
+    nm.RandomNumbers = np.random.default_rng(n).standard_normal((R, 12))
+    hist = nm.Solve()
+    E = O.kl_field(O.centroids(model.xyz, model.conn), [n, n, n], kl.table(), nm.RandomNumbers, mean=kl.mean,
+                   sigma=kl.sigma, mean_correction=kl.mean_correction)
+    cons = (model.dof < 0).astype(np.uint8)
+    for r in (0, R - 1):
+        t, u, info = O.block_newmark(n, n, n, cons, E[r], model.poisson, 1.0, 0.01, 0.001, 0.25, 0.5, dt, steps, 0.1,
+                                     1.0, 0, model.n_dofs, tip_dof=nm.tip_dof)
+        assert info["status"] == 0
+        assert np.abs(hist[r] - t).max() <= 1e-8 * np.abs(t).max()
+        assert np.abs(nm.Solutions[r] - u).max() <= 1e-7 * np.abs(u).max()
