@@ -56,8 +56,8 @@ namespace {
 
 constexpr int kEbeWarps = 8;   // warps per CTA
 constexpr int kEbeCheck = 8;   // iterations per chunk (graph launch) between host reads of the flags
-constexpr int kRgBlk = 64;     // nodes per work item of the operator passes: 8 warps x 8 nodes
-constexpr int kRgBlkU = 256;   // nodes per work item of the update pass: 8 warps x 32 nodes
+constexpr int kRgBlk = 8;      // nodes per work item of the operator passes: 8 warps x 1 node
+constexpr int kRgBlkU = 32;    // nodes per work item of the update passes: 8 warps x 4 nodes
 constexpr int kRgParts = 5;    // partial arrays per system over kRgBlk blocks
 enum { kPq = 0, kDrq = 1, kDqd = 2, kZr = 3, kRr = 4 };
 
@@ -155,6 +155,37 @@ __device__ __forceinline__ void rg_block_partials(const T (&v)[N], double (&sh)[
     dst(i)[l] = t;
   }
   __syncthreads();
+}
+
+constexpr int kRgFlight = 4;  // nodes of a warp in flight
+using RgOffsets = size_t[3 * kRgFlight];
+using RgNodes = int[kRgFlight];
+// Nodes n, n + 8, ... below n1 of a warp, N at a time and then one by one: body(count,
+// offsets of the three components of each, nodes). The body loads everything before
+// it stores, since the compiler cannot move a load across a store to another of the
+// system's vectors.
+template <class Body>
+__device__ __forceinline__ void rg_stream(int n, int n1, int Rp, int col, Body body) {
+  constexpr int N = kRgFlight;
+  RgOffsets o;
+  RgNodes nn;
+  auto offsets = [&](int m) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i < m) {
+        nn[i] = n + kEbeWarps * i;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o[3 * i + c] = ((size_t)nn[i] * 3 + c) * Rp + col;
+      }
+  };
+  for (; n + kEbeWarps * (N - 1) < n1; n += kEbeWarps * N) {
+    offsets(N);
+    body(std::integral_constant<int, N>{}, o, nn);
+  }
+  for (; n < n1; n += kEbeWarps) {
+    offsets(1);
+    body(std::integral_constant<int, 1>{}, o, nn);
+  }
 }
 
 __device__ __forceinline__ double* rg_part(const RgSys& S, int k, int blk, int col) {
@@ -307,12 +338,14 @@ __device__ __forceinline__ void rg_apply_item(const RgSys& S, int blk, int rb, d
   }
 }
 
-// Every G in one kernel at 128 registers a thread (2 CTAs an SM): each
-// variant gets registers for many gathers in flight. Compiled alone, G = 4
-// takes 80 registers (3 CTAs an SM) and runs 24 % slower at 32^3 x 512.
+// Bound by the latency of the gathers: 13 warps an SM were active on average with
+// items of 64 nodes, whose last wave left most SMs idle (313 us at 24^3 x 200, 111
+// for 20^3 and 12^3 x 64 together, 180 items there). A node a warp and three CTAs an SM (80 registers):
+// 241 and 70 us; two CTAs (128 registers) are 4 % slower over a solve, items of 16
+// nodes equal on large meshes and up to 25 % slower on small ones.
 // pq_only (the standard PCG of ebe_mg_solve): p.q alone, without the partials
 // of beta's expansion and their reads of r and D^-1.
-__global__ void __launch_bounds__(32 * kEbeWarps, 2) k_rg_apply(const RgSys* __restrict__ Sys,
+__global__ void __launch_bounds__(32 * kEbeWarps, 3) k_rg_apply(const RgSys* __restrict__ Sys,
                                                             const RgItem* __restrict__ items, int n_items,
                                                             const int* __restrict__ gact, int pq_only) {
   __shared__ double sh[kEbeWarps * 32];
@@ -331,9 +364,11 @@ __global__ void __launch_bounds__(32 * kEbeWarps, 2) k_rg_apply(const RgSys* __r
 
 // d += alpha p, r -= alpha q, p = D r + beta p; partials (D r).r and r.r. A
 // memory-bound pass with nothing to share between realization groups: work
-// items of 256 nodes and one group, one CTA each (few registers, long streams
-// per warp, two nodes in flight); items of groups without a running
-// realization skipped.
+// items of 32 nodes and one group, one CTA each, a warp's four nodes in flight
+// together; items of groups without a running realization skipped. (One node and
+// component after another in items of 256 nodes, a load's latency each:
+// k_vc_update 79 us at 24^3 x 200 and 60 for 20^3 and 12^3 x 64, 51 and 13 now;
+// k_vc_dir 58 and 55, 24 and 9.)
 __global__ void __launch_bounds__(32 * kEbeWarps) k_rg_update(const RgSys* __restrict__ Sys,
                                                              const RgItem* __restrict__ items, int n_items,
                                                              RgScal s) {
@@ -347,20 +382,27 @@ __global__ void __launch_bounds__(32 * kEbeWarps) k_rg_update(const RgSys* __res
     const int n1 = min(S.n_nodes, (I.blk + 1) * kRgBlkU);
     const float al = s.alpha[S.goff + col + lane], be = s.beta[S.goff + col + lane];
     double zr = 0.0, rr = 0.0;
-#pragma unroll 2
-    for (int n = I.blk * kRgBlkU + w; n < n1; n += kEbeWarps)
+    rg_stream(I.blk * kRgBlkU + w, n1, Rp, col + lane, [&](auto m, const RgOffsets& o, const RgNodes&) {
+      constexpr int M = 3 * decltype(m)::value;
+      float pv[M], qv[M], rv[M], dv[M], di[M];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const size_t o = ((size_t)n * 3 + c) * Rp + col + lane;
-        const float pv = S.p[o];
-        const float rv = fmaf(-al, S.q[o], S.r[o]);
-        S.d[o] = fmaf(al, pv, S.d[o]);
-        const float zv = S.dinv[o] * rv;
-        S.p[o] = fmaf(be, pv, zv);
-        S.r[o] = rv;
-        zr += (double)zv * (double)rv;
-        rr += (double)rv * (double)rv;
+      for (int i = 0; i < M; ++i) {
+        pv[i] = S.p[o[i]];
+        qv[i] = S.q[o[i]];
+        rv[i] = S.r[o[i]];
+        dv[i] = S.d[o[i]];
+        di[i] = S.dinv[o[i]];
       }
+#pragma unroll
+      for (int i = 0; i < M; ++i) {
+        const float rn = fmaf(-al, qv[i], rv[i]), zv = di[i] * rn;
+        S.d[o[i]] = fmaf(al, pv[i], dv[i]);
+        S.p[o[i]] = fmaf(be, pv[i], zv);
+        S.r[o[i]] = rn;
+        zr += (double)zv * (double)rn;
+        rr += (double)rn * (double)rn;
+      }
+    });
     const double v[2] = {zr, rr};
     rg_block_partials(v, sh, [&](int i) { return S.part_u + ((size_t)i * S.n_blk_u + I.blk) * Rp + col; });
   }
@@ -376,16 +418,22 @@ __global__ void k_rg_fold(const RgSys* __restrict__ Sys, const RgItem* __restric
     if (!all && !s.sreq[I.sys]) continue;
     const RgSys S = Sys[I.sys];
     const int n1 = min(S.n_nodes, (I.blk + 1) * kRgBlk);
-    for (int g = 0; g < I.G; ++g) {
-      const int col = I.rb + 32 * g + lane;
-      for (int n = I.blk * kRgBlk + w; n < n1; n += kEbeWarps)
+    for (int g = 0; g < I.G; ++g)
+      rg_stream(I.blk * kRgBlk + w, n1, S.Rp, I.rb + 32 * g + lane, [&](auto m, const RgOffsets& o, const RgNodes&) {
+        constexpr int M = 3 * decltype(m)::value;
+        double xv[M];
+        float dv[M];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const size_t o = ((size_t)n * 3 + c) * S.Rp + col;
-          S.x[o] += (double)S.d[o];
-          S.d[o] = 0.f;
+        for (int i = 0; i < M; ++i) {
+          xv[i] = S.x[o[i]];
+          dv[i] = S.d[o[i]];
         }
-    }
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+          S.x[o[i]] = xv[i] + (double)dv[i];
+          S.d[o[i]] = 0.f;
+        }
+      });
   }
 }
 
@@ -458,7 +506,15 @@ __global__ void __launch_bounds__(32 * kEbeWarps) k_rg_resid64(const RgSys* __re
 __device__ __forceinline__ double rg_sum(const double* __restrict__ part, int n_blk, int Rp, int r) {
   const int lane = threadIdx.x & 31;
   double v = 0.0;
-  for (int i = lane; i < n_blk; i += 32) v += part[(size_t)i * Rp + r];
+  int i = lane;
+  for (; i + 224 < n_blk; i += 256) {  // eight loads in flight, added in order
+    double t[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t[k] = part[(size_t)(i + 32 * k) * Rp + r];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v += t[k];
+  }
+  for (; i < n_blk; i += 32) v += part[(size_t)i * Rp + r];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -700,17 +756,27 @@ __global__ void __launch_bounds__(32 * kEbeWarps) k_vc_update(const RgSys* __res
     const int n1 = min(S.n_nodes, (I.blk + 1) * kRgBlkU);
     const float al = s.alpha[S.goff + col + lane];
     double rr = 0.0;
-#pragma unroll 2
-    for (int n = I.blk * kRgBlkU + w; n < n1; n += kEbeWarps)
+    rg_stream(I.blk * kRgBlkU + w, n1, Rp, col + lane, [&](auto m, const RgOffsets& o, const RgNodes& n) {
+      constexpr int N = decltype(m)::value;
+      float pv[3 * N], qv[3 * N], rv[3 * N], dv[3 * N];
+      int nl[N];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const size_t o = ((size_t)n * 3 + c) * Rp + col + lane;
-        const float rv = fmaf(-al, S.q[o], S.r[o]);
-        S.d[o] = fmaf(al, S.p[o], S.d[o]);
-        S.r[o] = rv;
-        if (S.lmap) S.rl[((size_t)__ldg(S.lmap + n) * 3 + c) * Rp + col + lane] = rv;  // the V-cycle's input
-        rr += (double)rv * (double)rv;
+      for (int i = 0; i < 3 * N; ++i) {
+        pv[i] = S.p[o[i]];
+        qv[i] = S.q[o[i]];
+        rv[i] = S.r[o[i]];
+        dv[i] = S.d[o[i]];
+        if (i < N) nl[i] = S.lmap ? __ldg(S.lmap + n[i]) : 0;
       }
+#pragma unroll
+      for (int i = 0; i < 3 * N; ++i) {
+        const float rn = fmaf(-al, qv[i], rv[i]);
+        S.d[o[i]] = fmaf(al, pv[i], dv[i]);
+        S.r[o[i]] = rn;
+        if (S.lmap) S.rl[((size_t)nl[i / 3] * 3 + i % 3) * Rp + col + lane] = rn;  // the V-cycle's input
+        rr += (double)rn * (double)rn;
+      }
+    });
     rg_block_partial(rr, sh, S.part_u + ((size_t)1 * S.n_blk_u + I.blk) * Rp + col);
   }
 }
@@ -726,14 +792,20 @@ __global__ void __launch_bounds__(32 * kEbeWarps) k_vc_dir(const RgSys* __restri
     const int Rp = S.Rp, col = I.rb;
     const int n1 = min(S.n_nodes, (I.blk + 1) * kRgBlkU);
     const float be = s.beta[S.goff + col + lane];
-#pragma unroll 2
-    for (int n = I.blk * kRgBlkU + w; n < n1; n += kEbeWarps)
+    rg_stream(I.blk * kRgBlkU + w, n1, Rp, col + lane, [&](auto m, const RgOffsets& o, const RgNodes& n) {
+      constexpr int N = decltype(m)::value;
+      float pv[3 * N], zv[3 * N];
+      int nl[N];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const size_t o = ((size_t)n * 3 + c) * Rp + col + lane;
-        const size_t oz = S.lmap ? ((size_t)__ldg(S.lmap + n) * 3 + c) * Rp + col + lane : o;
-        S.p[o] = fmaf(be, S.p[o], S.z[oz]);
+      for (int i = 0; i < N; ++i) nl[i] = S.lmap ? __ldg(S.lmap + n[i]) : n[i];
+#pragma unroll
+      for (int i = 0; i < 3 * N; ++i) {
+        pv[i] = S.p[o[i]];
+        zv[i] = S.z[((size_t)nl[i / 3] * 3 + i % 3) * Rp + col + lane];
       }
+#pragma unroll
+      for (int i = 0; i < 3 * N; ++i) S.p[o[i]] = fmaf(be, pv[i], zv[i]);
+    });
   }
 }
 
@@ -751,15 +823,21 @@ __global__ void __launch_bounds__(32 * kEbeWarps) k_vc_jacobi_z(const RgSys* __r
     const int Rp = S.Rp, col = I.rb;
     const int n1 = min(S.n_nodes, (I.blk + 1) * kRgBlkU);
     double zr = 0.0;
-#pragma unroll 2
-    for (int n = I.blk * kRgBlkU + w; n < n1; n += kEbeWarps)
+    rg_stream(I.blk * kRgBlkU + w, n1, Rp, col + lane, [&](auto m, const RgOffsets& o, const RgNodes&) {
+      constexpr int M = 3 * decltype(m)::value;
+      float rv[M], di[M];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const size_t o = ((size_t)n * 3 + c) * Rp + col + lane;
-        const float rv = S.r[o], zv = S.dinv[o] * rv;
-        S.z[o] = zv;
-        zr += (double)zv * (double)rv;
+      for (int i = 0; i < M; ++i) {
+        rv[i] = S.r[o[i]];
+        di[i] = S.dinv[o[i]];
       }
+#pragma unroll
+      for (int i = 0; i < M; ++i) {
+        const float zv = di[i] * rv[i];
+        S.z[o[i]] = zv;
+        zr += (double)zv * (double)rv[i];
+      }
+    });
     rg_block_partial(zr, sh, S.part_u + (size_t)I.blk * Rp + col);
   }
 }

@@ -134,3 +134,28 @@ def test_newmark_segments(ctx, n, R):
         assert info["status"] == 0
         assert np.abs(hist[r] - t).max() <= 1e-8 * np.abs(t).max()
         assert np.abs(nm.Solutions[r] - u).max() <= 1e-7 * np.abs(u).max()
+
+
+# moved nodes: node counts around the element-by-element work items (8 and 32
+# nodes), the last one short; by the diagonal (under 216 elements on odd axes) and by
+# the V-cycle; one to four realization groups
+@pytest.mark.parametrize("nx,ny,nz,R", [(1, 1, 1, 3), (3, 3, 3, 33), (3, 1, 2, 40), (4, 4, 4, 64), (6, 5, 8, 100)])
+def test_moved_node_counts(ctx, nx, ny, nz, R):
+    K = 6
+    model = M.clamped_block_model(nx, ny=ny, nz=nz)
+    rng = np.random.default_rng(R)
+    top = np.array([nx, ny, nz])
+    free = (model.xyz > 0.5).all(axis=1) | (model.xyz == top).any(axis=1)
+    model.xyz[free] += 0.1 * rng.uniform(-1, 1, (int(free.sum()), 3))
+    kl = M.LognormalStochasticCoefficientsProvider([nx, ny, nz], 0.3 * nx, K, 8)
+    mc = M.MonteCarloAnalyzerWithStochasticMaterial(ctx, model, kl, expansion_order=K, simulations=R, seed=3,
+                                                    mode="mixed", tolerance=1e-10)
+    mc.Initialize()
+    mc.Solve()
+    rows = (0, R - 1)
+    E = O.kl_field(O.centroids(model.xyz, model.conn), [nx, ny, nz], kl.table(), mc.RandomNumbers[list(rows)], sigma=0.3)
+    for i, r in enumerate(rows):
+        C = O.CSR(model.n_nodes, model.conn, model.dof, model.n_dofs)
+        C.assemble(O.h8_stiffness_batch(model.element_xyz(), E[i], model.poisson)[0])
+        xo, _ = C.pcg_jacobi(model.subdomains[0].RHS, tol=1e-13)
+        assert np.abs(mc.Solutions[r] - xo).max() <= 1e-8 * np.abs(xo).max()
