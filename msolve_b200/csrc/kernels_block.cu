@@ -1214,72 +1214,80 @@ __global__ void __launch_bounds__(kMThreads, 1)
 
 // ---------------------------------------------------------------- coarsest-level sweeps
 // All damped Jacobi sweeps of the coarsest level in one launch: a CTA holds the
-// whole level for its 32 realizations in shared memory (the iterate, b, omega
-// dinv, E and the mask, real nodes only). A sweep is two phases with a CTA
-// barrier after each: every (element pencil, x-plane) pair, one a warp, forms
-// the plane's corner contributions from the two elements next to it; then every
-// node sums the four pencils around it and steps the iterate in place. It is
-// bound by the latency of these two phases (0.6 us a sweep on 2 x 2 x 2
-// elements; 19 sweeps 41 -> 14 us against marching along x with a barrier a
-// plane). Every sweep is the arithmetic of k_lvl_op<kLvlSmooth> in the same
-// order, so the iterates are identical to the launch-per-sweep loop.
-constexpr int kCsX = 4 * 3 * 32;  // corner contributions of one (pencil, plane) pair
+// whole level for 8 realizations in shared memory (the iterate, b, omega dinv, E
+// and the mask, real nodes only). A sweep is two phases with a CTA barrier after
+// each: every (element pencil, x-plane) pair, 8 lanes, forms the plane's corner
+// contributions from the two elements next to it; then every node sums the four
+// pencils around it and steps the iterate in place. Every sweep is the arithmetic
+// of k_lvl_op<kLvlSmooth> in the same order, so the iterates are identical to the
+// launch-per-sweep loop. Bound by the latency of the two phases. With 32
+// realizations a CTA the shared-memory traffic of a phase took longer than its
+// latency while most SMs had nothing to do: 19 sweeps on 2 x 2 x 2 elements
+// 26 us a launch, 16 with 8. Strides: nodes 24 floats apart, pairs kCsX, so that the
+// four rows of a warp's access lie in different banks.
+constexpr int kCsR = 8;                  // realizations of a CTA
+constexpr int kCsSub = 32 / kCsR;        // pairs or nodes of a warp
+constexpr int kCsX = 4 * 3 * kCsR + 8;   // corner contributions of one (pencil, plane) pair, padded
+constexpr int kCsWarps = 16;             // at most
 inline size_t coarse_sweep_smem(const Lattice& L) {
   const size_t nn = (size_t)L.NX * L.NY * L.NZ, np = (size_t)(L.NY - 1) * (L.NZ - 1), ne = np * (L.NX - 1);
-  return sizeof(float) * (nn * 32 * 7 + ne * 32 + np * L.NX * kCsX) + sizeof(int2) * (nn + np * L.NX);
+  return sizeof(float) * (nn * kCsR * 7 + ne * kCsR + np * L.NX * kCsX) + sizeof(int2) * (nn + np * L.NX);
+}
+inline int coarse_sweep_threads(const Lattice& L) {  // a warp for every four nodes (there are fewer pairs)
+  return 32 * std::min(kCsWarps, (L.NX * L.NY * L.NZ + kCsSub - 1) / kCsSub);
 }
 template <bool kMass>
-__global__ void __launch_bounds__(kMWarps * 32, 1)
+__global__ void __launch_bounds__(kCsWarps * 32, 1)
     k_coarse_sweeps(Lattice L, const __grid_constant__ ModalC C, const uint8_t* __restrict__ mask,
                     const float* __restrict__ b, const float* __restrict__ dinv, const float* __restrict__ E,
                     float omega, int n_sweeps, const float* __restrict__ x, float* __restrict__ out) {
   extern __shared__ __align__(16) float smem_cs[];
   const int NX = L.NX, NY = L.NY, NZ = L.NZ, Rp = L.Rp;
   const int nn = NX * NY * NZ, np = (NY - 1) * (NZ - 1), ne = np * (NX - 1);
-  float* it = smem_cs;            // iterate [node][c][32]
-  float* bs = it + nn * 96;       // b [node][c][32]
-  float* ws = bs + nn * 96;       // omega dinv [node][32]
-  float* es = ws + nn * 32;       // E [element][32]
-  float* xbuf = es + ne * 32;     // [pencil][plane][corner][c][32]
+  float* it = smem_cs;               // iterate [node][c][kCsR]
+  float* bs = it + nn * 3 * kCsR;    // b [node][c][kCsR]
+  float* ws = bs + nn * 3 * kCsR;    // omega dinv [node][kCsR]
+  float* es = ws + nn * kCsR;        // E [element][kCsR]
+  float* xbuf = es + ne * kCsR;      // [pencil][plane][corner][c][kCsR]
   // index tables, so that the sweeps divide nothing: (pencil, plane) pair u -> its
   // node 0 and element (X - 1 below, X above; bit 30, 31: there is one); node i ->
   // offset of the exchange of pencil (J - 1, K - 1), and its neighbours and mask
   int2* utab = reinterpret_cast<int2*>(xbuf + np * NX * kCsX);
   int2* ntab = utab + np * NX;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int rr = blockIdx.x * 32 + lane;
+  const int lane = threadIdx.x % kCsR, w = threadIdx.x / kCsR, nw = blockDim.x / kCsR;
+  const int rr = blockIdx.x * kCsR + lane;
   // 0-based node (X, J, K), element (X, j, k) and pencil (j, k)
   auto cn = [&](int X, int J, int K) { return X + NX * (J + NY * K); };
   auto pn = [&](int X, int J, int K) { return (size_t)(X + 1) + (size_t)L.NXp * ((size_t)(J + 1) + (size_t)L.NYp * (K + 1)); };
-  for (int i = w; i < nn; i += kMWarps) {
+  for (int i = w; i < nn; i += nw) {
     const int X = i % NX, J = (i / NX) % NY, K = i / (NX * NY);
     const size_t pi = pn(X, J, K);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      it[(i * 3 + c) * 32 + lane] = x[(pi * 3 + c) * Rp + rr];
-      bs[(i * 3 + c) * 32 + lane] = b[(pi * 3 + c) * Rp + rr];
+      it[(i * 3 + c) * kCsR + lane] = x[(pi * 3 + c) * Rp + rr];
+      bs[(i * 3 + c) * kCsR + lane] = b[(pi * 3 + c) * Rp + rr];
     }
-    ws[i * 32 + lane] = omega * dinv[pi * Rp + rr];
+    ws[i * kCsR + lane] = omega * dinv[pi * Rp + rr];
     if (lane == 0)
       ntab[i] = make_int2(((J - 1 + (NY - 1) * (K - 1)) * NX + X) * kCsX,
                           (J < NY - 1) | (J > 0) << 1 | (K < NZ - 1) << 2 | (K > 0) << 3 | mask[pi] << 4);
   }
-  for (int u = threadIdx.x; u < np * NX; u += kMWarps * 32) {
+  for (int u = threadIdx.x; u < np * NX; u += blockDim.x) {
     const int X = u % NX, p = u / NX;
     utab[u] = make_int2(cn(X, p % (NY - 1), p / (NY - 1)) | (X > 0) << 30, (p * (NX - 1) + X) | (X < NX - 1) << 30);
   }
-  for (int i = w; i < ne; i += kMWarps) {
+  for (int i = w; i < ne; i += nw) {
     const int X = i % (NX - 1), p = i / (NX - 1);
-    es[i * 32 + lane] = E[pn(X, p % (NY - 1), p / (NY - 1)) * Rp + rr];
+    es[i * kCsR + lane] = E[pn(X, p % (NY - 1), p / (NY - 1)) * Rp + rr];
   }
   __syncthreads();
   for (int sw = 0; sw < n_sweeps; ++sw) {
     // corner contributions of plane X of pencil p: the part of the element below
     // it (upper face), then that of the element above it (lower face)
-    for (int u = w; u < np * NX; u += kMWarps) {
+    for (int u = w; u < np * NX; u += nw) {
       const int2 t = utab[u];
       const bool below = t.x >> 30, above = t.y >> 30;
-      const float* i0 = it + (t.x & 0x3fffffff) * 96 + lane;
+      const float* i0 = it + (t.x & 0x3fffffff) * 3 * kCsR + lane;
       auto plane = [&](int d, float (&B)[3][4]) {
         float v[2][2][3];
 #pragma unroll
@@ -1287,10 +1295,10 @@ __global__ void __launch_bounds__(kMWarps * 32, 1)
 #pragma unroll
           for (int az = 0; az < 2; ++az)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[ay][az][c] = i0[(d + ay * NX + az * NX * NY) * 96 + c * 32];
+            for (int c = 0; c < 3; ++c) v[ay][az][c] = i0[((d + ay * NX + az * NX * NY) * 3 + c) * kCsR];
         yz_forward(v, B);
       };
-      const float* ep = es + (t.y & 0x3fffffff) * 32 + lane;
+      const float* ep = es + (t.y & 0x3fffffff) * kCsR + lane;
       float T0[3][4], C1[3][4], Bo[3][4], Bc[3][4];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
@@ -1299,7 +1307,7 @@ __global__ void __launch_bounds__(kMWarps * 32, 1)
       plane(0, Bc);
       if (below) {
         plane(-1, Bo);
-        modal_apply<kMass>(C, ep[-32], Bo, Bc, T0, C1);
+        modal_apply<kMass>(C, ep[-kCsR], Bo, Bc, T0, C1);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c)
@@ -1317,13 +1325,13 @@ __global__ void __launch_bounds__(kMWarps * 32, 1)
 #pragma unroll
         for (int az = 0; az < 2; ++az)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) xb[((ay + 2 * az) * 3 + c) * 32] = y[ay][az][c];
+          for (int c = 0; c < 3; ++c) xb[((ay + 2 * az) * 3 + c) * kCsR] = y[ay][az][c];
     }
     __syncthreads();
-    for (int i = w; i < nn; i += kMWarps) {
+    for (int i = w; i < nn; i += nw) {
       const int2 t = ntab[i];
       const uint32_t mk = t.y >> 4;
-      const float wdv = ws[i * 32 + lane];
+      const float wdv = ws[i * kCsR + lane];
       // pencils around the node: (J, K), (J - 1, K), (J, K - 1), (J - 1, K - 1)
       const bool jh = t.y & 1, jl = t.y & 2, kh = t.y & 4, kl = t.y & 8;
       const float* xb = xbuf + t.x + lane;
@@ -1331,21 +1339,21 @@ __global__ void __launch_bounds__(kMWarps * 32, 1)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         float y = 0.f;
-        if (jh && kh) y += xb[sj + sk + (0 * 3 + c) * 32];
-        if (jl && kh) y += xb[sk + (1 * 3 + c) * 32];
-        if (jh && kl) y += xb[sj + (2 * 3 + c) * 32];
-        if (jl && kl) y += xb[(3 * 3 + c) * 32];
-        const int o = (i * 3 + c) * 32 + lane;
+        if (jh && kh) y += xb[sj + sk + (0 * 3 + c) * kCsR];
+        if (jl && kh) y += xb[sk + (1 * 3 + c) * kCsR];
+        if (jh && kl) y += xb[sj + (2 * 3 + c) * kCsR];
+        if (jl && kl) y += xb[(3 * 3 + c) * kCsR];
+        const int o = (i * 3 + c) * kCsR + lane;
         it[o] = ((mk >> c) & 1) ? 0.f : fmaf(wdv, bs[o] - y, it[o]);
       }
     }
     __syncthreads();  // the sweep's iterate is complete before the next one reads it
   }
-  for (int i = w; i < nn; i += kMWarps) {
+  for (int i = w; i < nn; i += nw) {
     const int X = i % NX, J = (i / NX) % NY, K = i / (NX * NY);
     const size_t pi = pn(X, J, K);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) out[(pi * 3 + c) * Rp + rr] = it[(i * 3 + c) * 32 + lane];
+    for (int c = 0; c < 3; ++c) out[(pi * 3 + c) * Rp + rr] = it[(i * 3 + c) * kCsR + lane];
   }
 }
 
@@ -3858,7 +3866,7 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
     res_c = g.x;
     if (B->sweeps > 1) {
       auto k = mass ? k_coarse_sweeps<true> : k_coarse_sweeps<false>;
-      k<<<Rp / 32, kMWarps * 32, g.sweep_smem, st>>>(g.L, g.MC, g.mask, g.b, g.dinv, g.E32, g.omega, B->sweeps - 1, g.x,
+      k<<<(B->R + kCsR - 1) / kCsR, coarse_sweep_threads(g.L), g.sweep_smem, st>>>(g.L, g.MC, g.mask, g.b, g.dinv, g.E32, g.omega, B->sweeps - 1, g.x,
                                                       g.t);
       res_c = g.t;
     }

@@ -159,3 +159,24 @@ def test_moved_node_counts(ctx, nx, ny, nz, R):
         C.assemble(O.h8_stiffness_batch(model.element_xyz(), E[i], model.poisson)[0])
         xo, _ = C.pcg_jacobi(model.subdomains[0].RHS, tol=1e-13)
         assert np.abs(mc.Solutions[r] - xo).max() <= 1e-8 * np.abs(xo).max()
+
+
+# all sweeps of the coarsest level in one launch against a launch a sweep, bit for
+# bit: 8 realizations a CTA, the last one short; coarsest levels with fewer nodes than
+# a CTA's lanes take at a time, and with several rounds of them
+@pytest.mark.parametrize("nx,ny,nz,R", [(6, 6, 6, 1), (4, 4, 4, 9), (40, 5, 5, 17), (10, 30, 26, 5)])
+def test_fused_coarsest_sweeps(ctx, nx, ny, nz, R):
+    model = M.clamped_block_model(nx, ny=ny, nz=nz)
+    kl = M.LognormalStochasticCoefficientsProvider([nx, ny, nz], 0.3 * nx, 8, 8)
+    out = []
+    for fused in (0, 1):
+        ctx.set_option("multigrid_fused_coarse", fused)
+        try:
+            mc = M.MonteCarloAnalyzerWithStochasticMaterial(ctx, model, kl, expansion_order=8, simulations=R, seed=2,
+                                                            mode="mixed", tolerance=1e-10)
+            mc.Initialize()
+            mc.Solve()
+        finally:
+            ctx.set_option("multigrid_fused_coarse", 1)
+        out.append((mc.Solutions.copy(), mc.Iterations.copy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
