@@ -20,7 +20,7 @@ e2e    = the same through the host-buffer entry point with pinned buffers: xi an
          returns with the copy done).
 fp64_dropin = the plain FP64 drop-in (assembled BSR + Jacobi PCG, one
          realization after another, MSG_MODE_FP64_BSR) on a sample of the batch.
-roofline = the dominant kernel (k_op_modal: fused PCG direction update and
+roofline = the dominant kernel (k_jacobi_op: fused PCG direction update and
          matrix-free FP32 operator), live per-launch CUDA event durations
          inside the timed region.
 cpu_baseline = the oracle (C++ FP64 restatement of the reference: assembled
@@ -46,7 +46,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "Hexa8 PCG solves/s at 1e-8 rel err, batched mixed vs plain FP64; p50/p99 latency"
-# DRAM traffic of one k_op_modal launch per realization on the 32^3 lattice: ncu capture
+# DRAM traffic of one k_jacobi_op launch per realization on the 32^3 lattice: ncu capture
 # at R = 512 (dram__bytes_read.sum 1,165.9 MB + dram__bytes_write.sum 845.5 MB) / 512
 OP_DRAM_BYTES_PER_REALIZATION = (1165.921e6 + 845.472e6) / 512
 # the same for the multigrid loop's direction + operator launch (packed k_lvl_op2<PcgZ>, 3 x 3
@@ -869,7 +869,7 @@ def main():
 
     # roofline of the dominant kernel, the fused direction + matrix-free FP32 operator
     # (live per-launch samples from the timed region): k_lvl_op<PcgZ> in the multigrid
-    # loop, k_op_modal in the Jacobi loop
+    # loop, k_jacobi_op in the Jacobi loop
     mg = ctx.get_option("multigrid") != 0
     op_ms = st["op_launch_ms"]
     nn = model.n_nodes
@@ -888,7 +888,7 @@ def main():
         op_bytes = 4.0 * Rp * ((3 + 3 + 3 + 3 + 3 + 3) * nn + ne)
         per_r = None if tensor else MG_OP_DRAM_BYTES_PER_REALIZATION
     else:
-        op_kernel = "k_op_modal (fused PCG direction update + matrix-free FP32 Hexa8 operator)"
+        op_kernel = "k_jacobi_op (fused PCG direction update + matrix-free FP32 Hexa8 operator)"
         op_bytes = 4.0 * Rp * ((3 + 3 + 3 + 1 + 3 + 3 + 3) * nn + ne)
         per_r = OP_DRAM_BYTES_PER_REALIZATION
     hbm, peak_kind = load_peaks()

@@ -1370,7 +1370,8 @@ __global__ void __launch_bounds__(kCsWarps * 32, 1)
 // realizations, which computed 16 element pencils for 9 nodes (1.78; here 32
 // for 21, 1.52) and had 3 times fewer, longer items: search-direction launch
 // 134 -> 103 us at 24^3 x 256 (2.2 rounds of items there took 3), 22.6 ->
-// 18.5 us at 8^3 x 64 (24 CTAs instead of 9), 776 -> 755 us at 32^3 x 1024.
+// 18.5 us at 8^3 x 64 (24 CTAs instead of 9), 776 -> 755 us at 32^3 x 1024; with
+// segments, 32-bit offsets and the loads' position in shared memory 99, 12.3 and 731.
 // Four items of one tile follow each other, so that CTAs next to each other
 // read whole 256-byte rows (a 16-realization row is 64 bytes; one group after
 // another re-read 35 % of the DRAM bytes). There is no producer warp: lane 0
@@ -2969,17 +2970,22 @@ int modal_coefficients(Context* ctx, const double* K576, const double* M576, dou
     if ((m & 4) && !az) s = -s;
     return s;
   };
+  // T^T A T one side after the other (term by term it was 36,864 dependent sums, 55 us
+  // for every level of every call)
+  double sg[8][8];  // [mode][corner]
+  for (int m = 0; m < 8; ++m)
+    for (int a = 0; a < 8; ++a) sg[m][a] = sgn(a, m);
   auto to_modal = [&](const double* A, std::vector<double>& Am) {
+    std::vector<double> H(576, 0.0);  // A T
     Am.assign(576, 0.0);
+    for (int i = 0; i < 24; ++i)
+      for (int m2 = 0; m2 < 8; ++m2)
+        for (int b = 0; b < 8; ++b)
+          for (int c2 = 0; c2 < 3; ++c2) H[i * 24 + 3 * m2 + c2] += sg[m2][b] * A[i * 24 + 3 * b + c2];
     for (int m = 0; m < 8; ++m)
-      for (int c = 0; c < 3; ++c)
-        for (int m2 = 0; m2 < 8; ++m2)
-          for (int c2 = 0; c2 < 3; ++c2) {
-            double s = 0;
-            for (int a = 0; a < 8; ++a)
-              for (int b = 0; b < 8; ++b) s += sgn(a, m) * sgn(b, m2) * A[(3 * a + c) * 24 + 3 * b + c2];
-            Am[(3 * m + c) * 24 + 3 * m2 + c2] = s;
-          }
+      for (int a = 0; a < 8; ++a)
+        for (int c = 0; c < 3; ++c)
+          for (int j = 0; j < 24; ++j) Am[(3 * m + c) * 24 + j] += sg[m][a] * H[(3 * a + c) * 24 + j];
   };
   std::vector<double> Km;
   to_modal(K576, Km);

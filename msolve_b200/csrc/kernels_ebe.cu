@@ -1106,8 +1106,8 @@ struct RgBatch {
 // Plan and carve a batch: per-system sizes (Rp a multiple of rp_multiple[i]),
 // one realization-group count G for all systems (the smallest of theirs; each
 // divides the next), the work items (per system and node block, the
-// realization ranges one after another: operator passes 64 nodes and G groups,
-// the update 256 nodes and one group, so that CTAs running at the same time
+// realization ranges one after another: operator passes 8 nodes and G groups,
+// the update 32 nodes and one group, so that CTAs running at the same time
 // cover whole rows [node * 3 + c][0 .. Rp) of the vectors) and the arena, with
 // a z vector for each system with want_z[i].
 static int rg_batch_plan(Context* ctx, const std::vector<RgInput>& in, const std::vector<int>& rp_multiple,

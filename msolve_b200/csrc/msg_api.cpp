@@ -136,15 +136,19 @@ int copy_out(Context* ctx, const std::vector<HostCopy>& outs, cudaStream_t st) {
   std::vector<Piece> pieces;
   size_t total = 0;
   std::vector<int> staged(outs.size(), 0);
-  for (size_t i = 0; i < outs.size(); ++i) {
+  size_t all = 0;
+  for (const HostCopy& o : outs) all += o.bytes;
+  // small outputs ask nothing about the memory or the host's processors
+  for (size_t i = 0; i < outs.size() && all >= kCopyMin; ++i) {
     cudaPointerAttributes at{};
     const bool known = cudaPointerGetAttributes(&at, outs[i].dst) == cudaSuccess;
     if (!known) cudaGetLastError();
     staged[i] = !known || at.type == cudaMemoryTypeUnregistered;
     if (staged[i]) total += outs[i].bytes;
   }
-  const int threads = std::min<int>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency() / 2));
-  const bool pool_copy = total >= kCopyMin && threads > 1;
+  const int threads =
+      total >= kCopyMin ? std::min<int>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency() / 2)) : 1;
+  const bool pool_copy = threads > 1;
   for (size_t i = 0; i < outs.size(); ++i) {
     const HostCopy& o = outs[i];
     if (!pool_copy || !staged[i]) {

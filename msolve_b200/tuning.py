@@ -6,8 +6,8 @@ FP64 stopping rule. The choices are:
 
   multigrid           V-cycle preconditioned loop (1; 2 also for systems with
                       a mass term) or the Jacobi loop (0);
-  multigrid_packed    level operators on 3 x 3 node tiles of 64 realizations
-                      (two per lane, packed FP32: 1) or of 32 realizations (0);
+  multigrid_packed    level operators on 7 x 3 node tiles of 16 realizations
+                      (two per lane, packed FP32: 1) or on 3 x 3 tiles of 32 (0);
   multigrid_levels    depth of the V-cycle.
 
 Which one is fastest depends on the lattice, the batch (the number of work
