@@ -47,12 +47,12 @@ sys.path.insert(0, ROOT)
 
 METRIC = "Hexa8 PCG solves/s at 1e-8 rel err, batched mixed vs plain FP64; p50/p99 latency"
 # DRAM traffic of one k_jacobi_op launch per realization on the 32^3 lattice: ncu capture
-# at R = 512 (dram__bytes_read.sum 1,165.9 MB + dram__bytes_write.sum 845.5 MB) / 512
-OP_DRAM_BYTES_PER_REALIZATION = (1165.921e6 + 845.472e6) / 512
-# the same for the multigrid loop's direction + operator launch (packed k_lvl_op2<PcgZ>, 3 x 3
-# node tiles), 32^3 lattice, ncu capture at R = 512: dram__bytes_read.sum 823.2 MB +
-# dram__bytes_write.sum 626.8 MB
-MG_OP_DRAM_BYTES_PER_REALIZATION = (823.197e6 + 626.791e6) / 512
+# at R = 512 (dram__bytes_read.sum 1,200.6 MB + dram__bytes_write.sum 851.5 MB) / 512
+OP_DRAM_BYTES_PER_REALIZATION = (1200.583e6 + 851.539e6) / 512
+# the same for the multigrid loop's direction + operator launch (packed k_lvl_op2<PcgZ>, 7 x 3
+# node tiles), 32^3 lattice, ncu capture at R = 512: dram__bytes_read.sum 849.5 MB +
+# dram__bytes_write.sum 626.1 MB
+MG_OP_DRAM_BYTES_PER_REALIZATION = (849.515e6 + 626.134e6) / 512
 
 
 def parse():
