@@ -1387,6 +1387,7 @@ constexpr int kQWarps = kQEJ * kQEK / kQPencils;    // 8 warps
 constexpr int kQThreads = 32 * kQWarps;
 constexpr int kQCtas = 2;                           // CTAs per SM
 constexpr int kQQuad = 64 / kQR;                    // items of one tile next to each other at most: 64 realizations, whole 256-byte rows
+static_assert(kQR % kCsR == 0, "a group of realizations is whole CTAs of the coarsest sweeps");
 constexpr int kQPJ = kQJ + 2, kQPK = kQK + 2;       // node patch 9 x 5
 static_assert(kQEJ % kQPencils == 0, "a warp's pencils lie in one row");
 // Work items of an operator launch: the planes of a tile of node pencils for a group
@@ -3872,8 +3873,10 @@ void gmg_vcycle(BlockSys* B, Scal& s, bool even, cudaStream_t st) {
     res_c = g.x;
     if (B->sweeps > 1) {
       auto k = mass ? k_coarse_sweeps<true> : k_coarse_sweeps<false>;
-      k<<<(B->R + kCsR - 1) / kCsR, coarse_sweep_threads(g.L), g.sweep_smem, st>>>(g.L, g.MC, g.mask, g.b, g.dinv, g.E32, g.omega, B->sweeps - 1, g.x,
-                                                      g.t);
+      // the groups that the operators' items cover: B->R itself is not in the graph's
+      // key, and the same graph serves every batch of these groups
+      k<<<B->groups * (kQR / kCsR), coarse_sweep_threads(g.L), g.sweep_smem, st>>>(
+          g.L, g.MC, g.mask, g.b, g.dinv, g.E32, g.omega, B->sweeps - 1, g.x, g.t);
       res_c = g.t;
     }
   } else {
@@ -3986,7 +3989,7 @@ int block_graph(Context* ctx, BlockSys* B, const LoopCfg& c, cudaGraphExec_t* ou
     }
     const int mm[5] = {B->mass ? 1 : 0, B->n_tiles_m, B->n_items_m, B->grid_m, B->tiles_jm};
     mix(mm, sizeof(mm));
-    const int gg[5] = {B->gmg ? 1 : 0, B->n_lvl, B->sweeps, B->pack ? 1 : 0, B->tc ? 1 : 0};
+    const int gg[6] = {B->gmg ? 1 : 0, B->n_lvl, B->sweeps, B->pack ? 1 : 0, B->tc ? 1 : 0, B->groups};
     mix(gg, sizeof(gg));
     {
       const CUtensorMap* t2[9] = {&B->tm2_rA, &B->tm2_rB, &B->tm2_qA, &B->tm2_qB, &B->tm2_pA,
