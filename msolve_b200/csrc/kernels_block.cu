@@ -3779,7 +3779,8 @@ LoopCfg loop_cfg(Context* ctx, const BlockSys* B, double tol, int chunk_cap) {
     // a multigrid iteration cuts the residual several-fold: check every few
     // iterations, replace the residual after a larger drop
     c.chunk = 2;
-    c.delta2 = ctx->mg_delta * ctx->mg_delta;
+    const double delta = gmg_delta(B->L.NX - 1, B->L.NY - 1, B->L.NZ - 1, ctx->mg_delta);
+    c.delta2 = delta * delta;
   }
   // ask for a check once sqrt(gamma / gamma0) is at tol/4 (single-reduction loop,
   // dinv-weighted norm), or once the recursive residual is at tol/2 (multigrid loop)

@@ -88,6 +88,7 @@ struct RgSys {
   // (lzr[(block * Rp + realization) * 2], lzr_blocks blocks)
   const double* lzr;
   int lzr_blocks;
+  double delta2;  // ebe_mg_solve: squared reliable-update factor
 };
 struct RgItem {
   int sys, blk, rb, G;  // nodes blk * 64 .., realizations rb .. rb + 32 G - 1
@@ -865,8 +866,7 @@ __global__ void k_vc_alpha(const RgSys* __restrict__ Sys, int Rtot, RgScal s) {
 }
 
 // beta = gamma_new / gamma with gamma_new = z.r, and the true-residual check on r.r
-__global__ void k_vc_beta(const RgSys* __restrict__ Sys, int Rtot, RgScal s, double tol2, double delta2,
-                          int max_it) {
+__global__ void k_vc_beta(const RgSys* __restrict__ Sys, int Rtot, RgScal s, double tol2, int max_it) {
   const int g = rg_warp_index();
   if (g >= Rtot) return;
   const int lane = threadIdx.x & 31;
@@ -881,7 +881,7 @@ __global__ void k_vc_beta(const RgSys* __restrict__ Sys, int Rtot, RgScal s, dou
   if (lane != 0) return;
   s.beta[g] = s.gamma[g] > 0.0 ? (float)(zr / s.gamma[g]) : 0.f;
   s.gamma[g] = zr;
-  rg_check(s, g, rr, tol2, delta2, max_it);
+  rg_check(s, g, rr, tol2, S.delta2, max_it);
 }
 
 // Starting scalars: ||b|| from the init partials, gamma = z.b, beta = 0 (p = z)
@@ -1365,6 +1365,10 @@ int ebe_mg_solve(Context* ctx, const std::vector<RgInput>& in, const std::vector
     while ((int)ctx->vc_pool.size() < n_vc) ctx->vc_pool.push_back(new DevMem[kWorkSlots]);
   for (int i = 0, k = 0; i < S; ++i) {
     b.sys[i].kind = use_vcycle[i] ? 1 : 0;
+    // each system's own reliable-update factor: its lattice's, or the Jacobi loop's
+    const double delta = use_vcycle[i] ? gmg_delta(lats[i]->nx, lats[i]->ny, lats[i]->nz, ctx->mg_delta)
+                                       : ctx->reliable_delta;
+    b.sys[i].delta2 = delta * delta;
     if (!use_vcycle[i]) continue;
     DevMem* own = n_vc > 1 ? ctx->vc_pool[k++] : nullptr;
     MSG_TRY(gmg_precond_create(ctx, lats[i], in[i].nu, in[i].kl, in[i].d_xi, in[i].R, bufs[i].Rp, own, &P[i]));
@@ -1424,9 +1428,8 @@ int ebe_mg_solve(Context* ctx, const std::vector<RgInput>& in, const std::vector
   k_vc_dir<<<g_u, 32 * kEbeWarps, 0, st>>>(dS, d_items_u, n_items_u, s);
   count_launch(ctx, 2 + S);
   MSG_CUDA(ctx, cudaGetLastError());
-  // two iterations to a graph launch (the multigrid loop's chunk), its reliable-update factor
-  constexpr int kChunk = 2;
-  const double delta2 = ctx->mg_delta * ctx->mg_delta, tol2 = 0.25 * tol * tol;
+  constexpr int kChunk = 2;  // two iterations to a graph launch (the multigrid loop's chunk)
+  const double tol2 = 0.25 * tol * tol;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   MSG_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1436,7 +1439,7 @@ int ebe_mg_solve(Context* ctx, const std::vector<RgInput>& in, const std::vector
     k_vc_alpha<<<g_scal, 32 * kEbeWarps, 0, st>>>(dS, Rtot, s);
     k_vc_update<<<g_u, 32 * kEbeWarps, 0, st>>>(dS, d_items_u, n_items_u, s);
     precondition(nullptr, false);
-    k_vc_beta<<<g_scal, 32 * kEbeWarps, 0, st>>>(dS, Rtot, s, tol2, delta2, max_it);
+    k_vc_beta<<<g_scal, 32 * kEbeWarps, 0, st>>>(dS, Rtot, s, tol2, max_it);
     k_vc_dir<<<g_u, 32 * kEbeWarps, 0, st>>>(dS, d_items_u, n_items_u, s);
   }
   k_rg_chunk_end_count<<<g_scal, 32 * kEbeWarps, 0, st>>>(Rtot, s);
