@@ -359,9 +359,9 @@ typedef struct {
  * reference's SolverPCG with the diagonal preconditioner) with the iterate in
  * FP64 and FP64 true residuals, to ||b - K x||/||b|| < tol in FP64 for each
  * realization. With the multigrid option on (the default), a system whose mesh
- * has the numbering of an nx x ny x nz lattice that coarsens (every side at
- * least 3; with an odd side, at least 216 elements; moved nodes allowed) is
- * preconditioned instead by the V-cycle of its cube lattice, and then the whole batch runs standard PCG (the operator, scalar
+ * has the numbering of an nx x ny x nz lattice that coarsens (the rule of the
+ * option "multigrid"; moved nodes allowed) is preconditioned instead by the
+ * V-cycle of its cube lattice, and then the whole batch runs standard PCG (the operator, scalar
  * and vector launches shared, one V-cycle per such system, the diagonal for
  * the others; two iterations to a graph launch). A system's results do not
  * depend on the other systems in the batch: the same bits alone and in any mix
@@ -461,8 +461,8 @@ int MSG_SERVE_STOP(MSG_CTX ctx);
  * batched lattice loop: 1, default, a geometric multigrid V-cycle for systems
  * without a mass term (static solves, serving), Jacobi for those with one
  * (Newmark); 2: the V-cycle for both; 0: Jacobi for both. The V-cycle needs a
- * lattice with every side at least 3 and, with an odd side, at least 216
- * elements; otherwise Jacobi runs),
+ * lattice with every side at least 3 and, with an odd side, every side at least 5
+ * and at least 216 elements; otherwise Jacobi runs),
  * "multigrid_levels" (lattice levels at most, fine level included, 2..6,
  * default 6; a level halves every axis, rounding up, while the shortest has more
  * than 2 elements),

@@ -42,14 +42,18 @@ inline int gmg_side(int n, int l) {
 // Lattice levels of an nx x ny x nz lattice, the fine one included (1: it does not
 // coarsen), at most max_levels: every axis halves while the shortest has more than
 // two elements. Below that the 20 coarsest-level sweeps (one launch) are cheaper
-// than a level: 2 x 2 x 2 elements from a cube of any side. Lattices with an odd
-// axis (and more of the Jacobi loop's cheaper iterations than V-cycles: 140 to 600
-// against 25 to 30) coarsen from 216 elements on: 5^3 x 64 took 3.3 ms by Jacobi and
-// 3.7 by V-cycles, 7^3 4.6 and 3.8, 15^3 13.6 and 5.6, 33^3 72 and 13.3.
+// than a level: 2 x 2 x 2 elements from a cube of any side. Lattices with an odd axis
+// coarsen from 216 elements on: 5^3 x 64 took 3.3 ms by Jacobi (140 to 600 of its
+// cheaper iterations against 25 to 30) and 3.7 by V-cycles, 7^3 4.6 and 3.8, 15^3 13.6
+// and 5.6, 33^3 72 and 13.3; and from five elements thick: on thinner ones the
+// coarsest level is large, its sweeps take a launch each and leave much of the error
+// (one realization by Jacobi and by V-cycles: 40 x 40 x 3 3.4 and 10.4 ms, 3 x 40 x 40
+// 21.6 and 46.6, 41 x 41 x 4 4.2 and 12.2; 5 x 40 x 40 26 and 13, 5 x 20 x 20 11.2 and 6.4).
 inline int gmg_level_count(int nx, int ny, int nz, int max_levels) {
-  if (((nx | ny | nz) & 1) && (int64_t)nx * ny * nz < 216) return 1;
+  const int lo = nx < ny ? (nx < nz ? nx : nz) : (ny < nz ? ny : nz);
+  if (((nx | ny | nz) & 1) && (lo < 5 || (int64_t)nx * ny * nz < 216)) return 1;
   int n = 1;
-  for (int m = nx < ny ? (nx < nz ? nx : nz) : (ny < nz ? ny : nz); n < max_levels && m > 2; m = (m + 1) / 2) ++n;
+  for (int m = lo; n < max_levels && m > 2; m = (m + 1) / 2) ++n;
   return n;
 }
 
