@@ -350,8 +350,10 @@ __global__ void __launch_bounds__(32 * kStWarps, kDu ? 2 : 4)
     if (stresses) put(sg, stresses);
     if (forces) {
       // CalcH8Forces: w B^T stresses of the lane's Gauss point, summed in Gauss order
+      // with the zeros of B, where a stress is not finite (by overflow too)
       double zf[3] = {0, 0, 0};
-      if (odd) {
+      const double total = ((sg[0] + sg[1]) + (sg[2] + sg[3])) + (sg[4] + sg[5]);
+      if (!(fabs(total) <= kMaxDouble)) {
         zf[0] = 0.0 * sg[1] + 0.0 * sg[2] + 0.0 * sg[4];
         zf[1] = 0.0 * sg[0] + 0.0 * sg[2] + 0.0 * sg[5];
         zf[2] = 0.0 * sg[0] + 0.0 * sg[1] + 0.0 * sg[3];

@@ -69,3 +69,21 @@ def test_values_that_are_not_finite(ctx, bad):
         fine = np.isfinite(want)
         assert np.array_equal(fine, np.isfinite(got)) and np.array_equal(np.isnan(want), np.isnan(got))
         assert np.abs(got[fine] - want[fine]).max() <= 1e-12 * np.abs(want[fine]).max()
+
+
+def test_stresses_that_overflow(ctx):
+    """Finite strains and moduli whose product is not: a stretch along x of 1e300 at a
+    modulus of 1e10 (its rounding in the other strains, 1e284, stays finite there). The
+    force of every node is then NaN, the sum of products of infinite stresses with the
+    zeros of B."""
+    model = M.clamped_block_model(3, ny=2, nz=2)
+    rng = np.random.default_rng(1)
+    E = rng.uniform(0.5, 2.0, (3, model.n_elems))
+    X = 0.01 * rng.standard_normal((3, model.n_dofs))
+    E[1] = 1e10
+    X[1] = 0.0
+    free = model.dof[:, 0] >= 0
+    X[1, model.dof[free, 0]] = 1e300 * model.xyz[free, 0]
+    for got, want in zip(recover(ctx, model, E, X, 0), oracle(model, E, X)):
+        assert np.array_equal(np.isfinite(want), np.isfinite(got)) and np.array_equal(np.isnan(want), np.isnan(got))
+    assert np.isnan(want[1]).all()
