@@ -926,24 +926,19 @@ struct PcgLaunch {
   size_t smem = 0;
 };
 
-// The resident kernels' shared memory, allowed once a context (the limit is a device's,
-// and other devices' contexts may live in the process) and always the same: other
-// threads' solves of other sizes share it.
-int pcg_resident_limit(Context* ctx) {
-  if (ctx->pcg_limit) return MSG_OK;
-  const void* ks[] = {(const void*)k_pcg_resident<1, 8>,       (const void*)k_pcg_resident<2, 4>,
-                      (const void*)k_pcg_resident<3, 4>,       (const void*)k_pcg_mixed_resident<1, 8>,
-                      (const void*)k_pcg_mixed_resident<2, 4>, (const void*)k_pcg_mixed_resident<3, 4>,
-                      (const void*)k_pcg_mixed_resident<4, 3>, (const void*)k_pcg_mixed_resident<5, 3>,
-                      (const void*)k_pcg_mixed_resident<6, 3>};
-  for (const void* k : ks)
-    MSG_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgResidentSmem));
-  ctx->pcg_limit = true;
+// The shared memory of a resident kernel, allowed when a context first launches it
+// (the limit is a device's, and other devices' contexts may live in the process) and
+// always the same: other threads' solves of other sizes share it.
+int pcg_resident_limit(Context* ctx, const void* kernel) {
+  std::vector<const void*>& done = ctx->pcg_limits;
+  if (std::find(done.begin(), done.end(), kernel) != done.end()) return MSG_OK;
+  MSG_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPcgResidentSmem));
+  done.push_back(kernel);
   return MSG_OK;
 }
 
 int pcg_cooperative(Context* ctx, const PcgLaunch& l, void** args, cudaStream_t s) {
-  if (l.smem) MSG_TRY(pcg_resident_limit(ctx));
+  if (l.smem) MSG_TRY(pcg_resident_limit(ctx, l.kernel));
   MSG_CUDA(ctx, cudaLaunchCooperativeKernel(l.kernel, dim3(l.grid), dim3(l.threads), args, l.smem, s));
   count_launch(ctx);
   return MSG_OK;

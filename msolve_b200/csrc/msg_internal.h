@@ -153,7 +153,7 @@ struct Context {
   int* h_flags = nullptr;           // 4 KB of pinned host memory, mapped into the device
   int* d_hflags = nullptr;          // the device's address of h_flags
   double* h_stage = nullptr;        // 8 KB of pinned host memory: small uploads issued as true async copies
-  bool pcg_limit = false;           // the resident PCG kernels' shared memory is allowed on the device
+  std::vector<const void*> pcg_limits;  // resident PCG kernels whose shared memory is allowed
   char* h_copy = nullptr;           // pinned pieces of copy_out (8 MB, on the first large output)
   cudaEvent_t copy_ev[2 * kCopyThreads] = {nullptr};
   // unit-cube element matrices already computed (kind 0: stiffness at E = 1
