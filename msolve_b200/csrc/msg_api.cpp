@@ -122,11 +122,29 @@ int workspace(Context* ctx, int slot, size_t bytes, void** out) {
   return MSG_OK;
 }
 
+// copy_out's pinned pieces and their events for that many threads, kept in the context;
+// false where they cannot be had.
+static bool pin_pieces(Context* ctx, int threads) {
+  cudaError_t e = cudaSuccess;
+  if (ctx->copy_threads < threads) {
+    if (ctx->h_copy) cudaFreeHost(ctx->h_copy);
+    ctx->h_copy = nullptr;
+    ctx->copy_threads = 0;
+    e = cudaMallocHost(&ctx->h_copy, 2 * (size_t)threads * kCopyPiece);
+    if (e == cudaSuccess) ctx->copy_threads = threads;
+  }
+  for (int i = 0; i < 2 * threads && e == cudaSuccess; ++i)
+    if (!ctx->copy_ev[i]) e = cudaEventCreateWithFlags(&ctx->copy_ev[i], cudaEventDisableTiming);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess;
+}
+
 // Device-to-host copies of outputs on stream st. Pageable memory is filled by a few
 // host threads, each through its own pair of pinned pieces: a plain copy is staged
 // by the driver on one thread, which also takes the page faults of an output that
 // was just allocated (3.8 GB/s; 92 MB of displacements in 20 ms, 6 ms here).
-// Complete on return then, otherwise (pinned or short outputs) enqueued on st.
+// Complete on return then, otherwise (pinned or short outputs, or no pinned pieces to
+// be had) enqueued on st.
 int copy_out(Context* ctx, const std::vector<HostCopy>& outs, cudaStream_t st) {
   struct Piece {
     char* dst;
@@ -148,7 +166,7 @@ int copy_out(Context* ctx, const std::vector<HostCopy>& outs, cudaStream_t st) {
   }
   const int threads =
       total >= kCopyMin ? std::min<int>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency() / 2)) : 1;
-  const bool pool_copy = threads > 1;
+  const bool pool_copy = threads > 1 && pin_pieces(ctx, threads);
   for (size_t i = 0; i < outs.size(); ++i) {
     const HostCopy& o = outs[i];
     if (!pool_copy || !staged[i]) {
@@ -160,10 +178,6 @@ int copy_out(Context* ctx, const std::vector<HostCopy>& outs, cudaStream_t st) {
                         std::min(kCopyPiece, o.bytes - at)});
   }
   if (pieces.empty()) return MSG_OK;
-  // pinned pieces and their events, kept in the context
-  if (!ctx->h_copy) MSG_CUDA(ctx, cudaMallocHost(&ctx->h_copy, 2 * kCopyThreads * kCopyPiece));
-  for (auto& e : ctx->copy_ev)
-    if (!e) MSG_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   std::atomic<int> failed{cudaSuccess};
   auto work = [&](int t) {
     cudaError_t e = cudaSetDevice(ctx->device);

@@ -154,7 +154,8 @@ struct Context {
   int* d_hflags = nullptr;          // the device's address of h_flags
   double* h_stage = nullptr;        // 8 KB of pinned host memory: small uploads issued as true async copies
   std::vector<const void*> pcg_limits;  // resident PCG kernels whose shared memory is allowed
-  char* h_copy = nullptr;           // pinned pieces of copy_out (8 MB, on the first large output)
+  char* h_copy = nullptr;           // pinned pieces of copy_out (1 MB a thread, on the first large output)
+  int copy_threads = 0;             // threads that h_copy holds pieces for
   cudaEvent_t copy_ev[2 * kCopyThreads] = {nullptr};
   // unit-cube element matrices already computed (kind 0: stiffness at E = 1
   // for (h, nu); 1: consistent mass for (h, rho)): later batches read no
