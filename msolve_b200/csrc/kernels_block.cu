@@ -1596,7 +1596,7 @@ __global__ void __launch_bounds__(kQThreads, kQCtas)
     auto realk = [&](int k) { return k >= 1 && k <= L.NZ - 1; };
     const bool real = realj(Je) && realk(Ke);
     const bool node_ok = node_lane && Je <= L.NY && Ke <= L.NZ;
-    // (32-bit offsets in pairs of realizations: a vector is far below 32 GB)
+    // (32-bit offsets, in pairs of realizations: block_setup refuses longer vectors)
     const uint32_t nrow = ((uint32_t)Je + (uint32_t)L.NYp * Ke) * L.NXp;
     const int rr2 = (g16 >> 1) + l2;  // float2 index of this lane's realization pair
     float2 al = z2, be = z2;
@@ -3308,6 +3308,11 @@ int block_setup(Context* ctx, Mesh* m, double nu, double rho, double cK, double 
   B->n_tiles = L.tiles_j * ((L.NZ + kTK - 1) / kTK);
   B->npad = (size_t)L.n_pad;
   B->nvec = B->npad * 3 * Rp;
+  // the operators index a vector's values in 32 bits (a batch of that size takes more
+  // than 200 GB of vectors)
+  if (B->nvec > UINT32_MAX)
+    return set_error(ctx, MSG_ERR_OUT_OF_MEMORY, "batch of %d realizations: %llu values a vector, at most %u (split it)",
+                     R, (unsigned long long)B->nvec, UINT32_MAX);
   B->interior = m->d_pad_interior.as<int>();
   B->mask = m->d_pad_mask.as<uint8_t>();
   B->cK = cK;

@@ -56,3 +56,17 @@ def test_memory_budget_is_enforced():
         mc.Solve()
     assert e.value.code == N.MSG_ERR_OUT_OF_MEMORY
     assert b"budget" in N.lib().MSG_LAST_ERROR(small.handle)
+
+
+def test_vectors_beyond_32_bit_offsets_are_refused(ctx):
+    """A batch whose vectors hold 2^32 values or more (33^3 padded nodes, 3 components,
+    40,000 realizations and padding) ends before anything of that size is allocated."""
+    with pytest.raises(M.MSolveError) as e:
+        mc = small_batch(ctx, 30, 40000, xi=np.zeros((40000, 12)))
+        mc.keep_solutions = False
+        mc.Solve()
+    assert e.value.code == N.MSG_ERR_OUT_OF_MEMORY
+    assert b"values a vector" in N.lib().MSG_LAST_ERROR(ctx.handle)
+    after = small_batch(ctx, 6, 8)
+    after.Solve()
+    assert (after.Residuals < 1e-10).all()
