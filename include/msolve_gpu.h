@@ -535,8 +535,10 @@ int MSG_STATS_RESET(MSG_CTX ctx);
  * it gives up, records the expiry in an error word and lets its kernel return;
  * the batch then ends with MSG_ERR_TIMEOUT and the context stays usable. This
  * entry launches one thread that waits, with `polls` polls (1 ... 2^24), on an
- * mbarrier that nothing completes: it returns MSG_ERR_TIMEOUT when the wait
- * expired as designed (MSG_OK would mean it completed). */
+ * mbarrier that nothing completes, and one CTA that waits as often in a grid-wide
+ * sum of the assembled PCG for an arrival that never comes: it returns
+ * MSG_ERR_TIMEOUT when both waits expired as designed (MSG_OK would mean that one
+ * completed). */
 int MSG_WAIT_SELFTEST(MSG_CTX ctx, int64_t polls);
 
 #ifdef __cplusplus

@@ -156,6 +156,7 @@ struct PcgGrid {
   unsigned* arrived;
   unsigned target;    // arrivals that complete the next sum
   int buf;
+  int spin = kPcgSpin;  // polls of a wait
 };
 
 // out[k] = sum over the grid of v[k], every thread of every CTA; what the CTAs
@@ -190,7 +191,7 @@ __device__ __forceinline__ bool grid_sum(PcgGrid& g, const double (&v)[K], doubl
       __threadfence();
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.arrived) : "memory");
       int good = 0;
-      for (int i = 0; i < kPcgSpin && !good; ++i) {
+      for (int i = 0; i < g.spin && !good; ++i) {
         unsigned n;
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(g.arrived) : "memory");
         good = (int)(n - g.target) >= 0;
@@ -812,6 +813,16 @@ __global__ void __launch_bounds__(32 * S * W, 1)
   PcgEnd::write(st, err, status, iterations, products);
 }
 
+// Self-test of the sum's bounded wait: one CTA, one arrival short of the target
+// (grid.target on entry), so that the sum gives up and the state stays not done, as a
+// solve's would.
+__global__ void __launch_bounds__(kPcgThreads) k_pcg_wait_selftest(PcgGrid grid, PcgState* st) {
+  const double v[1] = {1.0};
+  double t[1];
+  if (!grid_sum<kPcgWarps, 1>(grid, v, t)) return;
+  PcgEnd::write(st, t[0], MSG_OK, 0, 0);
+}
+
 __global__ void k_to_f32(size_t n, const double* __restrict__ a, float* __restrict__ b) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     b[i] = (float)a[i];
@@ -980,6 +991,19 @@ int pcg_finish(Context* ctx, PcgState* st, PcgState* host, cudaStream_t s) {
 }
 
 }  // namespace
+
+int pcg_wait_selftest(Context* ctx, int polls) {
+  DevMem head;
+  MSG_TRY(head.alloc(ctx, pcg_head_bytes(ctx)));
+  PcgState* st = pcg_state(ctx, head.ptr);
+  MSG_CUDA(ctx, cudaMemsetAsync(head.ptr, 0, pcg_head_bytes(ctx), ctx->stream));
+  PcgGrid g{head.as<double>(), &st->counter, 1u, 0, polls};
+  k_pcg_wait_selftest<<<1, kPcgThreads, 0, ctx->stream>>>(g, st);
+  count_launch(ctx);
+  MSG_CUDA(ctx, cudaGetLastError());
+  PcgState hs;
+  return pcg_finish(ctx, st, &hs, ctx->stream);
+}
 
 // Runs the device PCG on node-layout vectors (k_pcg, or k_pcg_mixed), one launch a solve.
 int pcg_solve_device(Context* ctx, Matrix* A, const double* d_b, double* d_x, int max_it, double tol, int* iterations,

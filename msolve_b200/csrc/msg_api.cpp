@@ -933,7 +933,10 @@ int MSG_WAIT_SELFTEST(MSG_CTX ctx, int64_t polls) {
     return set_error(ctx, MSG_ERR_INVALID_ARGUMENT, "wait self-test: polls must be in [1, 2^24]");
   int expired = 0;
   MSG_TRY(wait_selftest(ctx, (long)polls, &expired));
-  return expired ? set_error(ctx, MSG_ERR_TIMEOUT, "bounded wait expired (self-test)") : MSG_OK;
+  if (!expired) return MSG_OK;
+  const int st = pcg_wait_selftest(ctx, (int)polls);
+  if (st != MSG_ERR_TIMEOUT) return st;
+  return set_error(ctx, MSG_ERR_TIMEOUT, "bounded wait expired (self-test); %s", std::string(ctx->last_error).c_str());
 }
 
 int MSG_H8_KE_BATCH(MSG_CTX ctx, int n, const double* xyz, const double* E, double nu, double* Ke) {

@@ -381,6 +381,8 @@ int launch_to_f32(Context* ctx, size_t n, const double* a, float* b);
 // true-residual replacement (reliable updates), stop on the FP64 true residual.
 int pcg_solve_device(Context* ctx, Matrix* A, const double* d_b_node, double* d_x_node, int max_it, double tol,
                      int* iterations, double* rel_res, int* status, bool mixed = false);
+// Self-test of the bounded wait of the solves' grid-wide sums: MSG_ERR_TIMEOUT when it expires.
+int pcg_wait_selftest(Context* ctx, int polls);
 
 // KL field: E64/E32 [n_elems][Rp] (realization innermost) and/or E64 [R][n_elems].
 struct KLDevice {

@@ -70,3 +70,16 @@ def test_vectors_beyond_32_bit_offsets_are_refused(ctx):
     after = small_batch(ctx, 6, 8)
     after.Solve()
     assert (after.Residuals < 1e-10).all()
+
+
+def test_grid_sum_of_the_assembled_pcg_expires(ctx):
+    """The solve's wait for the other CTAs gives up too: its kernel returns, the call
+    reports the expiry, and the context still solves."""
+    assert N.lib().MSG_WAIT_SELFTEST(ctx.handle, 1 << 14) == N.MSG_ERR_TIMEOUT
+    assert b"grid barrier expired" in N.lib().MSG_LAST_ERROR(ctx.handle)
+    model = M.clamped_block_model(5)
+    solver = M.SolverPCG(ctx, model, 2000, 1e-10)
+    solver.matrix = M.GpuMesh(ctx, model).assemble(np.ones(model.n_elems), model.poisson)
+    x = solver.Solve()
+    b = model.subdomains[0].RHS
+    assert np.linalg.norm(b - solver.matrix.Multiply(x)) <= 1e-9 * np.linalg.norm(b)
