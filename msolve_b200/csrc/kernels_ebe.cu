@@ -56,7 +56,8 @@ namespace {
 
 constexpr int kEbeWarps = 8;   // warps per CTA
 constexpr int kEbeCheck = 8;   // iterations per chunk (graph launch) between host reads of the flags
-constexpr int kRgBlk = 8;      // nodes per work item of the operator passes: 8 warps x 1 node
+constexpr int kRgBlk = 8;      // nodes per work item of the operator passes: 8 warps x 1 node (the partial
+                               // sums then take 5 bytes a node and realization, the vectors 84)
 constexpr int kRgBlkU = 32;    // nodes per work item of the update passes: 8 warps x 4 nodes
 constexpr int kRgParts = 5;    // partial arrays per system over kRgBlk blocks
 enum { kPq = 0, kDrq = 1, kDqd = 2, kZr = 3, kRr = 4 };
@@ -91,7 +92,7 @@ struct RgSys {
   double delta2;  // ebe_mg_solve: squared reliable-update factor
 };
 struct RgItem {
-  int sys, blk, rb, G;  // nodes blk * 64 .., realizations rb .. rb + 32 G - 1
+  int sys, blk, rb, G;  // nodes from blk kRgBlk (kRgBlkU), realizations rb .. rb + 32 G - 1
 };
 // Batch-wide per-realization state, index = system goff + realization.
 struct RgScal {
@@ -410,7 +411,8 @@ __global__ void __launch_bounds__(32 * kEbeWarps) k_rg_update(const RgSys* __res
 }
 
 // x += d, d = 0 for the systems with a true residual pending (all = 1: every
-// system; a realization's d is 0 after its last true residual).
+// system; a realization's d is 0 after its last true residual). Items of the update
+// passes, one CTA each, a warp's four nodes in flight together.
 __global__ void k_rg_fold(const RgSys* __restrict__ Sys, const RgItem* __restrict__ items, int n_items, RgScal s,
                           int all) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -418,23 +420,22 @@ __global__ void k_rg_fold(const RgSys* __restrict__ Sys, const RgItem* __restric
     const RgItem I = items[it];
     if (!all && !s.sreq[I.sys]) continue;
     const RgSys S = Sys[I.sys];
-    const int n1 = min(S.n_nodes, (I.blk + 1) * kRgBlk);
-    for (int g = 0; g < I.G; ++g)
-      rg_stream(I.blk * kRgBlk + w, n1, S.Rp, I.rb + 32 * g + lane, [&](auto m, const RgOffsets& o, const RgNodes&) {
-        constexpr int M = 3 * decltype(m)::value;
-        double xv[M];
-        float dv[M];
+    const int n1 = min(S.n_nodes, (I.blk + 1) * kRgBlkU);
+    rg_stream(I.blk * kRgBlkU + w, n1, S.Rp, I.rb + lane, [&](auto m, const RgOffsets& o, const RgNodes&) {
+      constexpr int M = 3 * decltype(m)::value;
+      double xv[M];
+      float dv[M];
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-          xv[i] = S.x[o[i]];
-          dv[i] = S.d[o[i]];
-        }
+      for (int i = 0; i < M; ++i) {
+        xv[i] = S.x[o[i]];
+        dv[i] = S.d[o[i]];
+      }
 #pragma unroll
-        for (int i = 0; i < M; ++i) {
-          S.x[o[i]] = xv[i] + (double)dv[i];
-          S.d[o[i]] = 0.f;
-        }
-      });
+      for (int i = 0; i < M; ++i) {
+        S.x[o[i]] = xv[i] + (double)dv[i];
+        S.d[o[i]] = 0.f;
+      }
+    });
   }
 }
 
@@ -1250,13 +1251,12 @@ int ebe_ragged_solve(Context* ctx, const std::vector<RgInput>& in, int max_it, d
   count_launch(ctx);
   MSG_CUDA(ctx, cudaGetLastError());
   // persistent grids: the CTAs that fit on the device at once, at most one per item
-  int occ_apply = 1, occ_update = 1, occ_resid = 1;
+  int occ_apply = 1, occ_resid = 1;
   MSG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_apply, k_rg_apply, 32 * kEbeWarps, 0));
-  MSG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_update, k_rg_update, 32 * kEbeWarps, 0));
   MSG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_resid, k_rg_resid64, 32 * kEbeWarps, 0));
   auto grid_of = [&](int occ, int n) { return std::max(1, std::min(n, ctx->sm_count * std::max(1, occ))); };
   const int g_apply = grid_of(occ_apply, n_items), g_update = n_items_u;
-  const int g_resid = grid_of(occ_resid, n_items), g_fold = grid_of(occ_update, n_items);
+  const int g_resid = grid_of(occ_resid, n_items);
   const int g_scal = (Rtot + kEbeWarps - 1) / kEbeWarps;
   const RgSys* dS = b.d_sys;
   const RgItem* dI = b.d_items;
@@ -1300,7 +1300,7 @@ int ebe_ragged_solve(Context* ctx, const std::vector<RgInput>& in, int max_it, d
     if (h[0] == 0) continue;
     ++n_true;
     MSG_CUDA(ctx, cudaMemsetAsync(s.flags + 1, 0, sizeof(int), st));
-    k_rg_fold<<<g_fold, 32 * kEbeWarps, 0, st>>>(dS, dI, n_items, s, 0);
+    k_rg_fold<<<g_update, 32 * kEbeWarps, 0, st>>>(dS, dIu, n_items_u, s, 0);
     k_rg_resid64<<<g_resid, 32 * kEbeWarps, 0, st>>>(dS, dI, n_items, s);
     k_rg_true<<<g_scal, 32 * kEbeWarps, 0, st>>>(dS, Rtot, s, tol, max_it);
     k_rg_active<<<g_groups, 32 * kEbeWarps, 0, st>>>(n_groups, s);
@@ -1320,7 +1320,7 @@ int ebe_ragged_solve(Context* ctx, const std::vector<RgInput>& in, int max_it, d
   ctx->t_phase[3] = 0.0;
   // results (a realization stops right after its fold, so this adds 0 to it
   // unless it broke down or the chunk bound ended the loop)
-  k_rg_fold<<<g_fold, 32 * kEbeWarps, 0, st>>>(dS, dI, n_items, s, 1);
+  k_rg_fold<<<g_update, 32 * kEbeWarps, 0, st>>>(dS, dIu, n_items_u, s, 1);
   count_launch(ctx);
   return rg_results(ctx, in, bufs, sys, s, Rtot);
 }
@@ -1395,13 +1395,12 @@ int ebe_mg_solve(Context* ctx, const std::vector<RgInput>& in, const std::vector
   const RgSys* dS = b.d_sys;
   const int n_groups = Rtot / 32, g_groups = (n_groups + kEbeWarps - 1) / kEbeWarps;
   const int g_scal = (Rtot + kEbeWarps - 1) / kEbeWarps;
-  int occ_apply = 1, occ_resid = 1, occ_u = 1;
+  int occ_apply = 1, occ_resid = 1;
   MSG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_apply, k_rg_apply, 32 * kEbeWarps, 0));
   MSG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_resid, k_rg_resid64, 32 * kEbeWarps, 0));
-  MSG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k_rg_fold, 32 * kEbeWarps, 0));
   auto grid_of = [&](int occ, int n) { return std::max(1, std::min(n, ctx->sm_count * std::max(1, occ))); };
   const int g_apply = grid_of(occ_apply, n_items), g_resid = grid_of(occ_resid, n_items);
-  const int g_fold = grid_of(occ_u, n_items), g_u = n_items_u;
+  const int g_u = n_items_u;
   // z = M^-1 r of the systems in `which` (nullptr: all): V-cycles one system
   // after another, the diagonal for all the others in one launch. from_node:
   // r of the V-cycle systems in node layout (the start and the true
@@ -1474,7 +1473,7 @@ int ebe_mg_solve(Context* ctx, const std::vector<RgInput>& in, const std::vector
     MSG_CUDA(ctx, cudaStreamSynchronize(st));
     for (int i = 0; i < S; ++i) req[i] = hreq[i];
     MSG_CUDA(ctx, cudaMemsetAsync(s.flags + 1, 0, sizeof(int), st));
-    k_rg_fold<<<g_fold, 32 * kEbeWarps, 0, st>>>(dS, d_items, n_items, s, 0);
+    k_rg_fold<<<g_u, 32 * kEbeWarps, 0, st>>>(dS, d_items_u, n_items_u, s, 0);
     k_rg_resid64<<<g_resid, 32 * kEbeWarps, 0, st>>>(dS, d_items, n_items, s);
     MSG_TRY(precondition(&req, true));
     k_vc_true<<<g_scal, 32 * kEbeWarps, 0, st>>>(dS, Rtot, s, tol, max_it);
@@ -1493,7 +1492,7 @@ int ebe_mg_solve(Context* ctx, const std::vector<RgInput>& in, const std::vector
   ctx->t_phase[1] = loop_ms;
   ctx->t_phase[2] = n_true;
   ctx->t_phase[3] = 0.0;
-  k_rg_fold<<<g_fold, 32 * kEbeWarps, 0, st>>>(dS, d_items, n_items, s, 1);
+  k_rg_fold<<<g_u, 32 * kEbeWarps, 0, st>>>(dS, d_items_u, n_items_u, s, 1);
   count_launch(ctx);
   return rg_results(ctx, in, bufs, sys, s, Rtot);
 }
