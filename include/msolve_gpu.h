@@ -143,9 +143,11 @@ int MSG_MAT_DESTROY(MSG_MAT mat);
  * (ISAAR.MSolve.Solvers/PCG/SolverPCG.cs:105-149, simple search vector
  * SolverPCGSimpleSearchVectorCalculator.cs:18-41): x0 = 0, r0 = b, stop when
  * ||r_k|| / ||b|| < tol on the recursively updated r, skip if ||b|| <= 1e-25.
- * The whole loop runs on the device: one cooperative launch a solve (no host
- * round trip between iterations); MSG_ERR_TIMEOUT if its CTAs' bounded waits for
- * each other expire.
+ * The loop's scalars and decisions stay on the device: small matrices (up to 4,700
+ * nodes of a lattice on 148 SMs) are one cooperative launch a solve on at most a
+ * third of the SMs (MSG_ERR_TIMEOUT if its CTAs' bounded waits for each other
+ * expire), larger ones two launches an iteration, enqueued ahead of the host's look
+ * at the state, so that other streams' work runs beside a long solve.
  * iterations = the reference's count (loop index at the break); rel_res = last
  * ||r||/||b||. Returns MSG_ERR_NOT_CONVERGED if max_it was reached. */
 int MSG_PCG_SOLVE(MSG_MAT mat, const double* b, double* x, int max_it, double tol, int* iterations,
@@ -161,8 +163,8 @@ int MSG_PCG_SOLVE(MSG_MAT mat, const double* b, double* x, int max_it, double to
  * the search direction is kept, and the solve stops only when
  * ||b - K x|| / ||b|| < tol in FP64 (rel_res). iterations counts as
  * MSG_PCG_SOLVE. The FP32 copy of the values is built on first use. Like
- * MSG_PCG_SOLVE, one cooperative launch a solve, true-residual steps included.
- * No counterpart in the reference. */
+ * MSG_PCG_SOLVE, one cooperative launch (up to 9,400 nodes) or two launches an
+ * iteration, true-residual steps included. No counterpart in the reference. */
 int MSG_PCG_SOLVE_MIXED(MSG_MAT mat, const double* b, double* x, int max_it, double tol, int* iterations,
                         double* rel_res);
 

@@ -120,36 +120,107 @@ __global__ void k_node_to_dof(int n_dofs, const int* __restrict__ free_rows, con
 }
 
 // ------------------------------------------------------------------ PCG
-// Device-resident Jacobi-PCG: the whole solve is one cooperative launch. A CTA
-// owns a fixed set of 32-row slices; the phases of an iteration are separated by
-// grid-wide sums, in which every CTA adds all CTAs' partials itself in the same
-// fixed order, so that each holds the same scalars and takes the same branches
-// (deterministic results). FP64 loop, two sums an iteration:
+// Device-resident Jacobi-PCG. FP64 loop, two sums an iteration:
 //   1: p_new = z + beta p_old (formed at the gathered columns, written for own
 //      rows), q = K p_new, sum p.q -> alpha = z.r / p.q (breakdown check)
 //   2: r -= alpha q, x += alpha p_new, z = D^-1 r, sums r.r and z.r -> err =
 //      ||r||/||b||, convergence, beta
 // p is double-buffered by iteration parity so gathered columns are never read
-// while being overwritten.
+// while being overwritten. All sums are taken in a fixed order (deterministic
+// results).
 //
-// k_pcg_resident: while a matrix' values fit the SMs' shared memory (3 slices an
-// SM in FP64, 6 in FP32: 14,000 and 28,000 lattice nodes) they are copied there
-// once and an iteration reads only vectors from L2; it is bound by the two sums
-// (2.5 us each). k_pcg streams them: bound by HBM, or by L2 for matrices that
-// stay there. Two kernels an iteration in a graph spent the launch latency of
-// each and the last block's serial sum. Per iteration, then -> now: 10 x 4 x 4
-// 14.7 -> 6.7 us, 20^3 17.2 -> 7.4, 37 x 22 x 29 19.6 -> 14.4 (mixed 22.4 ->
-// 11.0), 32^3 20.7 -> 18.2, 48^3 55.7 -> 47.6, 64^3 111.7 -> 102.8 (5.7 TB/s;
-// mixed 63.5 -> 60.4). Reading blocks below the diagonal from their mirror images
-// (half the HBM bytes) was slower at 48^3 (57-60 us): L2 delivers no faster here.
+// k_pcg_resident: a matrix whose values fit the shared memory of a third of the SMs
+// (3 slices an SM in FP64, 6 in FP32: 4,700 and 9,400 lattice nodes on 148) is copied
+// there once, the whole solve is one cooperative launch, and its phases are separated
+// by grid-wide sums, in which every CTA adds all CTAs' partials itself; bound by the two
+// sums (2.5 us each): 10 x 4 x 4 5.8 us an iteration, 14^3 7.8, 20^3 mixed 10.7. It holds its
+// SMs until it ends, so it gets no more of them: with all 148, or with a cooperative
+// loop that streams larger matrices, a batch of 24^3 x 256 on another stream took 136
+// ms beside 20^3 solves and 1,296 beside 64^3 ones, and 13 to 39 beside launches that
+// end.
+//
+// k_pcg_product and k_pcg_step (k_pcgm_*): two launches an iteration for all other
+// matrices, enqueued ahead of the host's look at the state; a launch after the end of
+// the solve returns at once. The CTA that finishes last adds the partials. A launch
+// starts while the one before it ends and loads its first values meanwhile. Bound by
+// HBM, or by L2 and the two launches' latency for matrices that stay there: 20^3 13.0 us
+// an iteration, 37 x 22 x 29 16.6 (mixed 14.9), 32^3 18.8 (16.2), 48^3 52.9 (36.0), 64^3
+// 106 (63.7; HBM alone 88 and 47).
 
-constexpr int kPcgThreads = 256, kPcgWarps = kPcgThreads / 32;  // of the streaming kernels
-constexpr int kPcgMaxCtas = 4;     // CTAs an SM at most (sizes the partial sums)
-constexpr int kPcgSums = 3;        // values of a grid-wide sum at most
+constexpr int kPcgThreads = 256, kPcgWarps = kPcgThreads / 32;
+constexpr int kPcgSums = 3;        // values of a sum at most
+constexpr int kPcgMaxCtas = 8;     // CTAs an SM of a launch at most (sizes the partial sums)
 constexpr int kPcgSpin = 1 << 22;  // polls of a grid-wide sum before it gives up
 
-// Grid-wide sums of one solve: the CTAs' partial sums (two buffers, used in turn: a
-// CTA can be at most one sum ahead of another) and the arrival counter, cleared
+// v[k] of the CTA's threads summed and left in part[k][CTA] (thread 0 of the CTA has
+// passed a fence after it). NW: warps of the CTA.
+template <int NW, int K>
+__device__ __forceinline__ void leave_partials(double* part, const double (&v)[K]) {
+  __shared__ double sh[NW][K];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, G = gridDim.x;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double t = v[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (l == 0) sh[w][k] = t;
+  }
+  __syncthreads();  // (and every thread's stores of this phase are ordered before the fence)
+  if (w == 0) {
+    if (l < K) {
+      double t = 0;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) t += sh[i][l];
+      part[(size_t)l * G + blockIdx.x] = t;
+    }
+    __syncwarp();
+    if (l == 0) __threadfence();
+  }
+}
+
+// out[k] = the CTAs' partials added: thread t takes t, t + 32 NW, ... in order, then the
+// block's fixed tree. Every thread of the CTA gets it.
+template <int NW, int K>
+__device__ __forceinline__ void add_partials(const double* part, double (&out)[K]) {
+  __shared__ double sh[NW][K];
+  constexpr int T = 32 * NW;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, G = gridDim.x;
+  double t[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) t[k] = threadIdx.x < G ? __ldcg(part + (size_t)k * G + threadIdx.x) : 0.0;
+  int i = threadIdx.x + T;
+  for (; i + 3 * T < G; i += 4 * T) {  // four loads in flight, added in order
+    double u[K][4];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[k][j] = __ldcg(part + (size_t)k * G + i + j * T);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) t[k] += u[k][j];
+  }
+  for (; i < G; i += T)
+#pragma unroll
+    for (int k = 0; k < K; ++k) t[k] += __ldcg(part + (size_t)k * G + i);
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
+    if (l == 0) sh[w][k] = t[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double x = 0;
+#pragma unroll
+    for (int j = 0; j < NW; ++j) x += sh[j][k];
+    out[k] = x;
+  }
+}
+
+// Grid-wide sums of one cooperative solve: the CTAs' partial sums (two buffers, used in
+// turn: a CTA can be at most one sum ahead of another) and the arrival counter, cleared
 // before the launch.
 struct PcgGrid {
   double* part;       // [2][kPcgSums][grid]
@@ -161,68 +232,45 @@ struct PcgGrid {
 
 // out[k] = sum over the grid of v[k], every thread of every CTA; what the CTAs
 // wrote before is visible after. False when the bounded wait expired (the kernel
-// then returns). About 2.5 us over 26 to 592 CTAs; polling every CTA's partial sum
-// itself, without a counter, was faster below 30 CTAs only.
-template <int NW, int K>  // warps of the CTA, values
+// then returns).
+template <int NW, int K>
 __device__ __forceinline__ bool grid_sum(PcgGrid& g, const double (&v)[K], double (&out)[K]) {
-  __shared__ double sh[2][NW][K];
   __shared__ int ok;
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, G = gridDim.x;
+  const int G = gridDim.x;
   double* part = g.part + (size_t)g.buf * kPcgSums * G;
   g.buf ^= 1;
   g.target += G;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double t = v[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (l == 0) sh[0][w][k] = t;
-  }
-  __syncthreads();  // (and every thread's stores of this phase are ordered before the release)
-  if (w == 0) {
-    if (l < K) {
-      double t = 0;
-#pragma unroll
-      for (int i = 0; i < NW; ++i) t += sh[0][i][l];
-      part[(size_t)l * G + blockIdx.x] = t;
+  leave_partials<NW, K>(part, v);
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.arrived) : "memory");
+    int good = 0;
+    for (int i = 0; i < g.spin && !good; ++i) {
+      unsigned n;
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(g.arrived) : "memory");
+      good = (int)(n - g.target) >= 0;
     }
-    __syncwarp();
-    if (l == 0) {
-      __threadfence();
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(g.arrived) : "memory");
-      int good = 0;
-      for (int i = 0; i < g.spin && !good; ++i) {
-        unsigned n;
-        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(g.arrived) : "memory");
-        good = (int)(n - g.target) >= 0;
-      }
-      __threadfence();
-      ok = good;
-    }
+    __threadfence();
+    ok = good;
   }
   __syncthreads();
   if (!ok) return false;
-  // thread t adds the CTAs t, t + 32 NW, ... in order, then the block's fixed tree
-  double t[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) t[k] = threadIdx.x < G ? __ldcg(part + (size_t)k * G + threadIdx.x) : 0.0;
-  for (int i = threadIdx.x + (32 * NW); i < G; i += (32 * NW))
-#pragma unroll
-    for (int k = 0; k < K; ++k) t[k] += __ldcg(part + (size_t)k * G + i);
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
-    if (l == 0) sh[1][w][k] = t[k];
+  add_partials<NW, K>(part, out);
+  return true;
+}
+
+// The sum of a launch: true in the CTA that finishes last, which gets it.
+template <int NW, int K>
+__device__ __forceinline__ bool last_sum(double* part, unsigned* counter, const double (&v)[K], double (&out)[K]) {
+  __shared__ int last;
+  leave_partials<NW, K>(part, v);
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __threadfence();
   }
   __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double x = 0;
-#pragma unroll
-    for (int i = 0; i < NW; ++i) x += sh[1][i][k];
-    out[k] = x;
-  }
+  if (!last) return false;
+  add_partials<NW, K>(part, out);
+  if (threadIdx.x == 0) *counter = 0;  // for the next launch
   return true;
 }
 
@@ -241,11 +289,12 @@ __device__ __forceinline__ void block_row(const V (&a)[9], const V (&u)[3], doub
 // Part of a slice's row sums y = K u formed by warp w of the W that share the
 // slice (slots w, w + W, ...): U slots at a time, all their values requested
 // before use (kStream: evict-first, for matrices that do not stay in L2).
-// gather(c, u3) gives u at node c.
-template <int W, int U, bool kStream, class V, class Gather>
+// gather(c, u3) gives u at node c; first() runs when the first group's loads are under way.
+template <int W, int U, bool kStream, class V, class Gather, class First>
 __device__ __forceinline__ void slice_rows(int64_t s0, int64_t s1, int w, int lane, const int* __restrict__ col,
-                                           const V* __restrict__ val, Gather gather, double (&y)[3]) {
+                                           const V* __restrict__ val, Gather gather, double (&y)[3], First first) {
   y[0] = y[1] = y[2] = 0.0;
+  bool begin = true;
   for (int64_t s = s0 + w; s < s1; s += U * W) {
     V a[U][9];
     int c[U];
@@ -258,6 +307,8 @@ __device__ __forceinline__ void slice_rows(int64_t s0, int64_t s1, int w, int la
 #pragma unroll
       for (int k = 0; k < 9; ++k) a[u][k] = kStream ? __ldcs(v + k * 32) : __ldg(v + k * 32);
     }
+    if (begin) first();
+    begin = false;
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (c[u] >= 0) {  // (padding: -1)
@@ -274,12 +325,15 @@ struct PcgMat {
   const int* col;
 };
 
-// Visits the CTA's slices: f(slice, live) by all warps together, W warps a slice
-// (kPcgWarps / W slices at a time). The set is the same in every phase.
-template <int W, class F>
+// Visits the CTA's slices: f(slice) by all warps together, W warps a slice (kPcgWarps / W
+// slices at a time). kOnce: the launch has a CTA for every kPcgWarps / W slices.
+template <int W, bool kOnce, class F>
 __device__ __forceinline__ void for_slices(int n_slices, F f) {
   constexpr int S = kPcgWarps / W;
-  for (int base = blockIdx.x * S; base < n_slices; base += gridDim.x * S) f(base + (int)(threadIdx.x >> 5) / W);
+  if constexpr (kOnce)
+    f(blockIdx.x * S + (int)(threadIdx.x >> 5) / W);
+  else
+    for (int base = blockIdx.x * S; base < n_slices; base += gridDim.x * S) f(base + (int)(threadIdx.x >> 5) / W);
 }
 
 // y of the W warps of each slice summed in warp order; valid in warp 0 of the slice.
@@ -312,99 +366,135 @@ struct PcgEnd {  // how a solve ended (CTA 0 writes it)
   }
 };
 
-template <int W, bool kStream>
-__global__ void __launch_bounds__(kPcgThreads, 3)
-    k_pcg(PcgMat M, const double* __restrict__ val, const double* __restrict__ b, const double* __restrict__ dinv,
-          double* x, double* r, double* z, double* p0, double* p1, double* q, PcgGrid grid, PcgState* st, double tol,
-          int max_it) {
-  __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = warp % W;
-  const int n3 = 3 * M.n_rows;
-  // elementwise phases: the 96 components of a slice, dealt to its W warps
-  auto own = [&](auto f) {
-    for_slices<W>(M.n_slices, [&](int slice) {
-      if (slice >= M.n_slices) return;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int i = slice * 96 + k * 32 + lane;
-        if (k % W == w && i < n3) f(i);
-      }
-    });
-  };
-  double s2[2] = {0.0, 0.0}, t2[2], t1[1];
-  own([&](int i) {
+// Programmatic dependent launch: a launch's CTAs start while those of the launch before
+// it finish, load what no launch changes, and wait for its results here.
+__device__ __forceinline__ void wait_for_launch() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Whether the solve had ended before the launch began (it waits all the same).
+__device__ __forceinline__ bool over(const PcgState* st) {
+  if (!*reinterpret_cast<const volatile int*>(&st->done)) return false;
+  wait_for_launch();
+  return true;
+}
+
+// Elements i of a launch's vectors: f(i).
+template <class F>
+__device__ __forceinline__ void for_elements(int n, F f) {
+  for (int i = blockIdx.x * kPcgThreads + threadIdx.x; i < n; i += gridDim.x * kPcgThreads) f(i);
+}
+
+// Start of an FP64 solve: x = 0, r = b, z = D^-1 r, sums b.b and z.b.
+__global__ void __launch_bounds__(kPcgThreads)
+    k_pcg_start(int n3, const double* __restrict__ b, const double* __restrict__ dinv, double* x, double* r, double* z,
+                double* p0, double* part, PcgState* st) {
+  double v[2] = {0.0, 0.0}, t[2];
+  for_elements(n3, [&](int i) {
     const double bi = b[i], zi = dinv[i] * bi;
     r[i] = bi; x[i] = 0; z[i] = zi; p0[i] = 0;
-    s2[0] += bi * bi;
-    s2[1] += zi * bi;
+    v[0] += bi * bi;
+    v[1] += zi * bi;
   });
-  if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
-  const double bnorm = sqrt(t2[0]);
-  double zr = t2[1], beta = 0.0, err = 0.0;
-  if (!(bnorm > 1e-25)) {  // SolverPCG.cs:112
-    PcgEnd::write(st, 0.0, MSG_OK, 0, 0);
-    return;
-  }
-  for (int it = 0;; ++it) {
-    double* pold = (it & 1) ? p1 : p0;
-    double* pnew = (it & 1) ? p0 : p1;
-    double pq = 0.0;
-    for_slices<W>(M.n_slices, [&](int slice) {
-      const int row = slice * 32 + lane;
-      const bool live = slice < M.n_slices && row < M.n_rows;
-      double y[3] = {0.0, 0.0, 0.0};
-      auto dir = [&](int c, double (&u)[3]) {
+  if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
+  st->bnorm = sqrt(t[0]);
+  st->zr = t[1];
+  st->done = !(st->bnorm > 1e-25);  // SolverPCG.cs:112
+}
+
+// p_new = z + beta p_old, q = K p_new, alpha.
+template <int W, bool kStream>
+__global__ void __launch_bounds__(kPcgThreads, 3)
+    k_pcg_product(PcgMat M, const double* __restrict__ val, const double* z, double* p0, double* p1,
+                  double* __restrict__ q, double* part, PcgState* st) {
+  __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
+  if (over(st)) return;
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) % W;
+  double beta = 0.0, v[1] = {0.0}, t[1];
+  const double* pold = nullptr;
+  double* pnew = nullptr;
+  int it = 0, done = 0;
+  auto start = [&] {  // (once; the first slice's values are under way)
+    if (pnew) return;
+    wait_for_launch();
+    beta = st->beta;
+    it = st->it;
+    done = st->done;
+    pold = (it & 1) ? p1 : p0;
+    pnew = (it & 1) ? p0 : p1;
+  };
+  auto dir = [&](int c, double (&u)[3]) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) u[k] = z[3 * c + k] + beta * pold[3 * c + k];
-      };
-      if (live) slice_rows<W, 2, kStream>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val, dir, y);
-      join_warps<W>(y, ys);
-      if (w == 0 && live) {
-        double pn[3];
-        dir(row, pn);
+    for (int k = 0; k < 3; ++k) u[k] = z[3 * c + k] + beta * pold[3 * c + k];
+  };
+  for_slices<W, (W > 2)>(M.n_slices, [&](int slice) {
+    const int row = slice * 32 + lane;
+    const bool live = slice < M.n_slices && row < M.n_rows;
+    double y[3] = {0.0, 0.0, 0.0};
+    if (live) slice_rows<W, 2, kStream>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val, dir, y, start);
+    start();
+    join_warps<W>(y, ys);
+    if (w == 0 && live) {
+      double pn[3];
+      dir(row, pn);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          pnew[3 * row + k] = pn[k];
-          q[3 * row + k] = y[k];
-        }
-        pq += pn[0] * y[0] + pn[1] * y[1] + pn[2] * y[2];
+      for (int k = 0; k < 3; ++k) {
+        pnew[3 * row + k] = pn[k];
+        q[3 * row + k] = y[k];
       }
-    });
-    const double v1[1] = {pq};
-    if (!grid_sum<kPcgWarps, 1>(grid, v1, t1)) return;
-    if (!(t1[0] > 0) || isnan(t1[0])) {  // breakdown: p.q <= 0 or NaN
-      PcgEnd::write(st, err, MSG_ERR_BREAKDOWN, it, it + 1);
-      return;
+      v[0] += pn[0] * y[0] + pn[1] * y[1] + pn[2] * y[2];
     }
-    const double alpha = zr / t1[0];
-    s2[0] = s2[1] = 0.0;
-    own([&](int i) {
-      const double ri = r[i] - alpha * q[i], zi = dinv[i] * ri;
-      r[i] = ri;
-      x[i] += alpha * pnew[i];
-      z[i] = zi;
-      s2[0] += ri * ri;
-      s2[1] += zi * ri;
-    });
-    if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
-    err = sqrt(t2[0]) / bnorm;
-    if (err < tol) {
-      PcgEnd::write(st, err, MSG_OK, it, it + 1);
-      return;
-    }
-    if (it + 1 >= max_it) {
-      PcgEnd::write(st, err, MSG_ERR_NOT_CONVERGED, max_it, it + 1);
-      return;
-    }
-    beta = t2[1] / zr;
-    zr = t2[1];
+  });
+  if (done || !last_sum<kPcgWarps, 1>(part, &st->counter, v, t) || threadIdx.x) return;
+  st->matvecs = it + 1;
+  if (!(t[0] > 0) || isnan(t[0])) {  // breakdown: p.q <= 0 or NaN
+    st->status = MSG_ERR_BREAKDOWN;
+    st->iterations = it;
+    st->done = 1;
+  } else {
+    st->alpha = st->zr / t[0];
   }
 }
 
-// The same loop for matrices whose values fit the SMs' shared memory: a CTA, alone
-// on its SM, copies the values and columns of its S slices there once (W warps a
-// slice), and each thread keeps the r, x, D^-1 of its own component in registers,
-// so that an iteration reads only z and p_old at the gathered columns from L2.
+// r -= alpha q, x += alpha p_new, z = D^-1 r, err, beta.
+__global__ void __launch_bounds__(kPcgThreads)
+    k_pcg_step(int n3, const double* __restrict__ dinv, double* x, double* r, double* z, const double* p0,
+               const double* p1, const double* q, double* part, PcgState* st, double tol, int max_it) {
+  wait_for_launch();
+  if (st->done) return;
+  const int it = st->it;
+  const double alpha = st->alpha;
+  const double* p = (it & 1) ? p0 : p1;
+  double v[2] = {0.0, 0.0}, t[2];
+  for_elements(n3, [&](int i) {
+    const double ri = r[i] - alpha * q[i], zi = dinv[i] * ri;
+    r[i] = ri;
+    x[i] += alpha * p[i];
+    z[i] = zi;
+    v[0] += ri * ri;
+    v[1] += zi * ri;
+  });
+  if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
+  st->err = sqrt(t[0]) / st->bnorm;
+  if (st->err < tol) {
+    st->iterations = it;
+    st->done = 1;
+  } else if (it + 1 >= max_it) {
+    st->iterations = max_it;
+    st->status = MSG_ERR_NOT_CONVERGED;
+    st->done = 1;
+  }
+  st->beta = t[1] / st->zr;
+  st->zr = t[1];
+  st->it = it + 1;
+}
+
+// The same loop for matrices whose values fit the shared memory of a third of the SMs:
+// a CTA, alone on its SM, copies the values and columns of its S slices there once (W
+// warps a slice), and each thread keeps the r, x, D^-1 of its own component in
+// registers, so that an iteration reads only z and p_old at the gathered columns from
+// L2.
 constexpr int kPcgResidentSmem = 204 * 1024;
 template <class V>
 inline size_t pcg_resident_smem(int64_t slots) {  // of a CTA with that many slots
@@ -560,27 +650,13 @@ __global__ void __launch_bounds__(32 * S * W, 1)
 //      formed in the same pass), exact sums z.r and r.r -> gamma = z.r, and a
 //      true residual when ||r||/||b|| has dropped by delta since the last one or
 //      below tol: x += d, r = b - K64 x with the FP64 values (stop when
-//      ||r||/||b|| < tol in FP64), the direction kept.
-template <int W, bool kStream>
-__global__ void __launch_bounds__(kPcgThreads, 4)
-    k_pcg_mixed(PcgMat M, const double* __restrict__ val, const float* __restrict__ val32, const double* __restrict__ b,
-                const double* __restrict__ dinv, double* x, float* r32, float* p32, float* q32, float* d32,
-                float* dinv32, PcgGrid grid, PcgState* st, double tol, double delta, int max_it) {
-  __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = warp % W;
-  const int n3 = 3 * M.n_rows;
-  auto own = [&](auto f) {
-    for_slices<W>(M.n_slices, [&](int slice) {
-      if (slice >= M.n_slices) return;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int i = slice * 96 + k * 32 + lane;
-        if (k % W == w && i < n3) f(i);
-      }
-    });
-  };
-  double s2[2] = {0.0, 0.0}, t2[2], t3[3];
-  own([&](int i) {
+//      ||r||/||b|| < tol in FP64), the direction kept. The true residual takes the
+//      place of an iteration's two launches (x += d in the product's, r in the step's).
+__global__ void __launch_bounds__(kPcgThreads)
+    k_pcgm_start(int n3, const double* __restrict__ b, const double* __restrict__ dinv, double* x, float* r32,
+                 float* p32, float* d32, float* dinv32, double* part, PcgState* st) {
+  double v[2] = {0.0, 0.0}, t[2];
+  for_elements(n3, [&](int i) {
     const double bi = b[i];
     const float rv = (float)bi, dv = (float)dinv[i], zv = dv * rv;
     x[i] = 0;
@@ -588,108 +664,153 @@ __global__ void __launch_bounds__(kPcgThreads, 4)
     dinv32[i] = dv;
     p32[i] = zv;
     d32[i] = 0.f;
-    s2[0] += bi * bi;
-    s2[1] += (double)zv * (double)rv;
+    v[0] += bi * bi;
+    v[1] += (double)zv * (double)rv;
   });
-  if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
-  const double bnorm = sqrt(t2[0]);
-  double zr = t2[1], err = 0.0, err_ref = 1.0;
-  int status = MSG_OK, iterations = 0, it = 0, products = 0;
-  bool done = !(bnorm > 1e-25);  // SolverPCG.cs:112
-  while (!done) {
-    double s3[3] = {0.0, 0.0, 0.0};
-    for_slices<W>(M.n_slices, [&](int slice) {
+  if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
+  st->bnorm = sqrt(t[0]);
+  st->zr = t[1];
+  st->err_ref = 1.0;
+  st->done = !(st->bnorm > 1e-25);  // SolverPCG.cs:112
+}
+
+template <int W, bool kStream>
+__global__ void __launch_bounds__(kPcgThreads, 4)
+    k_pcgm_product(PcgMat M, const float* __restrict__ val32, double* x, const float* r32, const float* p32,
+                   float* q32, float* d32, const float* dinv32, double* part, PcgState* st) {
+  __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
+  if (over(st)) return;
+  const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) % W;
+  bool waited = false;
+  int need = 0, done = 0;
+  auto start = [&] {  // (once; the first slice's values are under way)
+    if (waited) return;
+    wait_for_launch();
+    waited = true;
+    need = st->need;
+    done = st->done;
+  };
+  double v[3] = {0.0, 0.0, 0.0}, t[3];
+  auto dir = [&](int c, float (&u)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) u[k] = p32[3 * c + k];
+  };
+  for_slices<W, (W > 2)>(M.n_slices, [&](int slice) {
+    if (need) return;
+    const int row = slice * 32 + lane;
+    const bool live = slice < M.n_slices && row < M.n_rows;
+    double y[3] = {0.0, 0.0, 0.0};
+    if (live) slice_rows<W, (W > 2 ? 4 : 3), kStream>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val32, dir, y, start);
+    start();
+    join_warps<W>(y, ys);
+    if (w == 0 && live && !need) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int i = 3 * row + k;
+        const float qf = (float)y[k], dv = dinv32[i];
+        q32[i] = qf;
+        v[0] += (double)p32[i] * (double)qf;
+        v[1] += (double)(dv * r32[i]) * (double)qf;
+        v[2] += (double)(dv * qf) * (double)qf;
+      }
+    }
+  });
+  if (done) return;
+  if (need) {
+    for_elements(3 * M.n_rows, [&](int i) {
+      x[i] += (double)d32[i];
+      d32[i] = 0.f;
+    });
+    return;
+  }
+  if (!last_sum<kPcgWarps, 3>(part, &st->counter, v, t) || threadIdx.x) return;
+  st->matvecs += 1;
+  if (!(t[0] > 0) || isnan(t[0])) {  // breakdown: p.q <= 0 or NaN
+    st->status = MSG_ERR_BREAKDOWN;
+    st->iterations = st->it;
+    st->done = 1;
+    return;
+  }
+  const double zr = st->zr, alpha = zr / t[0];
+  const double g1 = zr - 2.0 * alpha * t[1] + alpha * alpha * t[2];
+  st->alpha = alpha;
+  st->beta = g1 > 0.0 ? g1 / zr : 0.0;  // a non-positive estimate restarts from z
+}
+
+template <int W>
+__global__ void __launch_bounds__(kPcgThreads, 4)
+    k_pcgm_step(PcgMat M, const double* __restrict__ val, const double* __restrict__ b, const double* x, float* r32,
+                float* p32, const float* q32, float* d32, const float* dinv32, double* part, PcgState* st, double tol, double delta, int max_it) {
+  __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
+  wait_for_launch();
+  if (st->done) return;
+  const bool need = st->need;
+  double v[2] = {0.0, 0.0}, t[2];
+  if (need) {
+    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) % W;
+    for_slices<W, false>(M.n_slices, [&](int slice) {
       const int row = slice * 32 + lane;
       const bool live = slice < M.n_slices && row < M.n_rows;
       double y[3] = {0.0, 0.0, 0.0};
-      auto dir = [&](int c, float (&u)[3]) {
+      auto at = [&](int c, double (&u)[3]) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) u[k] = p32[3 * c + k];
+        for (int k = 0; k < 3; ++k) u[k] = x[3 * c + k];
       };
-      if (live) slice_rows<W, 2, kStream>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val32, dir, y);
+      if (live) slice_rows<W, 1, true>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val, at, y, [] {});
       join_warps<W>(y, ys);
       if (w == 0 && live) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           const int i = 3 * row + k;
-          const float qf = (float)y[k], dv = dinv32[i];
-          q32[i] = qf;
-          s3[0] += (double)p32[i] * (double)qf;
-          s3[1] += (double)(dv * r32[i]) * (double)qf;
-          s3[2] += (double)(dv * qf) * (double)qf;
+          const double ri = b[i] - y[k];
+          const float rv = (float)ri;
+          r32[i] = rv;
+          v[0] += ri * ri;
+          v[1] += (double)(dinv32[i] * rv) * (double)rv;
         }
       }
     });
-    if (!grid_sum<kPcgWarps, 3>(grid, s3, t3)) return;
-    ++products;
-    if (!(t3[0] > 0) || isnan(t3[0])) {  // breakdown: p.q <= 0 or NaN
-      status = MSG_ERR_BREAKDOWN;
-      iterations = it;
-      break;
-    }
-    const double alpha = zr / t3[0];
-    const double g1 = zr - 2.0 * alpha * t3[1] + alpha * alpha * t3[2];
-    const float al = (float)alpha, be = (float)(g1 > 0.0 ? g1 / zr : 0.0);  // a non-positive estimate restarts from z
-    s2[0] = s2[1] = 0.0;
-    own([&](int i) {
+  } else {
+    const float al = (float)st->alpha, be = (float)st->beta;
+    for_elements(3 * M.n_rows, [&](int i) {
       const float pv = p32[i], rn = fmaf(-al, q32[i], r32[i]), zv = dinv32[i] * rn;
       d32[i] = fmaf(al, pv, d32[i]);
       p32[i] = fmaf(be, pv, zv);
       r32[i] = rn;
-      s2[0] += (double)rn * (double)rn;
-      s2[1] += (double)zv * (double)rn;
+      v[0] += (double)rn * (double)rn;
+      v[1] += (double)zv * (double)rn;
     });
-    if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
-    err = sqrt(t2[0]) / bnorm;
-    zr = t2[1];
-    if (err < tol || err < delta * err_ref) {
-      own([&](int i) {
-        x[i] += (double)d32[i];
-        d32[i] = 0.f;
-      });
-      s2[0] = s2[1] = 0.0;
-      if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;  // x is complete
-      for_slices<W>(M.n_slices, [&](int slice) {
-        const int row = slice * 32 + lane;
-        const bool live = slice < M.n_slices && row < M.n_rows;
-        double y[3] = {0.0, 0.0, 0.0};
-        auto at = [&](int c, double (&u)[3]) {
-#pragma unroll
-          for (int k = 0; k < 3; ++k) u[k] = x[3 * c + k];
-        };
-        if (live) slice_rows<W, 1, true>(M.slice_ptr[slice], M.slice_ptr[slice + 1], w, lane, M.col, val, at, y);
-        join_warps<W>(y, ys);
-        if (w == 0 && live) {
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const int i = 3 * row + k;
-            const double ri = b[i] - y[k];
-            const float rv = (float)ri;
-            r32[i] = rv;
-            s2[0] += ri * ri;
-            s2[1] += (double)(dinv32[i] * rv) * (double)rv;
-          }
-        }
-      });
-      if (!grid_sum<kPcgWarps, 2>(grid, s2, t2)) return;
-      err = sqrt(t2[0]) / bnorm;
-      if (err < tol) {
-        iterations = it;
-        done = true;
-      } else {
-        zr = t2[1];
-        err_ref = err;
-      }
-    }
-    if (!done && it + 1 >= max_it) {
-      iterations = max_it;
-      status = MSG_ERR_NOT_CONVERGED;
-      done = true;
-    }
-    ++it;
   }
-  own([&](int i) { x[i] += (double)d32[i]; });  // a correction left by a solve that ended without a true residual
-  PcgEnd::write(st, err, status, iterations, products);
+  if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
+  const double err = sqrt(t[0]) / st->bnorm;
+  st->err = err;
+  if (!need && (err < tol || err < delta * st->err_ref)) {
+    st->zr = t[1];
+    st->need = 1;  // the next two launches
+    return;
+  }
+  const int it = st->it;
+  if (need) {
+    st->need = 0;
+    if (err < tol) {
+      st->iterations = it;
+      st->done = 1;
+      return;
+    }
+    st->err_ref = err;
+  }
+  st->zr = t[1];
+  if (it + 1 >= max_it) {
+    st->iterations = max_it;
+    st->status = MSG_ERR_NOT_CONVERGED;
+    st->done = 1;
+  }
+  st->it = it + 1;
+}
+
+// A correction left by a solve that ended without a true residual.
+__global__ void __launch_bounds__(kPcgThreads) k_pcgm_fold(int n3, double* x, const float* __restrict__ d32) {
+  for_elements(n3, [&](int i) { x[i] += (double)d32[i]; });
 }
 
 // The mixed loop on resident FP32 values (Resident): the thread keeps r, p, d, D^-1,
@@ -784,7 +905,7 @@ __global__ void __launch_bounds__(32 * S * W, 1)
                                [&](int c, double (&u)[3]) {
 #pragma unroll
                                  for (int k = 0; k < 3; ++k) u[k] = x[3 * c + k];
-                               }, y);
+                               }, y, [] {});
       spread(y);
       if (own) {
         const double ri = bi - qs[sl][e];
@@ -890,26 +1011,34 @@ int launch_node_to_dof(Context* ctx, const Mesh* m, const double* d_in, double* 
 
 namespace {
 
-// Warps that share a slice: 4 where the slices are fewer than 32 warps an SM
-// (a warp alone takes 27 slots one after another), 2 above (a CTA's share of the
-// slices is then even to a few percent: 64^3 is 9.7 rounds of 4 slices a CTA).
-bool pcg_small(const Context* ctx, const Mesh* m) { return m->pat.n_slices < ctx->sm_count * 32; }
+// Warps that share a slice (a warp alone takes its 27 slots one after another): as many
+// as keep the product's CTAs, `per_sm` an SM, in one round, 2 where none do. FP64, us an
+// iteration: 20^3 12.6 with 8, 13.3 with 4; 25^3 16.5 and 14.6; 32^3 25.6 with 8, 22.9
+// with 4, 18.2 with 2; 40^3 38.3 with 4, 39.1 with 2, 36.2 with 1; 48^3 54.8, 52.2, 56.6.
+constexpr int kPcgCtas = 3, kPcgmCtas = 4;  // CTAs an SM of the FP64 and the mixed product
+int pcg_warps(const Context* ctx, const Mesh* m, int per_sm) {
+  for (int W : {8, 4, 2, 1})
+    if ((int64_t)m->pat.n_slices * W <= (int64_t)kPcgWarps * per_sm * ctx->sm_count) return W;
+  return 2;
+}
 
 PcgMat pcg_mat(const Mesh* m) {
   return {m->n_nodes, m->pat.n_slices, m->d_slice_ptr.as<int64_t>(), m->d_col.as<int>()};
 }
 
-// CTAs of a solve: one per group of slices, at most those resident at once
-// (the kernels' CTAs wait for each other).
-int pcg_grid(Context* ctx, const Mesh* m, const void* kernel, bool small) {
-  const int per = small ? kPcgWarps / 4 : kPcgWarps / 2;
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kPcgThreads, 0) != cudaSuccess || occ < 1) occ = 1;
-  return std::max(1, std::min((m->pat.n_slices + per - 1) / per, ctx->sm_count * std::min(occ, kPcgMaxCtas)));
+// CTAs of the launches over slices (one round of them: 64^3 106 us an iteration, 110
+// with a CTA for every four slices) and over elements.
+int pcg_slice_ctas(const Context* ctx, const Mesh* m, int W, int per_sm) {
+  const int per = kPcgWarps / W;
+  return std::max(1, std::min((m->pat.n_slices + per - 1) / per, ctx->sm_count * per_sm));
+}
+int pcg_element_ctas(const Context* ctx, const Mesh* m) {
+  return std::max(1, std::min((3 * m->n_nodes + kPcgThreads - 1) / kPcgThreads, ctx->sm_count * kPcgMaxCtas));
 }
 
-// bytes of the partial sums, then the state
-size_t pcg_head_bytes(const Context* ctx) { return sizeof(double) * 2 * kPcgSums * kPcgMaxCtas * ctx->sm_count + 256; }
+// bytes of the partial sums (two buffers of a cooperative solve's CTAs, at most one an
+// SM; one of a launch's), then the state
+size_t pcg_head_bytes(const Context* ctx) { return sizeof(double) * kPcgSums * kPcgMaxCtas * ctx->sm_count + 256; }
 PcgState* pcg_state(const Context* ctx, void* head) {
   return reinterpret_cast<PcgState*>(static_cast<char*>(head) + pcg_head_bytes(ctx) - 256);
 }
@@ -919,11 +1048,12 @@ PcgState* pcg_state(const Context* ctx, void* head) {
 bool pcg_stream(const Mesh* m, size_t value_bytes) { return (size_t)m->pat.n_slots * 288 * value_bytes > (size_t)100 << 20; }
 
 // Slices an SM (at most `most`, the kernels' widest CTA) if the CTAs of a resident
-// solve fit, one an SM, with their slots in shared memory; 0 otherwise.
+// solve fit a third of the SMs, one an SM, with their slots in shared memory; 0
+// otherwise.
 template <class V>
 int pcg_resident(const Context* ctx, const Mesh* m, int most, size_t* smem) {
   const std::vector<int64_t>& sp = m->pat.slice_ptr;
-  const int ns = m->pat.n_slices, S = (ns + ctx->sm_count - 1) / ctx->sm_count;
+  const int sms = std::max(1, ctx->sm_count / 3), ns = m->pat.n_slices, S = (ns + sms - 1) / sms;
   if (S > most) return 0;
   int64_t slots = 0;
   for (int i = 0; i < ns; i += S) slots = std::max(slots, sp[std::min(i + S, ns)] - sp[i]);
@@ -955,16 +1085,57 @@ int pcg_cooperative(Context* ctx, const PcgLaunch& l, void** args, cudaStream_t 
   return MSG_OK;
 }
 
-// One FP64 solve on stream s: partial sums and state cleared, one cooperative launch.
+// A launch that may begin while the one before it ends (its kernel waits for it).
+template <class... Params, class... Args>
+void dependent(void (*kernel)(Params...), int grid, cudaStream_t s, Args... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(kPcgThreads);
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, Params(args)...);  // (its error is the next cudaGetLastError)
+}
+
+// The iterations of a solve in launches: iteration() enqueues one. They are enqueued
+// ahead of the host's look at the state by two rounds of about 0.4 ms each (the
+// launches after the end of the solve return at once, about 2 us a launch).
+template <class F>
+int pcg_iterate(Context* ctx, const Mesh* m, size_t value_bytes, PcgState* st, int max_it, F iteration, cudaStream_t s) {
+  static_assert(2 * 128 <= 4096 && sizeof(PcgState) <= 128, "two states fit the flag page");
+  const double us = 10.0 + (double)m->pat.n_slots * (288 * value_bytes) / 6e6;
+  const int round = std::min(max_it, (int)std::max(2.0, std::min(64.0, 400.0 / us)));
+  PcgState* h[2] = {reinterpret_cast<PcgState*>(ctx->h_flags), reinterpret_cast<PcgState*>(ctx->h_flags + 32)};
+  auto enqueue = [&](int k) -> int {
+    for (int i = 0; i < round; ++i) iteration();
+    MSG_CUDA(ctx, cudaGetLastError());
+    MSG_CUDA(ctx, cudaMemcpyAsync(h[k], st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
+    MSG_CUDA(ctx, cudaEventRecord(ctx->ev[k], s));
+    return MSG_OK;
+  };
+  MSG_TRY(enqueue(0));
+  for (int64_t n = 0, k = 0; n <= 2 * (int64_t)max_it + 2 * round; n += round, k ^= 1) {
+    MSG_TRY(enqueue((int)k ^ 1));
+    MSG_CUDA(ctx, cudaEventSynchronize(ctx->ev[k]));
+    if (h[k]->done) break;
+  }
+  return MSG_OK;
+}
+
+// One FP64 solve on stream s.
 int pcg_launch(Context* ctx, const Mesh* m, const double* val, const double* b, const double* dinv, double* x,
                double* r, double* z, double* p0, double* p1, double* q, void* head, double tol, int max_it,
                cudaStream_t s) {
   PcgMat M = pcg_mat(m);
   PcgState* st = pcg_state(ctx, head);
-  PcgGrid g{static_cast<double*>(head), &st->counter, 0u, 0};
+  double* part = static_cast<double*>(head);
   MSG_CUDA(ctx, cudaMemsetAsync(head, 0, pcg_head_bytes(ctx), s));
   PcgLaunch l;
   if (const int S = pcg_resident<double>(ctx, m, 3, &l.smem)) {
+    PcgGrid g{part, &st->counter, 0u, 0};
     l.kernel = S == 1 ? (const void*)k_pcg_resident<1, 8> : S == 2 ? (const void*)k_pcg_resident<2, 4>
                                                                    : (const void*)k_pcg_resident<3, 4>;
     l.threads = S == 1 ? 256 : 128 * S;
@@ -972,16 +1143,23 @@ int pcg_launch(Context* ctx, const Mesh* m, const double* val, const double* b, 
     void* args[] = {&M, &val, &b, &dinv, &x, &z, &p0, &p1, &g, &st, &tol, &max_it};
     return pcg_cooperative(ctx, l, args, s);
   }
-  l.smem = 0;
-  const bool small = pcg_small(ctx, m), stream = pcg_stream(m, sizeof(double));
-  l.kernel = small ? (stream ? (const void*)k_pcg<4, true> : (const void*)k_pcg<4, false>)
-                   : (stream ? (const void*)k_pcg<2, true> : (const void*)k_pcg<2, false>);
-  l.grid = pcg_grid(ctx, m, l.kernel, small);
-  void* args[] = {&M, &val, &b, &dinv, &x, &r, &z, &p0, &p1, &q, &g, &st, &tol, &max_it};
-  return pcg_cooperative(ctx, l, args, s);
+  const int W = pcg_warps(ctx, m, kPcgCtas), gs = pcg_slice_ctas(ctx, m, W, kPcgCtas), ge = pcg_element_ctas(ctx, m);
+  const int n3 = 3 * m->n_nodes;
+  const bool stream = pcg_stream(m, sizeof(double));
+  auto product = W == 8   ? k_pcg_product<8, false>  // (never that large)
+                 : W == 4 ? k_pcg_product<4, false>
+                 : W == 2 ? (stream ? k_pcg_product<2, true> : k_pcg_product<2, false>)
+                          : (stream ? k_pcg_product<1, true> : k_pcg_product<1, false>);
+  k_pcg_start<<<ge, kPcgThreads, 0, s>>>(n3, b, dinv, x, r, z, p0, part, st);
+  count_launch(ctx);
+  return pcg_iterate(ctx, m, sizeof(double), st, max_it, [&] {
+    dependent(product, gs, s, M, val, z, p0, p1, q, part, st);
+    dependent(k_pcg_step, ge, s, n3, dinv, x, r, z, p0, p1, q, part, st, tol, max_it);
+    count_launch(ctx, 2);
+  }, s);
 }
 
-// The state after a solve (its copy on the host); a solve whose grid barrier
+// The state after a solve (its copy on the host); a cooperative solve whose grid barrier
 // expired leaves it not done.
 int pcg_finish(Context* ctx, PcgState* st, PcgState* host, cudaStream_t s) {
   MSG_CUDA(ctx, cudaMemcpyAsync(host, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
@@ -1005,7 +1183,7 @@ int pcg_wait_selftest(Context* ctx, int polls) {
   return pcg_finish(ctx, st, &hs, ctx->stream);
 }
 
-// Runs the device PCG on node-layout vectors (k_pcg, or k_pcg_mixed), one launch a solve.
+// Runs the device PCG on node-layout vectors.
 int pcg_solve_device(Context* ctx, Matrix* A, const double* d_b, double* d_x, int max_it, double tol, int* iterations,
                      double* rel_res, int* status, bool mixed) {
   Mesh* m = A->mesh;
@@ -1044,14 +1222,23 @@ int pcg_solve_device(Context* ctx, Matrix* A, const double* d_b, double* d_x, in
       void* args[] = {&M, &val, &val32, &d_b, &dinv, &d_x, &p32, &g, &st, &tol, &delta, &max_it};
       MSG_TRY(pcg_cooperative(ctx, l, args, s));
     } else {
-      l.smem = 0;
-      const bool small = pcg_small(ctx, m), stream = pcg_stream(m, sizeof(float));
-      l.kernel = small ? (stream ? (const void*)k_pcg_mixed<4, true> : (const void*)k_pcg_mixed<4, false>)
-                       : (stream ? (const void*)k_pcg_mixed<2, true> : (const void*)k_pcg_mixed<2, false>);
-      l.grid = pcg_grid(ctx, m, l.kernel, small);
-      void* args[] = {&M,   &val, &val32,  &d_b, &dinv, &d_x, &r32,   &p32,
-                      &q32, &d32, &dinv32, &g,   &st,   &tol, &delta, &max_it};
-      MSG_TRY(pcg_cooperative(ctx, l, args, s));
+      const int W = pcg_warps(ctx, m, kPcgmCtas), gs = pcg_slice_ctas(ctx, m, W, kPcgmCtas), ge = pcg_element_ctas(ctx, m);
+      const int n3 = (int)n;
+      double* part = A->d_work.as<double>();
+      const bool stream = pcg_stream(m, sizeof(float));
+      auto product = W == 8   ? k_pcgm_product<8, false>
+                     : W == 4 ? k_pcgm_product<4, false>
+                     : W == 2 ? (stream ? k_pcgm_product<2, true> : k_pcgm_product<2, false>)
+                              : (stream ? k_pcgm_product<1, true> : k_pcgm_product<1, false>);
+      auto step = W == 8 ? k_pcgm_step<8> : W == 4 ? k_pcgm_step<4> : W == 2 ? k_pcgm_step<2> : k_pcgm_step<1>;
+      k_pcgm_start<<<ge, kPcgThreads, 0, s>>>(n3, d_b, dinv, d_x, r32, p32, d32, dinv32, part, st);
+      MSG_TRY(pcg_iterate(ctx, m, sizeof(float), st, max_it, [&] {
+        dependent(product, gs, s, M, val32, d_x, r32, p32, q32, d32, dinv32, part, st);
+        dependent(step, ge, s, M, val, d_b, d_x, r32, p32, q32, d32, dinv32, part, st, tol, delta, max_it);
+        count_launch(ctx, 2);
+      }, s));
+      k_pcgm_fold<<<ge, kPcgThreads, 0, s>>>(n3, d_x, d32);
+      count_launch(ctx, 2);
     }
   } else {
     MSG_TRY(pcg_launch(ctx, m, A->d_val.as<double>(), d_b, A->d_dinv.as<double>(), d_x, v, v + nv, v + 2 * nv,
@@ -1073,7 +1260,7 @@ int pcg_solve_device(Context* ctx, Matrix* A, const double* d_b, double* d_x, in
 // library holds this array until the process exits.
 constexpr int kNoAllocMaxNodes = 65536;
 constexpr size_t kNoAllocVecBytes = sizeof(double) * 3 * (size_t)kNoAllocMaxNodes;
-constexpr size_t kNoAllocBytes = 7 * kNoAllocVecBytes + sizeof(double) * 2 * kPcgSums * kPcgMaxCtas * 256 + 256;  // up to 256 SMs
+constexpr size_t kNoAllocBytes = 7 * kNoAllocVecBytes + sizeof(double) * kPcgSums * kPcgMaxCtas * 256 + 256;  // up to 256 SMs
 static_assert(sizeof(PcgState) <= 256, "the scalar state fits its slot");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -1105,6 +1292,7 @@ extern "C" int MSG_PCG_SOLVE_NOALLOC(MSG_MAT A, const double* b_dev, double* x_d
   Context* ctx = m->ctx;
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   MSG_CUDA(ctx, cudaSetDevice(ctx->device));
+  MSG_TRY(context_resources(ctx));  // (host memory and events)
   const int nr = m->n_nodes;
   if (nr > kNoAllocMaxNodes)
     return set_error(ctx, MSG_ERR_INVALID_ARGUMENT,

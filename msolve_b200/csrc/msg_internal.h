@@ -314,12 +314,16 @@ struct Mesh {
   std::mutex shadow_mu;
 };
 
-// How a device PCG solve ended, and the arrival counter of its grid-wide sums
-// (cleared before the launch; done stays 0 when their bounded wait expired).
+// Scalars of a device PCG solve and how it ended (done stays 0 when the bounded wait of
+// a cooperative solve expired), and the arrival counter of its sums. Cleared before it.
 struct PcgState {
   double err;
   int status, iterations, matvecs, done;
   unsigned int counter;
+  // between the launches of a solve that is not one launch; need: the mixed loop's next
+  // two launches take the FP64 true residual
+  int it, need;
+  double zr, alpha, beta, bnorm, err_ref;
 };
 
 struct Matrix {

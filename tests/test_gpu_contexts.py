@@ -2,6 +2,7 @@
 gives the status and the bits of the same call alone."""
 import ctypes as C
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -53,3 +54,52 @@ def test_matrices_of_other_widths_side_by_side(precision):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("n,precision", [(44, "fp64"), (44, "mixed"), (20, "fp64")])
+def test_a_solve_leaves_room_for_other_contexts(n, precision):
+    """Small solves and a batch beside solves that could fill the device take a fraction
+    of one of those, not its whole time for each launch that has to wait for its end.
+    (A 24^3 x 64 batch is some hundred launches of the whole device.)"""
+    ctx = M.Context(0)
+    model = M.clamped_block_model(n)
+    big = M.SolverPCG(ctx, model, 20000, 1e-10, precision)
+    big.matrix = M.GpuMesh(ctx, model).assemble(np.linspace(0.5, 2.0, model.n_elems), 0.3)
+
+    small_ctx = M.Context(0)
+    cantilever = M.cantilever_model()
+    small = M.SolverPCG(small_ctx, cantilever, 20000, 1e-7)
+    small.matrix = M.GpuMesh(small_ctx, cantilever).assemble(np.ones(cantilever.n_elems), 0.3)
+    block = M.clamped_block_model(24)
+    kl = M.LognormalStochasticCoefficientsProvider([24] * 3, 6.0, 10, 6)
+    batch = M.MonteCarloAnalyzerWithStochasticMaterial(small_ctx, block, kl, expansion_order=10, simulations=64, seed=1,
+                                                       mode="mixed", tolerance=1e-10, keep_solutions=False)
+    batch.Initialize()
+
+    def median(f, calls):
+        f()
+        t = []
+        for _ in range(calls):
+            t0 = time.perf_counter()
+            f()
+            t.append(time.perf_counter() - t0)
+        return sorted(t)[calls // 2]
+
+    alone = median(big.Solve, 5), median(small.Solve, 9), median(batch.Solve, 5)
+    stop = threading.Event()
+
+    def loop():
+        while not stop.is_set():
+            big.Solve()
+
+    t = threading.Thread(target=loop)
+    t.start()
+    try:
+        beside = median(small.Solve, 9), median(batch.Solve, 5)
+    finally:
+        stop.set()
+        t.join()
+    # a small solve's one launch never waits for the end of a big solve; the batch gets
+    # at least a quarter of the device
+    assert beside[0] <= alone[1] + 0.4 * alone[0], (alone, beside)
+    assert beside[1] <= 4.0 * alone[2], (alone, beside)

@@ -9,6 +9,7 @@ import pytest
 
 import msolve_b200 as M
 import oracle as O
+from msolve_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +66,41 @@ def test_pcg_streams_at_full_size(ctx):
     b = model.subdomains[0].RHS
     assert np.linalg.norm(b - A.Multiply(x[0])) <= 1e-9 * np.linalg.norm(b)
     assert np.abs(x[0] - x[1]).max() <= 1e-8 * np.abs(x[0]).max()
+
+
+# the largest matrices of one and two slices an SM on a third of 148 SMs and the next
+# ones (FP64), of six (mixed), and the first sizes of 4, 2 and 1 warps a slice
+@pytest.mark.parametrize("nx,ny,nz", [(11, 11, 10), (13, 13, 15), (14, 13, 14), (16, 15, 16), (20, 20, 20), (20, 21, 20),
+                                      (25, 24, 24), (37, 22, 29), (40, 40, 37)])
+def test_pcg_rule_edges(ctx, nx, ny, nz):
+    model = M.clamped_block_model(nx, ny=ny, nz=nz)
+    check(ctx, model, np.exp(0.3 * np.random.default_rng(nx).standard_normal(model.n_elems)))
+
+
+def test_pcg_several_rounds_of_slices(ctx):
+    """More slices than a launch's CTAs take at a time: mixed and FP64 agree to 1e-8."""
+    model = M.clamped_block_model(53, ny=53, nz=52)
+    A = M.GpuMesh(ctx, model).assemble(np.exp(0.3 * np.random.default_rng(5).standard_normal(model.n_elems)), 0.3)
+    x = []
+    for precision in ("fp64", "mixed"):
+        s = M.SolverPCG(ctx, model, 20000, 1e-11, precision)
+        s.matrix = A
+        x.append(s.Solve().copy())
+        assert np.array_equal(x[-1], s.Solve()), precision
+    b = model.subdomains[0].RHS
+    assert np.linalg.norm(b - A.Multiply(x[0])) <= 1e-9 * np.linalg.norm(b)
+    assert np.abs(x[0] - x[1]).max() <= 1e-8 * np.abs(x[0]).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n", [6, 18, 26])
+def test_pcg_limits(ctx, n, precision):
+    """A limit below, at and above a round of launches: the count is the limit."""
+    model = M.clamped_block_model(n)
+    A = M.GpuMesh(ctx, model).assemble(np.exp(0.3 * np.random.default_rng(1).standard_normal(model.n_elems)), 0.3)
+    for limit in (1, 2, 5, 70):
+        s = M.SolverPCG(ctx, model, limit, 1e-12, precision)
+        s.matrix = A
+        with pytest.raises(M.InvalidOperationError) as e:
+            s.Solve()
+        assert e.value.code == N.MSG_ERR_NOT_CONVERGED and s.iterations == limit
