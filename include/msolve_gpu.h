@@ -146,8 +146,8 @@ int MSG_MAT_DESTROY(MSG_MAT mat);
  * The loop's scalars and decisions stay on the device: small matrices (up to 4,700
  * nodes of a lattice on 148 SMs) are one cooperative launch a solve on at most a
  * third of the SMs (MSG_ERR_TIMEOUT if its CTAs' bounded waits for each other
- * expire), larger ones two launches an iteration, enqueued ahead of the host's look
- * at the state, so that other streams' work runs beside a long solve.
+ * expire), larger ones two launches an iteration, repeated by a graph's WHILE node,
+ * so that other streams' work runs beside a long solve.
  * iterations = the reference's count (loop index at the break); rel_res = last
  * ||r||/||b||. Returns MSG_ERR_NOT_CONVERGED if max_it was reached. */
 int MSG_PCG_SOLVE(MSG_MAT mat, const double* b, double* x, int max_it, double tol, int* iterations,

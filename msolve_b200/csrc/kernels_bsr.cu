@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include <cstddef>
+#include <cstring>
 
 #include "msg_internal.h"
 
@@ -140,12 +141,12 @@ __global__ void k_node_to_dof(int n_dofs, const int* __restrict__ free_rows, con
 // end.
 //
 // k_pcg_product and k_pcg_step (k_pcgm_*): two launches an iteration for all other
-// matrices, enqueued ahead of the host's look at the state; a launch after the end of
-// the solve returns at once. The CTA that finishes last adds the partials. A launch
-// starts while the one before it ends and loads its first values meanwhile. Bound by
-// HBM, or by L2 and the two launches' latency for matrices that stay there: 20^3 13.0 us
-// an iteration, 37 x 22 x 29 16.6 (mixed 14.9), 32^3 18.8 (16.2), 48^3 52.9 (36.0), 64^3
-// 106 (63.7; HBM alone 88 and 47).
+// matrices, repeated by a graph's WHILE node; a launch after the end of the solve
+// returns at once. The CTA that finishes last adds the partials. A launch starts while
+// the one before it ends and loads its first values meanwhile. Bound by HBM, or by L2
+// and the two launches' latency for matrices that stay there: 20^3 12.3 us an iteration,
+// 37 x 22 x 29 16.2 (mixed 14.2), 32^3 18.2 (15.4), 48^3 51 (35), 64^3 102 (62; HBM
+// alone 88 and 47).
 
 constexpr int kPcgThreads = 256, kPcgWarps = kPcgThreads / 32;
 constexpr int kPcgSums = 3;        // values of a sum at most
@@ -386,10 +387,24 @@ __device__ __forceinline__ void for_elements(int n, F f) {
   for (int i = blockIdx.x * kPcgThreads + threadIdx.x; i < n; i += gridDim.x * kPcgThreads) f(i);
 }
 
+// The loop of a solve whose launches a graph's WHILE node repeats (on = 0: the host
+// enqueues them).
+struct PcgLoop {
+  int on;
+  cudaGraphConditionalHandle handle;
+  __device__ void end() const {
+    if (on) cudaGraphSetConditional(handle, 0);
+  }
+};
+struct PcgLimits {
+  double tol, delta;  // delta: the mixed loop's reliable-update factor
+  int max_it;
+};
+
 // Start of an FP64 solve: x = 0, r = b, z = D^-1 r, sums b.b and z.b.
 __global__ void __launch_bounds__(kPcgThreads)
     k_pcg_start(int n3, const double* __restrict__ b, const double* __restrict__ dinv, double* x, double* r, double* z,
-                double* p0, double* part, PcgState* st) {
+                double* p0, double* part, PcgState* st, PcgLimits lim) {
   double v[2] = {0.0, 0.0}, t[2];
   for_elements(n3, [&](int i) {
     const double bi = b[i], zi = dinv[i] * bi;
@@ -398,6 +413,8 @@ __global__ void __launch_bounds__(kPcgThreads)
     v[1] += zi * bi;
   });
   if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
+  st->tol = lim.tol;
+  st->max_it = lim.max_it;
   st->bnorm = sqrt(t[0]);
   st->zr = t[1];
   st->done = !(st->bnorm > 1e-25);  // SolverPCG.cs:112
@@ -460,9 +477,12 @@ __global__ void __launch_bounds__(kPcgThreads, 3)
 // r -= alpha q, x += alpha p_new, z = D^-1 r, err, beta.
 __global__ void __launch_bounds__(kPcgThreads)
     k_pcg_step(int n3, const double* __restrict__ dinv, double* x, double* r, double* z, const double* p0,
-               const double* p1, const double* q, double* part, PcgState* st, double tol, int max_it) {
+               const double* p1, const double* q, double* part, PcgState* st, PcgLoop loop) {
   wait_for_launch();
-  if (st->done) return;
+  if (st->done) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) loop.end();
+    return;
+  }
   const int it = st->it;
   const double alpha = st->alpha;
   const double* p = (it & 1) ? p0 : p1;
@@ -476,15 +496,17 @@ __global__ void __launch_bounds__(kPcgThreads)
     v[1] += zi * ri;
   });
   if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
+  const int limit = st->max_it;
   st->err = sqrt(t[0]) / st->bnorm;
-  if (st->err < tol) {
+  if (st->err < st->tol) {
     st->iterations = it;
     st->done = 1;
-  } else if (it + 1 >= max_it) {
-    st->iterations = max_it;
+  } else if (it + 1 >= limit) {
+    st->iterations = limit;
     st->status = MSG_ERR_NOT_CONVERGED;
     st->done = 1;
   }
+  if (st->done) loop.end();
   st->beta = t[1] / st->zr;
   st->zr = t[1];
   st->it = it + 1;
@@ -654,7 +676,7 @@ __global__ void __launch_bounds__(32 * S * W, 1)
 //      place of an iteration's two launches (x += d in the product's, r in the step's).
 __global__ void __launch_bounds__(kPcgThreads)
     k_pcgm_start(int n3, const double* __restrict__ b, const double* __restrict__ dinv, double* x, float* r32,
-                 float* p32, float* d32, float* dinv32, double* part, PcgState* st) {
+                 float* p32, float* d32, float* dinv32, double* part, PcgState* st, PcgLimits lim) {
   double v[2] = {0.0, 0.0}, t[2];
   for_elements(n3, [&](int i) {
     const double bi = b[i];
@@ -668,6 +690,9 @@ __global__ void __launch_bounds__(kPcgThreads)
     v[1] += (double)zv * (double)rv;
   });
   if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
+  st->tol = lim.tol;
+  st->delta = lim.delta;
+  st->max_it = lim.max_it;
   st->bnorm = sqrt(t[0]);
   st->zr = t[1];
   st->err_ref = 1.0;
@@ -740,10 +765,13 @@ __global__ void __launch_bounds__(kPcgThreads, 4)
 template <int W>
 __global__ void __launch_bounds__(kPcgThreads, 4)
     k_pcgm_step(PcgMat M, const double* __restrict__ val, const double* __restrict__ b, const double* x, float* r32,
-                float* p32, const float* q32, float* d32, const float* dinv32, double* part, PcgState* st, double tol, double delta, int max_it) {
+                float* p32, const float* q32, float* d32, const float* dinv32, double* part, PcgState* st, PcgLoop loop) {
   __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
   wait_for_launch();
-  if (st->done) return;
+  if (st->done) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) loop.end();
+    return;
+  }
   const bool need = st->need;
   double v[2] = {0.0, 0.0}, t[2];
   if (need) {
@@ -782,28 +810,30 @@ __global__ void __launch_bounds__(kPcgThreads, 4)
     });
   }
   if (!last_sum<kPcgWarps, 2>(part, &st->counter, v, t) || threadIdx.x) return;
-  const double err = sqrt(t[0]) / st->bnorm;
+  const double err = sqrt(t[0]) / st->bnorm, tol = st->tol;
+  const int it = st->it, limit = st->max_it;
   st->err = err;
-  if (!need && (err < tol || err < delta * st->err_ref)) {
+  if (!need && (err < tol || err < st->delta * st->err_ref)) {
     st->zr = t[1];
     st->need = 1;  // the next two launches
     return;
   }
-  const int it = st->it;
   if (need) {
     st->need = 0;
     if (err < tol) {
       st->iterations = it;
       st->done = 1;
+      loop.end();
       return;
     }
     st->err_ref = err;
   }
   st->zr = t[1];
-  if (it + 1 >= max_it) {
-    st->iterations = max_it;
+  if (it + 1 >= limit) {
+    st->iterations = limit;
     st->status = MSG_ERR_NOT_CONVERGED;
     st->done = 1;
+    loop.end();
   }
   st->it = it + 1;
 }
@@ -1026,7 +1056,7 @@ PcgMat pcg_mat(const Mesh* m) {
   return {m->n_nodes, m->pat.n_slices, m->d_slice_ptr.as<int64_t>(), m->d_col.as<int>()};
 }
 
-// CTAs of the launches over slices (one round of them: 64^3 106 us an iteration, 110
+// CTAs of the launches over slices (one round of them: 64^3 102 us an iteration, 107
 // with a CTA for every four slices) and over elements.
 int pcg_slice_ctas(const Context* ctx, const Mesh* m, int W, int per_sm) {
   const int per = kPcgWarps / W;
@@ -1100,17 +1130,61 @@ void dependent(void (*kernel)(Params...), int grid, cudaStream_t s, Args... args
   cudaLaunchKernelEx(&c, kernel, Params(args)...);  // (its error is the next cudaGetLastError)
 }
 
-// The iterations of a solve in launches: iteration() enqueues one. They are enqueued
-// ahead of the host's look at the state by two rounds of about 0.4 ms each (the
-// launches after the end of the solve return at once, about 2 us a launch).
+// The iterations of a solve, iteration(loop) enqueues one. With a matrix (A) they are a
+// graph of its own, kept for its next solves with the same vectors, whose WHILE node
+// repeats kPcgRound of them until the solve ends, with no host in between (launched by
+// the host, 64^3 took 206 ms instead of 119 on a host with more busy processes than
+// processors). Without one (nothing may be allocated) the host enqueues them, two
+// rounds of about 0.4 ms ahead of its look at the state.
+constexpr int kPcgRound = 8;
 template <class F>
-int pcg_iterate(Context* ctx, const Mesh* m, size_t value_bytes, PcgState* st, int max_it, F iteration, cudaStream_t s) {
-  static_assert(2 * 128 <= 4096 && sizeof(PcgState) <= 128, "two states fit the flag page");
-  const double us = 10.0 + (double)m->pat.n_slots * (288 * value_bytes) / 6e6;
+int pcg_iterate(Context* ctx, const Mesh* m, Matrix* A, const void* b, const void* x, bool mixed, PcgState* st,
+                int max_it, F iteration, cudaStream_t s) {
+  if (A) {
+    PcgGraph& g = A->pcg_graph[mixed ? 1 : 0];
+    if (g.exec && (g.b != b || g.x != x)) {
+      cudaGraphExecDestroy(g.exec);
+      g.exec = nullptr;
+    }
+    if (!g.exec) {
+      struct Hold {
+        cudaGraph_t g = nullptr;
+        ~Hold() {
+          if (g) cudaGraphDestroy(g);
+        }
+      } graph;
+      MSG_CUDA(ctx, cudaGraphCreate(&graph.g, 0));
+      PcgLoop loop{1, 0};
+      MSG_CUDA(ctx, cudaGraphConditionalHandleCreate(&loop.handle, graph.g, 1, cudaGraphCondAssignDefault));
+      cudaGraphNodeParams wp = {};
+      wp.type = cudaGraphNodeTypeConditional;
+      wp.conditional.handle = loop.handle;
+      wp.conditional.type = cudaGraphCondTypeWhile;
+      wp.conditional.size = 1;
+      cudaGraphNode_t node = nullptr;
+      MSG_CUDA(ctx, cudaGraphAddNode(&node, graph.g, nullptr, 0, &wp));
+      cudaGraph_t body = wp.conditional.phGraph_out[0];
+      MSG_CUDA(ctx, cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+      for (int i = 0; i < kPcgRound; ++i) iteration(loop);
+      const cudaError_t le = cudaGetLastError(), ce = cudaStreamEndCapture(s, &body);
+      if (le != cudaSuccess || ce != cudaSuccess) return cuda_error(ctx, le != cudaSuccess ? le : ce, "PCG loop capture");
+      const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph.g, 0);
+      if (ie != cudaSuccess) {
+        g.exec = nullptr;
+        return cuda_error(ctx, ie, "cudaGraphInstantiate");
+      }
+      g.b = b;
+      g.x = x;
+    }
+    MSG_CUDA(ctx, cudaGraphLaunch(g.exec, s));
+    return MSG_OK;
+  }
+  static_assert(sizeof(PcgState) <= 128, "two states in the flag page's first 256 bytes");
+  const double us = 10.0 + (double)m->pat.n_slots * 288 * (mixed ? sizeof(float) : sizeof(double)) / 6e6;
   const int round = std::min(max_it, (int)std::max(2.0, std::min(64.0, 400.0 / us)));
   PcgState* h[2] = {reinterpret_cast<PcgState*>(ctx->h_flags), reinterpret_cast<PcgState*>(ctx->h_flags + 32)};
   auto enqueue = [&](int k) -> int {
-    for (int i = 0; i < round; ++i) iteration();
+    for (int i = 0; i < round; ++i) iteration(PcgLoop{0, 0});
     MSG_CUDA(ctx, cudaGetLastError());
     MSG_CUDA(ctx, cudaMemcpyAsync(h[k], st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
     MSG_CUDA(ctx, cudaEventRecord(ctx->ev[k], s));
@@ -1125,10 +1199,10 @@ int pcg_iterate(Context* ctx, const Mesh* m, size_t value_bytes, PcgState* st, i
   return MSG_OK;
 }
 
-// One FP64 solve on stream s.
+// One FP64 solve on stream s (A: the matrix, where a graph may be allocated).
 int pcg_launch(Context* ctx, const Mesh* m, const double* val, const double* b, const double* dinv, double* x,
                double* r, double* z, double* p0, double* p1, double* q, void* head, double tol, int max_it,
-               cudaStream_t s) {
+               cudaStream_t s, Matrix* A) {
   PcgMat M = pcg_mat(m);
   PcgState* st = pcg_state(ctx, head);
   double* part = static_cast<double*>(head);
@@ -1150,27 +1224,31 @@ int pcg_launch(Context* ctx, const Mesh* m, const double* val, const double* b, 
                  : W == 4 ? k_pcg_product<4, false>
                  : W == 2 ? (stream ? k_pcg_product<2, true> : k_pcg_product<2, false>)
                           : (stream ? k_pcg_product<1, true> : k_pcg_product<1, false>);
-  k_pcg_start<<<ge, kPcgThreads, 0, s>>>(n3, b, dinv, x, r, z, p0, part, st);
+  k_pcg_start<<<ge, kPcgThreads, 0, s>>>(n3, b, dinv, x, r, z, p0, part, st, PcgLimits{tol, 0.0, max_it});
   count_launch(ctx);
-  return pcg_iterate(ctx, m, sizeof(double), st, max_it, [&] {
+  return pcg_iterate(ctx, m, A, b, x, false, st, max_it, [&](PcgLoop loop) {
     dependent(product, gs, s, M, val, z, p0, p1, q, part, st);
-    dependent(k_pcg_step, ge, s, n3, dinv, x, r, z, p0, p1, q, part, st, tol, max_it);
-    count_launch(ctx, 2);
+    dependent(k_pcg_step, ge, s, n3, dinv, x, r, z, p0, p1, q, part, st, loop);
   }, s);
 }
 
 // The state after a solve (its copy on the host); a cooperative solve whose grid barrier
-// expired leaves it not done.
+// expired leaves it not done. Copied to pinned memory and then waited for: a copy to
+// pageable memory waits inside the driver, and calls of other contexts with it (a batch
+// beside long solves took the whole time of one in three of four processes).
 int pcg_finish(Context* ctx, PcgState* st, PcgState* host, cudaStream_t s) {
-  MSG_CUDA(ctx, cudaMemcpyAsync(host, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
+  MSG_CUDA(ctx, cudaMemcpyAsync(ctx->h_flags, st, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
   MSG_CUDA(ctx, cudaStreamSynchronize(s));
+  std::memcpy(host, ctx->h_flags, sizeof(PcgState));
   if (!host->done) return set_error(ctx, MSG_ERR_TIMEOUT, "PCG: a bounded grid barrier expired");
+  if (host->it > 0) count_launch(ctx, 2 * host->matvecs);  // of a solve in launches
   return MSG_OK;
 }
 
 }  // namespace
 
 int pcg_wait_selftest(Context* ctx, int polls) {
+  MSG_TRY(context_resources(ctx));
   DevMem head;
   MSG_TRY(head.alloc(ctx, pcg_head_bytes(ctx)));
   PcgState* st = pcg_state(ctx, head.ptr);
@@ -1231,18 +1309,18 @@ int pcg_solve_device(Context* ctx, Matrix* A, const double* d_b, double* d_x, in
                      : W == 2 ? (stream ? k_pcgm_product<2, true> : k_pcgm_product<2, false>)
                               : (stream ? k_pcgm_product<1, true> : k_pcgm_product<1, false>);
       auto step = W == 8 ? k_pcgm_step<8> : W == 4 ? k_pcgm_step<4> : W == 2 ? k_pcgm_step<2> : k_pcgm_step<1>;
-      k_pcgm_start<<<ge, kPcgThreads, 0, s>>>(n3, d_b, dinv, d_x, r32, p32, d32, dinv32, part, st);
-      MSG_TRY(pcg_iterate(ctx, m, sizeof(float), st, max_it, [&] {
+      k_pcgm_start<<<ge, kPcgThreads, 0, s>>>(n3, d_b, dinv, d_x, r32, p32, d32, dinv32, part, st,
+                                              PcgLimits{tol, delta, max_it});
+      MSG_TRY(pcg_iterate(ctx, m, A, d_b, d_x, true, st, max_it, [&](PcgLoop loop) {
         dependent(product, gs, s, M, val32, d_x, r32, p32, q32, d32, dinv32, part, st);
-        dependent(step, ge, s, M, val, d_b, d_x, r32, p32, q32, d32, dinv32, part, st, tol, delta, max_it);
-        count_launch(ctx, 2);
+        dependent(step, ge, s, M, val, d_b, d_x, r32, p32, q32, d32, dinv32, part, st, loop);
       }, s));
       k_pcgm_fold<<<ge, kPcgThreads, 0, s>>>(n3, d_x, d32);
       count_launch(ctx, 2);
     }
   } else {
     MSG_TRY(pcg_launch(ctx, m, A->d_val.as<double>(), d_b, A->d_dinv.as<double>(), d_x, v, v + nv, v + 2 * nv,
-                       v + 3 * nv, v + 4 * nv, A->d_work.ptr, tol, max_it, s));
+                       v + 3 * nv, v + 4 * nv, A->d_work.ptr, tol, max_it, s, A));
   }
   PcgState hs;
   MSG_TRY(pcg_finish(ctx, st, &hs, s));
@@ -1283,8 +1361,9 @@ using namespace msg;
 // The device Jacobi-PCG of MSG_PCG_SOLVE, for callers that must not allocate
 // device memory during the solve: the solve's working vectors live in the
 // fixed scratch array above instead of buffers from cudaMalloc, and the
-// right-hand side and solution are the caller's device buffers. The kernel and
-// its launch shape are MSG_PCG_SOLVE's.
+// right-hand side and solution are the caller's device buffers. The kernels and
+// their launch shapes are MSG_PCG_SOLVE's; the host enqueues them (a graph takes device
+// memory).
 extern "C" int MSG_PCG_SOLVE_NOALLOC(MSG_MAT A, const double* b_dev, double* x_dev, int max_it, double tol,
                                      int* iterations, double* rel_res) {
   if (!A || !b_dev || !x_dev || max_it <= 0 || !(tol > 0)) return MSG_ERR_INVALID_ARGUMENT;
@@ -1313,7 +1392,7 @@ extern "C" int MSG_PCG_SOLVE_NOALLOC(MSG_MAT A, const double* b_dev, double* x_d
   MSG_CUDA(ctx, cudaMemsetAsync(bn, 0, sizeof(double) * n, s));
   MSG_TRY(launch_dof_to_node(ctx, m, b_dev, bn, 1, 0, 0));
   MSG_TRY(pcg_launch(ctx, m, A->d_val.as<double>(), bn, A->d_dinv.as<double>(), xn, v[0], v[1], v[2], v[3], v[4],
-                     head, tol, max_it, s));
+                     head, tol, max_it, s, nullptr));
   MSG_TRY(launch_node_to_dof(ctx, m, xn, x_dev, 1, 0, 0));
   PcgState hs;
   MSG_TRY(pcg_finish(ctx, st, &hs, s));

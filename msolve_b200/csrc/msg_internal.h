@@ -324,6 +324,19 @@ struct PcgState {
   // two launches take the FP64 true residual
   int it, need;
   double zr, alpha, beta, bnorm, err_ref;
+  double tol, delta;
+  int max_it;
+};
+
+// The loop of a matrix's solves that are not one launch, for one pair of vectors.
+struct PcgGraph {
+  cudaGraphExec_t exec = nullptr;
+  const void *b = nullptr, *x = nullptr;
+  PcgGraph() = default;
+  PcgGraph(const PcgGraph&) = delete;
+  ~PcgGraph() {
+    if (exec) cudaGraphExecDestroy(exec);
+  }
 };
 
 struct Matrix {
@@ -333,6 +346,7 @@ struct Matrix {
   DevMem d_bn, d_xn, d_bd;  // node-layout b and x, DOF-layout staging of the host entry points
   DevMem d_dinv;  // [n_nodes*3]
   DevMem d_work;  // PCG workspace: partial sums, state, vectors (node layout)
+  PcgGraph pcg_graph[2];  // FP64, mixed
 
 };
 
