@@ -395,6 +395,12 @@ struct PcgLoop {
   __device__ void end() const {
     if (on) cudaGraphSetConditional(handle, 0);
   }
+  // One launch of the step: the loop's bound, and its end once the solve is over. (At
+  // most two steps an iteration, so that the bound is never the reason to stop.)
+  __device__ void step(PcgState* st, bool over) const {
+    if (!on || blockIdx.x > 0 || threadIdx.x > 0) return;
+    if (over || ++st->steps > 2LL * st->max_it + 2) cudaGraphSetConditional(handle, 0);
+  }
 };
 struct PcgLimits {
   double tol, delta;  // delta: the mixed loop's reliable-update factor
@@ -479,10 +485,9 @@ __global__ void __launch_bounds__(kPcgThreads)
     k_pcg_step(int n3, const double* __restrict__ dinv, double* x, double* r, double* z, const double* p0,
                const double* p1, const double* q, double* part, PcgState* st, PcgLoop loop) {
   wait_for_launch();
-  if (st->done) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) loop.end();
-    return;
-  }
+  const bool over = st->done;
+  loop.step(st, over);
+  if (over) return;
   const int it = st->it;
   const double alpha = st->alpha;
   const double* p = (it & 1) ? p0 : p1;
@@ -768,10 +773,9 @@ __global__ void __launch_bounds__(kPcgThreads, 4)
                 float* p32, const float* q32, float* d32, const float* dinv32, double* part, PcgState* st, PcgLoop loop) {
   __shared__ double ys[W > 1 ? kPcgWarps : 1][3][32];
   wait_for_launch();
-  if (st->done) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) loop.end();
-    return;
-  }
+  const bool over = st->done;
+  loop.step(st, over);
+  if (over) return;
   const bool need = st->need;
   double v[2] = {0.0, 0.0}, t[2];
   if (need) {

@@ -326,6 +326,7 @@ struct PcgState {
   double zr, alpha, beta, bnorm, err_ref;
   double tol, delta;
   int max_it;
+  long long steps;
 };
 
 // The loop of a matrix's solves that are not one launch, for one pair of vectors.
